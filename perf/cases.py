@@ -400,6 +400,7 @@ def run(state):
         with torch.cuda.stream(state["stream"]):
             return fields_of(m, range(12 if c["moist"] else 7), c["mixed"])
     if k == "nested":
+        state["n"].wait()  # the members are the set's until its launched steps are done
         for m in state["models"]:
             m.restore_snapshot()
             m.sync()
