@@ -417,6 +417,25 @@ def test_column_kernel_variants_agree(vg):
             m.set_tuning()
 
 
+@pytest.mark.parametrize("dt,n_sub", [(0.5, 1), (1.0, 3)])
+@pytest.mark.parametrize("dims", [(5, 3, 7), (33, 17, 41), (63, 2, 33), (64, 9, 80), (70, 9, 81), (97, 96, 13),
+                                  (24, 20, 161), (8, 6, 203)])
+def test_level_split_column_kernel_edges(vg, oc, dims, dt, n_sub):
+    """The built-in level-split column kernel at its edges (a last chunk of one
+    level, the longest chunks, 64 columns exactly, rows that run on into each
+    other, above the columns of the short-chunk form, columns too tall for it;
+    a stage's only substep) against the oracle, at the bound of the ragged
+    grids above and inside the substep's horizontal acoustic limit."""
+    nx, ny, nz = dims
+    t = small_setup(vg, nx=nx, ny=ny, nz=nz, zeta_stretch=1.0, bubble_xc=nx * 125.0, bubble_yc=ny * 125.0,
+                    **STEP_CASES[3])
+    with vg.Model(t, vg.MIXED) as m:
+        o = oc.Model(oracle_setup(oc, t), "port")
+        m.step(dt, n_sub, 2)
+        assert o.rk3_step(dt, n_sub) == 0 and o.rk3_step(dt, n_sub) == 0
+        assert_state_close(vg, t, m.state(), o.state(), 2 * TOLMX, range(7), "level-split column kernel %s" % (dims,))
+
+
 def test_autotune_keeps_the_update(vg):
     """The autotuner only chooses among launch shapes of the same update: a run
     after tuning matches the run before it to FP32 rounding (1e-6 of each

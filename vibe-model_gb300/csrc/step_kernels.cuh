@@ -108,14 +108,16 @@ void mixed_fb_substep(const Dims& d, const Tab& t, const Flags& fl, const WS& wi
                       cudaStream_t stream);
 int mixed_hevi_substep(const Dims& d, const Tab& t, const Flags& fl, const WS& win, const WS& wout, float dtau,
                        const float* lu /* 3*nz: a, cprime, inv_denom */, unsigned* err, cudaStream_t stream);
-// returns nonzero when a TMA descriptor cannot be made
+// returns nonzero when a TMA descriptor cannot be made. apply_uv: win is the
+// output of a substep whose u/v update (and deferred corrections) are still
+// to be applied; last: no further substep follows in the stage
 int mixed_hevi_column(const Dims& d, const Tab& t, const Flags& fl, const WS& win, const WS& wout, float dtau,
-                      const float* lu, bool apply_uv, unsigned* err, cudaStream_t stream);
+                      const float* lu, bool apply_uv, bool last, unsigned* err, cudaStream_t stream);
 void mixed_uv_backward(const Dims& d, const Tab& t, const WS& win, const WS& wout, float dtau, cudaStream_t stream);
 // whether the column kernel chosen for this grid defers its w/rho'
 // corrections to the reader (then the last substep of a stage is finished
 // by mixed_uv_fix instead of mixed_uv_backward, and mixed_finish gets defer)
-bool mixed_hevi_defers(const Dims& d);
+bool mixed_hevi_defers(const Dims& d, const Flags& fl);
 // u/v backward update and the deferred w/rho' corrections, in place
 void mixed_uv_fix(const Dims& d, const Tab& t, const Flags& fl, const WS& s, float dtau, cudaStream_t stream);
 // adjoint of mixed_fb_substep, in place on bars of (u, v, w, rho', pi')

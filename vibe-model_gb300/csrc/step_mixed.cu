@@ -833,7 +833,8 @@ bool tune_of(const Dims& d, MixedTune* t) {
 }
 
 constexpr int kDefaultHeviRing = 4;  // single-domain column kernel: 0 = register ring
-constexpr int kDefaultHeviPar = 0;   // levels per thread of the level-split column kernel (0 = off)
+constexpr int kMaxChunks = 20;       // chunks (warps) per block of the level-split column kernel at most
+constexpr long kChunkSmall = 9000;   // ... which takes 4 levels a warp up to this many columns
 constexpr int kDefaultHeviTwo = 2;   // ring depth of the two-columns-per-thread kernel (0 = off)
 constexpr bool kDefaultHeviTma = true;  // TMA-fed two-column kernel (VIBE_GB300_HEVI_TMA=0 turns it off; candidate 4)
 constexpr bool kDefaultHeviDefer = true;  // ... with the w/rho' corrections deferred to the reader (candidate 5)
@@ -2291,228 +2292,232 @@ size_t hevi_tma_smem_bytes(int nz) {
   return 128 + ((size_t)kColRing * kColSlot + 10 * (size_t)(nz + 1)) * sizeof(float);
 }
 
-// ---- the same HEVI column update with the levels split over threads ------
-// The column system's LU factors (la, lc, li) depend on the level only, so
-// both recurrences, dp(k) = (rhs(k) - la(k) dp(k-1)) li(k) and
+// ---- the HEVI column update with the levels split over warps ---------------
+// The column system's LU factors depend on the level only, so both
+// recurrences, dp(k) = rhs(k) li(k) - m(k) dp(k-1) with m = la li and
 // x(k) = dp(k) - lc(k) x(k+1), split into chunks of kM levels: each thread
-// solves its chunk with a zero carry and the chunks are joined by a scan of
-// the carries, dp(k) = dpl(k) + G(k) dp(k0-1) with G(k) = prod_{l=k0..k}
-// (-la(l) li(l)), and x(k) = xl(k) + H(k) x(k0+kM) with H(k) = prod_{l=k..
-// k0+kM-1} (-lc(l)). A block is 32 consecutive columns (one warp per chunk,
-// so every level's load is one 128-byte row) by C = ceil(nz/kM) chunks; every
-// thread issues all the loads of its chunk at once and nothing is parked
-// between sweeps. Same arithmetic per level as hevi_body; the carries change
-// the rounding of the tridiagonal solve only.
+// solves its chunk with a zero carry and adds the chunk's carry times
+// G(k) = prod_{l=k0..k} (-m(l)), or H(k) = prod_{l=k..k0+kn-1} (-lc(l)). Every
+// warp folds the carries of the chunks below (above) it by itself, so a block
+// meets at two barriers instead of two per level, and a column's latency is
+// that of one chunk instead of 2 nz levels. A warp is 64 consecutive points of
+// the padded plane (two adjacent columns a lane, every row access an aligned
+// 8-byte load or store; rows run on into each other, so only the P - nx
+// padding points idle) by one chunk; a block is the C = ceil(nz/kM) chunks of
+// its 64 points. Per-level constants lie in float4 tables with the step's
+// scalars folded in. The eliminated pi' never leaves the registers: 40 B/cell
+// of traffic, against 48 of the sweeping kernel.
+// All but a stage's last substep leave w and rho' as their explicit parts w~
+// and rho~ (the deferred form of hevi_tma_body<true>: the next substep applies
+// the implicit corrections to its input), so a chunk carries only its dp
+// values; the last one (`last`) reads its own w~ and rho~ back and corrects
+// them, and what remains of the stage is the u/v update.
+// Bound by latency at small grids (load, two barriers, store), by DRAM and the
+// loads in flight at large ones.
+size_t hevi_chunk_smem_bytes(int nz, int m) {
+  const int C = (nz + m - 1) / m;
+  return ((size_t)(3 * nz + 1)) * sizeof(float4) + (size_t)64 * C * sizeof(float2);
+}
 template <int kM>
-__device__ __forceinline__ void hevi_par_body(const Dims& d, const Tab& t, const Flags& fl, const WS& win,
-                                              const WS& wout, float dtau, const float* __restrict__ lu,
-                                              int apply_uv, float cdx, float cdy, int bx, int by) {
-  extern __shared__ float s_tab[];
+__device__ __forceinline__ void hevi_chunk_body(const Dims& d, const Tab& t, const Flags& fl, const WS& win,
+                                                const WS& wout, float dtau, const float* __restrict__ lu,
+                                                int apply_uv, int last, float cdx, float cdy, int bx) {
+  extern __shared__ float4 s_split[];
   const int nz = d.nz;
   const int C = blockDim.y;
-  float* s_tfz = s_tab;                    // nz+1
-  float* s_idzw = s_tfz + (nz + 1);        // nz+1
-  float* s_rfz = s_idzw + (nz + 1);        // nz+1
-  float* s_idzc = s_rfz + (nz + 1);        // nz
-  float* s_kap = s_idzc + nz;              // nz
-  float* s_la = s_kap + nz;                // nz
-  float* s_lc = s_la + nz;                 // nz
-  float* s_li = s_lc + nz;                 // nz
-  float* s_r0 = s_li + nz;                 // nz
-  float* s_t0 = s_r0 + nz;                 // nz
-  float* s_a = s_t0 + nz;                  // C x 32: chunk result with zero carry
-  float* s_g = s_a + C * 32;               // C x 32: its carry coefficient
-  float* s_e = s_g + C * 32;               // (C+1) x 32: scanned carries
-  float* s_x = s_e + (C + 1) * 32;         // C x 32: x at each chunk's top level
+  float4* ta = s_split;          // nz+1: face k: explicit and implicit pressure-gradient factor, rfz; level k: H
+  float4* tb = ta + (nz + 1);    // nz: idzc, dtau kap, r0, t0
+  float4* tc = tb + nz;          // nz: li, m = la li, lc, G
+  float2* sf = reinterpret_cast<float2*>(tc + nz);  // C x 32: dp at each chunk's last level, zero carry
+  float2* sx = sf + 32 * C;                         // C x 32: x at each chunk's first level, zero carry
   const int tx = threadIdx.x, c = threadIdx.y;
-  const int tid = c * 32 + tx, nthr = 32 * C;
-  for (int e = tid; e <= nz; e += nthr) {
-    s_tfz[e] = t.tfz[e];
-    s_idzw[e] = t.idzw[e];
-    s_rfz[e] = t.rfz[e];
-    if (e < nz) {
-      s_idzc[e] = t.idzc[e];
-      s_kap[e] = t.kap[e];
-      s_la[e] = lu[e];
-      s_lc[e] = lu[nz + e];
-      s_li[e] = lu[2 * nz + e];
-      s_r0[e] = t.r0c[e];
-      s_t0[e] = t.t0c[e];
-    }
-  }
-  __syncthreads();
-  const int i = bx * 32 + tx;
-  const int j = by;
+  const int tid = c * 32 + tx;
+  const int e = bx * 64 + 2 * tx;
+  const int j = e / d.P, i = e - j * d.P;
   const bool active = i < d.nx && j < d.ny;
+  const bool two = i + 1 < d.nx;
   const int k0 = c * kM;
   const int kn = imin(kM, nz - k0);  // >= 1: C = ceil(nz / kM)
+  const unsigned pl = (unsigned)d.plane;
+  const unsigned col = active ? (unsigned)e : 0u;
+  // 32-bit offsets from the fields' bases (the mixed path's fields have fewer
+  // than 2^32 points); the inputs are other buffers than the outputs, so the
+  // read-only loads may pass the stores
+  auto ld2 = [&](int q, unsigned o) { return __ldg(reinterpret_cast<const float2*>(win.f[q] + o)); };
+  auto ld1 = [&](int q, unsigned o) { return __ldg(win.f[q] + o); };
+  auto st2 = [&](int q, unsigned o, float2 v) {
+    if (two) *reinterpret_cast<float2*>(wout.f[q] + o) = v;
+    else wout.f[q][o] = v.x;
+  };
+  unsigned o = (unsigned)k0 * pl + col;
+  float2 pk = ld2(PI, o), wk = ld2(W, o);
+  const float2 pm = ld2(PI, k0 > 0 ? o - pl : o);
   const float b = (float)fl.hevi_beta, ob = 1.f - b;
   const float cpf = (float)kCp;
-  const size_t pl = d.plane;
-  const size_t col = active ? (size_t)j * d.P + i : 0;
-  const float* __restrict__ U0 = win.f[U] + col;
-  const float* __restrict__ V0 = win.f[V] + col;
-  const float* __restrict__ W0 = win.f[W] + col;
-  const float* __restrict__ P0 = win.f[PI] + col;
-  const float* __restrict__ R0 = win.f[RHO] + col;
-  float* __restrict__ Wo = wout.f[W] + col;
-  float* __restrict__ Po = wout.f[PI] + col;
-  float* __restrict__ Ro = wout.f[RHO] + col;
-  float* __restrict__ Uo = wout.f[U] + col;
-  float* __restrict__ Vo = wout.f[V] + col;
-  const size_t vn = d.P;
-  const float dxi = t.dx_inv, dyi = t.dy_inv;
-  const int ow = (i > 0) ? -1 : 0, oe = (i + 1 < d.nx) ? 1 : 0;
-  const long long os = (j > 0) ? -(long long)vn : 0, on = (j + 1 < d.ny) ? (long long)vn : 0;
-  const bool last_i = (i == d.nx - 1), last_j = (j == d.ny - 1);
-
-  float pv[kM + 2];  // p'(k0-1+q), 0 outside [0, nz)
-  float wv[kM + 1];  // w(face k0+q)
-  float wt[kM + 1];  // w with the explicit pressure gradient, faces k0..k0+kM
-  float rhs[kM], rs[kM], dp[kM], gq[kM];
-#pragma unroll
-  for (int q = 0; q < kM + 2; ++q) {
-    const int kk = k0 - 1 + q;
-    pv[q] = (active && kk >= 0 && kk < nz && q <= kn + 1) ? P0[(size_t)kk * pl] : 0.f;
+  for (int k = tid; k <= nz; k += 32 * C) {
+    const float g = (k > 0 && k < nz) ? cpf * t.tfz[k] * t.idzw[k] : 0.f;  // no gradient on the ground and the lid
+    float G = 1.f, H = 1.f;
+    if (k < nz) {
+      const int lo = k / kM * kM, hi = imin(lo + kM, nz);
+      for (int l = lo; l <= k; ++l) G *= -lu[l] * lu[2 * nz + l];
+      for (int l = k; l < hi; ++l) H *= -lu[nz + l];
+      tb[k] = make_float4(t.idzc[k], dtau * t.kap[k], t.r0c[k], t.t0c[k]);
+      tc[k] = make_float4(lu[2 * nz + k], lu[k] * lu[2 * nz + k], lu[nz + k], G);
+    }
+    ta[k] = make_float4(dtau * ob * g, dtau * b * g, t.rfz[k], H);
   }
-#pragma unroll
-  for (int q = 0; q < kM + 1; ++q) {
-    const int f = k0 + q;
-    wv[q] = (active && q <= kn && f <= nz) ? W0[(size_t)f * pl] : 0.f;
+  const int vn = d.P;
+  const float dxi = t.dx_inv, dyi = t.dy_inv, db = dtau * b;
+  // single neighbours as in hevi2_body (the idle points read column 0 alone)
+  const int ou2 = two ? 2 : 1;
+  const int opw = (active && i > 0) ? -1 : 0;
+  const int ope = !active ? 0 : (i + 2 < d.nx) ? 2 : (two ? 1 : 0);
+  const int ops = (active && j > 0) ? -vn : 0, opn = (active && j + 1 < d.ny) ? vn : 0;
+  const bool last_j = (j == d.ny - 1), last_i = (i + 2 >= d.nx);
+  __syncthreads();
+  float2 dp[kM], wt, prev = make_float2(0.f, 0.f);
+  {
+    const float4 A = ta[k0];
+    const float gx = pk.x - pm.x, gy = pk.y - pm.y;
+    if (apply_uv) {  // the input's deferred correction of w
+      wk.x -= A.y * gx;
+      wk.y -= A.y * gy;
+    }
+    wt = make_float2(wk.x - A.x * gx, wk.y - A.x * gy);
   }
-#pragma unroll
-  for (int q = 0; q < kM + 1; ++q) {
-    const int f = k0 + q;
-    wt[q] = wv[q];
-    if (q <= kn && f >= 1 && f < nz)
-      wt[q] = wv[q] - dtau * ob * cpf * s_tfz[f] * (pv[q + 1] - pv[q]) * s_idzw[f];
-  }
-  float w_top = 0.f;  // w(face k0+kn)
-#pragma unroll
-  for (int q = 0; q < kM + 1; ++q)
-    if (q == kn) w_top = wv[q];
-  float prev = 0.f, g = 1.f, d_last = 0.f, g_last = 1.f;
 #pragma unroll
   for (int q = 0; q < kM; ++q) {
-    rhs[q] = rs[q] = dp[q] = 0.f;
-    gq[q] = 1.f;
     if (q < kn) {
       const int k = k0 + q;
-      if (active) {
-        const size_t o = (size_t)k * pl;
-        const float p_k = pv[q + 1];
-        float u0 = U0[o], u1 = U0[o + 1], v0 = V0[o], v1 = V0[o + vn];
-        if (apply_uv) {
-          const float tx_ = s_t0[k] * cdx, ty_ = s_t0[k] * cdy;
-          u0 += tx_ * (p_k - P0[o + ow]);
-          u1 += tx_ * (P0[o + oe] - p_k);
-          v0 += ty_ * (p_k - P0[o + os]);
-          v1 += ty_ * (P0[o + on] - p_k);
-        }
-        const float Dh = -(s_r0[k] * ((u1 - u0) * dxi + (v1 - v0) * dyi));
-        Uo[o] = u0;
-        Vo[o] = v0;
-        if (last_i) Uo[o + 1] = u1;
-        if (last_j) Vo[o + vn] = v1;
-        const float rk = s_rfz[k], rk1 = s_rfz[k + 1], idz = s_idzc[k];
-        const float dv_old = -(rk1 * wv[q + 1] - rk * wv[q]) * idz;
-        const float dv_t = -(rk1 * wt[q + 1] - rk * wt[q]) * idz;
-        const float S = Dh + ob * dv_old;
-        rhs[q] = p_k + dtau * s_kap[k] * (S + b * dv_t);
-        rs[q] = R0[o] + dtau * S;
+      float2 wk1 = ld2(W, o + pl), pk1 = ld2(PI, k + 1 < nz ? o + pl : o);
+      const float2 fu = ld2(U, o), fv0 = ld2(V, o), fv1 = ld2(V, o + vn);
+      float2 r = ld2(RHO, o);
+      const float fu2 = ld1(U, o + ou2);
+      float u0x = fu.x, u0y = fu.y, u1y = fu2, v0x = fv0.x, v0y = fv0.y, v1x = fv1.x, v1y = fv1.y, u1x;
+      const float4 A0 = ta[k], A1 = ta[k + 1], B = tb[k], Ck = tc[k];
+      const float gx = pk1.x - pk.x, gy = pk1.y - pk.y;
+      if (apply_uv) {
+        const float2 fs = ld2(PI, o + ops), fn = ld2(PI, o + opn);
+        const float fpw = ld1(PI, o + opw), fpe = ld1(PI, o + ope);
+        const float tx_ = B.w * cdx, ty_ = B.w * cdy;
+        u0x += tx_ * (pk.x - fpw);
+        u0y += tx_ * (pk.y - pk.x);
+        u1x = two ? u0y : fu2;  // the face between the two columns; face nx has no gradient
+        u1y += tx_ * (fpe - pk.y);
+        v0x += ty_ * (pk.x - fs.x);
+        v0y += ty_ * (pk.y - fs.y);
+        v1x += ty_ * (fn.x - pk.x);
+        v1y += ty_ * (fn.y - pk.y);
+        wk1.x -= A1.y * gx;
+        wk1.y -= A1.y * gy;
+        r.x += db * ((A0.z * wk.x - A1.z * wk1.x) * B.x);
+        r.y += db * ((A0.z * wk.y - A1.z * wk1.y) * B.x);
+      } else {
+        u1x = fu.y;
       }
-      dp[q] = (rhs[q] - s_la[k] * prev) * s_li[k];
-      prev = dp[q];
-      g *= -s_la[k] * s_li[k];
-      gq[q] = g;
-      d_last = dp[q];
-      g_last = g;
+      const float2 wt1 = make_float2(wk1.x - A1.x * gx, wk1.y - A1.x * gy);
+      const float sx_ = ob * ((A0.z * wk.x - A1.z * wk1.x) * B.x) - B.z * ((u1x - u0x) * dxi + (v1x - v0x) * dyi);
+      const float sy_ = ob * ((A0.z * wk.y - A1.z * wk1.y) * B.x) - B.z * ((u1y - u0y) * dxi + (v1y - v0y) * dyi);
+      const float rx = pk.x + B.y * (sx_ + b * ((A0.z * wt.x - A1.z * wt1.x) * B.x));
+      const float ry = pk.y + B.y * (sy_ + b * ((A0.z * wt.y - A1.z * wt1.y) * B.x));
+      prev = make_float2(rx * Ck.x - Ck.y * prev.x, ry * Ck.x - Ck.y * prev.y);
+      dp[q] = prev;
+      if (active) {
+        st2(W, o, wt);
+        st2(U, o, make_float2(u0x, u0y));
+        st2(V, o, make_float2(v0x, v0y));
+        st2(RHO, o, make_float2(r.x + dtau * sx_, r.y + dtau * sy_));
+        if (last_i) wout.f[U][o + ou2] = two ? u1y : u1x;  // face nx
+        if (last_j) st2(V, o + vn, make_float2(v1x, v1y));
+      }
+      pk = pk1;
+      wk = wk1;
+      wt = wt1;
+      o += pl;
+    } else {
+      dp[q] = make_float2(0.f, 0.f);
     }
   }
-  s_a[tid] = d_last;
-  s_g[tid] = g_last;
+  if (active && k0 + kn == nz) st2(W, o, wt);
+  sf[tid] = prev;
   __syncthreads();
-  if (c == 0) {  // forward carries: s_e[cc] = dp(last level of chunk cc-1)
-    float e = 0.f;
-    s_e[tx] = 0.f;
-    for (int cc = 0; cc < C; ++cc) {
-      e = s_a[cc * 32 + tx] + s_g[cc * 32 + tx] * e;
-      s_e[(cc + 1) * 32 + tx] = e;
-    }
+  float2 in = make_float2(0.f, 0.f);  // dp(k0 - 1)
+  for (int cc = 0; cc < c; ++cc) {
+    const float2 f = sf[cc * 32 + tx];
+    const float g = tc[(cc + 1) * kM - 1].w;
+    in = make_float2(f.x + g * in.x, f.y + g * in.y);
   }
-  __syncthreads();
-  const float ein = s_e[tid];
-  float hq[kM];
 #pragma unroll
-  for (int q = 0; q < kM; ++q) dp[q] += gq[q] * ein;
-  float nxt = 0.f, h = 1.f;
-#pragma unroll
-  for (int q = kM - 1; q >= 0; --q) {
-    hq[q] = 1.f;
+  for (int q = 0; q < kM; ++q)
     if (q < kn) {
-      const int k = k0 + q;
-      dp[q] = dp[q] - s_lc[k] * nxt;  // local x with zero carry from above
-      nxt = dp[q];
-      h *= -s_lc[k];
-      hq[q] = h;
+      const float g = tc[k0 + q].w;
+      dp[q].x += g * in.x;
+      dp[q].y += g * in.y;
     }
-  }
-  s_a[tid] = dp[0];
-  s_g[tid] = hq[0];
-  __syncthreads();
-  if (c == 0) {  // backward carries: s_e[cc] = x(first level of chunk cc), s_e[C] = 0
-    float x = 0.f;
-    s_e[C * 32 + tx] = 0.f;
-    for (int cc = C - 1; cc >= 0; --cc) {
-      x = s_a[cc * 32 + tx] + s_g[cc * 32 + tx] * x;
-      s_e[cc * 32 + tx] = x;
-    }
-  }
-  __syncthreads();
-  const float xin = s_e[(c + 1) * 32 + tx];  // x(k0 + kn), 0 above the top
-  float x_last = 0.f;
+  float2 nx = make_float2(0.f, 0.f);
 #pragma unroll
-  for (int q = 0; q < kM; ++q) {
-    dp[q] += hq[q] * xin;  // dp now holds x
-    if (q == kn - 1) x_last = dp[q];
-  }
-  s_x[tid] = x_last;
+  for (int q = kM - 1; q >= 0; --q)
+    if (q < kn) {  // x with zero carry from above
+      const float l = tc[k0 + q].z;
+      dp[q].x -= l * nx.x;
+      dp[q].y -= l * nx.y;
+      nx = dp[q];
+    }
+  sx[tid] = dp[0];
   __syncthreads();
+  const float2 below = in;  // dp(k0 - 1), which gives x(k0 - 1) below
+  in = make_float2(0.f, 0.f);  // x(k0 + kn)
+  for (int cc = C - 1; cc > c; --cc) {
+    const float2 f = sx[cc * 32 + tx];
+    const float h = ta[cc * kM].w;
+    in = make_float2(f.x + h * in.x, f.y + h * in.y);
+  }
   if (!active) return;
-  const float xprev = (c > 0) ? s_x[tid - 32] : 0.f;
-  // final w on faces k0..k0+kn, then rho' and the outputs
-  float wn[kM + 1];
+  o = (unsigned)k0 * pl + col;
 #pragma unroll
-  for (int q = 0; q < kM + 1; ++q) {
-    const int f = k0 + q;
-    wn[q] = wt[q];
-    if (q <= kn && f >= 1 && f < nz) {
-      const float xf = (q < kn) ? dp[q] : xin;
-      const float xb = (q == 0) ? xprev : dp[q - 1];
-      wn[q] = wt[q] - dtau * b * cpf * s_tfz[f] * (xf - xb) * s_idzw[f];
+  for (int q = 0; q < kM; ++q)
+    if (q < kn) {
+      const float h = ta[k0 + q].w;
+      dp[q].x += h * in.x;
+      dp[q].y += h * in.y;
+      st2(PI, o + q * pl, dp[q]);
     }
+  if (!last) return;
+  auto back = [&](int q, unsigned at) {  // this thread's own stores
+    if (two) return *reinterpret_cast<const float2*>(wout.f[q] + at);
+    return make_float2(wout.f[q][at], 0.f);
+  };
+  float2 wb = back(W, o);  // w at the level's lower face
+  if (c > 0) {
+    const float l = tc[k0 - 1].z, a = ta[k0].y;
+    wb.x -= a * (dp[0].x - (below.x - l * dp[0].x));
+    wb.y -= a * (dp[0].y - (below.y - l * dp[0].y));
   }
 #pragma unroll
-  for (int q = 0; q < kM; ++q) {
+  for (int q = 0; q < kM; ++q)
     if (q < kn) {
       const int k = k0 + q;
-      const size_t o = (size_t)k * pl;
-      const float dv_new = -(s_rfz[k + 1] * wn[q + 1] - s_rfz[k] * wn[q]) * s_idzc[k];
-      Ro[o] = rs[q] + dtau * b * dv_new;
-      Po[o] = dp[q];
-      Wo[o] = wn[q];
+      const float4 A0 = ta[k], A1 = ta[k + 1];
+      const float iz = tb[k].x;
+      const bool top = q + 1 >= kn;
+      const float2 xf = top ? in : dp[q + 1 < kM ? q + 1 : q];
+      const float2 wf = top ? wt : back(W, o + pl);
+      const float2 wn = make_float2(wf.x - A1.y * (xf.x - dp[q].x), wf.y - A1.y * (xf.y - dp[q].y));
+      const float2 r = back(RHO, o);
+      st2(RHO, o, make_float2(r.x + db * ((A0.z * wb.x - A1.z * wn.x) * iz),
+                              r.y + db * ((A0.z * wb.y - A1.z * wn.y) * iz)));
+      st2(W, o, wb);
+      wb = wn;
+      o += pl;
     }
-  }
-  if (k0 + kn == nz) Wo[(size_t)nz * pl] = w_top;
 }
 
-template <int kM>
-__global__ void __launch_bounds__(640, 2) k_mx_hevi_par(const __grid_constant__ Dims d, const __grid_constant__ Tab t,
-                                                      const __grid_constant__ Flags fl, const __grid_constant__ WS win,
-                                                      const __grid_constant__ WS wout, float dtau,
-                                                      const float* __restrict__ lu, int apply_uv, float cdx,
-                                                      float cdy) {
-  hevi_par_body<kM>(d, t, fl, win, wout, dtau, lu, apply_uv, cdx, cdy, blockIdx.x, blockIdx.y);
+template <int kM, int kThreads, int kBlocks>
+__global__ void __launch_bounds__(kThreads, kBlocks) k_mx_hevi_chunk(
+    const __grid_constant__ Dims d, const __grid_constant__ Tab t, const __grid_constant__ Flags fl,
+    const __grid_constant__ WS win, const __grid_constant__ WS wout, float dtau, const float* __restrict__ lu,
+    int apply_uv, int last, float cdx, float cdy) {
+  hevi_chunk_body<kM>(d, t, fl, win, wout, dtau, lu, apply_uv, last, cdx, cdy, blockIdx.x);
 }
 
 template <int kPF, int kRing>
@@ -2557,27 +2562,47 @@ size_t hevi_smem_bytes(int nz, int ring) {
   return (10 * (size_t)(nz + 1) + (size_t)ring * 11 * 128) * sizeof(float);
 }
 
-// Levels per thread of the level-split column kernel (0 = one thread per
-// column, hevi_body); VIBE_GB300_HEVI_PAR=0|4|8 overrides the built-in choice.
-int hevi_par_levels(int nz) {
-  static int v = -1;
-  if (v < 0) {
-    v = kDefaultHeviPar;
+// Levels per warp of the level-split column kernel for a launch over `columns`
+// columns, 0 = the sweeping kernels. VIBE_GB300_HEVI_PAR=0 turns it off, 4 or
+// 8 fixes the levels. Eight chunks (256 threads, 4 blocks an SM at 64
+// registers) measured best from 128 x 128 up; below, where the blocks do not
+// fill the SMs twice, shorter chunks without the register limit (a launch at
+// 64 x 64 x 40: 10.8 us, 14.7 with 8 levels; the sweeping kernel 50.8; at
+// 193 x 193 x 60 23 against 75, at 512 x 512 x 80 179 against 187).
+// Moist models keep the sweeping kernel: the carries round differently, and
+// the saturation adjustment turns a difference in the last bits of theta and
+// pi into 6e-5 of qc within two steps (cloud water is the small difference of
+// vapour and saturation), though either rounding is as good.
+int hevi_chunk_levels(int nz, long columns, const Flags& fl) {
+  static int env = -2;
+  if (env == -2) {
+    int v = -1;
     if (const char* e = std::getenv("VIBE_GB300_HEVI_PAR")) {
       const int x = std::atoi(e);
       if (x == 0 || x == 4 || x == 8) v = x;
     }
+    env = v;
   }
-  if (v == 0) return 0;
-  int m = v;
-  if ((nz + m - 1) / m > 20) m = 8;       // at most 20 chunks (640 threads)
-  return ((nz + m - 1) / m > 20) ? 0 : m;  // taller columns: one thread per column
+  if (env == 0 || fl.moist) return 0;
+  int m = env;
+  if (m < 0) m = columns <= kChunkSmall ? 4 : nz <= 48 ? 6 : nz <= 64 ? 8 : 10;
+  if ((nz + m - 1) / m > kMaxChunks) m = 10;
+  return (nz + m - 1) / m <= kMaxChunks ? m : 0;  // taller columns: one thread per column
 }
-
-size_t hevi_par_smem_bytes(int nz, int m) {
-  const int C = (nz + m - 1) / m;
-  return (10 * (size_t)(nz + 1) + (size_t)32 * (4 * C + 1)) * sizeof(float);
-}
+int hevi_chunk_blocks(const Dims& d) { return ((d.ny - 1) * d.P + d.nx + 63) / 64; }
+// Kernel<levels, threads, blocks an SM> for m levels of nz, m from hevi_chunk_levels
+#define VGB_CHUNK_LAUNCH(Kernel, m, nz, blocks, st, ...)                                                        \
+  do {                                                                                                          \
+    const int C_ = ((nz) + (m) - 1) / (m);                                                                      \
+    const dim3 b_(32, C_);                                                                                      \
+    const size_t sm_ = hevi_chunk_smem_bytes(nz, m);                                                            \
+    if ((m) == 4) Kernel<4, 640, 1><<<blocks, b_, sm_, st>>>(__VA_ARGS__);                                      \
+    else if ((m) == 6) Kernel<6, 256, 4><<<blocks, b_, sm_, st>>>(__VA_ARGS__);                                 \
+    else if ((m) == 8 && C_ <= 8) Kernel<8, 256, 4><<<blocks, b_, sm_, st>>>(__VA_ARGS__);                      \
+    else if ((m) == 8) Kernel<8, 640, 1><<<blocks, b_, sm_, st>>>(__VA_ARGS__);                                 \
+    else if (C_ <= 8) Kernel<10, 256, 4><<<blocks, b_, sm_, st>>>(__VA_ARGS__);                                 \
+    else Kernel<10, 640, 1><<<blocks, b_, sm_, st>>>(__VA_ARGS__);                                              \
+  } while (0)
 
 // Ring depth of the two-columns-per-thread kernel (0 = off);
 // VIBE_GB300_HEVI_TWO=0|2|3|4 overrides the built-in choice.
@@ -2613,14 +2638,16 @@ bool hevi_defer() {
   return v != 0;
 }
 
-// the column kernel variant for this grid among the TMA ones: 4 TMA,
-// 5 TMA with deferred corrections, -1 neither
-int hevi_tma_variant(const Dims& d) {
+// the column kernel variant for this grid among the TMA and the level-split
+// ones: 4 TMA, 5 TMA with deferred corrections, 6 level-split, -1 neither
+int hevi_tma_variant(const Dims& d, const Flags& fl) {
   MixedTune tn;
   bool tma = hevi_tma(), defer = hevi_defer();
   if (tune_of(d, &tn) && tn.column >= 0) {
     tma = tn.column == 4 || tn.column == 5;
     defer = tn.column == 5;
+  } else if (hevi_chunk_levels(d.nz, (long)d.nx * d.ny, fl)) {
+    return 6;
   }
   if (!tma || hevi_tma_smem_bytes(d.nz) > 48 * 1024) return -1;
   return defer ? 5 : 4;
@@ -2631,7 +2658,7 @@ size_t hevi2_smem_bytes(int nz, int ring) {
 }
 
 int mixed_hevi_column(const Dims& d, const Tab& t, const Flags& fl, const WS& win, const WS& wout, float dtau,
-                      const float* lu, bool apply_uv, unsigned* err, cudaStream_t stream) {
+                      const float* lu, bool apply_uv, bool last, unsigned* err, cudaStream_t stream) {
   MixedTune tn;
   const bool tuned = tune_of(d, &tn) && tn.column >= 0;
   int r2 = hevi_two_ring(), ring = hevi_ring();
@@ -2639,7 +2666,15 @@ int mixed_hevi_column(const Dims& d, const Tab& t, const Flags& fl, const WS& wi
     r2 = (tn.column == 2) ? 2 : (tn.column == 3 ? 3 : 0);
     ring = (tn.column == 1) ? 4 : 0;
   }
-  if (const int v = hevi_tma_variant(d); v >= 0) {
+  const int v = hevi_tma_variant(d, fl);
+  if (v == 6) {
+    const int m = hevi_chunk_levels(d.nz, (long)d.nx * d.ny, fl);
+    const float cdx = -(float)kCp * dtau * t.dx_inv, cdy = -(float)kCp * dtau * t.dy_inv;
+    VGB_CHUNK_LAUNCH(k_mx_hevi_chunk, m, d.nz, hevi_chunk_blocks(d), stream, d, t, fl, win, wout, dtau, lu,
+                     apply_uv ? 1 : 0, last ? 1 : 0, cdx, cdy);
+    return 0;
+  }
+  if (v >= 0) {
     ColumnMaps C;
     if (!column_maps(d, win, wout, C)) return -1;
     const dim3 bc(32, 4);
@@ -2662,17 +2697,6 @@ int mixed_hevi_column(const Dims& d, const Tab& t, const Flags& fl, const WS& wi
     if (r2 == 4) k_mx_hevi_col2<4><<<g, bc, sm, stream>>>(d, t, fl, win, wout, dtau, lu, au, cdx, cdy);
     else if (r2 == 3) k_mx_hevi_col2<3><<<g, bc, sm, stream>>>(d, t, fl, win, wout, dtau, lu, au, cdx, cdy);
     else k_mx_hevi_col2<2><<<g, bc, sm, stream>>>(d, t, fl, win, wout, dtau, lu, au, cdx, cdy);
-    return 0;
-  }
-  if (const int m = tuned ? 0 : hevi_par_levels(d.nz)) {
-    const dim3 bp(32, (d.nz + m - 1) / m);
-    const dim3 gp((d.nx + 31) / 32, d.ny);
-    const float cdx = -(float)kCp * dtau * t.dx_inv, cdy = -(float)kCp * dtau * t.dy_inv;
-    const size_t sm = hevi_par_smem_bytes(d.nz, m);
-    if (m == 4)
-      k_mx_hevi_par<4><<<gp, bp, sm, stream>>>(d, t, fl, win, wout, dtau, lu, apply_uv ? 1 : 0, cdx, cdy);
-    else
-      k_mx_hevi_par<8><<<gp, bp, sm, stream>>>(d, t, fl, win, wout, dtau, lu, apply_uv ? 1 : 0, cdx, cdy);
     return 0;
   }
   const dim3 bc(32, 4);
@@ -2702,7 +2726,7 @@ void mixed_uv_backward(const Dims& d, const Tab& t, const WS& win, const WS& wou
   k_mx_fb_mom<<<g3(d.nx + 1, d.ny + 1, d.nz, b), b, 0, stream>>>(d, t, win, wout, dtau, 0);
 }
 
-bool mixed_hevi_defers(const Dims& d) { return hevi_tma_variant(d) == 5; }
+bool mixed_hevi_defers(const Dims& d, const Flags& fl) { return hevi_tma_variant(d, fl) == 5; }
 
 void mixed_uv_fix(const Dims& d, const Tab& t, const Flags& fl, const WS& s, float dtau, cudaStream_t stream) {
   const dim3 b(32, 4);
@@ -2711,9 +2735,9 @@ void mixed_uv_fix(const Dims& d, const Tab& t, const Flags& fl, const WS& s, flo
 
 int mixed_hevi_substep(const Dims& d, const Tab& t, const Flags& fl, const WS& win, const WS& wout, float dtau,
                        const float* lu, unsigned* err, cudaStream_t stream) {
-  if (mixed_hevi_column(d, t, fl, win, wout, dtau, lu, false, err, stream)) return -1;
+  if (mixed_hevi_column(d, t, fl, win, wout, dtau, lu, false, true, err, stream)) return -1;
   // in place: u, v were copied by the column kernel
-  if (mixed_hevi_defers(d)) mixed_uv_fix(d, t, fl, wout, dtau, stream);
+  if (mixed_hevi_defers(d, fl)) mixed_uv_fix(d, t, fl, wout, dtau, stream);
   else mixed_uv_backward(d, t, wout, wout, dtau, stream);
   return 0;
 }
@@ -2816,7 +2840,7 @@ struct HeviArgs {  // 64-byte aligned through its CUtensorMap members
   WS win, wout;
   float dtau, cdx, cdy;
   const float* lu;
-  int apply_uv, gx, gy;
+  int apply_uv, last, gx, gy;
 };
 struct UvArgs {
   Dims d;
@@ -2882,6 +2906,15 @@ __global__ void __launch_bounds__(128, 7) k_b_hevi_tmad(const HeviArgs* __restri
                       l / a.gx);
 }
 
+template <int kM, int kThreads, int kBlocks>
+__global__ void __launch_bounds__(kThreads, kBlocks) k_b_hevi_chunk(const HeviArgs* __restrict__ A,
+                                                                    const int* __restrict__ start, int nd) {
+  const int dom = find_domain(start, nd);
+  const HeviArgs& a = A[dom];
+  hevi_chunk_body<kM>(a.d, a.t, a.fl, a.win, a.wout, a.dtau, a.lu, a.apply_uv, a.last, a.cdx, a.cdy,
+                      (int)blockIdx.x - start[dom]);
+}
+
 __global__ void k_b_uv(const UvArgs* __restrict__ A, const int* __restrict__ start, int nd) {
   const int dom = find_domain(start, nd);
   const UvArgs& a = A[dom];
@@ -2926,6 +2959,7 @@ struct MixedBatch {
   std::vector<Launch> seq;
   std::vector<void*> allocs;
   size_t hevi_smem = 0;
+  int split = 0, nz = 0;  // split > 0: the level-split column body with that many levels per warp
   bool hevi_tma = false;  // TMA-fed column body (else the cp.async two-column body)
   bool defer = false;     // the TMA body defers its w/rho' corrections (u/v launches become fix-ups)
   bool spec = false;      // the stage body with the flags of the kSpec composition fixed
@@ -2962,10 +2996,15 @@ MixedBatch* mixed_batch_build(const std::vector<MixedDomain>& doms, const Flags&
     if (m.d.nz != nz) return nullptr;
   auto* b = new MixedBatch();
   b->err = err;
-  b->hevi_tma = hevi_tma() && hevi_tma_smem_bytes(nz) <= 48 * 1024;
+  long columns = 0;  // one launch runs all of them
+  for (const auto& m : doms) columns += (long)m.d.nx * m.d.ny;
+  b->nz = nz;
+  b->split = hevi_chunk_levels(nz, columns, fl);
+  b->hevi_tma = !b->split && hevi_tma() && hevi_tma_smem_bytes(nz) <= 48 * 1024;
   b->defer = b->hevi_tma && hevi_defer();
   b->spec = stage_spec(fl);
-  b->hevi_smem = b->hevi_tma ? hevi_tma_smem_bytes(nz) : hevi2_smem_bytes(nz, kBatchTwoRing);
+  b->hevi_smem = b->split ? hevi_chunk_smem_bytes(nz, b->split)
+                          : b->hevi_tma ? hevi_tma_smem_bytes(nz) : hevi2_smem_bytes(nz, kBatchTwoRing);
   const double dts[3] = {dt / 3.0, dt / 2.0, dt};
   const int nd = (int)doms.size();
   auto sub_out = [&](const MixedDomain& m, int n) { return (n & 1) ? m.WB : m.WA; };
@@ -3015,11 +3054,12 @@ MixedBatch* mixed_batch_build(const std::vector<MixedDomain>& doms, const Flags&
         a.cdy = -(float)kCp * dtau * m.t.dy_inv;
         a.lu = m.lu + (size_t)stage * 3 * nz;
         a.apply_uv = n > 0;
+        a.last = n == n_sub - 1;
         if (b->hevi_tma && !column_maps(m.d, a.win, a.wout, a.C)) ok = false;
         a.gx = ceil_div(m.d.nx, 64);  // two columns per thread
         a.gy = ceil_div(m.d.ny, 4);
         start[q] = hb;
-        hb += a.gx * a.gy;
+        hb += b->split ? hevi_chunk_blocks(m.d) : a.gx * a.gy;
       }
       ok = ok && upload_launch(b, 1, 0, ha, start, hb);
     }
@@ -3091,7 +3131,9 @@ void mixed_batch_enqueue(const MixedBatch* b, cudaStream_t s) {
           k_b_stage<false, false><<<L.blocks, dim3(TX, TY), 0, s>>>((const StageArgs*)L.args, L.start, L.nd, b->err);
         break;
       case 1:
-        if (b->defer)
+        if (b->split)
+          VGB_CHUNK_LAUNCH(k_b_hevi_chunk, b->split, b->nz, L.blocks, s, (const HeviArgs*)L.args, L.start, L.nd);
+        else if (b->defer)
           k_b_hevi_tmad<<<L.blocks, dim3(32, 4), b->hevi_smem, s>>>((const HeviArgs*)L.args, L.start, L.nd, b->err);
         else if (b->hevi_tma)
           k_b_hevi_tma<<<L.blocks, dim3(32, 4), b->hevi_smem, s>>>((const HeviArgs*)L.args, L.start, L.nd, b->err);
