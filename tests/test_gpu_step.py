@@ -193,6 +193,32 @@ def test_consistent_hevi_substep_fp64(vg, oc, beta):
         assert_state_close(vg, s, m.state(), o.state(), TOL64, range(7), "consistent HEVI substep")
 
 
+@pytest.mark.parametrize("pgf", [0, 1])
+@pytest.mark.parametrize("dims", [(5, 3, 7), (33, 17, 8), (31, 1, 9), (40, 9, 81), (24, 20, 160), (8, 6, 161)])
+def test_hevi_level_split_fp64(vg, oc, dims, pgf):
+    """The FP64 level-split HEVI substep (flat grid, uniform reference state) at
+    its edges (a last chunk of one level, one chunk, more than ten chunks, the
+    tallest columns, columns too tall for it) against the oracle, inside the
+    substep's horizontal acoustic limit, and its adjoint by the dot product:
+    the bounds of the substep and of the HEVI adjoint elsewhere, 1e-12."""
+    nx, ny, nz = dims
+    s = small_setup(vg, nx=nx, ny=ny, nz=nz, zeta_stretch=1.0, ref_kind=1, acoustic_mode=2, hevi_beta=0.6,
+                    pgf_perturbation=pgf, bubble_xc=nx * 125.0, bubble_yc=ny * 125.0)
+    with vg.Model(s, vg.FP64) as m:
+        o = oc.Model(oracle_setup(oc, s), "port")
+        for _ in range(2):
+            m.hevi_substep(0.4)
+            o.hevi_substep(0.4)
+        assert_state_close(vg, s, m.state(), o.state(), TOL64, range(7), "HEVI substep %s" % (dims,))
+        rng = np.random.default_rng(11)
+        x, y = ([a * rng.standard_normal(m.size(sp)) for a, sp in zip((1.0, 1.0, 0.5, 1e-3, 1e-4), m.ACOUSTIC_FIELDS)]
+                for _ in range(2))
+        tx, ay = m.hevi_tl(0.4, 3, x), m.hevi_ad(0.4, 3, y)
+        lhs, rhs = (float(sum(np.dot(p, q) for p, q in zip(a, b))) for a, b in ((tx, y), (x, ay)))
+        norm = np.sqrt(sum(np.dot(p, p) for p in tx) * sum(np.dot(q, q) for q in y))
+        assert abs(lhs - rhs) <= 1e-12 * norm, (lhs, rhs, norm)
+
+
 def test_sponge_fp64(vg, oc):
     s = small_setup(vg, sponge_alpha=0.3, sponge_start_fraction=0.5)
     with vg.Model(s, vg.FP64) as m:

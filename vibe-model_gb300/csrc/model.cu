@@ -124,6 +124,11 @@ struct vibe_gb300_model {
   unsigned* h_err = nullptr;      // pinned
   double* h_pin = nullptr;        // pinned staging
   size_t pin_n = 0;
+  // FP64 HEVI substep on uniform grids: Metric::hevi tables of the last few dtau
+  static constexpr int kHeviSlots = 6;
+  double* d_hevi[kHeviSlots] = {};
+  double hevi_dtau[kHeviSlots] = {};
+  int hevi_next = 0;
   double cfg_dt = -1.0;
   int cfg_nsub = -1;
   int kmin = 0;
@@ -548,6 +553,88 @@ int configure_dt(vibe_gb300_model* m, double dt, int n_sub) {
   return 0;
 }
 
+// The metric of an FP64 HEVI substep of dtau: with the per-level coefficient
+// table (Metric::hevi) on flat grids with a uniform reference state, where the
+// fast build's level-split kernels take it; without (the per-column kernels)
+// for terrain, the bit-exact build, columns above 160 levels, or a column
+// matrix whose pivots are not all safely away from zero. A table depends on
+// the model and dtau only; it is laid out once per dtau (a step uses three)
+// and uploaded on the model's stream, behind the launches that read the slot
+// it replaces.
+int hevi_metric(vibe_gb300_model* m, double dtau, Metric* out) {
+  *out = m->met;
+  out->hevi = nullptr;
+  const int nz = m->d.nz, C = (nz + kHevi64M - 1) / kHevi64M;
+  if (!m->uniform || m->f64 != &kFp64Fast || C > kHevi64Chunks) return 0;
+  for (int s = 0; s < vibe_gb300_model::kHeviSlots; ++s)
+    if (m->d_hevi[s] && m->hevi_dtau[s] == dtau) {
+      out->hevi = m->d_hevi[s];
+      return 0;
+    }
+  const auto& hs = m->hs;
+  const int cx = m->nsx[RHO], cy = m->nsy[RHO], R = nz + 1;
+  auto ref = [&](int w, int k) { return hs.ref[w][soff(cx, cy, 0, 0, iclamp(k, 0, nz - 1))]; };
+  auto dz = [&](int k) {
+    const int kk = iclamp(k, 0, nz - 1);
+    return dmax((hs.zeta[kk + 1] - hs.zeta[kk]) * m->su.z_top, 1.0);
+  };
+  const double b = m->su.hevi_beta;
+  std::vector<double> t((size_t)kH_rows * R, 0.0), sub(nz), sup(nz);
+  auto at = [&](int row, int k) -> double& { return t[(size_t)row * R + k]; };
+  for (int k = 0; k <= nz; ++k) {
+    const double rf = 0.5 * (ref(2, k - 1) + ref(2, k)), tf = 0.5 * (ref(0, k - 1) + ref(0, k));
+    at(kH_rf, k) = rf;
+    if (k > 0 && k < nz) {
+      at(kH_ae, k) = dtau * (1.0 - b) * kCp * tf / dz(k);
+      at(kH_ai, k) = dtau * b * kCp * tf / dz(k);
+    }
+    if (k < nz) at(kH_ra, k) = rf / dz(k);
+    if (k > 0) at(kH_rb, k) = rf / dz(k - 1);
+  }
+  for (int k = 0; k < nz; ++k) {
+    const double kap = (kRd / kCv) * (ref(1, k) / dmax(ref(2, k), 1e-8));
+    at(kH_idz, k) = 1.0 / dz(k);
+    at(kH_dk, k) = dtau * kap;
+    at(kH_r0, k) = ref(2, k);
+    at(kH_p0, k) = ref(1, k);
+    at(kH_cu, k) = dtau * kCp * ref(0, k) / m->su.dx;
+    at(kH_cv, k) = dtau * kCp * ref(0, k) / m->su.dy;
+    const double ck = (dtau * b) * (dtau * b) * kap / dz(k);
+    auto Tf = [&](int f) { return (f == 0 || f == nz) ? 0.0 : at(kH_rf, f) * kCp * 0.5 * (ref(0, f - 1) + ref(0, f)) / dz(f); };
+    sub[k] = -ck * Tf(k);
+    sup[k] = -ck * Tf(k + 1);
+    const double diag = 1.0 + ck * (Tf(k) + Tf(k + 1));
+    const double piv = (k == 0) ? diag : diag - sub[k] * at(kH_lc, k - 1);
+    if (!(std::fabs(piv) > 1e-6 && std::fabs(piv) < 1e30)) return 0;
+    at(kH_li, k) = 1.0 / piv;
+    at(kH_m, k) = sub[k] / piv;
+    at(kH_lc, k) = (k + 1 < nz) ? sup[k] / piv : 0.0;
+  }
+  for (int k = 0; k < nz; ++k) {  // the transpose: sub-diagonal sup(k-1), super-diagonal sub(k+1), the same pivots
+    at(kH_mT, k) = (k > 0) ? sup[k - 1] * at(kH_li, k) : 0.0;
+    at(kH_lcT, k) = (k + 1 < nz) ? sub[k + 1] * at(kH_li, k) : 0.0;
+  }
+  for (int k = 0; k < nz; ++k) {
+    const bool first = k % kHevi64M == 0;
+    at(kH_G, k) = -at(kH_m, k) * (first ? 1.0 : at(kH_G, k - 1));
+    at(kH_GT, k) = -at(kH_mT, k) * (first ? 1.0 : at(kH_GT, k - 1));
+  }
+  for (int k = nz - 1; k >= 0; --k) {
+    const bool top = k == nz - 1 || k % kHevi64M == kHevi64M - 1;
+    at(kH_H, k) = -at(kH_lc, k) * (top ? 1.0 : at(kH_H, k + 1));
+    at(kH_HT, k) = -at(kH_lcT, k) * (top ? 1.0 : at(kH_HT, k + 1));
+  }
+  const int s = m->hevi_next;
+  if (!m->d_hevi[s])
+    if (int rc = dalloc(m, &m->d_hevi[s], t.size())) return rc;
+  CUDA_OK(cudaMemcpyAsync(m->d_hevi[s], t.data(), t.size() * sizeof(double), cudaMemcpyHostToDevice, m->stream));
+  CUDA_OK(cudaStreamSynchronize(m->stream));  // t goes out of scope
+  m->hevi_dtau[s] = dtau;
+  m->hevi_next = (s + 1) % vibe_gb300_model::kHeviSlots;
+  out->hevi = m->d_hevi[s];
+  return 0;
+}
+
 // reference HEVI coefficients from column (0,0), acoustic_substep.cpp:38-65
 int ref_hevi_coefficients(vibe_gb300_model* m, double dtau) {
   const int nz = m->d.nz;
@@ -707,13 +794,16 @@ int enqueue_one_step(vibe_gb300_model* m, double dt, int n_sub) {
         const double dtau = dts[stage] / (double)n_sub;
         if (m->fl.acoustic_mode == 1)
           if (int rc = ref_hevi_coefficients(m, dtau)) return rc;
+        Metric hm;
+        if (m->fl.acoustic_mode == 2)
+          if (int rc = hevi_metric(m, dtau, &hm)) return rc;
         for (int n = 0; n < n_sub; ++n) {
           Span sp(m, 1);
           if (m->fl.acoustic_mode == 0) m->f64->fb_substep(d, m->met, m->fl, S1, dtau, m->stream);
           else if (m->fl.acoustic_mode == 1)
             m->f64->ref_hevi_substep(d, m->met, S1, dtau, m->d_tri, m->d_tri + d.nz, m->d_tri + 2 * d.nz, m->scratch,
                                   m->d_err, m->stream);
-          else m->f64->cons_hevi_substep(d, m->met, m->fl, S1, m->tmp, m->scratch, dtau, m->d_err, m->stream);
+          else m->f64->cons_hevi_substep(d, hm, m->fl, S1, m->tmp, m->scratch, dtau, m->d_err, m->stream);
         }
         Span sp(m, 2);
         m->f64->nonfinite(d, S1, m->d_err, m->stream);
@@ -1210,6 +1300,9 @@ int acoustic_linear(vibe_gb300_model* m, double dtau, int n_sub, const double* c
     st[kLinField[f]] = m->lin[f];
     if (int rc = upload_storage(m, kLinField[f], in[f], &m->lin[f], 1)) return rc;
   }
+  Metric hm;
+  if (hevi)
+    if (int rc = hevi_metric(m, dtau, &hm)) return rc;
   Flags lf = m->fl;
   lf.pgf_pert = 0;  // gradient of pi' itself: the substep is linear
   double* tmp[NSPECIES] = {};
@@ -1218,8 +1311,8 @@ int acoustic_linear(vibe_gb300_model* m, double dtau, int n_sub, const double* c
   tmp[PI] = m->lin_tmp[2];
   for (int n = 0; n < n_sub; ++n) {
     if (hevi) {
-      if (adjoint) m->f64->hevi_substep_ad(m->d, m->met, lf, st, m->lin_dh, m->lin_scr, dtau, m->d_err, m->stream);
-      else m->f64->cons_hevi_substep(m->d, m->met, lf, st, tmp, m->lin_scr, dtau, m->d_err, m->stream);
+      if (adjoint) m->f64->hevi_substep_ad(m->d, hm, lf, st, m->lin_dh, m->lin_scr, dtau, m->d_err, m->stream);
+      else m->f64->cons_hevi_substep(m->d, hm, lf, st, tmp, m->lin_scr, dtau, m->d_err, m->stream);
     } else {
       if (adjoint) m->f64->fb_substep_ad(m->d, m->met, st, dtau, m->stream);
       else m->f64->fb_substep(m->d, m->met, lf, st, dtau, m->stream);
@@ -1376,7 +1469,9 @@ int vibe_gb300_hevi_substep(vibe_gb300_model* m, double dtau) {
       m->f64->ref_hevi_substep(m->d, m->met, m->S[m->cur], dtau, m->d_tri, m->d_tri + m->d.nz, m->d_tri + 2 * m->d.nz,
                             m->scratch, m->d_err, m->stream);
     } else {
-      m->f64->cons_hevi_substep(m->d, m->met, m->fl, m->S[m->cur], m->tmp, m->scratch, dtau, m->d_err, m->stream);
+      Metric hm;
+      if (int rc = hevi_metric(m, dtau, &hm)) return rc;
+      m->f64->cons_hevi_substep(m->d, hm, m->fl, m->S[m->cur], m->tmp, m->scratch, dtau, m->d_err, m->stream);
     }
   } else {
     // single substep: factors for this dtau in stage slot 0
@@ -2471,6 +2566,9 @@ int stl_substeps(vibe_gb300_model* m, int stage, double dtau, int n_sub, double*
   const Dims& d = m->d;
   const bool hevi = m->fl.acoustic_mode == 2;
   if (m->precision == VIBE_GB300_FP64) {
+    Metric hm;
+    if (hevi)
+      if (int rc = hevi_metric(m, dtau, &hm)) return rc;
     Flags lf = m->fl;
     lf.pgf_pert = 0;  // the linear part: the gradient of the perturbation of pi
     double* tmp[NSPECIES] = {};
@@ -2479,10 +2577,10 @@ int stl_substeps(vibe_gb300_model* m, int stage, double dtau, int n_sub, double*
     tmp[PI] = m->lin_tmp[2];
     for (int n = 0; n < n_sub; ++n) {
       if (adjoint) {
-        if (hevi) m->f64->hevi_substep_ad(d, m->met, lf, x, m->lin_dh, m->lin_scr, dtau, m->d_err, m->stream);
+        if (hevi) m->f64->hevi_substep_ad(d, hm, lf, x, m->lin_dh, m->lin_scr, dtau, m->d_err, m->stream);
         else m->f64->fb_substep_ad(d, m->met, x, dtau, m->stream);
       } else {
-        if (hevi) m->f64->cons_hevi_substep(d, m->met, lf, x, tmp, m->lin_scr, dtau, m->d_err, m->stream);
+        if (hevi) m->f64->cons_hevi_substep(d, hm, lf, x, tmp, m->lin_scr, dtau, m->d_err, m->stream);
         else m->f64->fb_substep(d, m->met, lf, x, dtau, m->stream);
       }
     }

@@ -646,6 +646,140 @@ __global__ void k_chevi_column(Dims d, Metric m, Flags fl, CS s, double* __restr
   for (int k = 0; k <= nz; ++k) w_out[IDX(i, j, k)] = S(WN, k);
 }
 
+#ifndef VGB_FP64_EXACT
+// The same substep on flat grids with a uniform reference state, levels split
+// over warps. Its column matrix is one per level there, factored once on the
+// host (Metric::hevi): no division and no per-column coefficient is left, and
+// the two recurrences split into chunks of kHevi64M levels joined by carries
+// (as in the mixed path's level-split kernel: dp(k) = dp0(k) + G(k) dp(k0-1),
+// x(k) = x0(k) + H(k) x(k0+kn)). A warp is 32 consecutive points of the padded
+// plane by one chunk, a block the chunks of its columns. w, rho and pi are
+// updated in place: a chunk reads its inputs (its own and the two levels
+// beside it) before the first barrier and writes after the second. The points
+// of the ghost column and row get the zeros the substep leaves there.
+// Bound by the FP64 pipe: about 30 FP64 operations per cell, where the
+// sweeping kernel above spends ~250 (divisions, per-column coefficients).
+template <int kBlocks>
+__global__ void __launch_bounds__(32 * kHevi64Chunks / kBlocks, kBlocks)
+    k_chevi_chunk(Dims d, const double* __restrict__ tab, double inv_dx, double inv_dy, double b, double dtau, int pert,
+                  const double* __restrict__ u, const double* __restrict__ v, double* __restrict__ w,
+                  double* __restrict__ rho, double* __restrict__ pi) {
+  constexpr int kM = kHevi64M;
+  extern __shared__ double sh64[];
+  const int nz = d.nz, C = blockDim.y, R = nz + 1;
+  double* sf = sh64;            // C x 32: dp at each chunk's last level, zero carry
+  double* sx = sh64 + 32 * C;   // C x 32: x at each chunk's first level, zero carry
+  const int tx = threadIdx.x, c = threadIdx.y, tid = c * 32 + tx;
+  const int e = blockIdx.x * 32 + tx;
+  const int j = e / d.P, i = e - j * d.P;
+  const bool active = i < d.nx && j < d.ny;
+  const bool ghost = !active && i <= d.nx && j <= d.ny;
+  const int k0 = c * kM, kn = imin(kM, nz - k0);
+  const size_t pl = d.plane, col = active ? (size_t)e : 0;
+  auto T = [&](int row, int k) { return __ldg(tab + row * R + k); };
+  const double ob = 1.0 - b;
+  double pv[kM + 2], wv[kM + 1], rs[kM], dp[kM];
+#pragma unroll
+  for (int q = 0; q < kM + 2; ++q) {
+    const int k = k0 - 1 + q;
+    pv[q] = (active && k >= 0 && k < nz && q <= kn + 1) ? pi[(size_t)k * pl + col] - (pert ? T(kH_p0, k) : 0.0) : 0.0;
+  }
+#pragma unroll
+  for (int q = 0; q < kM + 1; ++q) wv[q] = (active && q <= kn) ? w[(size_t)(k0 + q) * pl + col] : 0.0;
+  double prev = 0.0, fo = 0.0, ft = 0.0;  // rho0_f w and rho0_f w~ at the level's lower face
+  if (active) {
+    const double r = T(kH_rf, k0);
+    fo = r * wv[0];
+    wv[0] -= T(kH_ae, k0) * (pv[1] - pv[0]);
+    ft = r * wv[0];
+  }
+#pragma unroll
+  for (int q = 0; q < kM; ++q) {
+    rs[q] = dp[q] = 0.0;
+    if (q < kn && active) {
+      const int k = k0 + q;
+      const size_t o = (size_t)k * pl + col;
+      const double r1 = T(kH_rf, k + 1), iz = T(kH_idz, k);
+      const double fo1 = r1 * wv[q + 1];
+      wv[q + 1] -= T(kH_ae, k + 1) * (pv[q + 2] - pv[q + 1]);  // w~ at the upper face
+      const double ft1 = r1 * wv[q + 1];
+      const double dh = -T(kH_r0, k) * ((u[o + 1] - u[o]) * inv_dx + (v[o + d.P] - v[o]) * inv_dy);
+      const double S = dh + (ob * iz) * (fo - fo1);
+      const double z = T(kH_dk, k) * (S + (b * iz) * (ft - ft1));
+      // the total first, as the reference forms it (its rounding at pi ~ 1 is part of its result)
+      const double p0 = pert ? T(kH_p0, k) : 0.0;
+      const double rhs = pert ? ((pv[q + 1] + p0) + z) - p0 : pv[q + 1] + z;
+      rs[q] = rho[o] + dtau * S;
+      prev = rhs * T(kH_li, k) - T(kH_m, k) * prev;
+      dp[q] = prev;
+      fo = fo1;
+      ft = ft1;
+    }
+  }
+  sf[tid] = prev;
+  __syncthreads();
+  double below = 0.0;  // dp(k0 - 1)
+  for (int cc = 0; cc < c; ++cc) below = sf[cc * 32 + tx] + T(kH_G, (cc + 1) * kM - 1) * below;
+  double nxt = 0.0;
+#pragma unroll
+  for (int q = kM - 1; q >= 0; --q)
+    if (q < kn) {  // x with zero carry from above
+      dp[q] += T(kH_G, k0 + q) * below;
+      dp[q] -= T(kH_lc, k0 + q) * nxt;
+      nxt = dp[q];
+    }
+  sx[tid] = dp[0];
+  __syncthreads();
+  double above = 0.0;  // x(k0 + kn)
+  for (int cc = C - 1; cc > c; --cc) above = sx[cc * 32 + tx] + T(kH_H, cc * kM) * above;
+  if (ghost) {
+    const size_t g = (size_t)e;
+    for (int q = 0; q < kn; ++q) {
+      const size_t o = (size_t)(k0 + q) * pl + g;
+      w[o] = rho[o] = pi[o] = 0.0;
+    }
+    if (k0 + kn == nz) w[(size_t)nz * pl + g] = 0.0;
+  }
+  if (!active) return;
+#pragma unroll
+  for (int q = 0; q < kM; ++q)
+    if (q < kn) dp[q] += T(kH_H, k0 + q) * above;
+  double wb = wv[0];
+  if (c > 0) wb -= T(kH_ai, k0) * (dp[0] - (below - T(kH_lc, k0 - 1) * dp[0]));
+  double fn = T(kH_rf, k0) * wb;
+#pragma unroll
+  for (int q = 0; q < kM; ++q)
+    if (q < kn) {
+      const int k = k0 + q;
+      const size_t o = (size_t)k * pl + col;
+      const double xf = (q + 1 < kn) ? dp[q + 1 < kM ? q + 1 : q] : above;
+      const double wn = wv[q + 1] - T(kH_ai, k + 1) * (xf - dp[q]);
+      const double fn1 = T(kH_rf, k + 1) * wn;
+      rho[o] = rs[q] + (dtau * b * T(kH_idz, k)) * (fn - fn1);
+      pi[o] = dp[q] + (pert ? T(kH_p0, k) : 0.0);
+      w[o] = wb;
+      wb = wn;
+      fn = fn1;
+    }
+  if (k0 + kn == nz) w[(size_t)nz * pl + col] = wb;
+}
+
+// Its horizontal momentum: u += dtau (-cp theta0 d(pi)/dx) on the inner faces
+// (the clamped ones see no difference); pi0 is the same on both sides of a
+// face, so pi and pi' have one gradient
+__global__ void k_uv_chunk(Dims d, const double* __restrict__ tab, const double* __restrict__ pi,
+                           double* __restrict__ u, double* __restrict__ v) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int j = blockIdx.y * blockDim.y + threadIdx.y;
+  const int k = blockIdx.z;
+  if (i >= d.nx || j >= d.ny) return;
+  const size_t c = IDX(i, j, k);
+  const double p = pi[c];
+  if (i > 0) u[c] -= __ldg(tab + kH_cu * (d.nz + 1) + k) * (p - pi[c - 1]);
+  if (j > 0) v[c] -= __ldg(tab + kH_cv * (d.nz + 1) + k) * (p - pi[c - d.P]);
+}
+#endif
+
 __global__ void k_uv_backward(Dims d, Metric m, Flags fl, CS s, double* __restrict__ u, double* __restrict__ v,
                               double dtau) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -897,6 +1031,129 @@ __global__ void k_hevi_ad_column(Dims d, Metric m, Flags fl, double* __restrict_
   }
 }
 
+#ifndef VGB_FP64_EXACT
+// Adjoint of k_chevi_chunk + k_uv_chunk, the same split: the gradient of u and
+// v transposed is gathered here (bar_pi at a cell from its four faces), then
+// the column part of k_hevi_ad_column with the transposed factors of
+// Metric::hevi, in place on bar_w and bar_pi; bar of Dh goes to k_dh_ad_chunk.
+// bar_rho passes through. The ghost points' bars do not reach the input.
+template <int kBlocks>
+__global__ void __launch_bounds__(32 * kHevi64Chunks / kBlocks, kBlocks)
+    k_hevi_ad_chunk(Dims d, const double* __restrict__ tab, double b, double dtau, const double* __restrict__ bu,
+                    const double* __restrict__ bv, double* __restrict__ bw, double* __restrict__ brho,
+                    double* __restrict__ bpi, double* __restrict__ bdh) {
+  constexpr int kM = kHevi64M;
+  extern __shared__ double sh64[];
+  const int nz = d.nz, C = blockDim.y, R = nz + 1;
+  double* sf = sh64;
+  double* sx = sh64 + 32 * C;
+  const int tx = threadIdx.x, c = threadIdx.y, tid = c * 32 + tx;
+  const int e = blockIdx.x * 32 + tx;
+  const int j = e / d.P, i = e - j * d.P;
+  const bool active = i < d.nx && j < d.ny;
+  const bool ghost = !active && i <= d.nx && j <= d.ny;
+  const int k0 = c * kM, kn = imin(kM, nz - k0);
+  const size_t pl = d.plane, col = active ? (size_t)e : 0;
+  auto T = [&](int row, int k) { return __ldg(tab + row * R + k); };
+  const double ob = 1.0 - b, db = dtau * b;
+  double br[kM + 2], bn[kM + 1], y[kM];  // bar_rho(k0-1+q); bar of w_new, faces k0..k0+kn; bar_x, then y
+#pragma unroll
+  for (int q = 0; q < kM + 2; ++q) {
+    const int k = k0 - 1 + q;
+    br[q] = (active && k >= 0 && k < nz && q <= kn + 1) ? brho[(size_t)k * pl + col] : 0.0;
+  }
+#pragma unroll
+  for (int q = 0; q < kM + 1; ++q) {
+    const int k = k0 + q;
+    bn[q] = 0.0;
+    if (active && q <= kn)
+      bn[q] = bw[(size_t)k * pl + col] + db * (T(kH_ra, k) * br[q + 1] - T(kH_rb, k) * br[q]);
+  }
+  double prev = 0.0;
+#pragma unroll
+  for (int q = 0; q < kM; ++q) {
+    y[q] = 0.0;
+    if (q < kn && active) {
+      const int k = k0 + q;
+      const size_t o = (size_t)k * pl + col;
+      const double gu = (i + 1 < d.nx ? bu[o + 1] : 0.0) - (i > 0 ? bu[o] : 0.0);
+      const double gv = (j + 1 < d.ny ? bv[o + d.P] : 0.0) - (j > 0 ? bv[o] : 0.0);
+      const double x = bpi[o] + T(kH_cu, k) * gu + T(kH_cv, k) * gv + (T(kH_ai, k + 1) * bn[q + 1] - T(kH_ai, k) * bn[q]);
+      prev = x * T(kH_li, k) - T(kH_mT, k) * prev;
+      y[q] = prev;
+    }
+  }
+  sf[tid] = prev;
+  __syncthreads();
+  double below = 0.0;
+  for (int cc = 0; cc < c; ++cc) below = sf[cc * 32 + tx] + T(kH_GT, (cc + 1) * kM - 1) * below;
+  double nxt = 0.0;
+#pragma unroll
+  for (int q = kM - 1; q >= 0; --q)
+    if (q < kn) {
+      y[q] += T(kH_GT, k0 + q) * below;
+      y[q] -= T(kH_lcT, k0 + q) * nxt;
+      nxt = y[q];
+    }
+  sx[tid] = y[0];
+  __syncthreads();
+  double above = 0.0;  // y(k0 + kn)
+  for (int cc = C - 1; cc > c; --cc) above = sx[cc * 32 + tx] + T(kH_HT, cc * kM) * above;
+  if (ghost) {
+    const size_t g = (size_t)e;
+    for (int q = 0; q < kn; ++q) {
+      const size_t o = (size_t)(k0 + q) * pl + g;
+      bw[o] = brho[o] = bpi[o] = 0.0;
+    }
+    if (k0 + kn == nz) bw[(size_t)nz * pl + g] = 0.0;
+  }
+  if (!active) return;
+#pragma unroll
+  for (int q = 0; q < kM; ++q)
+    if (q < kn) y[q] += T(kH_HT, k0 + q) * above;
+  // bar of pstar's kappa factor at level k, times dtau kappa
+  const double ybelow = c > 0 ? below - T(kH_lcT, k0 - 1) * y[0] : 0.0;
+  double km = c > 0 ? T(kH_dk, k0 - 1) * ybelow : 0.0;
+  double kc = T(kH_dk, k0) * y[0];
+  double brm = br[0], brc = br[1];
+  // face k0: bar of w~ (from w_new and dv_t), then bar of w (from dv_old)
+  double wtb = bn[0] + b * (T(kH_ra, k0) * kc - T(kH_rb, k0) * km);
+#pragma unroll
+  for (int q = 0; q < kM; ++q)
+    if (q < kn) {
+      const int k = k0 + q;
+      const size_t o = (size_t)k * pl + col;
+      const double dc = dtau * brc + kc, dm = dtau * brm + km;  // bar of Dh
+      bdh[o] = dc;
+      bw[o] = wtb + ob * (T(kH_ra, k) * dc - T(kH_rb, k) * dm);
+      // the upper face
+      const bool in = k + 1 < nz;
+      const double kt = (q + 1 < kn) ? T(kH_dk, k + 1) * y[q + 1 < kM ? q + 1 : q] : (in ? T(kH_dk, k + 1) * above : 0.0);
+      const double wt1 = bn[q + 1] + b * (T(kH_ra, k + 1) * kt - T(kH_rb, k + 1) * kc);
+      bpi[o] = y[q] + T(kH_ae, k + 1) * wt1 - T(kH_ae, k) * wtb;
+      if (k + 1 == nz) bw[o + pl] = wt1 - ob * T(kH_rb, nz) * dc;
+      wtb = wt1;
+      km = kc;
+      kc = kt;
+      brm = brc;
+      brc = br[q + 2];
+    }
+}
+
+// Dh = -rho0 (du/dx + dv/dy) transposed on the uniform grid
+__global__ void k_dh_ad_chunk(Dims d, const double* __restrict__ tab, double inv_dx, double inv_dy,
+                              const double* __restrict__ bdh, double* __restrict__ bu, double* __restrict__ bv) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int j = blockIdx.y * blockDim.y + threadIdx.y;
+  const int k = blockIdx.z;
+  if (i > d.nx || j > d.ny) return;
+  const size_t c = IDX(i, j, k);
+  const double r0 = __ldg(tab + kH_r0 * (d.nz + 1) + k);
+  if (j < d.ny) bu[c] += (r0 * inv_dx) * ((i < d.nx ? bdh[c] : 0.0) - (i > 0 ? bdh[c - 1] : 0.0));
+  if (i < d.nx) bv[c] += (r0 * inv_dy) * ((j < d.ny ? bdh[c] : 0.0) - (j > 0 ? bdh[c - d.P] : 0.0));
+}
+#endif
+
 // The forward substep copies the column solve's whole w, rho, pi outputs back,
 // whose ghost column i = nx and ghost row j = ny it never writes (zeros): those
 // outputs do not depend on the input, so their bars do not reach it
@@ -1003,6 +1260,21 @@ void FP64_FN(fp64_fb_substep_ad)(const Dims& d, const Metric& m, double* const* 
 
 void FP64_FN(fp64_hevi_substep_ad)(const Dims& d, const Metric& m, const Flags& fl, double* const* bar, double* bdh,
                                    double* scratch, double dtau, unsigned* err, cudaStream_t stream) {
+#ifndef VGB_FP64_EXACT
+  if (m.hevi) {
+    const int C = (d.nz + kHevi64M - 1) / kHevi64M, g = (int)((d.plane + 31) / 32);
+    const size_t sm = 64 * (size_t)C * sizeof(double);
+    if (C <= kHevi64Chunks / 2)
+      k_hevi_ad_chunk<2><<<g, dim3(32, C), sm, stream>>>(d, m.hevi, fl.hevi_beta, dtau, bar[U], bar[V], bar[W],
+                                                         bar[RHO], bar[PI], bdh);
+    else
+      k_hevi_ad_chunk<1><<<g, dim3(32, C), sm, stream>>>(d, m.hevi, fl.hevi_beta, dtau, bar[U], bar[V], bar[W],
+                                                         bar[RHO], bar[PI], bdh);
+    k_dh_ad_chunk<<<grid3(d, d.nx + 1, d.ny + 1, d.nz, kBlk), kBlk, 0, stream>>>(d, m.hevi, m.inv_dx, m.inv_dy, bdh,
+                                                                                bar[U], bar[V]);
+    return;
+  }
+#endif
   k_fbad_pi<<<grid3(d, d.nx, d.ny, d.nz, kBlk), kBlk, 0, stream>>>(d, m, bar[U], bar[V], bar[W], bar[PI], dtau, 0);
   k_hevi_ad_column<<<dim3((d.nx + 31) / 32, (d.ny + 3) / 4), dim3(32, 4), 0, stream>>>(d, m, fl, bar[W], bar[RHO],
                                                                                       bar[PI], bdh, scratch, dtau,
@@ -1032,6 +1304,20 @@ void FP64_FN(fp64_ref_hevi_substep)(const Dims& d, const Metric& m, double* cons
 
 void FP64_FN(fp64_cons_hevi_substep)(const Dims& d, const Metric& m, const Flags& fl, double* const* st, double* const* tmp,
                             double* scratch, double dtau, unsigned* err, cudaStream_t stream) {
+#ifndef VGB_FP64_EXACT
+  if (m.hevi) {
+    const int C = (d.nz + kHevi64M - 1) / kHevi64M, g = (int)((d.plane + 31) / 32);
+    const size_t sm = 64 * (size_t)C * sizeof(double);
+    if (C <= kHevi64Chunks / 2)
+      k_chevi_chunk<2><<<g, dim3(32, C), sm, stream>>>(d, m.hevi, m.inv_dx, m.inv_dy, fl.hevi_beta, dtau, fl.pgf_pert,
+                                                       st[U], st[V], st[W], st[RHO], st[PI]);
+    else
+      k_chevi_chunk<1><<<g, dim3(32, C), sm, stream>>>(d, m.hevi, m.inv_dx, m.inv_dy, fl.hevi_beta, dtau, fl.pgf_pert,
+                                                       st[U], st[V], st[W], st[RHO], st[PI]);
+    k_uv_chunk<<<grid3(d, d.nx, d.ny, d.nz, kBlk), kBlk, 0, stream>>>(d, m.hevi, st[PI], st[U], st[V]);
+    return;
+  }
+#endif
   // column solve reads the old state, writes w/rho/pi into tmp, copied back
   const CS s = to_cs(st);
   const dim3 b2(32, 4);

@@ -54,7 +54,39 @@ struct Metric {
   const double* rho0;
   double f0, beta;       // Coriolis (coriolis.cpp:25-41)
   double inv_dx, inv_dy; // 1/dx, 1/dy (the fast FP64 build multiplies by them)
+  // flat grids with a horizontally uniform reference state: the consistent
+  // HEVI substep's per-level coefficients for one dtau (Hevi64Row rows of
+  // nz + 1 doubles), else null
+  const double* hevi = nullptr;
 };
+
+// Rows of Metric::hevi. Face rows (k = 0..nz) are zero on the ground and the
+// lid where the substep takes no gradient there.
+enum Hevi64Row {
+  kH_ae,   // face: dtau (1-b) cp theta0_f / dz_f
+  kH_ai,   // face: dtau b cp theta0_f / dz_f
+  kH_rf,   // face: rho0_f
+  kH_idz,  // 1/dz
+  kH_dk,   // dtau kappa
+  kH_r0,   // rho0
+  kH_p0,   // pi0
+  kH_li,   // 1/pivot of the column matrix
+  kH_m,    // a/pivot
+  kH_lc,   // c/pivot (0 on the last level)
+  kH_G,    // prod_{l = chunk start..k} (-m)
+  kH_H,    // prod_{l = k..chunk end} (-lc)
+  kH_mT,   // the same four of the transposed matrix (same pivots)
+  kH_lcT,
+  kH_GT,
+  kH_HT,
+  kH_ra,   // face: rho0_f / dz(k), 0 on the lid
+  kH_rb,   // face: rho0_f / dz(k-1), 0 on the ground
+  kH_cu,   // dtau cp theta0 / dx
+  kH_cv,   // dtau cp theta0 / dy
+  kH_rows
+};
+constexpr int kHevi64M = 8;         // levels per warp of the FP64 level-split kernels
+constexpr int kHevi64Chunks = 20;   // warps per block at most: nz <= 160
 
 // Composition switches (same meaning as the setup struct in vibe_gb300.h).
 struct Flags {
