@@ -124,6 +124,75 @@ def test_tendency_dot_product(vg, mixed, tol, weno):
         assert abs(lhs - rhs) <= tol * max(abs(lhs), abs(rhs)), (lhs, rhs)
 
 
+def test_tendency_tl_below_the_upwind_switch(vg):
+    """Winds below 1e-3 m/s, where the Lax-Friedrichs weight is the constant
+    and both WENO5 sides enter a face: the bounds of the test above (the
+    perturbed winds stay below the switch for every e)."""
+    s, m = case(vg, vg.FP64, u_background=0.0)
+    with m:
+        x0 = m.state()
+        rng = np.random.default_rng(12)
+        dx = perturb(vg, s, m, 13)
+        for sp in (0, 1, 2):
+            v = vg.interior(s, sp, x0[sp])
+            v[...] = rng.uniform(-8e-4, 8e-4, v.shape)
+            v = vg.interior(s, sp, dx[sp])
+            v[...] = rng.uniform(-1e-2, 1e-2, v.shape)
+        m.set_state(x0)
+        tl = m.tendency_tl(dx)
+
+        def tend(x):
+            m.set_state(x)
+            return m.slow_tendency()
+
+        curves = u_curve(tend, x0, dx, tl, lambda sp, a: tendency_box(vg, s, sp, a), (4,))
+        assert min(curves[4]) < 1e-4, curves[4]
+
+
+@pytest.mark.parametrize("mixed,tol", [(False, 1e-10), (True, 1e-5)])
+@pytest.mark.parametrize("form", ["slow_winds", "moist", "terrain_total", "one_row"])
+def test_tendency_dot_product_forms(vg, mixed, tol, form):
+    """<TL dx, y> = <dx, AD y> of the slow tendency on the forms the written-out
+    adjoints branch on: winds below the upwind switch, moisture species with
+    zeros and the positivity clip, terrain with the total pressure gradient
+    and unsplit fast terms (FP64 only) under the beta-plane, a 1-cell wide
+    grid. The bounds of the dot product above."""
+    kw = dict(slow_winds=dict(u_background=0.0), moist=dict(moist=1, qv_surface=0.01),
+              terrain_total=dict(terrain_kind=1, hill_h=400.0, hill_a=9000.0, hill_xc=30000.0, hill_yc=24000.0,
+                                 pgf_perturbation=0, split_fast=0, coriolis=2, w_rigid=0),
+              one_row=dict(nx=1, ny=6, nz=4))[form]
+    if mixed and form == "terrain_total":
+        pytest.skip("the mixed path needs flat terrain and the perturbation gradient")
+    if form != "terrain_total":
+        s, m = case(vg, vg.MIXED if mixed else vg.FP64, **kw)
+    else:  # without the steps of case(): this composition diverges within a few
+        s = vg.Setup.defaults(nx=20, ny=16, nz=12, dx=3000.0, dy=3000.0, z_top=12000.0, zeta_first=1.0,
+                              zeta_stretch=1.05, ref_kind=1, bv_n=0.01, u_background=10.0, shear_u=0.001, advection=5,
+                              weno_scalars=1, weno_advective=1, acoustic_mode=0, qv_surface=0.0, **kw)
+        m = vg.Model(s, vg.FP64)
+    with m:
+        rng = np.random.default_rng(14)
+        st = m.state()
+        if form == "slow_winds":
+            for sp in (0, 1, 2):
+                v = vg.interior(s, sp, st[sp])
+                v[...] = rng.uniform(-8e-4, 8e-4, v.shape)
+        if form == "moist":
+            for sp in range(6, 12):  # positive, zero and slightly negative cells
+                v = vg.interior(s, sp, st[sp])
+                v[...] = np.maximum(rng.normal(0.0, 1e-3, v.shape), -1e-5) * (rng.random(v.shape) < 0.7)
+        m.set_state(st)
+        dx, y = perturb(vg, s, m, 15), perturb(vg, s, m, 16)
+        for q in (dx, y):
+            for sp in range(6, 12 if form == "moist" else 6):
+                v = vg.interior(s, sp, q[sp])
+                v[...] = 1e-3 * rng.standard_normal(v.shape)
+        lhs = vdot(m.tendency_tl(dx), y)
+        rhs = vdot(dx, m.tendency_ad(y))
+        norm = max(abs(lhs), abs(rhs))
+        assert abs(lhs - rhs) <= tol * norm, (lhs, rhs)
+
+
 def test_step_tl_matches_central_differences(vg):
     """(M(x + e dx) - M(x - e dx)) / 2e -> TL(dx) for one model step (FP64);
     the model's state is left as it was."""

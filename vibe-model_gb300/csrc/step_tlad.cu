@@ -16,11 +16,13 @@
 //     and dR (the tangent-linear). The WENO5 weights and the Lax-Friedrichs
 //     switch at |u| = 1e-3 are differentiated exactly; where the positivity
 //     clip of the moisture species is active the derivative is zero.
-//   * The adjoint evaluates the same point function once per load, with a
-//     unit derivative on that load alone (forward mode, one column of the
-//     point's Jacobian row per pass), and adds (dR/dload) * bar_R to the bar
-//     of the loaded point with atomicAdd. Loads that alias through index
-//     clamps add up, so the scatter is the exact transpose of the tangent.
+//   * The adjoint adds (dR/dload) * bar_R to the bar of each loaded point with
+//     atomicAdd, the derivatives written out beside the point function they
+//     belong to (ad_u, ad_v, ad_w, ad_rho; wgrad_ for a WENO5 face, in reverse
+//     mode). Loads that alias through index clamps add up, so the scatter is
+//     the exact transpose of the tangent. The rarely used point functions
+//     (divergence damping, central scalars) are evaluated once per load with a
+//     unit derivative on that load alone (ad_scatter).
 //   * A WENO5 face flux is shared by the two cells beside the face, so its
 //     adjoint runs per face: bar_F is gathered from the two cells' bars (zero
 //     where the clip is active) and then scattered to the face's six loads.
@@ -308,36 +310,114 @@ __device__ __forceinline__ Jet<R> pt_scalar_nc(const Dims& d, const Metric& m, c
 }
 
 // WENO5 left-biased reconstruction (Advection::weno5_reconstruct,
-// advection.cpp:62-98; the right-biased one is this of the reversed stencil)
+// advection.cpp:62-98; the right-biased one is this of the reversed stencil).
+// The weights d_k / s_k^2 are scaled by (s0 s1 s2)^2: no 1/s^2 of s ~ 1e-6.
 template <class R>
-__device__ __forceinline__ Jet<R> weno_left_(Jet<R> qm2, Jet<R> qm1, Jet<R> q0, Jet<R> q1, Jet<R> q2) {
-  using T = Jet<R>;
-  const double s6 = 1.0 / 6.0;
-  const T v0 = (2.0 * qm2 - 7.0 * qm1 + 11.0 * q0) * s6;
-  const T v1 = (-qm1 + 5.0 * q0 + 2.0 * q1) * s6;
-  const T v2 = (2.0 * q0 + 5.0 * q1 - q2) * s6;
-  const T e0 = qm2 - 2.0 * qm1 + q0, f0 = qm2 - 4.0 * qm1 + 3.0 * q0;
-  const T e1 = qm1 - 2.0 * q0 + q1, f1 = qm1 - q1;
-  const T e2 = q0 - 2.0 * q1 + q2, f2 = 3.0 * q0 - 4.0 * q1 + q2;
-  const T s0 = (13.0 / 12.0) * (e0 * e0) + 0.25 * (f0 * f0) + 1e-6;
-  const T s1 = (13.0 / 12.0) * (e1 * e1) + 0.25 * (f1 * f1) + 1e-6;
-  const T s2 = (13.0 / 12.0) * (e2 * e2) + 0.25 * (f2 * f2) + 1e-6;
-  // the weights d_k / s_k^2 scaled by (s0 s1 s2)^2: no 1/s^2 of s ~ 1e-6, so
-  // the derivatives of the normalisation do not cancel large numbers
-  const T p12 = s1 * s2, p02 = s0 * s2, p01 = s0 * s1;
-  const T a0 = 0.1 * (p12 * p12), a1 = 0.6 * (p02 * p02), a2 = 0.3 * (p01 * p01);
+__device__ __forceinline__ R weno_left_(const R (&z)[5]) {
+  const R s6 = (R)(1.0 / 6.0), c13 = (R)(13.0 / 12.0);
+  const R v0 = ((R)2 * z[0] - (R)7 * z[1] + (R)11 * z[2]) * s6;
+  const R v1 = (-z[1] + (R)5 * z[2] + (R)2 * z[3]) * s6;
+  const R v2 = ((R)2 * z[2] + (R)5 * z[3] - z[4]) * s6;
+  const R e0 = z[0] - (R)2 * z[1] + z[2], f0 = z[0] - (R)4 * z[1] + (R)3 * z[2];
+  const R e1 = z[1] - (R)2 * z[2] + z[3], f1 = z[1] - z[3];
+  const R e2 = z[2] - (R)2 * z[3] + z[4], f2 = (R)3 * z[2] - (R)4 * z[3] + z[4];
+  const R s0 = c13 * (e0 * e0) + (R)0.25 * (f0 * f0) + (R)1e-6;
+  const R s1 = c13 * (e1 * e1) + (R)0.25 * (f1 * f1) + (R)1e-6;
+  const R s2 = c13 * (e2 * e2) + (R)0.25 * (f2 * f2) + (R)1e-6;
+  const R p12 = s1 * s2, p02 = s0 * s2, p01 = s0 * s1;
+  const R a0 = (R)0.1 * (p12 * p12), a1 = (R)0.6 * (p02 * p02), a2 = (R)0.3 * (p01 * p01);
   return (a0 * v0 + a1 * v1 + a2 * v2) / (a0 + a1 + a2);
 }
 // Lax-Friedrichs face flux 0.5 (u (qL + qR) - max(|u|, 1e-3) (qR - qL)),
-// advection.cpp:160-170
+// advection.cpp:160-170: u times the upwind side alone for |u| >= 1e-3
 template <class R>
-__device__ __forceinline__ Jet<R> weno_flux_(Jet<R> qm2, Jet<R> qm1, Jet<R> q0, Jet<R> q1, Jet<R> q2, Jet<R> vel) {
-  const Jet<R> ql = weno_left_<R>(qm2, qm1, q0, q1, q2);
-  const Jet<R> qr = weno_left_<R>(q2, q1, q0, qm1, qm2);
-  Jet<R> alpha{(R)1e-3, (R)0};
-  if (vel.v >= (R)1e-3) alpha = vel;
-  else if (vel.v <= (R)-1e-3) alpha = -vel;
-  return 0.5 * (vel * (ql + qr) - alpha * (qr - ql));
+__device__ __forceinline__ R wflux_value_(const R (&z)[5], R vel) {
+  const bool up = vel >= (R)0;
+  R y[5], yo[5];
+#pragma unroll
+  for (int m = 0; m < 5; ++m) {
+    y[m] = up ? z[m] : z[4 - m];
+    yo[m] = up ? z[4 - m] : z[m];
+  }
+  const R q = weno_left_<R>(y);
+  if (fabs(vel) >= (R)1e-3) return vel * q;
+  const R r = weno_left_<R>(yo);
+  const R ql = up ? q : r, qr = up ? r : q;
+  return (R)0.5 * (vel * (ql + qr) - (R)1e-3 * (qr - ql));
+}
+// Value and gradient of the upwind reconstruction weno_left_:
+// q and dq/dz of its five stencil values. With w_k the normalised
+// weights, q = sum w_k v_k and d(w_k) = w_k (dln a_k - sum ..) give
+//   dq = sum_k w_k dv_k - 2 sum_k w_k (v_k - q) ds_k / s_k,
+// one reverse pass instead of one forward pass per stencil value.
+template <class R>
+__device__ __forceinline__ R wgrad_left_(const R (&z)[5], R (&g)[5]) {
+  const R s6 = (R)(1.0 / 6.0), c13 = (R)(13.0 / 12.0);
+  const R v0 = ((R)2 * z[0] - (R)7 * z[1] + (R)11 * z[2]) * s6;
+  const R v1 = (-z[1] + (R)5 * z[2] + (R)2 * z[3]) * s6;
+  const R v2 = ((R)2 * z[2] + (R)5 * z[3] - z[4]) * s6;
+  const R e0 = z[0] - (R)2 * z[1] + z[2], f0 = z[0] - (R)4 * z[1] + (R)3 * z[2];
+  const R e1 = z[1] - (R)2 * z[2] + z[3], f1 = z[1] - z[3];
+  const R e2 = z[2] - (R)2 * z[3] + z[4], f2 = (R)3 * z[2] - (R)4 * z[3] + z[4];
+  const R s0 = c13 * (e0 * e0) + (R)0.25 * (f0 * f0) + (R)1e-6;
+  const R s1 = c13 * (e1 * e1) + (R)0.25 * (f1 * f1) + (R)1e-6;
+  const R s2 = c13 * (e2 * e2) + (R)0.25 * (f2 * f2) + (R)1e-6;
+  const R p12 = s1 * s2, p02 = s0 * s2, p01 = s0 * s1;
+  const R a0 = (R)0.1 * (p12 * p12), a1 = (R)0.6 * (p02 * p02), a2 = (R)0.3 * (p01 * p01);
+  R w0, w1, w2, h0, h1, h2;  // weights and weights / s
+  if (sizeof(R) == 8) {  // one division, by (a0 + a1 + a2) s0 s1 s2 (below 1e-300 only for s far under the 1e-6 floor)
+    const R s012 = s0 * p12, r = (R)1 / ((a0 + a1 + a2) * s012);
+    h0 = a0 * p12 * r, h1 = a1 * p02 * r, h2 = a2 * p01 * r;
+    w0 = h0 * s0, w1 = h1 * s1, w2 = h2 * s2;
+  } else {
+    const R r = (R)1 / (a0 + a1 + a2);
+    w0 = a0 * r, w1 = a1 * r, w2 = a2 * r;
+    h0 = w0 / s0, h1 = w1 / s1, h2 = w2 / s2;
+  }
+  const R q = w0 * v0 + w1 * v1 + w2 * v2;
+  // d s_k = 13/6 e_k de_k + 1/2 f_k df_k, times -2 w_k (v_k - q) / s_k
+  h0 *= q - v0, h1 *= q - v1, h2 *= q - v2;
+  const R x0 = (R)(13.0 / 3.0) * h0 * e0, y0 = h0 * f0;
+  const R x1 = (R)(13.0 / 3.0) * h1 * e1, y1 = h1 * f1;
+  const R x2 = (R)(13.0 / 3.0) * h2 * e2, y2 = h2 * f2;
+  w0 *= s6, w1 *= s6, w2 *= s6;
+  g[0] = x0 + y0 + (R)2 * w0;
+  g[1] = -(R)2 * x0 - (R)4 * y0 - (R)7 * w0 + x1 + y1 - w1;
+  g[2] = x0 + (R)3 * y0 + (R)11 * w0 - (R)2 * x1 + (R)5 * w1 + x2 + (R)3 * y2 + (R)2 * w2;
+  g[3] = x1 - y1 + (R)2 * w1 - (R)2 * x2 - (R)4 * y2 + (R)5 * w2;
+  g[4] = x2 + y2 - w2;
+  return q;
+}
+// wflux_value_ and its derivatives: to the five stencil values and to
+// the wind. For |vel| >= 1e-3 the flux is vel times the upwind reconstruction
+// alone; below, the Lax-Friedrichs weight is the constant 1e-3.
+template <class R>
+__device__ __forceinline__ R wgrad_(const R (&z)[5], R vel, R (&g)[5], R& gvel) {
+  const bool up = vel >= (R)0;
+  R y[5], h[5];
+#pragma unroll
+  for (int m = 0; m < 5; ++m) y[m] = up ? z[m] : z[4 - m];
+  const R q = wgrad_left_<R>(y, h);
+  if (fabs(vel) >= (R)1e-3) {
+#pragma unroll
+    for (int m = 0; m < 5; ++m) g[m] = vel * (up ? h[m] : h[4 - m]);
+    gvel = q;
+    return vel * q;
+  }
+  R yo[5], ho[5];
+#pragma unroll
+  for (int m = 0; m < 5; ++m) yo[m] = y[4 - m];
+  const R qo = wgrad_left_<R>(yo, ho);  // the reversed side; h and ho are in the order of y and yo
+  const R cu = (R)0.5 * (fabs(vel) + (R)1e-3), co = (R)0.5 * (fabs(vel) - (R)1e-3);
+  const R sg = up ? (R)1 : (R)-1;
+#pragma unroll
+  for (int m = 0; m < 5; ++m) {
+    const R a = cu * h[m] + co * ho[4 - m];  // in the order of y
+    if (up) g[m] = a;
+    else g[4 - m] = -a;
+  }
+  gvel = (R)0.5 * (q + qo);
+  return sg * (cu * q + co * qo);
 }
 // The face flux of direction dir (0 x, 1 y, 2 z) at face index (i, j, k)
 // (k_weno_faces' stencil CL(f-3..f+1) and the normal wind at the face), as
@@ -346,20 +426,12 @@ __device__ __forceinline__ Jet<R> weno_flux_(Jet<R> qm2, Jet<R> qm1, Jet<R> q0, 
 // derivative) changes only the c u part. The small shifted values keep FP32
 // accurate; a cell combines G with c and its own q without cancelling the
 // large c u terms of its faces (pt_wcell).
-template <class R, class Ld>
-__device__ __forceinline__ Jet<R> pt_wface(const Dims& d, Ld& L, int q, int dir, int i, int j, int k, double c) {
-  Jet<R> z[5];
-  int di = 0, dj = 0, dk = 0;
-  if (dir == 0) di = 1;
-  else if (dir == 1) dj = 1;
-  else dk = 1;
+__device__ __forceinline__ void wface_points(const Dims& d, int dir, int i, int j, int k, size_t (&o)[5]) {
+  const int di = dir == 0, dj = dir == 1, dk = dir == 2;
 #pragma unroll
-  for (int m = 0; m < 5; ++m) {
-    const int a = iclamp(i + (m - 3) * di, 0, d.nx - 1), b = iclamp(j + (m - 3) * dj, 0, d.ny - 1);
-    z[m] = L(q, d.idx(a, b, iclamp(k + (m - 3) * dk, 0, d.nz - 1)), c);
-  }
-  const Jet<R> vel = LD(dir == 0 ? U : (dir == 1 ? V : W), i, j, k);
-  return weno_flux_<R>(z[0], z[1], z[2], z[3], z[4], vel);
+  for (int m = 0; m < 5; ++m)
+    o[m] = d.idx(iclamp(i + (m - 3) * di, 0, d.nx - 1), iclamp(j + (m - 3) * dj, 0, d.ny - 1),
+                 iclamp(k + (m - 3) * dk, 0, d.nz - 1));
 }
 // c of the face at index (i, j, k): q at the stencil's centre (the cell at
 // the face's index, clamped)
@@ -465,16 +537,23 @@ __global__ void k_tl_wface(Dims d, const __grid_constant__ F12 b, const __grid_c
   const double sh = wface_shift(d, b.f[q], i, j, k);
   for (int dir = 0; dir < 3; ++dir) {
     if (!face_exists(d, dir, i, j, k)) continue;
-    Jet<R> f;
+    const int vq = dir == 0 ? U : (dir == 1 ? V : W);
+    size_t o[5];
+    wface_points(d, dir, i, j, k, o);
+    R z[5];
+#pragma unroll
+    for (int m = 0; m < 5; ++m) z[m] = (R)(b.f[q][o[m]] - sh);
+    const R vel = (R)b.f[vq][c];
     if (with_t) {
-      TlLoad<R> L{&b, &p};
-      f = pt_wface<R>(d, L, q, dir, i, j, k, sh);
-      F.t[dir][c] = (double)f.d;
+      R g[5], gvel;
+      F.v[dir][c] = (double)wgrad_<R>(z, vel, g, gvel);
+      R t = gvel * (R)p.f[vq][c];
+#pragma unroll
+      for (int m = 0; m < 5; ++m) t += g[m] * (R)p.f[q][o[m]];
+      F.t[dir][c] = (double)t;
     } else {
-      ValLoad<R> L{&b};
-      f = pt_wface<R>(d, L, q, dir, i, j, k, sh);
+      F.v[dir][c] = (double)wflux_value_<R>(z, vel);
     }
-    F.v[dir][c] = (double)f.v;
     F.c[dir][c] = sh;
   }
 }
@@ -506,6 +585,165 @@ __device__ __forceinline__ void ad_scatter(const F12& b, const B12& bar, double 
   }
 }
 
+// The written-out adjoints: each adds lam * (derivative of the point function
+// named) to the bar of every point that function loads, the derivatives taken
+// in R as the tangent takes them.
+struct BarAdd {
+  const B12& bi;
+  double lam;
+  __device__ __forceinline__ void operator()(int q, size_t c, double coef) const { atomicAdd(&bi.f[q][c], coef * lam); }
+};
+#define BV(q, c) ((R)b.f[q][c])
+#define BP(c) ((R)(b.f[PI][c] - (fl.pgf_pert ? m.pi0[c] : 0.0)))
+#define BT(c) ((R)(b.f[THETA][c] - (fl.split_fast ? m.th0[c] : 0.0)))
+
+template <class R>
+__device__ __forceinline__ void ad_u(const Dims& d, const Metric& m, const Flags& fl, const F12& b, const B12& bi,
+                                     double lam, int i, int j, int k) {
+  const int nx = d.nx, ny = d.ny, nz = d.nz;
+  const int ip = imin(i, nx - 1), im = imax(i - 1, 0), jm = imax(j - 1, 0), kp = imin(k + 1, nz - 1);
+  const R idx = (R)m.inv_dx, hy = (R)(0.5 * m.inv_dy);
+  const R hz = (R)(1.0 / (2.0 * (dzeta_(m, d, imin(k, nz - 1)) * scale_(m, d, ip, j))));
+  const size_t cm = d.idx(im, j, k), cp = d.idx(ip, j, k);
+  const size_t cn = d.idx(ip, imin(j + 1, ny - 1), k), cs = d.idx(ip, jm, k);
+  const size_t ct = d.idx(ip, j, kp), cb = d.idx(ip, j, imax(k - 1, 0));
+  const size_t v0 = d.idx(im, jm, k), v1 = d.idx(ip, jm, k);
+  const R um = BV(U, cm), up = BV(U, cp);
+  const R uc = (R)0.5 * (um + up), ux = (up - um) * idx;
+  const R uy = (BV(U, cn) - BV(U, cs)) * hy, uz = (BV(U, ct) - BV(U, cb)) * hz;
+  const R vc = (R)0.25 * (BV(V, v0) + BV(V, v1) + BV(V, cm) + BV(V, cp));
+  const R wc = (R)0.5 * (BV(W, cp) + BV(W, ct));
+  const R th = (R)0.5 * (BT(cm) + BT(cp)), dp = BP(cp) - BP(cm);
+  const R g = (R)kCp * idx;
+  const BarAdd add{bi, lam};
+  add(U, cp, (double)-((R)0.5 * ux + uc * idx));
+  add(U, cm, (double)(uc * idx - (R)0.5 * ux));
+  add(U, cn, (double)-(vc * hy));
+  add(U, cs, (double)(vc * hy));
+  add(U, ct, (double)-(wc * hz));
+  add(U, cb, (double)(wc * hz));
+  const double cv = (double)((R)0.25 * ((fl.coriolis ? (R)corf_(m, fl, d, j) : (R)0) - uy));
+  add(V, v0, cv);
+  add(V, v1, cv);
+  add(V, cm, cv);
+  add(V, cp, cv);
+  const double cw = (double)-((R)0.5 * uz);
+  add(W, cp, cw);
+  add(W, ct, cw);
+  const double ch = (double)-((R)0.5 * g * dp);
+  add(THETA, cm, ch);
+  add(THETA, cp, ch);
+  add(PI, cp, (double)-(g * th));
+  add(PI, cm, (double)(g * th));
+}
+
+template <class R>
+__device__ __forceinline__ void ad_v(const Dims& d, const Metric& m, const Flags& fl, const F12& b, const B12& bi,
+                                     double lam, int i, int j, int k) {
+  const int nx = d.nx, ny = d.ny, nz = d.nz;
+  const int jp = imin(j, ny - 1), jm = imax(j - 1, 0), ia = imax(i - 1, 0), kp = imin(k + 1, nz - 1);
+  const R idy = (R)m.inv_dy, hx = (R)(0.5 * m.inv_dx);
+  const R hz = (R)(1.0 / (2.0 * (dzeta_(m, d, imin(k, nz - 1)) * scale_(m, d, i, jp))));
+  const size_t cm = d.idx(i, jm, k), cp = d.idx(i, jp, k);
+  const size_t ce = d.idx(imin(i + 1, nx - 1), jp, k), cw = d.idx(ia, jp, k);
+  const size_t ct = d.idx(i, jp, kp), cb = d.idx(i, jp, imax(k - 1, 0));
+  const size_t u0 = d.idx(ia, jm, k);
+  const R vm = BV(V, cm), vp = BV(V, cp);
+  const R vc = (R)0.5 * (vm + vp), vy = (vp - vm) * idy;
+  const R vx = (BV(V, ce) - BV(V, cw)) * hx, vz = (BV(V, ct) - BV(V, cb)) * hz;
+  const R uc = (R)0.25 * (BV(U, u0) + BV(U, cm) + BV(U, cw) + BV(U, cp));
+  const R wc = (R)0.5 * (BV(W, cp) + BV(W, ct));
+  const R th = (R)0.5 * (BT(cm) + BT(cp)), dp = BP(cp) - BP(cm);
+  const R g = (R)kCp * idy;
+  const BarAdd add{bi, lam};
+  add(V, cp, (double)-((R)0.5 * vy + vc * idy));
+  add(V, cm, (double)(vc * idy - (R)0.5 * vy));
+  add(V, ce, (double)-(uc * hx));
+  add(V, cw, (double)(uc * hx));
+  add(V, ct, (double)-(wc * hz));
+  add(V, cb, (double)(wc * hz));
+  const double cu = (double)-((R)0.25 * (vx + (fl.coriolis ? (R)corf_(m, fl, d, j) : (R)0)));
+  add(U, u0, cu);
+  add(U, cm, cu);
+  add(U, cw, cu);
+  add(U, cp, cu);
+  const double cz = (double)-((R)0.5 * vz);
+  add(W, cp, cz);
+  add(W, ct, cz);
+  const double ch = (double)-((R)0.5 * g * dp);
+  add(THETA, cm, ch);
+  add(THETA, cp, ch);
+  add(PI, cp, (double)-(g * th));
+  add(PI, cm, (double)(g * th));
+}
+
+template <class R>
+__device__ __forceinline__ void ad_w(const Dims& d, const Metric& m, const Flags& fl, const F12& b, const B12& bi,
+                                     double lam, int i, int j, int k) {
+  const int nx = d.nx, ny = d.ny, nz = d.nz;
+  const int kc = imin(imax(k, 0), nz - 1), kt = imin(k, nz), km = imax(k - 1, 0);
+  const double dz = dzeta_(m, d, kc) * scale_(m, d, i, j);
+  const R hx = (R)(0.5 * m.inv_dx), hy = (R)(0.5 * m.inv_dy), iz = (R)(1.0 / dz), iz1 = (R)(1.0 / dmax(dz, 1.0));
+  const size_t ct = d.idx(i, j, kt), cc = d.idx(i, j, kc), cb = d.idx(i, j, km);
+  const size_t ce = d.idx(imin(i + 1, nx - 1), j, kt), cw = d.idx(imax(i - 1, 0), j, kt);
+  const size_t cn = d.idx(i, imin(j + 1, ny - 1), kt), cs = d.idx(i, imax(j - 1, 0), kt);
+  const R wt = BV(W, ct);
+  const R wc = (R)0.5 * (BV(W, cc) + wt), wz = (wt - BV(W, cb)) * iz;
+  const R wx = (BV(W, ce) - BV(W, cw)) * hx, wy = (BV(W, cn) - BV(W, cs)) * hy;
+  const R uc = (R)0.5 * (BV(U, cc) + BV(U, cc + 1)), vc = (R)0.5 * (BV(V, cc) + BV(V, cc + d.P));
+  const R th = (R)0.5 * (BT(cb) + BT(cc)), dp = BP(cc) - BP(cb);
+  const R g = (R)kCp * iz1;
+  const BarAdd add{bi, lam};
+  add(W, ct, (double)-((R)0.5 * wz + wc * iz));
+  add(W, cc, (double)-((R)0.5 * wz));
+  add(W, cb, (double)(wc * iz));
+  add(W, ce, (double)-(uc * hx));
+  add(W, cw, (double)(uc * hx));
+  add(W, cn, (double)-(vc * hy));
+  add(W, cs, (double)(vc * hy));
+  const double cu = (double)-((R)0.5 * wx), cv = (double)-((R)0.5 * wy);
+  add(U, cc, cu);
+  add(U, cc + 1, cu);
+  add(V, cc, cv);
+  add(V, cc + d.P, cv);
+  const R ch = (R)0.5 * g * dp;
+  add(THETA, cb, (double)-ch);
+  add(THETA, cc, (double)((R)kG * (R)(1.0 / dmax(m.th0[cc], 1.0)) - ch));
+  add(PI, cc, (double)-(g * th));
+  add(PI, cb, (double)(g * th));
+  add(QV, cc, (double)((R)kG * (R)kBuoyMoist));
+  for (int q = QC; q <= QG; ++q) add(q, cc, (double)-(R)kG);
+}
+
+template <class R>
+__device__ __forceinline__ void ad_rho(const Dims& d, const Metric& m, const Flags& fl, const F12& b, const B12& bi,
+                                       double lam, int i, int j, int k) {
+  const int nx = d.nx, ny = d.ny, nz = d.nz;
+  const bool sp = fl.split_fast;
+  const R idx = (R)m.inv_dx, idy = (R)m.inv_dy, iz = (R)(1.0 / dmax(dzeta_(m, d, k) * scale_(m, d, i, j), 1.0));
+  const size_t c = d.idx(i, j, k), e = c + 1, n = c + d.P;
+  const size_t w = d.idx(imax(i - 1, 0), j, k), s = d.idx(i, imax(j - 1, 0), k);
+  const size_t t = d.idx(i, j, imin(k + 1, nz - 1)), l = d.idx(i, j, imax(k - 1, 0)), tf = c + d.plane;
+  auto rr = [&](size_t p, size_t p0) { return (R)(b.f[RHO][p] - (sp ? m.rho0[p0] : 0.0)); };
+  const R rc = rr(c, c);
+  const R ue = BV(U, e), uw = BV(U, c), vn = BV(V, n), vs = BV(V, c), wt = BV(W, tf), wb = BV(W, c);
+  const R h = (R)0.5;
+  const BarAdd add{bi, lam};
+  add(U, e, (double)-(idx * (h * (rc + rr(e, i + 1 < nx ? e : c)))));
+  add(U, c, (double)(idx * (h * (rr(w, w) + rc))));
+  add(V, n, (double)-(idy * (h * (rc + rr(n, j + 1 < ny ? n : c)))));
+  add(V, c, (double)(idy * (h * (rr(s, s) + rc))));
+  add(W, tf, (double)-(iz * (h * (rc + rr(t, t)))));
+  add(W, c, (double)(iz * (h * (rr(l, l) + rc))));
+  add(RHO, e, (double)-(h * ue * idx));
+  add(RHO, w, (double)(h * uw * idx));
+  add(RHO, n, (double)-(h * vn * idy));
+  add(RHO, s, (double)(h * vs * idy));
+  add(RHO, t, (double)-(h * wt * iz));
+  add(RHO, l, (double)(h * wb * iz));
+  add(RHO, c, (double)-(h * ((ue - uw) * idx + (vn - vs) * idy + (wt - wb) * iz)));
+}
+
 template <class R>
 __global__ void k_ad_faces(Dims d, Metric m, Flags fl, const __grid_constant__ F12 b, const __grid_constant__ F12 bo,
                            const __grid_constant__ B12 bi) {
@@ -515,11 +753,11 @@ __global__ void k_ad_faces(Dims d, Metric m, Flags fl, const __grid_constant__ F
   if (i > d.nx || j > d.ny || k > d.nz) return;
   const size_t c = d.idx(i, j, k);
   if (j < d.ny && k < d.nz && bo.f[U][c] != 0.0)
-    ad_scatter<R>(b, bi, bo.f[U][c], [&](AdLoad<R>& L) { return pt_u<R>(d, m, fl, L, i, j, k); });
+    ad_u<R>(d, m, fl, b, bi, bo.f[U][c], i, j, k);
   if (i < d.nx && k < d.nz && bo.f[V][c] != 0.0)
-    ad_scatter<R>(b, bi, bo.f[V][c], [&](AdLoad<R>& L) { return pt_v<R>(d, m, fl, L, i, j, k); });
+    ad_v<R>(d, m, fl, b, bi, bo.f[V][c], i, j, k);
   if (i < d.nx && j < d.ny && bo.f[W][c] != 0.0)
-    ad_scatter<R>(b, bi, bo.f[W][c], [&](AdLoad<R>& L) { return pt_w<R>(d, m, fl, L, i, j, k); });
+    ad_w<R>(d, m, fl, b, bi, bo.f[W][c], i, j, k);
 }
 
 template <class R>
@@ -531,7 +769,7 @@ __global__ void k_ad_cells(Dims d, Metric m, Flags fl, const __grid_constant__ F
   if (i >= d.nx || j >= d.ny || k >= d.nz) return;
   const size_t c = d.idx(i, j, k);
   if (bo.f[RHO][c] != 0.0)
-    ad_scatter<R>(b, bi, bo.f[RHO][c], [&](AdLoad<R>& L) { return pt_rho<R>(d, m, fl, L, i, j, k); });
+    ad_rho<R>(d, m, fl, b, bi, bo.f[RHO][c], i, j, k);
   if (fl.div_damp > 0.0 && bo.f[PI][c] != 0.0)
     ad_scatter<R>(b, bi, bo.f[PI][c], [&](AdLoad<R>& L) { return pt_pi<R>(d, m, fl, L, i, j, k); });
   if (!fl.weno_scalars) {
@@ -617,17 +855,16 @@ __global__ void k_ad_wface(Dims d, Metric m, Flags fl, const __grid_constant__ F
       extra = sh * lamG;
     }
     const int vq = dir == 0 ? U : (dir == 1 ? V : W);
-    AdLoad<R> L{&b, 0, 0, -1, 0};
-    for (int seed = 0; seed < kMaxLoads; ++seed) {
-      L.seed = seed;
-      L.n = 0;
-      L.hq = -1;
-      const Jet<R> g = pt_wface<R>(d, L, q, dir, i, j, k, sh);
-      if (L.hq < 0) break;
-      double v = (double)g.d * lamG;
-      if (L.hq == vq) v += extra;
-      if (v != 0.0) atomicAdd(&bi.f[L.hq][L.hc], v);
-    }
+    size_t o[5];
+    wface_points(d, dir, i, j, k, o);
+    R z[5], g[5], gvel;
+#pragma unroll
+    for (int n = 0; n < 5; ++n) z[n] = (R)(b.f[q][o[n]] - sh);
+    const size_t c = d.idx(i, j, k);
+    wgrad_<R>(z, (R)b.f[vq][c], g, gvel);
+#pragma unroll
+    for (int n = 0; n < 5; ++n) atomicAdd(&bi.f[q][o[n]], (double)g[n] * lamG);
+    atomicAdd(&bi.f[vq][c], (double)gvel * lamG + extra);
   }
 }
 
@@ -726,7 +963,8 @@ void tend_ad_t(const Dims& d, const Metric& m, const Flags& fl, double* const* b
     const FaceArr F = face_arr(d, face);
     for (int q = THETA; q <= scalar_last(fl); ++q) {
       if (q == PI) continue;
-      k_tl_wface<R><<<grid3_(d, d.nx + 1, d.ny + 1, d.nz + 1, kB), kB, 0, s>>>(d, b, b, q, F, 0);
+      if (q >= QV)  // the clip's test needs the cell's value
+        k_tl_wface<R><<<grid3_(d, d.nx + 1, d.ny + 1, d.nz + 1, kB), kB, 0, s>>>(d, b, b, q, F, 0);
       k_ad_wcell<R><<<grid3_(d, d.nx, d.ny, d.nz, kB), kB, 0, s>>>(d, m, fl, b, q, F, bar_out[q], cell_scr, bi);
       k_ad_wface<R><<<grid3_(d, d.nx + 1, d.ny + 1, d.nz + 1, kB), kB, 0, s>>>(d, m, fl, b, q, cell_scr, bi);
     }
