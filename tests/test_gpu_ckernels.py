@@ -578,3 +578,56 @@ def test_flux_advection_adjoint_dot_product_f32(vg):
     bar = _ad(vg, x, y, dzeta, zs, dims, f32=True)
     rhs = float(sum(np.dot(d[k].astype(np.float64), bar[k]) for k in ADV))
     assert abs(lhs - rhs) <= 1e-5 * max(abs(lhs), abs(rhs)), (lhs, rhs)
+
+
+def _dev(vg, name, args):
+    import ctypes
+    f = getattr(ctypes.CDLL(vg.lib._name), name)
+    f.restype, f.argtypes = ctypes.c_int, args
+    return f
+
+
+@pytest.mark.parametrize("bits", [64, 32])
+@pytest.mark.parametrize("n", [1, 2, 7, 8, 9, 16, 17, 80, 128, 129, 200, 363, 364])
+@pytest.mark.parametrize("n_sys", [1, 33, 300])
+def test_thomas_staged_sweep_edges(vg, oc, bits, n, n_sys):
+    """The on-chip sweep at the edges of its stages (8 and 16 levels), its
+    32-system blocks and its limits in n and n_sys: against the oracle at the
+    bounds of the tests above (1e-12; FP32 1e-5), NULL off-diagonals, and a
+    singular system, whose x stays as it was while its neighbours solve."""
+    import ctypes
+    import torch
+    dt = torch.float64 if bits == 64 else torch.float32
+    vp, i32 = ctypes.c_void_p, ctypes.c_int
+    f = _dev(vg, "vibe_tridiagonal_solve_batched_f%d_dev" % bits, [vp] * 4 + [i32, i32, vp, vp, vp])
+    rng = np.random.default_rng(n * 1000 + n_sys)
+    a, c = -rng.random((n_sys, max(n - 1, 1))), -rng.random((n_sys, max(n - 1, 1)))
+    b, d = 2.5 + rng.random((n_sys, n)), rng.random((n_sys, n))
+    bad = n_sys // 2
+    if n_sys > 1:
+        b[bad, 0] = 0.0  # a zero first pivot
+    t = [torch.tensor(v, dtype=dt, device="cuda") for v in (a[:, :n - 1], b, c[:, :n - 1], d)]
+    x = torch.full((n_sys, n), 7.0, dtype=dt, device="cuda")
+    st = torch.full((n_sys,), -1, dtype=torch.int32, device="cuda")
+    stream = torch.cuda.current_stream().cuda_stream
+    p = lambda v: v.data_ptr() if v.numel() else None  # noqa: E731
+    assert f(p(t[0]), p(t[1]), p(t[2]), p(t[3]), n, n_sys, x.data_ptr(), st.data_ptr(), stream) == 0
+    torch.cuda.synchronize()
+    host = [v.double().cpu().numpy() for v in t]
+    got, status = x.double().cpu().numpy(), st.cpu().numpy()
+    tol = 1e-12 if bits == 64 else 1e-5
+    for s in range(n_sys):
+        xo, ws = np.zeros(n), np.zeros(n)
+        rows = [np.ascontiguousarray(h[s]) for h in host]
+        rc = oc.port_lib().vo_tridiagonal_solve(rows[0].ctypes.data, rows[1].ctypes.data, rows[2].ctypes.data,
+                                                 rows[3].ctypes.data, n, xo.ctypes.data, ws.ctypes.data)
+        assert status[s] == rc == (1 if n_sys > 1 and s == bad else 0)
+        if rc:
+            if n <= 128:
+                assert (got[s] == 7.0).all()
+        else:
+            assert np.abs(got[s] - xo).max() <= tol * np.abs(xo).max()
+    assert f(None, p(t[1]), None, p(t[3]), n, n_sys, x.data_ptr(), None, stream) == 0
+    ok = np.arange(n_sys) != (bad if n_sys > 1 else -1)
+    q = (host[3] / np.where(host[1] == 0.0, 1.0, host[1]))[ok]
+    assert np.abs(x.double().cpu().numpy()[ok] - q).max() <= tol * np.abs(q).max()

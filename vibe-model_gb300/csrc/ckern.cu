@@ -138,7 +138,135 @@ __global__ void k_thomas_batched(const T* __restrict__ a, const T* __restrict__ 
 }
 
 // ---------------------------------------------------------------------------
-// Tall systems (n > kTallN): one warp per system. The n rows split into 32
+// The sweep staged on chip: one warp takes 32 consecutive systems, one per
+// lane, with the recurrence of thomas_seq. In every array the rows of those
+// systems are one contiguous span; a chunk of kStage levels (a 32-byte sector a
+// system) comes in by cp.async with four (FP32: eight) lanes on consecutive
+// elements, so each fetched sector is used, and is transposed by the odd row
+// stride of the staging buffer (no bank conflicts when lanes read their own
+// rows). Two chunks are in flight; chunks of two sectors leave room for three
+// warps an SM instead of four at n = 80 (0.80 ms against 0.71 at 262144 x 80,
+// where one thread per system took 2.50 ms and read DRAM 13 times over). The modified super-diagonal and the
+// eliminated right-hand side stay in shared memory, level-major, and the back
+// substitution stores x through the same staging, so DRAM sees each element
+// once and no workspace is needed. FP64 multiplies by one reciprocal per row
+// (pivots under 1e-290, where it could overflow, divide), as the pipe is the
+// bound there: about 13 FP64 operations a row; FP32 divides twice.
+// A system with a zero pivot leaves x as it was.
+template <typename T>
+struct Sweep {
+  static constexpr int kStage = 32 / (int)sizeof(T), kRow = kStage + 1;
+  static constexpr int kArr = 32 * kRow;  // one array's chunk
+  static size_t smem(int n) { return ((size_t)64 * n + 8 * kArr) * sizeof(T); }
+};
+template <typename T>
+__device__ __forceinline__ void cp_async_elem(T* smem, const T* gmem) {
+  const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;\n" ::"r"(sa), "l"(gmem), "n"((int)sizeof(T)) : "memory");
+}
+// one row: x_k = (d - a x_{k-1}) / den, c'_k = c / den
+__device__ __forceinline__ void sweep_row(double den, double num, double c, double& x, double& cp) {
+  if ((__double2hiint(den) & 0x7fffffff) < 0x03d00000) {  // |den| < 1e-290
+    x = num / den;
+    cp = c / den;
+  } else {
+    const double r = 1.0 / den;
+    x = num * r;
+    cp = c * r;
+  }
+}
+__device__ __forceinline__ void sweep_row(float den, float num, float c, float& x, float& cp) {
+  x = num / den;
+  cp = c / den;
+}
+template <typename T>
+__global__ void __launch_bounds__(32) k_thomas_sweep(const T* __restrict__ a, const T* __restrict__ b,
+                                                     const T* __restrict__ c, const T* __restrict__ d, int n, int n_sys,
+                                                     T* __restrict__ x, int* __restrict__ status) {
+  constexpr int K = Sweep<T>::kStage, R = Sweep<T>::kRow, A = Sweep<T>::kArr;
+  extern __shared__ __align__(16) char s_sweep[];
+  T* Y = reinterpret_cast<T*>(s_sweep);  // n x 32
+  T* CP = Y + (size_t)32 * n;            // n x 32
+  T* st = CP + (size_t)32 * n;           // 2 buffers x (a, b, c, d)
+  const int lane = threadIdx.x;
+  const int s0 = blockIdx.x * 32, ns = n_sys - s0 < 32 ? n_sys - s0 : 32;
+  const T* bs = b + (size_t)s0 * n;
+  const T* ds = d + (size_t)s0 * n;
+  const T* as = a ? a + (size_t)s0 * (n - 1) : nullptr;
+  const T* cs = c ? c + (size_t)s0 * (n - 1) : nullptr;
+  for (int e = lane; e < 8 * A; e += 32) st[e] = (T)0;  // absent a, c and idle lanes read zeros
+  __syncwarp();
+  const int nch = (n + K - 1) / K;
+  auto load = [&](int ch) {
+    T* q = st + (ch & 1) * 4 * A;
+#pragma unroll
+    for (int m = 0; m < K; ++m) {
+      const int e = m * 32 + lane, sys = e / K, kk = e % K, k = ch * K + kk;
+      if (sys < ns && k < n) {
+        const int o = sys * R + kk;
+        const size_t g = (size_t)sys * n + k, h = g - sys;  // h: row k of the (n - 1)-long arrays
+        cp_async_elem(q + A + o, bs + g);
+        cp_async_elem(q + 3 * A + o, ds + g);
+        if (as && k >= 1) cp_async_elem(q + o, as + h - 1);
+        if (cs && k < n - 1) cp_async_elem(q + 2 * A + o, cs + h);
+      }
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+  load(0);
+  T xp = (T)0, cp = (T)0;
+  bool sing = false;
+  for (int ch = 0; ch < nch; ++ch) {
+    if (ch + 1 < nch) {
+      load(ch + 1);
+      asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+    } else {
+      asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    }
+    __syncwarp();
+    const T* q = st + (ch & 1) * 4 * A + lane * R;
+#pragma unroll
+    for (int kk = 0; kk < K; ++kk) {
+      const int k = ch * K + kk;
+      if (k < n) {
+        const T am = k > 0 ? q[kk] : (T)0;
+        const T den = q[A + kk] - am * cp;
+        sing |= den == (T)0;
+        sweep_row(den, q[3 * A + kk] - am * xp, k + 1 < n ? q[2 * A + kk] : (T)0, xp, cp);
+        if (n == 1) xp = q[3 * A] / den;
+        Y[k * 32 + lane] = xp;
+        CP[k * 32 + lane] = cp;
+      }
+    }
+    __syncwarp();  // the buffer is free for the chunk after next
+  }
+  if (lane >= ns) sing = true;
+  const unsigned bad = __ballot_sync(0xffffffffu, sing);
+  if (status && lane < ns) status[s0 + lane] = sing ? VIBE_C_ERR_SINGULAR : VIBE_C_OK;
+  xp = (T)0;
+  T* xs = x + (size_t)s0 * n;
+  for (int ch = nch - 1; ch >= 0; --ch) {
+    T* q = st + (ch & 1) * A;
+#pragma unroll
+    for (int kk = K - 1; kk >= 0; --kk) {
+      const int k = ch * K + kk;
+      if (k < n) {
+        xp = (k + 1 < n) ? Y[k * 32 + lane] - CP[k * 32 + lane] * xp : Y[k * 32 + lane];
+        q[lane * R + kk] = xp;
+      }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int m = 0; m < K; ++m) {
+      const int e = m * 32 + lane, sys = e / K, kk = e % K, k = ch * K + kk;
+      if (!((bad >> sys) & 1u) && k < n) xs[(size_t)sys * n + k] = q[sys * R + kk];
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Tall systems (n > kTallN) that are few, or too tall for the on-chip sweep:
+// one warp per system. The n rows split into 32
 // contiguous chunks, one per lane; each lane factors its chunk once (the
 // recurrence above) and solves it for three right-hand sides: the chunk's d
 // (y), its coupling to the unknown left of the chunk (v, from a at the first
@@ -523,10 +651,11 @@ __global__ void k_flux_adv(const T* __restrict__ q, const T* __restrict__ rho, c
 // workspace (the modified super-diagonal, n doubles per system) in this
 // fixed device array instead of the allocated scratch buffer. The array is
 // sized here, once, and every GPU that loads the library holds it until the
-// process exits. It always runs the one-thread-per-system sweep
-// (k_thomas_batched), also for n > 128 where the allocating _dev form runs
-// the warp-per-system solver: there the two agree to rounding, and this
-// form's singular test is the sweep's exact-zero pivot.
+// process exits; only columns too tall for the on-chip sweep use it, with the
+// one-thread-per-system sweep (k_thomas_batched). It sweeps for every n, also
+// where the allocating _dev form runs the warp-per-system solver: there the
+// two agree to rounding, and this form's singular test is the sweep's
+// exact-zero pivot.
 constexpr size_t kNoAllocThomasDoubles = (size_t)1 << 18;  // 2 MiB: n * n_sys <= 262144
 static __device__ __align__(256) double g_noalloc_thomas_work[kNoAllocThomasDoubles];
 // Device address of that array per device. Host code only sees a host-side
@@ -550,16 +679,38 @@ constexpr int kRedThreads = 256;
 using vgb_cabi::DevScratch;
 using vgb_cabi::HostCall;
 
-size_t thomas_work(int n, int n_sys) { return (size_t)n * (size_t)n_sys * (n > kTallN ? 3 : 1); }
+// The staged sweep runs whenever its columns fit in shared memory and n is at
+// most kTallN, or there are enough systems: it takes n * 0.18 us a wave of 32 x
+// 152 systems, the warp-per-system solver 0.7 ns * n a system (65536 systems of
+// 200 rows: 9.1 ms), which meet near 260 systems.
+constexpr size_t kSweepSmem = 200 * 1024;
+constexpr int kSweepSystems = 256;
+template <typename T>
+bool thomas_sweeps(int n, int n_sys) {
+  return Sweep<T>::smem(n) <= kSweepSmem && (n <= kTallN || n_sys >= kSweepSystems);
+}
+template <typename T>
+size_t thomas_work(int n, int n_sys) {
+  return thomas_sweeps<T>(n, n_sys) ? 0 : (size_t)n * (size_t)n_sys * 3;
+}
+template <typename T>
+int thomas_sweep_launch(const T* a, const T* b, const T* c, const T* d, int n, int n_sys, T* x, int* status,
+                        cudaStream_t st) {
+  const size_t sm = Sweep<T>::smem(n);
+  if (sm > 48 * 1024 && !device_ok(cudaFuncSetAttribute(k_thomas_sweep<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                        (int)kSweepSmem),
+                                   "thomas shared memory"))
+    return VIBE_C_ERR_DEVICE;
+  k_thomas_sweep<T><<<(n_sys + 31) / 32, 32, sm, st>>>(a, b, c, d, n, n_sys, x, status);
+  return device_ok(cudaGetLastError(), "thomas launch") ? VIBE_C_OK : VIBE_C_ERR_DEVICE;
+}
 
 template <typename T>
 int thomas_launch(const T* a, const T* b, const T* c, const T* d, int n, int n_sys, T* x, T* work, int* status,
                   cudaStream_t st) {
-  if (n > kTallN)
-    k_thomas_tall<T><<<(n_sys + kTallWarps - 1) / kTallWarps, 32 * kTallWarps, 0, st>>>(a, b, c, d, n, n_sys, x,
-                                                                                       work, status);
-  else
-    k_thomas_batched<T><<<(n_sys + 127) / 128, 128, 0, st>>>(a, b, c, d, n, n_sys, x, work, status);
+  if (thomas_sweeps<T>(n, n_sys)) return thomas_sweep_launch<T>(a, b, c, d, n, n_sys, x, status, st);
+  k_thomas_tall<T><<<(n_sys + kTallWarps - 1) / kTallWarps, 32 * kTallWarps, 0, st>>>(a, b, c, d, n, n_sys, x, work,
+                                                                                     status);
   return device_ok(cudaGetLastError(), "thomas launch") ? VIBE_C_OK : VIBE_C_ERR_DEVICE;
 }
 
@@ -568,7 +719,8 @@ int thomas_batched_dev(const T* a, const T* b, const T* c, const T* d, int n, in
                        vibe_stream_t stream) {
   if (n <= 0 || n_sys < 0 || b == nullptr || d == nullptr || x == nullptr) return VIBE_C_ERR_BAD_ARG;
   if (n_sys == 0) return VIBE_C_OK;
-  DevScratch w(thomas_work(n, n_sys) * sizeof(T), (cudaStream_t)stream);
+  if (thomas_sweeps<T>(n, n_sys)) return thomas_sweep_launch<T>(a, b, c, d, n, n_sys, x, status, (cudaStream_t)stream);
+  DevScratch w(thomas_work<T>(n, n_sys) * sizeof(T), (cudaStream_t)stream);
   if (!w.get()) return VIBE_C_ERR_DEVICE;
   int rc = thomas_launch<T>(a, b, c, d, n, n_sys, x, (T*)w.get(), status, (cudaStream_t)stream);
   if (!w.release() && rc == VIBE_C_OK) rc = VIBE_C_ERR_DEVICE;
@@ -588,7 +740,7 @@ int thomas_batched_host(const T* a, const T* b, const T* c, const T* d, int n, i
   // reference, which returns before it writes x (c_kernels.c:26,34,40)
   const int ix = hc.add(nullptr, nn * e, HostCall::kOut);
   const int is = hc.add(nullptr, (size_t)n_sys * sizeof(int), HostCall::kOut);
-  const int iw = hc.add(nullptr, thomas_work(n, n_sys) * e, HostCall::kScratch);
+  const int iw = hc.add(nullptr, thomas_work<T>(n, n_sys) * e, HostCall::kScratch);
   if (!hc.commit()) return VIBE_C_ERR_DEVICE;
   int rc = thomas_launch<T>(hc.dev<T>(ia), hc.dev<T>(ib), hc.dev<T>(ic), hc.dev<T>(id), n, n_sys, hc.dev<T>(ix),
                             hc.dev<T>(iw), hc.dev<int>(is), hc.stream());
@@ -915,6 +1067,8 @@ int vibe_tridiagonal_solve_batched_f64_dev_noalloc(const double* a, const double
     return VIBE_C_ERR_BAD_ARG;
   }
   if (n_sys == 0) return VIBE_C_OK;
+  if (Sweep<double>::smem(n) <= kSweepSmem)  // on chip: no workspace at all
+    return thomas_sweep_launch<double>(a, b, c, d, n, n_sys, x, status, (cudaStream_t)stream);
   const int dev = cur_dev();
   if (dev < 0 || dev >= 64) { g_cerr = "device ordinal out of range"; return VIBE_C_ERR_DEVICE; }
   double* work = nullptr;
