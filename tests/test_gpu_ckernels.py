@@ -631,3 +631,33 @@ def test_thomas_staged_sweep_edges(vg, oc, bits, n, n_sys):
     ok = np.arange(n_sys) != (bad if n_sys > 1 else -1)
     q = (host[3] / np.where(host[1] == 0.0, 1.0, host[1]))[ok]
     assert np.abs(x.double().cpu().numpy()[ok] - q).max() <= tol * np.abs(q).max()
+
+
+@pytest.mark.parametrize("bits", [64, 32])
+@pytest.mark.parametrize("dims", [(1, 1, 1), (1, 5, 2), (5, 3, 3), (31, 8, 4), (32, 9, 5), (62, 7, 9), (63, 17, 13)])
+def test_flux_advection_tile_edges(vg, oc, bits, dims):
+    """Tiles of 31 x 8 columns and chunks of levels, wrapped rows and columns on
+    small periodic grids: against the oracle at the bounds above (1e-12; FP32
+    1e-4)."""
+    import ctypes
+    import torch
+    nx, ny, nz = dims
+    dt = torch.float64 if bits == 64 else torch.float32
+    vp, i32 = ctypes.c_void_p, ctypes.c_int
+    real = ctypes.c_double if bits == 64 else ctypes.c_float
+    f = _dev(vg, "vibe_advect_scalar_flux_f%d_dev" % bits, [vp] * 7 + [i32] * 3 + [real] * 3 + [vp, vp])
+    rng = np.random.default_rng(nx * 100 + ny)
+    n = nx * ny * nz
+    fields = [rng.random(n), 0.5 + rng.random(n), 20 * rng.random(n) - 10, 20 * rng.random(n) - 10,
+              rng.random(n) - 0.5, 0.01 + 0.01 * rng.random(nz), 500.0 * rng.random(nx * ny)]
+    t = [torch.tensor(v, dtype=dt, device="cuda") for v in fields]
+    host = [np.ascontiguousarray(v.double().cpu().numpy()) for v in t]
+    for zs in (True, False):
+        out = torch.full((n,), float("nan"), dtype=dt, device="cuda")
+        args = [v.data_ptr() for v in t[:6]] + [t[6].data_ptr() if zs else None]
+        assert f(*args, nx, ny, nz, 900.0, 1100.0, 20000.0, out.data_ptr(), torch.cuda.current_stream().cuda_stream) == 0
+        ref = np.full(n, np.nan)
+        oc.port_lib().vo_advect_scalar_flux(*[h.ctypes.data for h in host[:6]], host[6].ctypes.data if zs else None,
+                                             nx, ny, nz, 900.0, 1100.0, 20000.0, ref.ctypes.data)
+        tol = 1e-12 if bits == 64 else 1e-4
+        assert np.abs(out.double().cpu().numpy() - ref).max() <= tol * np.abs(ref).max() or np.abs(ref).max() == 0.0

@@ -606,39 +606,72 @@ __global__ void k_cfl_final(const T* __restrict__ partials, int nb, T* __restric
   }
 }
 
-// flux advection (c_kernels.c:209-286), one thread per cell
+// flux advection (c_kernels.c:209-286). Every face flux is computed once: a
+// warp is 32 consecutive columns, whose west fluxes serve the 31 cells between
+// them (the neighbour's by shuffle); a block's nine rows of south fluxes serve
+// eight rows of cells through shared memory; a thread marches up the levels
+// and keeps its lower face's flux. With one division per cell that is about 30
+// FP64 operations, the bound, where one thread per cell with its six faces
+// spent 70 and three index divisions. The halves of the two means are exact
+// powers of two and are applied once.
+// x < 1 and x > 1e-12 on the integer pipe (a NaN rho makes the fluxes NaN
+// whatever the divisor)
+__device__ __forceinline__ bool below_one(double x) { return __double2hiint(x) < 0x3ff00000; }
+__device__ __forceinline__ bool below_one(float x) { return x < 1.f; }
+__device__ __forceinline__ bool above_floor(double x) { return __double_as_longlong(x) > __double_as_longlong(1e-12); }
+__device__ __forceinline__ bool above_floor(float x) { return x > 1e-12f; }
+constexpr int kFluxRows = 8, kFluxCols = 31;
 template <typename T>
-__global__ void k_flux_adv(const T* __restrict__ q, const T* __restrict__ rho, const T* __restrict__ u,
-                           const T* __restrict__ v, const T* __restrict__ w, const T* __restrict__ dzeta,
-                           const T* __restrict__ zs, int nx, int ny, int nz, T dx, T dy, T z_top, T* __restrict__ dqdt) {
-  const size_t nxy = (size_t)nx * ny, n = nxy * nz;
-  const T inv_dx = (T)1 / dx, inv_dy = (T)1 / dy, hf = (T)0.5;
-  for (size_t idx = blockIdx.x * (size_t)blockDim.x + threadIdx.x; idx < n; idx += (size_t)gridDim.x * blockDim.x) {
-    const int k = (int)(idx / nxy);
-    const int j = (int)((idx / nx) % ny);
-    const int i = (int)(idx % nx);
-    const size_t base_k = (size_t)k * nxy;
-    const T scale = zs ? (z_top - zs[(size_t)j * nx + i]) : z_top;
-    T dz = dzeta[k] * scale;
-    if (dz < (T)1) dz = (T)1;
-    const size_t c = idx;
-    const size_t e = base_k + (size_t)j * nx + (size_t)((i + 1) % nx);
-    const size_t ws = base_k + (size_t)j * nx + (size_t)((i + nx - 1) % nx);
-    const T fxE = u[e] * (hf * (rho[c] + rho[e])) * (hf * (q[c] + q[e]));
-    const T fxW = u[c] * (hf * (rho[ws] + rho[c])) * (hf * (q[ws] + q[c]));
-    const size_t nn = base_k + (size_t)((j + 1) % ny) * nx + (size_t)i;
-    const size_t ss = base_k + (size_t)((j + ny - 1) % ny) * nx + (size_t)i;
-    const T fyN = v[nn] * (hf * (rho[c] + rho[nn])) * (hf * (q[c] + q[nn]));
-    const T fyS = v[c] * (hf * (rho[ss] + rho[c])) * (hf * (q[ss] + q[c]));
-    T fzT = 0, fzB = 0;
-    if (k > 0 && k + 1 < nz) {
-      const size_t t = c + nxy, b = c - nxy;
-      fzT = w[t] * (hf * (rho[c] + rho[t])) * (hf * (q[c] + q[t]));
-      fzB = w[c] * (hf * (rho[b] + rho[c])) * (hf * (q[b] + q[c]));
+__global__ void __launch_bounds__(32 * (kFluxRows + 1)) k_flux_adv(
+    const T* __restrict__ q, const T* __restrict__ rho, const T* __restrict__ u, const T* __restrict__ v,
+    const T* __restrict__ w, const T* __restrict__ dzeta, const T* __restrict__ zs, int nx, int ny, int nz, T dx, T dy,
+    T z_top, T* __restrict__ dqdt, int xtiles, int kz) {
+  __shared__ T sy[2][kFluxRows + 1][32];
+  const size_t nxy = (size_t)nx * ny;
+  const int lane = threadIdx.x, row = threadIdx.y;
+  const int i0 = (int)(blockIdx.x % (unsigned)xtiles) * kFluxCols, j0 = (int)(blockIdx.x / (unsigned)xtiles) * kFluxRows;
+  const int k0 = blockIdx.y * kz, k1 = k0 + kz < nz ? k0 + kz : nz;
+  const int i = (i0 + lane) % nx, j = (j0 + row) % ny;  // periodic; the columns and rows past the grid wrap onto it
+  const int im = i > 0 ? i - 1 : nx - 1, js = j > 0 ? j - 1 : ny - 1;
+  const bool cells = row < kFluxRows;  // the last row only has south fluxes
+  const bool mine = cells && lane < kFluxCols && i0 + lane < nx && j0 + row < ny;
+  const size_t c = (size_t)j * nx + i, cs = (size_t)js * nx + i, cw = (size_t)j * nx + im;
+  const T ax = (T)0.25 * ((T)1 / dx), ay = (T)0.25 * ((T)1 / dy);
+  const T scale = zs ? (z_top - zs[c]) : z_top;
+  size_t o = (size_t)k0 * nxy;
+  T qc = q[o + c], rc = rho[o + c], fb = 0;
+  if (cells && k0 > 0) fb = w[o + c] * (rho[o - nxy + c] + rc) * (q[o - nxy + c] + qc);
+  for (int k = k0; k < k1; ++k, o += nxy) {
+    const T fs = v[o + c] * (rho[o + cs] + rc) * (q[o + cs] + qc);
+    sy[k & 1][row][lane] = fs;
+    T qt = 0, rt = 0, ft = 0, fw = 0, fe = 0;
+    if (k + 1 < nz) {
+      qt = q[o + nxy + c];
+      rt = rho[o + nxy + c];
     }
-    const T div = (fxE - fxW) * inv_dx + (fyN - fyS) * inv_dy + (fzT - fzB) / dz;
-    const T rr = (rho[idx] > (T)1e-12) ? rho[idx] : (T)1e-12;
-    dqdt[idx] = -div / rr;
+    if (cells) {
+      if (k + 1 < nz) ft = w[o + nxy + c] * (rc + rt) * (qc + qt);
+      T qw = __shfl_up_sync(0xffffffffu, qc, 1), rw = __shfl_up_sync(0xffffffffu, rc, 1);
+      if (lane == 0) {
+        qw = q[o + cw];
+        rw = rho[o + cw];
+      }
+      fw = u[o + c] * (rw + rc) * (qw + qc);
+      fe = __shfl_down_sync(0xffffffffu, fw, 1);
+    }
+    __syncthreads();  // (the buffer of two levels ago: every thread read it before the barrier in between)
+    if (mine) {
+      const T fn = sy[k & 1][row + 1][lane];
+      T dz = dzeta[k] * scale;
+      if (below_one(dz)) dz = (T)1;
+      const T rr = above_floor(rc) ? rc : (T)1e-12;
+      const T h = (fe - fw) * ax + (fn - fs) * ay;
+      const T z = (k > 0 && k + 1 < nz) ? (T)0.25 * (ft - fb) : (T)0;
+      dqdt[o + c] = -(h * dz + z) / (dz * rr);
+    }
+    qc = qt;
+    rc = rt;
+    fb = ft;
   }
 }
 
@@ -888,8 +921,16 @@ int flux_dev(const T* q, const T* rho, const T* u, const T* v, const T* w, const
   if (!q || !rho || !u || !v || !w || !dzeta || !dqdt || nx < 0 || ny < 0 || nz < 0) return VIBE_C_ERR_BAD_ARG;
   const size_t n = (size_t)nx * ny * nz;
   if (n == 0) return VIBE_C_OK;
-  const int blocks = (int)((n + 255) / 256 < 65535 ? (n + 255) / 256 : 65535);
-  k_flux_adv<T><<<blocks, 256, 0, (cudaStream_t)stream>>>(q, rho, u, v, w, dzeta, zs, nx, ny, nz, dx, dy, z_top, dqdt);
+  // level chunks for about 24 blocks an SM, so that the last wave weighs little,
+  // of at least 4 levels (a chunk computes its first lower face again)
+  const int xt = (nx + kFluxCols - 1) / kFluxCols;
+  const size_t tiles = (size_t)xt * ((ny + kFluxRows - 1) / kFluxRows);
+  const int want = tiles >= 3648 ? 1 : (int)(3648 / tiles);
+  int kz = (nz + want - 1) / want;
+  if (kz < 4) kz = 4;
+  if (kz < (nz + 65534) / 65535) kz = (nz + 65534) / 65535;
+  k_flux_adv<T><<<dim3((unsigned)tiles, (nz + kz - 1) / kz), dim3(32, kFluxRows + 1), 0, (cudaStream_t)stream>>>(
+      q, rho, u, v, w, dzeta, zs, nx, ny, nz, dx, dy, z_top, dqdt, xt, kz);
   return device_ok(cudaGetLastError(), "flux advection launch") ? VIBE_C_OK : VIBE_C_ERR_DEVICE;
 }
 
