@@ -661,3 +661,60 @@ def test_flux_advection_tile_edges(vg, oc, bits, dims):
                                              nx, ny, nz, 900.0, 1100.0, 20000.0, ref.ctypes.data)
         tol = 1e-12 if bits == 64 else 1e-4
         assert np.abs(out.double().cpu().numpy() - ref).max() <= tol * np.abs(ref).max() or np.abs(ref).max() == 0.0
+
+
+@pytest.mark.parametrize("kind", ["plain", "calm", "tiny", "huge", "nonfinite", "odd_metric"])
+@pytest.mark.parametrize("dims", [(1, 1, 1), (7, 5, 3), (129, 3, 17), (64, 40, 8)])
+def test_cfl_scan_bounds_change_no_bit(vg, oc, kind, dims):
+    """The FP32 bounds skip cells, never a maximum: the scan equals the oracle's
+    bit for bit on ordinary, resting, subnormal, overflowing and non-finite
+    winds and on a metric with negative and huge entries."""
+    nx, ny, nz = dims
+    n = nx * ny * nz
+    rng = np.random.default_rng(n)
+    u, v, w = (20.0 * rng.standard_normal(n) for _ in range(3))
+    dz, zs, dt = 0.01 + 0.02 * rng.random(nz), 500.0 * rng.random(nx * ny), 6.0
+    if kind == "calm":
+        u, v, w = np.zeros(n), np.zeros(n), np.zeros(n)
+    elif kind == "tiny":
+        u, v, w = (1e-40 * a for a in (u, v, w))
+        u[n // 2] = 1e-310
+    elif kind == "huge":
+        u, v, w = (10.0 ** rng.uniform(20, 150, n) * np.sign(a) for a in (u, v, w))
+    elif kind == "nonfinite":
+        u[n // 3], v[n // 2], w[n - 1] = np.nan, -np.inf, np.nan
+    elif kind == "odd_metric":
+        dz, zs = rng.standard_normal(nz) * 10.0 ** rng.uniform(-3, 3, nz), 40000.0 * rng.random(nx * ny)
+    with np.errstate(all="ignore"):
+        for step in (dt, -dt, 1e-40):
+            r, mw, mdz = vg.cfl_scan(u, v, w, dz, zs, nx, ny, nz, 900.0, 1100.0, 20000.0, step)
+            a, b = ctypes.c_double(), ctypes.c_double()
+            ro = oc.port_lib().vo_cfl_scan(u.ctypes.data, v.ctypes.data, w.ctypes.data, dz.ctypes.data, zs.ctypes.data,
+                                            nx, ny, nz, 900.0, 1100.0, 20000.0, step, ctypes.byref(a), ctypes.byref(b))
+            assert (r, mdz) == (ro, b.value), (step, r, ro, mdz, b.value)
+            assert mw == a.value or abs(mw - a.value) <= 2.3e-16 * a.value, (mw, a.value)  # the sum's FMA contraction
+
+
+@pytest.mark.parametrize("kind", ["narrow", "wide", "cancel", "subnormal", "rising"])
+@pytest.mark.parametrize("n", [1, 255, 4097, 300000])
+def test_neumaier_integer_sum(vg, kind, n):
+    """Sums whose exponents stay in, leave and move the integer accumulator's
+    window, against math.fsum: one rounding of the result plus the compensated
+    sum's second-order bound, 4 eps |s| + 4 n eps^2 sum|x|."""
+    import math
+    rng = np.random.default_rng(n)
+    x = rng.standard_normal(n)
+    if kind == "wide":
+        x = x * 10.0 ** rng.uniform(-150, 150, n)
+    elif kind == "cancel":
+        x = x * 10.0 ** rng.uniform(0, 30, n)
+        x[n // 2:2 * (n // 2)] = -x[:n // 2]
+    elif kind == "subnormal":
+        x = x * 1e-310
+    elif kind == "rising":
+        x = np.sort(np.abs(x) * 10.0 ** rng.uniform(-300, 300, n))
+    got, ref = vg.neumaier_sum(x), math.fsum(x)
+    eps = 2.0 ** -52
+    assert abs(got - ref) <= 4 * eps * abs(ref) + 4 * n * eps * eps * np.abs(x).sum() + 5e-324, (got, ref)
+    x[n // 2] = np.inf  # the compensation of an infinite sum is inf - inf, as in the reference
+    assert np.isnan(vg.neumaier_sum(x))

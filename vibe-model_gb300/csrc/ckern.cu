@@ -484,15 +484,19 @@ __device__ __forceinline__ Neu<T> neu_merge(Neu<T> a, Neu<T> b) {
   a.c += b.c;
   return a;
 }
+constexpr int kNeuThreads = 256;
 template <typename T>
 __device__ Neu<T> neu_block(Neu<T> v) {
   __shared__ T sh_s[32], sh_c[32];
-  for (int off = 16; off > 0; off >>= 1) {
-    Neu<T> o;
-    o.s = __shfl_down_sync(0xffffffffu, v.s, off);
-    o.c = __shfl_down_sync(0xffffffffu, v.c, off);
-    v = neu_merge(v, o);
-  }
+  // (lanes with empty pairs, as the integer sums leave them, need no merging)
+  const bool lane0 = (threadIdx.x & 31) == 0;
+  if (__any_sync(0xffffffffu, !lane0 && (v.s != (T)0 || v.c != (T)0)))
+    for (int off = 16; off > 0; off >>= 1) {
+      Neu<T> o;
+      o.s = __shfl_down_sync(0xffffffffu, v.s, off);
+      o.c = __shfl_down_sync(0xffffffffu, v.c, off);
+      v = neu_merge(v, o);
+    }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (lane == 0) { sh_s[warp] = v.s; sh_c[warp] = v.c; }
   __syncthreads();
@@ -509,12 +513,121 @@ __device__ Neu<T> neu_block(Neu<T> v) {
   }
   return v;
 }
+// Exact sum of doubles in integers: each lane's 128-bit fixed-point accumulator
+// holds multiples of 2^(base - 1075) of elements whose exponent field lies in
+// [base, base + 54]; an element is its 53-bit mantissa shifted by its exponent
+// over the base, ~20 integer instructions where Neumaier's addition takes six
+// on the FP64 pipe, which issues 1/32 of the integer rate here. The window is
+// common to the warp, so the lanes' accumulators add up in integers too: the
+// FP64 work is one conversion per warp. 107 bits leave 2^20 additions of
+// headroom, 2^13 a lane and 2^5 for the lanes used. Elements above the window
+// move it (the accumulators go to the lanes' compensated pairs first);
+// elements below it, subnormals, infinities and NaN are added to the lane's
+// pair as before. value() is exact to the two doubles of a pair.
+struct ExactSum {
+  static constexpr int kSpan = 54, kAbove = 8, kRounds = 1024;
+  unsigned long long lo = 0;
+  long long hi = 0;
+  int base = 1 << 20;  // no window yet
+  __device__ __forceinline__ void plus(unsigned long long l, long long h) {
+    const unsigned long long t = lo + l;
+    hi += h + (long long)(t < lo);
+    lo = t;
+  }
+  __device__ __forceinline__ Neu<double> value() const {
+    Neu<double> v{0.0, 0.0};
+    if (lo == 0 && hi == 0) return v;
+    const bool neg = hi < 0;
+    unsigned long long l = lo, h = (unsigned long long)hi;
+    if (neg) {
+      l = ~l + 1;
+      h = ~h + (l == 0);
+    }
+    // three parts of at most 43 bits, each an exact double
+    const double p[3] = {(double)(l & 0x7ffffffffffull), (double)((l >> 43) | ((h & 0x3fffffull) << 21)),
+                         (double)(h >> 22)};
+    const int w[3] = {0, 43, 86};
+    for (int q = 2; q >= 0; --q) {
+      if (p[q] == 0.0) continue;
+      const double x = ldexp(p[q], base - 1075 + w[q]);
+      neu_add(v, neg ? -x : x);
+    }
+    return v;
+  }
+  __device__ __forceinline__ void flush(Neu<double>& pair) {
+    pair = neu_merge(pair, value());
+    lo = 0;
+    hi = 0;
+  }
+  static __device__ __forceinline__ int exponent(double x) { return (__double2hiint(x) >> 20) & 0x7ff; }
+  // top: the warp's largest finite exponent field among the elements to come
+  __device__ __forceinline__ void window(int top, Neu<double>& pair) {
+    if (top == 0 || (unsigned)(top - base) <= (unsigned)kSpan || (top < base && base < 4096)) return;
+    flush(pair);
+    base = top + kAbove - kSpan;
+  }
+  __device__ __forceinline__ void add(double x, Neu<double>& pair) {
+    const unsigned long long bits = (unsigned long long)__double_as_longlong(x);
+    const int ef = exponent(x);
+    const unsigned s = (unsigned)(ef - base);
+    if (s > (unsigned)kSpan || ef == 0) {
+      if (bits << 1) neu_add(pair, x);  // (a zero adds nothing)
+      return;
+    }
+    const unsigned long long m = (bits & 0xfffffffffffffull) | 0x10000000000000ull;
+    const unsigned long long sg = (unsigned long long)((long long)bits >> 63);  // all ones for negative elements
+    // two's complement: the inverted bits of a negative element, and one
+    plus((m << s) ^ sg, (long long)(((m >> 1) >> (63 - s)) ^ sg));
+    plus(sg & 1, 0);
+  }
+};
 // each block sums a contiguous chunk; partials[2*block] = (s, c)
 template <typename T>
-__global__ void k_neu_partial(const T* __restrict__ x, size_t n, size_t chunk, T* __restrict__ partials) {
+__global__ void __launch_bounds__(kNeuThreads) k_neu_partial(const T* __restrict__ x, size_t n, size_t chunk,
+                                                             T* __restrict__ partials) {
   const size_t lo = (size_t)blockIdx.x * chunk, hi = lo + chunk < n ? lo + chunk : n;
   Neu<T> v{(T)0, (T)0};
-  for (size_t e = lo + threadIdx.x; e < hi; e += blockDim.x) neu_add(v, x[e]);
+  constexpr int kU = 8;  // loads in flight per thread
+  if constexpr (sizeof(T) == 8) {
+    ExactSum acc;
+    int rounds = 0;
+    for (size_t e0 = lo; e0 < hi; e0 += kU * kNeuThreads) {  // the same trips for every lane
+      T q[kU];
+      int top = 0;
+#pragma unroll
+      for (int m = 0; m < kU; ++m) {
+        const size_t e = e0 + m * kNeuThreads + threadIdx.x;
+        q[m] = e < hi ? x[e] : (T)0;
+      }
+#pragma unroll
+      for (int m = 0; m < kU; ++m) {
+        const int ef = ExactSum::exponent(q[m]);
+        top = max(top, ef == 0x7ff ? 0 : ef);
+      }
+      acc.window(__reduce_max_sync(0xffffffffu, top), v);
+      if (++rounds == ExactSum::kRounds) {
+        acc.flush(v);
+        rounds = 0;
+      }
+#pragma unroll
+      for (int m = 0; m < kU; ++m) acc.add(q[m], v);
+    }
+    for (int off = 16; off > 0; off >>= 1)  // lane 0 gets the warp's sum
+      acc.plus(__shfl_down_sync(0xffffffffu, acc.lo, off), __shfl_down_sync(0xffffffffu, acc.hi, off));
+    // the warps' sums, one per lane of the first warp: one conversion for all
+    __shared__ ExactSum part[kNeuThreads / 32];
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = acc;
+    __syncthreads();
+    if (threadIdx.x < kNeuThreads / 32) part[threadIdx.x].flush(v);
+  } else {
+    for (size_t e0 = lo + threadIdx.x; e0 < hi; e0 += kU * kNeuThreads) {
+      T q[kU];
+#pragma unroll
+      for (int m = 0; m < kU; ++m) q[m] = e0 + m * kNeuThreads < hi ? x[e0 + m * kNeuThreads] : (T)0;
+#pragma unroll
+      for (int m = 0; m < kU; ++m) neu_add(v, q[m]);
+    }
+  }
   v = neu_block(v);
   if (threadIdx.x == 0) { partials[2 * blockIdx.x] = v.s; partials[2 * blockIdx.x + 1] = v.c; }
 }
@@ -526,6 +639,7 @@ __global__ void k_neu_final(const T* __restrict__ partials, int nb, T* __restric
   if (threadIdx.x == 0) *out = v.s + v.c;
 }
 
+constexpr int kCflThreads = 256;
 // CFL scan (c_kernels.c:148-186): per cell dz = max(dzeta[k]*scale, 1),
 // speed = sqrt(u^2+v^2+w^2), cfl = dt*(|u|/dx + |v|/dy + |w|/dz); block maxima
 // of (cfl, speed) and min of dz, then one block merges.
@@ -551,36 +665,130 @@ __device__ __forceinline__ void max3_block(T& a, T& b, T& c) {  // max, max, min
     }
   }
 }
+// Most cells cannot raise a maximum, and finding that out in FP64 costs three
+// divisions a cell. So a cell's CFL number and squared speed are first bounded
+// from above in FP32 (within 2.1e-5), from the doubles' upper bits (integer
+// instructions; a conversion would issue at the FP64 rate). A cell is evaluated
+// in FP64 only if its bound exceeds the block's best so far and is not so far
+// under the largest bound of the block's tile that the cell holding that one
+// must win: a handful of cells per block. The maxima are those of the FP64
+// values, bit for bit. The bounds assume ordinary positive dt, dx, dy
+// (`plain`); else, and where a bound is not finite, cells are evaluated.
+// The minimum of dz over a column is dz at the smallest (or, where the column's
+// depth is negative, the largest) dzeta: a product rounds monotonically.
+__device__ __forceinline__ float trunc_abs(double x) {  // |x| rounded toward zero; tiny values up to 2^-126
+  const unsigned h = (unsigned)__double2hiint(x) & 0x7fffffffu, l = (unsigned)__double2loint(x);
+  if (h >= 0x47f00000u) return __int_as_float(0x7f800000);
+  if (h < 0x38100000u) return (h | l) ? 1.17549435e-38f : 0.f;
+  return __uint_as_float(((h - 0x38000000u) << 3) | (l >> 29));
+}
+__device__ __forceinline__ float trunc_abs(float x) { return fabsf(x); }
+__device__ __forceinline__ float trunc_signed(double x) {  // rounded toward zero; NaN and 2^128 up: NaN, infinity
+  const int h = __double2hiint(x), m = h & 0x7fffffff;
+  float f = m < 0x38100000 ? 0.f : trunc_abs(x);
+  if (m > 0x7ff00000 || (m == 0x7ff00000 && __double2loint(x))) f = __int_as_float(0x7fc00000);
+  return copysignf(f, __int_as_float(h));
+}
+__device__ __forceinline__ float trunc_signed(float x) { return x; }
+__device__ __forceinline__ unsigned down_bits(double x) { return __float_as_uint(__double2float_rd(x)); }
+__device__ __forceinline__ unsigned down_bits(float x) { return __float_as_uint(x); }
+constexpr int kCflLevels = 4;  // levels of one tile
 template <typename T>
-__global__ void k_cfl_partial(const T* __restrict__ u, const T* __restrict__ v, const T* __restrict__ w,
-                              const T* __restrict__ dzeta, const T* __restrict__ zs, int nx, int ny, int nz, T dx, T dy,
-                              T z_top, T dt, T* __restrict__ partials) {
-  const size_t n = (size_t)nx * ny * nz, nxy = (size_t)nx * ny;  // (no negative dimension reaches here)
+__global__ void __launch_bounds__(kCflThreads, 4) k_cfl_partial(const T* __restrict__ u, const T* __restrict__ v,
+                                                             const T* __restrict__ w, const T* __restrict__ dzeta,
+                                                             const T* __restrict__ zs, int nx, int ny, int nz, T dx,
+                                                             T dy, T z_top, T dt, size_t tiles,
+                                                             T* __restrict__ partials) {
+  const size_t nxy = (size_t)nx * ny;  // (no negative dimension reaches here)
+  const size_t ctiles = (nxy + kCflThreads - 1) / kCflThreads;
+  const bool plain = dt >= (T)1e-30 && dt <= (T)1e30 && dx >= (T)1e-30 && dx <= (T)1e30 && dy >= (T)1e-30 && dy <= (T)1e30;
+  const float up = 1.00002f;  // above the rounding of the bounds (a few 1e-6)
+  const float bdt = (float)dt * up, bdx = 1.f / (float)dx, bdy = 1.f / (float)dy;
   // the largest squared speed, one square root at the end: a correctly
   // rounded square root is monotone, so the maximum of the roots is the root
   // of the maximum, bit for bit
   T worst = 0, mw2 = 0, mdz = (T)1e30;
-  const size_t S = (size_t)gridDim.x * blockDim.x;
-  size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-  if (e < n) {
-    // the cell's level and column, stepped along with e (no division per cell)
-    size_t k = e / nxy, col = e - k * nxy;
-    const size_t sk = S / nxy, sc = S - sk * nxy;
-    for (; e < n; e += S) {
-      const T uu = u[e], vv = v[e], ww = w[e];
-      const T scale = zs ? (z_top - zs[col]) : z_top;
-      T dz = dzeta[k] * scale;
+  // best[0..1]: the block's maxima of the two, rounded down, as float bits
+  // (non-negative floats order as their bits); seen[..]: a tile's largest bounds
+  __shared__ unsigned best[2], seen[2][2];
+  if (threadIdx.x < 2) best[threadIdx.x] = seen[0][threadIdx.x] = 0u;
+  __syncthreads();
+  int par = 0;
+  T dlo = (T)NAN, dhi = (T)NAN;
+  for (int k = threadIdx.x & 31; k < nz; k += 32) {
+    dlo = fmin(dlo, dzeta[k]);
+    dhi = fmax(dhi, dzeta[k]);
+  }
+  for (int off = 16; off > 0; off >>= 1) {
+    dlo = fmin(dlo, __shfl_xor_sync(0xffffffffu, dlo, off));
+    dhi = fmax(dhi, __shfl_xor_sync(0xffffffffu, dhi, off));
+  }
+  for (size_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    const size_t kt = tile / ctiles, col = (tile - kt * ctiles) * kCflThreads + threadIdx.x;
+    const int k0 = (int)kt * kCflLevels;
+    const bool in = col < nxy;
+    const T scale = zs ? (in ? z_top - zs[col] : (T)1) : z_top;
+    const float fscale = (float)scale;
+    if (in && k0 == 0) {
+      T dz = fmin(dlo * scale, dhi * scale);
       if (dz < (T)1) dz = (T)1;
       mdz = fmin(mdz, dz);
-      mw2 = fmax(mw2, uu * uu + vv * vv + ww * ww);
-      worst = fmax(worst, dt * (fabs(uu) / dx + fabs(vv) / dy + fabs(ww) / dz));
-      col += sc;
-      k += sk;
-      if (col >= nxy) {
-        col -= nxy;
-        ++k;
+    }
+    T qu[kCflLevels], qv[kCflLevels], qw[kCflLevels];
+#pragma unroll
+    for (int m = 0; m < kCflLevels; ++m) {
+      const size_t e = (size_t)(k0 + m) * nxy + col;
+      const bool on = in && k0 + m < nz;
+      qu[m] = on ? u[e] : (T)0;
+      qv[m] = on ? v[e] : (T)0;
+      qw[m] = on ? w[e] : (T)0;
+    }
+    float ec[kCflLevels], es[kCflLevels], tc = 0.f, ts = 0.f;
+#pragma unroll
+    for (int m = 0; m < kCflLevels; ++m) {
+      const int k = k0 + m < nz ? k0 + m : nz - 1;
+      const float fu = trunc_abs(qu[m]), fv = trunc_abs(qv[m]), fw = trunc_abs(qw[m]);
+      const float some = (fu + fv + fw > 0.f) ? 1e-36f : 0.f;  // products below 2^-126 count as that much
+      float fdz = trunc_signed(dzeta[k]) * fscale;
+      if (fdz < 1.f) fdz = 1.f;
+      ec[m] = bdt * (fu * bdx + fv * bdy + fw * __frcp_rn(fdz)) + some;
+      if (fdz > 3e38f) ec[m] = __int_as_float(0x7f800000);  // out of FP32's range: no bound
+      es[m] = up * (fu * fu + fv * fv + fw * fw) + some;
+      tc = fmaxf(tc, ec[m]);
+      ts = fmaxf(ts, es[m]);
+    }
+    if (plain) {
+      const unsigned wc = __reduce_max_sync(0xffffffffu, __float_as_uint(tc));
+      const unsigned ws = __reduce_max_sync(0xffffffffu, __float_as_uint(ts));
+      if ((threadIdx.x & 31) == 0) {
+        atomicMax(&seen[par][0], wc);
+        atomicMax(&seen[par][1], ws);
       }
     }
+    __syncthreads();
+    // (another warp may raise best meanwhile: any value read is a maximum already reached)
+    const float bc = __uint_as_float(best[0]), bs = __uint_as_float(best[1]);
+    const float mc = __uint_as_float(seen[par][0]), ms = __uint_as_float(seen[par][1]);
+    // under these a cell cannot be the tile's maximum (no such limit where a bound is tiny or not finite)
+    const float lc = (mc > 1e-30f && mc < 3e38f) ? mc * 0.99995f : 0.f, ls = (ms > 1e-30f && ms < 3e38f) ? ms * 0.99995f : 0.f;
+    if (threadIdx.x < 2) seen[par ^ 1][threadIdx.x] = 0u;
+#pragma unroll
+    for (int m = 0; m < kCflLevels; ++m) {
+      const int k = k0 + m;
+      const T uu = qu[m], vv = qv[m], ww = qw[m];
+      if (in && k < nz && (!plain || (!(ec[m] <= bc) && !(ec[m] < lc)))) {
+        T dz = dzeta[k] * scale;
+        if (dz < (T)1) dz = (T)1;
+        worst = fmax(worst, dt * (fabs(uu) / dx + fabs(vv) / dy + fabs(ww) / dz));
+        atomicMax(&best[0], down_bits(worst));
+      }
+      if (in && k < nz && (!plain || (!(es[m] <= bs) && !(es[m] < ls)))) {
+        mw2 = fmax(mw2, uu * uu + vv * vv + ww * ww);
+        atomicMax(&best[1], down_bits(mw2));
+      }
+    }
+    par ^= 1;
+    __syncthreads();  // seen[par] is clear, best is settled
   }
   T mw = sqrt(mw2);
   max3_block(worst, mw, mdz);
@@ -700,8 +908,8 @@ static __device__ __align__(256) double g_noalloc_thomas_work[kNoAllocThomasDoub
 std::mutex g_noalloc_mu;
 double* g_noalloc_ptr[64] = {};
 
-constexpr int kRedBlocks = 304;  // 2 x 152 SMs
 constexpr int kRedThreads = 256;
+constexpr int kNeuBlocks = 608, kCflBlocks = 608;  // 4 x 152 SMs
 
 // ---- entry points, one template per ABI function: T = double (the
 // reference's *_f64 names) or float (the *_f32 twins its header reserves,
@@ -839,8 +1047,11 @@ T bilinear_host(const T* f, int halo, int nsx, int nsy, int nz, T xi, T yj, int 
 template <typename T>
 int cfl_launch(const T* u, const T* v, const T* w, const T* dzeta, const T* zs, int nx, int ny, int nz, T dx, T dy,
                T z_top, T dt, T* out3, T* part, cudaStream_t st) {
-  k_cfl_partial<T><<<kRedBlocks, kRedThreads, 0, st>>>(u, v, w, dzeta, zs, nx, ny, nz, dx, dy, z_top, dt, part);
-  k_cfl_final<T><<<1, kRedThreads, 0, st>>>(part, kRedBlocks, out3);
+  const size_t ctiles = ((size_t)nx * ny + kCflThreads - 1) / kCflThreads;
+  const size_t tiles = ctiles * (((size_t)nz + kCflLevels - 1) / kCflLevels);
+  const int nb = (int)(tiles < 1 ? 1 : tiles < (size_t)kCflBlocks ? tiles : (size_t)kCflBlocks);
+  k_cfl_partial<T><<<nb, kCflThreads, 0, st>>>(u, v, w, dzeta, zs, nx, ny, nz, dx, dy, z_top, dt, tiles, part);
+  k_cfl_final<T><<<1, kRedThreads, 0, st>>>(part, nb, out3);
   return device_ok(cudaGetLastError(), "cfl launch") ? VIBE_C_OK : VIBE_C_ERR_DEVICE;
 }
 
@@ -848,7 +1059,7 @@ template <typename T>
 int cfl_dev(const T* u, const T* v, const T* w, const T* dzeta, const T* zs, int nx, int ny, int nz, T dx, T dy,
             T z_top, T dt, T* out3, vibe_stream_t stream) {
   if (!u || !v || !w || !dzeta || !out3 || nx < 0 || ny < 0 || nz < 0) return VIBE_C_ERR_BAD_ARG;
-  DevScratch part((size_t)3 * kRedBlocks * sizeof(T), (cudaStream_t)stream);
+  DevScratch part((size_t)3 * kCflBlocks * sizeof(T), (cudaStream_t)stream);
   if (!part.get()) return VIBE_C_ERR_DEVICE;
   int rc = cfl_launch<T>(u, v, w, dzeta, zs, nx, ny, nz, dx, dy, z_top, dt, out3, (T*)part.get(),
                          (cudaStream_t)stream);
@@ -872,7 +1083,7 @@ T cfl_host(const T* u, const T* v, const T* w, const T* dzeta, const T* zs, int 
   const int iu = hc.add(u, n * e, HostCall::kIn), iv = hc.add(v, n * e, HostCall::kIn),
             iw = hc.add(w, n * e, HostCall::kIn), iz = hc.add(dzeta, nzp * e, HostCall::kIn),
             izs = hc.add(zs, zs ? nxy * e : 0, HostCall::kIn), io = hc.add(r, 3 * e, HostCall::kOut),
-            ip = hc.add(nullptr, (size_t)3 * kRedBlocks * e, HostCall::kScratch);
+            ip = hc.add(nullptr, (size_t)3 * kCflBlocks * e, HostCall::kScratch);
   bool ok = hc.commit();
   ok = ok && cfl_launch<T>(hc.dev<T>(iu), hc.dev<T>(iv), hc.dev<T>(iw), hc.dev<T>(iz), hc.dev<T>(izs), nx, ny, nz, dx,
                            dy, z_top, dt, hc.dev<T>(io), hc.dev<T>(ip), hc.stream()) == VIBE_C_OK;
@@ -885,16 +1096,19 @@ T cfl_host(const T* u, const T* v, const T* w, const T* dzeta, const T* zs, int 
 
 template <typename T>
 int neu_launch(const T* x, size_t n, T* out, T* part, cudaStream_t st) {
-  const size_t chunk = (n + kRedBlocks - 1) / kRedBlocks;
-  k_neu_partial<T><<<kRedBlocks, kRedThreads, 0, st>>>(x, n, chunk > 0 ? chunk : 1, part);
-  k_neu_final<T><<<1, kRedThreads, 0, st>>>(part, kRedBlocks, out);
+  // blocks of at least 2048 elements (8 a thread), at most kNeuBlocks
+  const size_t want = (n + 2047) / 2048;
+  const int nb = (int)(want < 1 ? 1 : want < (size_t)kNeuBlocks ? want : (size_t)kNeuBlocks);
+  const size_t chunk = (n + nb - 1) / nb;
+  k_neu_partial<T><<<nb, kNeuThreads, 0, st>>>(x, n, chunk > 0 ? chunk : 1, part);
+  k_neu_final<T><<<1, kRedThreads, 0, st>>>(part, nb, out);
   return device_ok(cudaGetLastError(), "neumaier launch") ? VIBE_C_OK : VIBE_C_ERR_DEVICE;
 }
 
 template <typename T>
 int neu_dev(const T* x, size_t n, T* out, vibe_stream_t stream) {
   if (!x || !out) return VIBE_C_ERR_BAD_ARG;
-  DevScratch part((size_t)2 * kRedBlocks * sizeof(T), (cudaStream_t)stream);
+  DevScratch part((size_t)2 * kNeuBlocks * sizeof(T), (cudaStream_t)stream);
   if (!part.get()) return VIBE_C_ERR_DEVICE;
   int rc = neu_launch<T>(x, n, out, (T*)part.get(), (cudaStream_t)stream);
   if (!part.release() && rc == VIBE_C_OK) rc = VIBE_C_ERR_DEVICE;
@@ -908,7 +1122,7 @@ T neu_host(const T* x, size_t n) {
   T r = (T)NAN;
   HostCall hc;
   const int ix = hc.add(x, n * e, HostCall::kIn), io = hc.add(&r, e, HostCall::kOut),
-            ip = hc.add(nullptr, (size_t)2 * kRedBlocks * e, HostCall::kScratch);
+            ip = hc.add(nullptr, (size_t)2 * kNeuBlocks * e, HostCall::kScratch);
   bool ok = hc.commit();
   ok = ok && neu_launch<T>(hc.dev<T>(ix), n, hc.dev<T>(io), hc.dev<T>(ip), hc.stream()) == VIBE_C_OK;
   ok = hc.finish() && ok;
