@@ -108,6 +108,7 @@ struct vibe_gb300_model {
   double* wface = nullptr;  // FP64 path: WENO face fluxes of one scalar
   double *d_dzeta = nullptr, *d_scale = nullptr, *d_sponge = nullptr;
   double *d_th0 = nullptr, *d_pi0 = nullptr, *d_rho0 = nullptr;
+  double *d_inv_dzeta = nullptr, *d_inv_scale = nullptr, *d_inv_th0 = nullptr;
   double* d_stage_in = nullptr;   // staging for FieldT <-> device layout
   double* d_tri = nullptr;        // reference HEVI coefficients (3*nz)
   float* W0[NSPECIES] = {};
@@ -376,6 +377,12 @@ template <class T>
 void unpack(const Dims& d, int nsx, int nsy, int nsz, int ni, int nj, int nk, const T* src, double* dst,
             cudaStream_t s) {
   k_unpack_t<T><<<dim3((nsx + 31) / 32, (nsy + 7) / 8, nsz), dim3(32, 8), 0, s>>>(d, nsx, nsy, ni, nj, nk, src, dst);
+}
+
+// 1 / max(x, 1)
+__global__ void k_inv_floor1(size_t n, const double* __restrict__ x, double* __restrict__ out) {
+  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x)
+    out[e] = 1.0 / dmax(x[e], 1.0);
 }
 
 // rigid ground and lid (w_rigid): w = 0 on the k = 0 and k = nz faces
@@ -1065,6 +1072,9 @@ int vibe_gb300_model_create(const vibe_gb300_setup* s, int precision, vibe_gb300
   rc = rc ? rc : dalloc(m, &m->d_th0, nfield);
   rc = rc ? rc : dalloc(m, &m->d_pi0, nfield);
   rc = rc ? rc : dalloc(m, &m->d_rho0, nfield);
+  rc = rc ? rc : dalloc(m, &m->d_inv_dzeta, (size_t)nz);
+  rc = rc ? rc : dalloc(m, &m->d_inv_scale, (size_t)nx * ny);
+  rc = rc ? rc : dalloc(m, &m->d_inv_th0, nfield);
   rc = rc ? rc : dalloc(m, &m->d_err, (size_t)1);
   rc = rc ? rc : dalloc(m, &m->d_tri, 3 * (size_t)nz);
   if (!rc && precision == VIBE_GB300_FP64) {
@@ -1094,6 +1104,12 @@ int vibe_gb300_model_create(const vibe_gb300_setup* s, int precision, vibe_gb300
       cudaMemcpy(m->d_scale, sc.data(), sc.size() * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess ||
       cudaMemcpy(m->d_sponge, m->hs.sponge.data(), nz * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess)
     return bail(fail(VIBE_GB300_EDEVICE, "metric upload failed"));
+  for (double& v : dz) v = 1.0 / v;
+  for (double& v : sc) v = 1.0 / v;
+  if (cudaMemcpy(m->d_inv_dzeta, dz.data(), nz * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess ||
+      cudaMemcpy(m->d_inv_scale, sc.data(), sc.size() * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess)
+    return bail(fail(VIBE_GB300_EDEVICE, "metric upload failed"));
+  m->met.inv_dzeta = m->d_inv_dzeta; m->met.inv_scale = m->d_inv_scale; m->met.inv_th0 = m->d_inv_th0;
   m->met.dx = s->dx; m->met.dy = s->dy; m->met.z_top = s->z_top;
   m->met.inv_dx = 1.0 / s->dx; m->met.inv_dy = 1.0 / s->dy;
   m->met.dzeta = m->d_dzeta; m->met.scale = m->d_scale; m->met.sponge = m->d_sponge;
@@ -1103,6 +1119,7 @@ int vibe_gb300_model_create(const vibe_gb300_setup* s, int precision, vibe_gb300
     dst[0] = m->d_th0;
     if ((rc = upload_storage(m, RHO, m->hs.ref[0].data(), dst, 1))) return bail(rc);
     CUDA_OK(cudaStreamSynchronize(m->stream));
+    k_inv_floor1<<<1024, 256, 0, m->stream>>>(nfield, m->d_th0, m->d_inv_th0);
     dst[0] = m->d_pi0;
     if ((rc = upload_storage(m, RHO, m->hs.ref[1].data(), dst, 1))) return bail(rc);
     CUDA_OK(cudaStreamSynchronize(m->stream));
@@ -2625,7 +2642,7 @@ int stl_substeps(vibe_gb300_model* m, int stage, double dtau, int n_sub, double*
 // diagonal, so each is its own adjoint)
 int stl_sponge_rigid(vibe_gb300_model* m, double dt, double* const* x) {
   Metric mz = m->met;
-  mz.th0 = mz.pi0 = mz.rho0 = m->stl_zero;
+  mz.th0 = mz.pi0 = mz.rho0 = m->stl_zero;  // (the sponge reads nothing else of the metric but its profile)
   m->f64->sponge(m->d, mz, x, m->kmin, dt, m->stream);
   if (m->fl.w_rigid)
     k_rigid_w<<<dim3((m->d.nx + 31) / 32, (m->d.ny + 7) / 8), dim3(32, 8), 0, m->stream>>>(m->d, x[W]);

@@ -93,38 +93,40 @@ __device__ inline double weno_face(double qm2, double qm1, double q0, double q1,
   return 0.5 * (vel * (ql + qr) - alpha * (qr - ql));
 }
 #else
-// The same face flux with the arithmetic arranged for the FP64 pipe: the
-// right-biased reconstruction is the left-biased one of the reversed
-// stencil (same three smoothness indicators, reversed), the weights
-// a_k = d_k / s_k^2 (s_k = eps + beta_k) are normalised with one division
-// by scaling numerator and denominator with (s0 s1 s2)^2, the 1/6 is a
-// multiplication, and for |vel| >= 1e-3 the Lax-Friedrichs flux
+// The same face flux with the arithmetic arranged for the FP64 pipe. All is
+// written in the four differences of the stencil: the right-biased
+// reconstruction is the left-biased one of the reversed stencil (the same
+// differences, reversed and negated, and the same three smoothness
+// indicators, reversed), taken relative to the centre value; the weights
+// a_k = d_k / s_k^2 (s_k = 4 (eps + beta_k), whose factor cancels) are
+// normalised with one division by scaling numerator and denominator with
+// (s0 s1 s2)^2; and for |vel| >= 1e-3 the Lax-Friedrichs flux
 // 0.5*(vel*(ql+qr) - |vel|*(qr-ql)) is vel times the upwind reconstruction
-// alone. Equal to the reference's to rounding.
-__device__ inline double weno_left_d(double qm2, double qm1, double q0, double q1, double q2, double s0, double s1,
-                                     double s2) {
-  const double sixth = 1.0 / 6.0;
-  const double v0 = (2.0 * qm2 - 7.0 * qm1 + 11.0 * q0) * sixth;
-  const double v1 = (-qm1 + 5.0 * q0 + 2.0 * q1) * sixth;
-  const double v2 = (2.0 * q0 + 5.0 * q1 - q2) * sixth;
+// alone: about 48 FP64 operations a face. A flat stencil, whose reconstruction
+// is its value, takes none of them: most of the moisture fields of most
+// atmospheres are zero. Equal to the reference's to rounding.
+__device__ inline double weno_left_d(double d1, double d2, double d3, double d4, double s0, double s1, double s2) {
+  const double v0 = 5.0 * d2 - 2.0 * d1, v1 = d2 + 2.0 * d3, v2 = 4.0 * d3 - d4;  // 6 (v_k - q0)
   const double p01 = s0 * s1, p02 = s0 * s2, p12 = s1 * s2;
-  const double w0 = 0.1 * (p12 * p12), w1 = 0.6 * (p02 * p02), w2 = 0.3 * (p01 * p01);
-  return (w0 * v0 + w1 * v1 + w2 * v2) / (w0 + w1 + w2);
+  const double w0 = (0.1 * p12) * p12, w1 = (0.6 * p02) * p02, w2 = (0.3 * p01) * p01;
+  return (w0 * v0 + w1 * v1 + w2 * v2) / (6.0 * (w0 + w1 + w2));
 }
 __device__ inline double weno_face(double qm2, double qm1, double q0, double q1, double q2, double vel) {
-  const double eps = 1e-6;
-  const double e0 = qm2 - 2.0 * qm1 + q0, f0 = qm2 - 4.0 * qm1 + 3.0 * q0;
-  const double e1 = qm1 - 2.0 * q0 + q1, f1 = qm1 - q1;
-  const double e2 = q0 - 2.0 * q1 + q2, f2 = 3.0 * q0 - 4.0 * q1 + q2;
-  const double s0 = eps + (13.0 / 12.0) * (e0 * e0) + 0.25 * (f0 * f0);
-  const double s1 = eps + (13.0 / 12.0) * (e1 * e1) + 0.25 * (f1 * f1);
-  const double s2 = eps + (13.0 / 12.0) * (e2 * e2) + 0.25 * (f2 * f2);
+  const double d1 = qm1 - qm2, d2 = q0 - qm1, d3 = q1 - q0, d4 = q2 - q1;
+  const long long flat = __double_as_longlong(d1) | __double_as_longlong(d2) | __double_as_longlong(d3) |
+                         __double_as_longlong(d4);
+  if ((flat << 1) == 0) return vel * q0;
+  const double e0 = d2 - d1, e1 = d3 - d2, e2 = d4 - d3;
+  const double f0 = e0 + 2.0 * d2, f1 = d2 + d3, f2 = e2 - 2.0 * d3;
+  const double s0 = f0 * f0 + (4e-6 + ((13.0 / 3.0) * e0) * e0);
+  const double s1 = f1 * f1 + (4e-6 + ((13.0 / 3.0) * e1) * e1);
+  const double s2 = f2 * f2 + (4e-6 + ((13.0 / 3.0) * e2) * e2);
   const bool up = vel >= 0.0;
-  const double a0 = up ? qm2 : q2, a1 = up ? qm1 : q1, a3 = up ? q1 : qm1, a4 = up ? q2 : qm2;
-  const double t0 = up ? s0 : s2, t2 = up ? s2 : s0;
-  const double rec = weno_left_d(a0, a1, q0, a3, a4, t0, s1, t2);
+  const double rec = q0 + weno_left_d(up ? d1 : -d4, up ? d2 : -d3, up ? d3 : -d2, up ? d4 : -d1, up ? s0 : s2, s1,
+                                      up ? s2 : s0);
   if (fabs(vel) >= 1e-3) return vel * rec;
-  const double oth = weno_left_d(a4, a3, q0, a1, a0, t2, s1, t0);
+  const double oth = q0 + weno_left_d(up ? -d4 : d1, up ? -d3 : d2, up ? -d2 : d3, up ? -d1 : d4, up ? s2 : s0, s1,
+                                      up ? s0 : s2);
   const double ql = up ? rec : oth, qr = up ? oth : rec;
   return 0.5 * (vel * (ql + qr) - 1e-3 * (qr - ql));
 }
@@ -196,10 +198,26 @@ __device__ inline double ac_w(const CS& s, const Metric& m, const Dims& d, const
   return -kCp * t0 * dpi(s, m, d, fl, i, j, kc, i, j, km) / dz;
 }
 
+#ifndef VGB_FP64_EXACT
+// 1 / (dzeta(k) scale(i, j)) and the spacing's 1 m floor
+__device__ inline double idz_at(const Metric& m, const Dims& d, int i, int j, int k) {
+  return m.inv_dzeta[iclamp(k, 0, d.nz - 1)] * m.inv_scale[(size_t)iclamp(j, 0, d.ny - 1) * d.nx + iclamp(i, 0, d.nx - 1)];
+}
+__device__ inline double floor1(double idz) { return idz > 1.0 ? 1.0 : idz; }  // 1 / max(dz, 1)
+// theta less what split_fast moves to the substeps, pi or pi'
+__device__ inline double th_slow(const CS& s, const Metric& m, const Flags& fl, size_t c) {
+  return fl.split_fast ? s.f[THETA][c] - m.th0[c] : s.f[THETA][c];
+}
+__device__ inline double pi_grad(const CS& s, const Metric& m, const Flags& fl, size_t c) {
+  return fl.pgf_pert ? s.f[PI][c] - m.pi0[c] : s.f[PI][c];
+}
+#endif
+
 // ---- slow tendencies, equations.cpp:60-150 -------------------------------
 
 // u faces: Advection::momentum u-part (advection.cpp:260-278), Coriolis
 // (coriolis.cpp:51-59), PGF (equations.cpp:72-80) [- acoustic u if split].
+#ifdef VGB_FP64_EXACT
 __global__ void k_tend_u(Dims d, Metric m, Flags fl, CS s, double* __restrict__ out) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
@@ -232,7 +250,34 @@ __global__ void k_tend_u(Dims d, Metric m, Flags fl, CS s, double* __restrict__ 
   if (fl.split_fast) acc -= ac_u(s, m, d, fl, i, j, k);
   out[IDX(i, j, k)] = acc;
 }
+#else
+// (fast build: the slow part of the pressure gradient taken directly with
+// theta - theta0 instead of the two terms that cancel, reciprocals for the
+// spacings)
+__global__ void k_tend_u(Dims d, Metric m, Flags fl, CS s, double* __restrict__ out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int j = blockIdx.y * blockDim.y + threadIdx.y;
+  const int k = blockIdx.z;
+  if (i > d.nx || j >= d.ny || k >= d.nz) return;
+  const int nx = d.nx, ny = d.ny, nz = d.nz;
+  const int ip = imin(i, nx - 1), im = imax(i - 1, 0), jm = imax(j - 1, 0);
+  const size_t cm = IDX(im, j, k), cp = IDX(ip, j, k), ct = IDX(ip, j, imin(k + 1, nz - 1));
+  const double hz = 0.5 * idz_at(m, d, ip, j, k);
+  const double um = s.f[U][cm], up = s.f[U][cp];
+  const double uy = SF(U, ip, imin(j + 1, ny - 1), k) - SF(U, ip, jm, k);
+  const double uz = s.f[U][ct] - SF(U, ip, j, imax(k - 1, 0));
+  const double vs = (SF(V, im, jm, k) + SF(V, ip, jm, k)) + (s.f[V][cm] + s.f[V][cp]);
+  const double ws = s.f[W][cp] + s.f[W][ct];
+  const double vc = 0.25 * vs;
+  double acc = fl.coriolis ? cor_f(m, fl, d, j) * vc : 0.0;
+  acc -= (0.5 * m.inv_dx) * ((um + up) * (up - um)) + (0.5 * m.inv_dy) * (vc * uy) + (0.5 * hz) * (ws * uz);
+  const double th = th_slow(s, m, fl, cm) + th_slow(s, m, fl, cp);
+  acc -= (0.5 * kCp * m.inv_dx) * (th * (pi_grad(s, m, fl, cp) - pi_grad(s, m, fl, cm)));
+  out[IDX(i, j, k)] = acc;
+}
+#endif
 
+#ifdef VGB_FP64_EXACT
 __global__ void k_tend_v(Dims d, Metric m, Flags fl, CS s, double* __restrict__ out) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
@@ -265,7 +310,31 @@ __global__ void k_tend_v(Dims d, Metric m, Flags fl, CS s, double* __restrict__ 
   if (fl.split_fast) acc -= ac_v(s, m, d, fl, i, j, k);
   out[IDX(i, j, k)] = acc;
 }
+#else
+__global__ void k_tend_v(Dims d, Metric m, Flags fl, CS s, double* __restrict__ out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int j = blockIdx.y * blockDim.y + threadIdx.y;
+  const int k = blockIdx.z;
+  if (i >= d.nx || j > d.ny || k >= d.nz) return;
+  const int nx = d.nx, ny = d.ny, nz = d.nz;
+  const int jp = imin(j, ny - 1), jm = imax(j - 1, 0), ia = imax(i - 1, 0);
+  const size_t cm = IDX(i, jm, k), cp = IDX(i, jp, k), ct = IDX(i, jp, imin(k + 1, nz - 1));
+  const double hz = 0.5 * idz_at(m, d, i, jp, k);
+  const double vm = s.f[V][cm], vp = s.f[V][cp];
+  const double vx = SF(V, imin(i + 1, nx - 1), jp, k) - SF(V, ia, jp, k);
+  const double vz = s.f[V][ct] - SF(V, i, jp, imax(k - 1, 0));
+  const double us = (SF(U, ia, jm, k) + s.f[U][cm]) + (SF(U, ia, jp, k) + s.f[U][cp]);
+  const double ws = s.f[W][cp] + s.f[W][ct];
+  const double uc = 0.25 * us;
+  double acc = fl.coriolis ? -cor_f(m, fl, d, j) * uc : 0.0;
+  acc -= (0.5 * m.inv_dy) * ((vm + vp) * (vp - vm)) + (0.5 * m.inv_dx) * (uc * vx) + (0.5 * hz) * (ws * vz);
+  const double th = th_slow(s, m, fl, cm) + th_slow(s, m, fl, cp);
+  acc -= (0.5 * kCp * m.inv_dy) * (th * (pi_grad(s, m, fl, cp) - pi_grad(s, m, fl, cm)));
+  out[IDX(i, j, k)] = acc;
+}
+#endif
 
+#ifdef VGB_FP64_EXACT
 __global__ void k_tend_w(Dims d, Metric m, Flags fl, CS s, double* __restrict__ out) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
@@ -299,6 +368,29 @@ __global__ void k_tend_w(Dims d, Metric m, Flags fl, CS s, double* __restrict__ 
   if (fl.split_fast) acc -= ac_w(s, m, d, fl, i, j, k);
   out[IDX(i, j, k)] = acc;
 }
+#else
+__global__ void k_tend_w(Dims d, Metric m, Flags fl, CS s, double* __restrict__ out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int j = blockIdx.y * blockDim.y + threadIdx.y;
+  const int k = blockIdx.z;
+  if (i >= d.nx || j >= d.ny || k > d.nz) return;
+  const int nx = d.nx, ny = d.ny, nz = d.nz;
+  const int kc = imin(k, nz - 1), km = imax(k - 1, 0);
+  const size_t ct = IDX(i, j, k), cc = IDX(i, j, kc), cb = IDX(i, j, km);
+  const double iz = idz_at(m, d, i, j, kc);
+  const double wt = s.f[W][ct];
+  const double wx = SF(W, imin(i + 1, nx - 1), j, k) - SF(W, imax(i - 1, 0), j, k);
+  const double wy = SF(W, i, imin(j + 1, ny - 1), k) - SF(W, i, imax(j - 1, 0), k);
+  const double us = s.f[U][cc] + s.f[U][cc + 1], vs = s.f[V][cc] + s.f[V][cc + d.P];
+  double acc = -((0.25 * m.inv_dx) * (us * wx) + (0.25 * m.inv_dy) * (vs * wy) +
+                 (0.5 * iz) * ((s.f[W][cc] + wt) * (wt - s.f[W][cb])));
+  const double th = th_slow(s, m, fl, cb) + th_slow(s, m, fl, cc);
+  acc -= (0.5 * kCp * floor1(iz)) * (th * (pi_grad(s, m, fl, cc) - pi_grad(s, m, fl, cb)));
+  const double thp = s.f[THETA][cc] - m.th0[cc];
+  const double qcond = s.f[QC][cc] + s.f[QR][cc] + s.f[QI][cc] + s.f[QS][cc] + s.f[QG][cc];
+  out[ct] = acc + kG * (thp * m.inv_th0[cc] + kBuoyMoist * s.f[QV][cc] - qcond);
+}
+#endif
 
 // Advection::scalar_nonconservative, advection.cpp:224-244
 __device__ double adv_nc(const CS& s, const Metric& m, const Dims& d, const Flags& fl, int q, int i, int j, int k) {
@@ -345,8 +437,11 @@ __global__ void k_weno_cells(Dims d, Metric m, Flags fl, CS s, int q, const doub
   const int k = blockIdx.z;
   if (i >= d.nx || j >= d.ny || k >= d.nz) return;
   const size_t c = IDX(i, j, k);
+#ifdef VGB_FP64_EXACT
   const double dz = dzeta(m, d, k) * scale_at(m, d, i, j);
-  const double idz = 1.0 / dz;
+#else
+  const double idz = idz_at(m, d, i, j, k);
+#endif
   const double qc = SF(q, i, j, k);
   const double fe = fx[IDX(i + 1, j, k)], fw = fx[c];
   const double fn = fy[IDX(i, j + 1, k)], fs = fy[c];
@@ -395,6 +490,21 @@ __global__ void k_tend_cells(Dims d, Metric m, Flags fl, CS s, MS out, const dou
   if (i >= d.nx || j >= d.ny || k >= d.nz) return;
   const int nz = d.nz;
   const size_t c = IDX(i, j, k);
+#ifndef VGB_FP64_EXACT
+  {  // face by face with rho - rho0 where the linear part belongs to the substeps
+    // (there rho0 at the clamped neighbour stands beside rho's ghost line)
+    const bool sp = fl.split_fast;
+    auto rr = [&](size_t p, size_t p0) { return sp ? s.f[RHO][p] - m.rho0[p0] : s.f[RHO][p]; };
+    const size_t w = IDX(imax(i - 1, 0), j, k), t0 = IDX(i, imax(j - 1, 0), k);
+    const size_t up = IDX(i, j, imin(k + 1, nz - 1)), dn = IDX(i, j, imax(k - 1, 0));
+    const size_t e = c + 1, n = c + d.P;
+    const double rc = rr(c, c);
+    const double fx = s.f[U][e] * (rc + rr(e, i + 1 < d.nx ? e : c)) - s.f[U][c] * (rr(w, w) + rc);
+    const double fy = s.f[V][n] * (rc + rr(n, j + 1 < d.ny ? n : c)) - s.f[V][c] * (rr(t0, t0) + rc);
+    const double fz = s.f[W][c + d.plane] * (rc + rr(up, up)) - s.f[W][c] * (rr(dn, dn) + rc);
+    out.f[RHO][c] = -((0.5 * m.inv_dx) * fx + (0.5 * m.inv_dy) * fy + (0.5 * floor1(idz_at(m, d, i, j, k))) * fz);
+  }
+#else
   {
     const double dz = dmax(dzeta(m, d, k) * scale_at(m, d, i, j), 1.0);
     const double fx = SF(U, i + 1, j, k) * 0.5 * (SF(RHO, i, j, k) + SF(RHO, i + 1, j, k)) -
@@ -407,6 +517,7 @@ __global__ void k_tend_cells(Dims d, Metric m, Flags fl, CS s, MS out, const dou
     if (fl.split_fast) r -= mass_div0(s, m, d, i, j, k);
     out.f[RHO][c] = r;
   }
+#endif
   {
     double r = 0.0;
     if (fl.div_damp > 0.0) {
@@ -427,15 +538,17 @@ __global__ void k_tend_cells(Dims d, Metric m, Flags fl, CS s, MS out, const dou
   }
 }
 
-// s = s0 + a * R over one field's interior (+ faces). Ghost points untouched.
-__global__ void k_axpy_field(Dims d, int ni, int nj, int nk, const double* __restrict__ s0,
-                             const double* __restrict__ r, double a, double* __restrict__ out) {
+// s = s0 + a * R over every field's interior (+ faces), one launch for all of
+// them. Ghost points untouched.
+__global__ void k_axpy_fields(Dims d, CS s0, CS r, double a, MS out) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int k = blockIdx.z;
-  if (i >= ni || j >= nj || k >= nk) return;
+  if (i > d.nx || j > d.ny) return;
   const size_t c = d.idx(i, j, k);
-  out[c] = s0[c] + a * r[c];
+#pragma unroll
+  for (int q = 0; q < NSPECIES; ++q)
+    if (i < d.nx + (q == U) && j < d.ny + (q == V) && k < d.nz + (q == W)) out.f[q][c] = s0.f[q][c] + a * r.f[q][c];
 }
 
 // ---- explicit forward-backward substep, runge_kutta.cpp:65-75 -----------
@@ -1246,10 +1359,8 @@ void FP64_FN(fp64_slow_tendency)(const Dims& d, const Metric& m, const Flags& fl
 
 void FP64_FN(fp64_stage_update)(const Dims& d, double* const* s0, double* const* tend, double a, double* const* out,
                        cudaStream_t stream) {
-  for (int q = 0; q < NSPECIES; ++q) {
-    const int ni = d.nx + (q == U), nj = d.ny + (q == V), nk = d.nz + (q == W);
-    k_axpy_field<<<grid3(d, ni, nj, nk, kBlk), kBlk, 0, stream>>>(d, ni, nj, nk, s0[q], tend[q], a, out[q]);
-  }
+  k_axpy_fields<<<grid3(d, d.nx + 1, d.ny + 1, d.nz + 1, kBlk), kBlk, 0, stream>>>(d, to_cs(s0), to_cs(tend),
+                                                                                               a, to_ms(out));
 }
 
 void FP64_FN(fp64_fb_substep_ad)(const Dims& d, const Metric& m, double* const* bar, double dtau, cudaStream_t stream) {

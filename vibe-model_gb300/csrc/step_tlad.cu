@@ -137,12 +137,11 @@ constexpr int kMaxLoads = 48;  // more than any point function below reads
 #define LDS(q, i, j, k, ref) L((q), d.idx((i), (j), (k)), (ref))
 #define LDC(q, i, j, k) L((q), d.idx(iclamp((i), 0, d.nx - 1), iclamp((j), 0, d.ny - 1), iclamp((k), 0, d.nz - 1)))
 
-__device__ __forceinline__ double dzeta_(const Metric& m, const Dims& d, int k) {
-  return m.dzeta[iclamp(k, 0, d.nz - 1)];
+// 1 / (dzeta(k) scale(i, j)) at clamped indices
+__device__ __forceinline__ double idz_(const Metric& m, const Dims& d, int i, int j, int k) {
+  return m.inv_dzeta[iclamp(k, 0, d.nz - 1)] * m.inv_scale[(size_t)iclamp(j, 0, d.ny - 1) * d.nx + iclamp(i, 0, d.nx - 1)];
 }
-__device__ __forceinline__ double scale_(const Metric& m, const Dims& d, int i, int j) {
-  return m.scale[(size_t)iclamp(j, 0, d.ny - 1) * d.nx + iclamp(i, 0, d.nx - 1)];
-}
+__device__ __forceinline__ double floor1_(double idz) { return idz > 1.0 ? 1.0 : idz; }  // 1 / max(dz, 1)
 __device__ __forceinline__ double ref_(const double* f, const Dims& d, int i, int j, int k) {
   return f[d.idx(i, j, k)];
 }
@@ -166,12 +165,12 @@ __device__ __forceinline__ Jet<R> pt_u(const Dims& d, const Metric& m, const Fla
   using T = Jet<R>;
   const int nx = d.nx, ny = d.ny, nz = d.nz;
   const int ip = imin(i, nx - 1), im = imax(i - 1, 0);
-  const double dz = dzeta_(m, d, imin(k, nz - 1)) * scale_(m, d, ip, j);
+  const double hz = 0.5 * idz_(m, d, ip, j, k);
   const T um = LD(U, im, j, k), up = LD(U, ip, j, k);
   const T uc = 0.5 * (um + up);
   const T ux = (up - um) * m.inv_dx;
   const T uy = (LD(U, ip, imin(j + 1, ny - 1), k) - LD(U, ip, imax(j - 1, 0), k)) * (0.5 * m.inv_dy);
-  const T uz = (LD(U, ip, j, imin(k + 1, nz - 1)) - LD(U, ip, j, imax(k - 1, 0))) * (1.0 / (2.0 * dz));
+  const T uz = (LD(U, ip, j, imin(k + 1, nz - 1)) - LD(U, ip, j, imax(k - 1, 0))) * hz;
   const T vc = 0.25 * (LD(V, im, imax(j - 1, 0), k) + LD(V, ip, imax(j - 1, 0), k) + LD(V, im, j, k) + LD(V, ip, j, k));
   const T wc = 0.5 * (LD(W, ip, j, k) + LD(W, ip, j, imin(k + 1, nz - 1)));
   T acc = -(uc * ux + vc * uy + wc * uz);
@@ -188,12 +187,12 @@ __device__ __forceinline__ Jet<R> pt_v(const Dims& d, const Metric& m, const Fla
   using T = Jet<R>;
   const int nx = d.nx, ny = d.ny, nz = d.nz;
   const int jp = imin(j, ny - 1), jm = imax(j - 1, 0);
-  const double dz = dzeta_(m, d, imin(k, nz - 1)) * scale_(m, d, i, jp);
+  const double hz = 0.5 * idz_(m, d, i, jp, k);
   const T vm = LD(V, i, jm, k), vp = LD(V, i, jp, k);
   const T vc = 0.5 * (vm + vp);
   const T vy = (vp - vm) * m.inv_dy;
   const T vx = (LD(V, imin(i + 1, nx - 1), jp, k) - LD(V, imax(i - 1, 0), jp, k)) * (0.5 * m.inv_dx);
-  const T vz = (LD(V, i, jp, imin(k + 1, nz - 1)) - LD(V, i, jp, imax(k - 1, 0))) * (1.0 / (2.0 * dz));
+  const T vz = (LD(V, i, jp, imin(k + 1, nz - 1)) - LD(V, i, jp, imax(k - 1, 0))) * hz;
   const int ia = imax(i - 1, 0);
   const T uc = 0.25 * (LD(U, ia, jm, k) + LD(U, i, jm, k) + LD(U, ia, jp, k) + LD(U, i, jp, k));
   const T wc = 0.5 * (LD(W, i, jp, k) + LD(W, i, jp, imin(k + 1, nz - 1)));
@@ -211,24 +210,23 @@ __device__ __forceinline__ Jet<R> pt_w(const Dims& d, const Metric& m, const Fla
   using T = Jet<R>;
   const int nx = d.nx, ny = d.ny, nz = d.nz;
   const int kc = imin(imax(k, 0), nz - 1), kt = imin(k, nz), km = imax(k - 1, 0);
-  const double dz = dzeta_(m, d, kc) * scale_(m, d, i, j);
+  const double iz = idz_(m, d, i, j, kc);
   const T wt = LD(W, i, j, kt);
   const T wc = 0.5 * (LD(W, i, j, kc) + wt);
-  const T wz = (wt - LD(W, i, j, km)) * (1.0 / dz);
+  const T wz = (wt - LD(W, i, j, km)) * iz;
   const T wx = (LD(W, imin(i + 1, nx - 1), j, kt) - LD(W, imax(i - 1, 0), j, kt)) * (0.5 * m.inv_dx);
   const T wy = (LD(W, i, imin(j + 1, ny - 1), kt) - LD(W, i, imax(j - 1, 0), kt)) * (0.5 * m.inv_dy);
   const T uc = 0.5 * (LD(U, i, j, kc) + LD(U, i + 1, j, kc));
   const T vc = 0.5 * (LD(V, i, j, kc) + LD(V, i, j + 1, kc));
   T acc = -(uc * wx + vc * wy + wc * wz);
-  const double dz1 = dmax(dz, 1.0);
   const bool sp = fl.split_fast;
   const T th = 0.5 * (LDS(THETA, i, j, km, sp ? ref_(m.th0, d, i, j, km) : 0.0) +
                       LDS(THETA, i, j, kc, sp ? ref_(m.th0, d, i, j, kc) : 0.0));
-  acc = acc - kCp * (th * dpi_<R>(d, m, fl, L, i, j, kc, i, j, km)) * (1.0 / dz1);
+  acc = acc - kCp * (th * dpi_<R>(d, m, fl, L, i, j, kc, i, j, km)) * floor1_(iz);
   const double th0 = ref_(m.th0, d, i, j, kc);
   const T thp = LDS(THETA, i, j, kc, th0);
   const T qcond = LD(QC, i, j, kc) + LD(QR, i, j, kc) + LD(QI, i, j, kc) + LD(QS, i, j, kc) + LD(QG, i, j, kc);
-  return acc + kG * (thp * (1.0 / dmax(th0, 1.0)) + kBuoyMoist * LD(QV, i, j, kc) - qcond);
+  return acc + kG * (thp * ref_(m.inv_th0, d, i, j, kc) + kBuoyMoist * LD(QV, i, j, kc) - qcond);
 }
 
 // rho cell (i, j, k): the mass-flux divergence of k_tend_cells; with
@@ -240,7 +238,7 @@ __device__ __forceinline__ Jet<R> pt_rho(const Dims& d, const Metric& m, const F
   const int nx = d.nx, ny = d.ny, nz = d.nz;
   const bool sp = fl.split_fast;
   const double* r0 = m.rho0;
-  const double dz = dmax(dzeta_(m, d, k) * scale_(m, d, i, j), 1.0);
+  const double iz = floor1_(idz_(m, d, i, j, k));
   // rho at point p minus (with split) rho0 at point p0 (mass_div0 reads rho0
   // at clamped neighbours where the flux reads rho's ghost line)
   auto rr = [&](int a, int b, int c, int a0, int b0, int c0) {
@@ -257,7 +255,7 @@ __device__ __forceinline__ Jet<R> pt_rho(const Dims& d, const Metric& m, const F
   const T tz = 0.5 * (rc + rr(i, j, kp, i, j, kp));
   const T bz = 0.5 * (rr(i, j, km, i, j, km) + rc);
   const T fz = LD(W, i, j, k + 1) * tz - LD(W, i, j, k) * bz;
-  return -(fx * m.inv_dx + fy * m.inv_dy + fz * (1.0 / dz));
+  return -(fx * m.inv_dx + fy * m.inv_dy + fz * iz);
 }
 
 // pi cell: second-order divergence damping (damping.cpp:48-53)
@@ -287,7 +285,7 @@ template <class R, class Ld>
 __device__ __forceinline__ Jet<R> pt_scalar_nc(const Dims& d, const Metric& m, const Flags& fl, Ld& L, int q, int i,
                                                int j, int k) {
   using T = Jet<R>;
-  const double dz = dzeta_(m, d, k) * scale_(m, d, i, j);
+  const double idz = idz_(m, d, i, j, k);
   const T ua = 0.5 * (LD(U, i, j, k) + LD(U, i + 1, j, k));
   const T va = 0.5 * (LD(V, i, j, k) + LD(V, i, j + 1, k));
   const T wa = 0.5 * (LD(W, i, j, k) + LD(W, i, j, k + 1));
@@ -300,7 +298,7 @@ __device__ __forceinline__ Jet<R> pt_scalar_nc(const Dims& d, const Metric& m, c
   const T gy = gradc_<R>(w3 ? LDC(q, i, j - 3, k) : z, w2 ? LDC(q, i, j - 2, k) : z, LDC(q, i, j - 1, k),
                          LDC(q, i, j + 1, k), w2 ? LDC(q, i, j + 2, k) : z, w3 ? LDC(q, i, j + 3, k) : z,
                          1.0 / m.dy, o);
-  const T gz = (LDC(q, i, j, k + 1) - LDC(q, i, j, k - 1)) * (0.5 / dz);
+  const T gz = (LDC(q, i, j, k + 1) - LDC(q, i, j, k - 1)) * (0.5 * idz);
   T r = -(ua * gx + va * gy + wa * gz);
   if (q >= QV) {
     const T qc = LD(q, i, j, k);
@@ -332,6 +330,7 @@ __device__ __forceinline__ R weno_left_(const R (&z)[5]) {
 // advection.cpp:160-170: u times the upwind side alone for |u| >= 1e-3
 template <class R>
 __device__ __forceinline__ R wflux_value_(const R (&z)[5], R vel) {
+  if (z[0] == z[1] && z[1] == z[2] && z[2] == z[3] && z[3] == z[4]) return vel * z[2];
   const bool up = vel >= (R)0;
   R y[5], yo[5];
 #pragma unroll
@@ -352,6 +351,12 @@ __device__ __forceinline__ R wflux_value_(const R (&z)[5], R vel) {
 // one reverse pass instead of one forward pass per stencil value.
 template <class R>
 __device__ __forceinline__ R wgrad_left_(const R (&z)[5], R (&g)[5]) {
+  if (z[0] == z[1] && z[1] == z[2] && z[2] == z[3] && z[3] == z[4]) {
+    // a flat stencil (most moisture fields are zero): the linear weights, whose derivatives vanish
+    g[0] = (R)(2.0 / 60.0), g[1] = (R)(-13.0 / 60.0), g[2] = (R)(47.0 / 60.0), g[3] = (R)(27.0 / 60.0);
+    g[4] = (R)(-3.0 / 60.0);
+    return z[2];
+  }
   const R s6 = (R)(1.0 / 6.0), c13 = (R)(13.0 / 12.0);
   const R v0 = ((R)2 * z[0] - (R)7 * z[1] + (R)11 * z[2]) * s6;
   const R v1 = (-z[1] + (R)5 * z[2] + (R)2 * z[3]) * s6;
@@ -465,8 +470,7 @@ template <class R, class Ld>
 __device__ __forceinline__ Jet<R> pt_wcell(const Dims& d, const Metric& m, const Flags& fl, Ld& L, const FaceArr& F,
                                            bool with_t, int q, int i, int j, int k, bool clip = true) {
   using T = Jet<R>;
-  const double dz = dzeta_(m, d, k) * scale_(m, d, i, j);
-  const double idz = 1.0 / dz;
+  const double idz = idz_(m, d, i, j, k);
   const T qc = LD(q, i, j, k);
   const bool vert = (k + 2 < d.nz || k >= 2);
   const bool adv = fl.weno_advective;
@@ -603,7 +607,7 @@ __device__ __forceinline__ void ad_u(const Dims& d, const Metric& m, const Flags
   const int nx = d.nx, ny = d.ny, nz = d.nz;
   const int ip = imin(i, nx - 1), im = imax(i - 1, 0), jm = imax(j - 1, 0), kp = imin(k + 1, nz - 1);
   const R idx = (R)m.inv_dx, hy = (R)(0.5 * m.inv_dy);
-  const R hz = (R)(1.0 / (2.0 * (dzeta_(m, d, imin(k, nz - 1)) * scale_(m, d, ip, j))));
+  const R hz = (R)(0.5 * idz_(m, d, ip, j, k));
   const size_t cm = d.idx(im, j, k), cp = d.idx(ip, j, k);
   const size_t cn = d.idx(ip, imin(j + 1, ny - 1), k), cs = d.idx(ip, jm, k);
   const size_t ct = d.idx(ip, j, kp), cb = d.idx(ip, j, imax(k - 1, 0));
@@ -643,7 +647,7 @@ __device__ __forceinline__ void ad_v(const Dims& d, const Metric& m, const Flags
   const int nx = d.nx, ny = d.ny, nz = d.nz;
   const int jp = imin(j, ny - 1), jm = imax(j - 1, 0), ia = imax(i - 1, 0), kp = imin(k + 1, nz - 1);
   const R idy = (R)m.inv_dy, hx = (R)(0.5 * m.inv_dx);
-  const R hz = (R)(1.0 / (2.0 * (dzeta_(m, d, imin(k, nz - 1)) * scale_(m, d, i, jp))));
+  const R hz = (R)(0.5 * idz_(m, d, i, jp, k));
   const size_t cm = d.idx(i, jm, k), cp = d.idx(i, jp, k);
   const size_t ce = d.idx(imin(i + 1, nx - 1), jp, k), cw = d.idx(ia, jp, k);
   const size_t ct = d.idx(i, jp, kp), cb = d.idx(i, jp, imax(k - 1, 0));
@@ -682,8 +686,8 @@ __device__ __forceinline__ void ad_w(const Dims& d, const Metric& m, const Flags
                                      double lam, int i, int j, int k) {
   const int nx = d.nx, ny = d.ny, nz = d.nz;
   const int kc = imin(imax(k, 0), nz - 1), kt = imin(k, nz), km = imax(k - 1, 0);
-  const double dz = dzeta_(m, d, kc) * scale_(m, d, i, j);
-  const R hx = (R)(0.5 * m.inv_dx), hy = (R)(0.5 * m.inv_dy), iz = (R)(1.0 / dz), iz1 = (R)(1.0 / dmax(dz, 1.0));
+  const double idz = idz_(m, d, i, j, kc);
+  const R hx = (R)(0.5 * m.inv_dx), hy = (R)(0.5 * m.inv_dy), iz = (R)idz, iz1 = (R)floor1_(idz);
   const size_t ct = d.idx(i, j, kt), cc = d.idx(i, j, kc), cb = d.idx(i, j, km);
   const size_t ce = d.idx(imin(i + 1, nx - 1), j, kt), cw = d.idx(imax(i - 1, 0), j, kt);
   const size_t cn = d.idx(i, imin(j + 1, ny - 1), kt), cs = d.idx(i, imax(j - 1, 0), kt);
@@ -708,7 +712,7 @@ __device__ __forceinline__ void ad_w(const Dims& d, const Metric& m, const Flags
   add(V, cc + d.P, cv);
   const R ch = (R)0.5 * g * dp;
   add(THETA, cb, (double)-ch);
-  add(THETA, cc, (double)((R)kG * (R)(1.0 / dmax(m.th0[cc], 1.0)) - ch));
+  add(THETA, cc, (double)((R)kG * (R)m.inv_th0[cc] - ch));
   add(PI, cc, (double)-(g * th));
   add(PI, cb, (double)(g * th));
   add(QV, cc, (double)((R)kG * (R)kBuoyMoist));
@@ -720,7 +724,7 @@ __device__ __forceinline__ void ad_rho(const Dims& d, const Metric& m, const Fla
                                        double lam, int i, int j, int k) {
   const int nx = d.nx, ny = d.ny, nz = d.nz;
   const bool sp = fl.split_fast;
-  const R idx = (R)m.inv_dx, idy = (R)m.inv_dy, iz = (R)(1.0 / dmax(dzeta_(m, d, k) * scale_(m, d, i, j), 1.0));
+  const R idx = (R)m.inv_dx, idy = (R)m.inv_dy, iz = (R)floor1_(idz_(m, d, i, j, k));
   const size_t c = d.idx(i, j, k), e = c + 1, n = c + d.P;
   const size_t w = d.idx(imax(i - 1, 0), j, k), s = d.idx(i, imax(j - 1, 0), k);
   const size_t t = d.idx(i, j, imin(k + 1, nz - 1)), l = d.idx(i, j, imax(k - 1, 0)), tf = c + d.plane;
@@ -800,11 +804,11 @@ __global__ void k_ad_wcell(Dims d, Metric m, Flags fl, const __grid_constant__ F
   if (lam == 0.0 || !fl.weno_advective) return;
   // the cell's own q enters r (beyond its faces' G) through (q - c_f) u_f:
   // dr/dq = div; the winds' part is scattered per face (k_ad_wface)
-  const double dz = dzeta_(m, d, k) * scale_(m, d, i, j);
+  const double idz = idz_(m, d, i, j, k);
   const bool vert = (k + 2 < d.nz || k >= 2);
   R div = ((R)b.f[U][d.idx(i + 1, j, k)] - (R)b.f[U][c]) * (R)m.inv_dx +
           ((R)b.f[V][d.idx(i, j + 1, k)] - (R)b.f[V][c]) * (R)m.inv_dy;
-  if (vert) div += ((R)b.f[W][d.idx(i, j, k + 1)] - (R)b.f[W][c]) * (R)(1.0 / dz);
+  if (vert) div += ((R)b.f[W][d.idx(i, j, k + 1)] - (R)b.f[W][c]) * (R)idz;
   atomicAdd(&bi.f[q][c], (double)div * lam);
 }
 
@@ -839,8 +843,8 @@ __global__ void k_ad_wface(Dims d, Metric m, Flags fl, const __grid_constant__ F
     } else {
       hasR = k < d.nz && (k + 2 < d.nz || k >= 2);
       hasL = k >= 1 && (lk + 2 < d.nz || lk >= 2);
-      invR = hasR ? 1.0 / (dzeta_(m, d, k) * scale_(m, d, i, j)) : 0.0;
-      invL = hasL ? 1.0 / (dzeta_(m, d, lk) * scale_(m, d, i, j)) : 0.0;
+      invR = hasR ? idz_(m, d, i, j, k) : 0.0;
+      invL = hasL ? idz_(m, d, i, j, lk) : 0.0;
     }
     const double aR = hasR ? ebar[d.idx(i, j, k)] * invR : 0.0;
     const double aL = hasL ? ebar[d.idx(li, lj, lk)] * invL : 0.0;

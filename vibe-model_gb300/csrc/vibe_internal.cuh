@@ -54,6 +54,11 @@ struct Metric {
   const double* rho0;
   double f0, beta;       // Coriolis (coriolis.cpp:25-41)
   double inv_dx, inv_dy; // 1/dx, 1/dy (the fast FP64 build multiplies by them)
+  // reciprocals the fast FP64 build and the TL/AD multiply by: an FP64
+  // division costs about nine FP64 operations
+  const double* inv_dzeta;  // nz: 1/dzeta
+  const double* inv_scale;  // nx*ny: 1/scale
+  const double* inv_th0;    // 3-D: 1/max(theta0, 1)
   // flat grids with a horizontally uniform reference state: the consistent
   // HEVI substep's per-level coefficients for one dtau (Hevi64Row rows of
   // nz + 1 doubles), else null
