@@ -108,6 +108,28 @@ def test_multigrid_bicgstab_converges_to_1e10(vg, oc, kind, dims):
     assert np.abs(sols[3] - sols[4]).max() <= 1e-8 * np.abs(sols[3]).max()
 
 
+@pytest.mark.parametrize("dims,levels", [((33, 17, 5), 3), ((63, 9, 24), 2), ((9, 65, 88), 2), ((8, 9, 300), 2),
+                                         ((64, 64, 87), 5), ((129, 130, 3), 5)])
+def test_multigrid_odd_grids(vg, oc, dims, levels):
+    """Aggregates of half the width at every odd size, the coarsest grid held
+    on chip up to 87 levels and read from memory above, the FP64 smoother
+    without its tiles (300 levels): the oracle's operator finds the relative
+    residual below the tolerance asked for, twice in a row from one solver,
+    with the same bits."""
+    nx, ny, nz = dims
+    s = hc.si_setup(oc, nx=nx, ny=ny, nz=nz, zeta_first=20000.0 / nz, zeta_stretch=1.0)
+    a, b, f, dzeta, zs = hc.si_problem(oc, s)
+    port = oc.Model(s, "port")
+    fn = np.sqrt(np.sum(oc.interior(s, 3, f) ** 2))
+    for kind in (3, 4):
+        for tol in (1e-10, 1e-6):
+            with make(vg, s, kind, dzeta, zs, tol=tol) as h:
+                rc, x = h.solve(a, b, f)
+                assert rc == 0 and h.levels() == levels
+                assert port.helmholtz_residual_l2(a, b, f, x) / fn < tol
+                assert np.array_equal(h.solve(a, b, f)[1], x)
+
+
 def test_bad_arguments(vg, oc):
     s = hc.si_setup(oc, nx=8, ny=8, nz=4)
     dzeta = np.full(4, 0.25)

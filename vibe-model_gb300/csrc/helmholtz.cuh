@@ -14,6 +14,8 @@ struct HGeo {
   double dx, dy;
   const double* dzeta;  // nz
   const double* scale;  // nx*ny: z_top - zs(i,j)
+  const double* inv_dzeta;  // 1/dzeta
+  const double* inv_scale;  // 1/scale
   __host__ __device__ size_t n() const { return (size_t)nx * ny * nz; }
 };
 
@@ -27,6 +29,12 @@ void hz_jacobi_prec(const HGeo& g, const double* a, const double* b, double* pre
 // column tridiagonal solve of VerticalTridiagonalSolver; cp, dp: n scratch
 void hz_vertical_solve(const HGeo& g, const double* a, const double* b, const double* f, double* x, double* cp,
                        double* dp, unsigned* err, cudaStream_t s);
+
+// r = f - A x for the refinement loop of the multigrid solvers: the same
+// operator with each face flux computed once and reciprocal spacings (equal to
+// the reference's order to rounding)
+void hz_residual(const HGeo& g, const double* a, const double* b, const double* f, const double* x, double* r,
+                 cudaStream_t s);
 
 // ---- deterministic FP64 reductions: sum over n of x*y (y may equal x) into
 // out[slot]; partials: >= kRedBlocks doubles per slot ----

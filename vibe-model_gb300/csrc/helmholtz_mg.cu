@@ -22,9 +22,15 @@
 // keep nz (semi-coarsening); coarse couplings are the 2x2 aggregates: cT,
 // cB, cD averaged, the horizontal face couplings summed over the two fine
 // faces of the coarse face and divided by 8 (= the rediscretised
-// a/(2h)^2). Residuals are restricted by the 2x2 mean (computed and
+// a/(2h)^2). An odd nx or ny leaves a last aggregate of half the width, whose
+// equation is kept in the volume-weighted form (sums over the cells there
+// are), which keeps the couplings of its faces symmetric. Residuals are restricted by the 2x2 mean (computed and
 // restricted in one pass) and corrections prolonged piecewise constant.
-// V(1,1) cycle, the coarsest grid smoothed 8 times in one block. The
+// V(1,1) cycle, the coarsest grid smoothed kCoarseSweeps times in one cluster
+// launch. The half sweep before a restriction leaves the residual zero on its
+// colour, so only the other colour's is computed and restricted; the one after
+// a prolongation overwrites its colour, so the correction is added where it
+// reads the other colour and never stored. The
 // BiCGSTAB loop runs on the device as a conditional CUDA graph.
 #include <cmath>
 #include <cstdio>
@@ -59,6 +65,7 @@ struct MgSolver {
   T *x, *r, *r0, *p, *v, *s, *t, *ph, *sh;  // Krylov vectors (fine level)
   double* part = nullptr;                   // 2 x kMgRedBlocks partial sums
   double* sc = nullptr;                     // device scalars
+  unsigned* done = nullptr;                 // blocks of a reducing kernel that are through
   double* hsc = nullptr;                    // pinned host copy
   std::vector<void*> allocs;
   // the iteration loop as a CUDA graph: a WHILE node around one iteration,
@@ -66,6 +73,7 @@ struct MgSolver {
   // yet, 1 = built, -1 = not available: the host loop runs instead)
   int graph_state = 0;
   int coarse_ctas = 0;  // CTAs of the one-cluster coarsest smoothing (0: one launch per half sweep)
+  bool coarse_resident = false;  // ... whose CTAs keep their one tile per colour in shared memory
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t gexec = nullptr;
 };
@@ -109,6 +117,64 @@ __device__ __forceinline__ T apply_at(const MgLevel<T>& l, const T* __restrict__
   return y;
 }
 
+// ---- the FP64 residual of the refinement loop ----
+// Tiles of 31 x 8 columns marching up the levels: a warp's 32 lanes hold the
+// west-face fluxes of 31 cells and the next one's (by shuffle), nine rows the
+// south-face fluxes of eight (through shared memory), and a thread carries its
+// lower face: each flux a (x - x) once, the spacings as reciprocals. About 20
+// FP64 operations a cell, the bound (one thread per cell with six faces and
+// three divisions, in the reference's order, took 539 us at 256 x 256 x 64).
+constexpr int kResRows = 8, kResCols = 31;
+__global__ void __launch_bounds__(32 * (kResRows + 1)) k_residual64(HGeo g, const double* __restrict__ a,
+                                                                    const double* __restrict__ b,
+                                                                    const double* __restrict__ f,
+                                                                    const double* __restrict__ x,
+                                                                    double* __restrict__ r, int xtiles, int kz) {
+  __shared__ double sy[2][kResRows + 1][32];
+  const int lane = threadIdx.x, row = threadIdx.y;
+  const int i0 = (int)(blockIdx.x % (unsigned)xtiles) * kResCols, j0 = (int)(blockIdx.x / (unsigned)xtiles) * kResRows;
+  const int k0 = blockIdx.y * kz, k1 = imin(k0 + kz, g.nz);
+  const int i = i0 + lane, j = j0 + row;
+  const bool in = i < g.nx && j < g.ny;  // (outside: the clamped cell's values, whose fluxes are not used)
+  const bool cells = row < kResRows;
+  const size_t pl = (size_t)g.nx * g.ny;
+  const size_t c = (size_t)imin(j, g.ny - 1) * g.nx + imin(i, g.nx - 1);
+  const double hx = 0.5 / (g.dx * g.dx), hy = 0.5 / (g.dy * g.dy), is = g.inv_scale[c];
+  size_t o = (size_t)k0 * pl + c;
+  double ac = a[o], xc = x[o], fb = 0.0;
+  if (cells && k0 > 0) fb = (a[o - pl] + ac) * (xc - x[o - pl]);
+  for (int k = k0; k < k1; ++k, o += pl) {
+    // boundary faces carry no flux: the south face of row 0, and the faces beyond the grid
+    const double fs = (j > 0 && j < g.ny) ? (a[o - g.nx] + ac) * (xc - x[o - g.nx]) : 0.0;
+    sy[k & 1][row][lane] = fs;
+    double at = 0.0, xt = 0.0, ft = 0.0, fw = 0.0, fe = 0.0;
+    if (k + 1 < g.nz) {
+      at = a[o + pl];
+      xt = x[o + pl];
+    }
+    if (cells) {
+      if (k + 1 < g.nz) ft = (ac + at) * (xt - xc);
+      double aw = __shfl_up_sync(0xffffffffu, ac, 1), xw = __shfl_up_sync(0xffffffffu, xc, 1);
+      if (lane == 0 && i > 0) {
+        aw = a[o - 1];
+        xw = x[o - 1];
+      }
+      if (i > 0 && i < g.nx) fw = (aw + ac) * (xc - xw);
+      fe = __shfl_down_sync(0xffffffffu, fw, 1);
+    }
+    __syncthreads();  // (the buffer of two levels ago was read before the barrier in between)
+    if (cells && in && lane < kResCols) {
+      const double iz = g.inv_dzeta[k] * is;
+      const double hz = (unsigned)__double2hiint(iz) < 0x3ff00000u ? 0.5 * iz * iz : 0.5;  // 1/2 / max(dz, 1)^2
+      const double fn = sy[k & 1][row + 1][lane];
+      r[o] = f[o] + ((fe - fw) * hx + (fn - fs) * hy + (ft - fb) * hz - b[o] * xc);
+    }
+    ac = at;
+    xc = xt;
+    fb = ft;
+  }
+}
+
 // ---- coefficient set-up ----
 template <typename T>
 __global__ void k_fine_coefs(HGeo g, const double* __restrict__ a, const double* __restrict__ b, MgLevel<T> l) {
@@ -134,11 +200,38 @@ __global__ void k_coarse_coefs(MgLevel<T> f, MgLevel<T> cl) {
     cell_of(c, cl.nx, cl.ny, I, J, k);
     const size_t f00 = (size_t)k * pf + (size_t)(2 * J) * f.nx + 2 * I;
     const size_t f10 = f00 + 1, f01 = f00 + f.nx, f11 = f01 + 1;
-    cl.cE[c] = (f.cE[f10] + f.cE[f11]) * (T)0.125;
-    cl.cN[c] = (f.cN[f01] + f.cN[f11]) * (T)0.125;
-    cl.cT[c] = (f.cT[f00] + f.cT[f10] + f.cT[f01] + f.cT[f11]) * (T)0.25;
-    cl.cB[c] = (f.cB[f00] + f.cB[f10] + f.cB[f01] + f.cB[f11]) * (T)0.25;
-    cl.cD[c] = (f.cD[f00] + f.cD[f10] + f.cD[f01] + f.cD[f11]) * (T)0.25;
+    if (2 * I + 1 < f.nx && 2 * J + 1 < f.ny) {
+      // (a face beside a last cell of half the width: centres 1.5 h apart instead of 2 h)
+      const T wE = (T)(2 * I + 3 == f.nx ? 1.0 / 6.0 : 0.125), wN = (T)(2 * J + 3 == f.ny ? 1.0 / 6.0 : 0.125);
+      cl.cE[c] = (f.cE[f10] + f.cE[f11]) * wE;
+      cl.cN[c] = (f.cN[f01] + f.cN[f11]) * wN;
+      cl.cT[c] = (f.cT[f00] + f.cT[f10] + f.cT[f01] + f.cT[f11]) * (T)0.25;
+      cl.cB[c] = (f.cB[f00] + f.cB[f10] + f.cB[f01] + f.cB[f11]) * (T)0.25;
+      cl.cD[c] = (f.cD[f00] + f.cD[f10] + f.cD[f01] + f.cD[f11]) * (T)0.25;
+      continue;
+    }
+    // the last column or row of an odd grid: the same sums over the cells there
+    // are, so the equation carries the cell's share of a full one's volume
+    const bool x2 = 2 * I + 1 < f.nx, y2 = 2 * J + 1 < f.ny;
+    T t = f.cT[f00], bb = f.cB[f00], dd = f.cD[f00], ce = 0, cn = 0;
+    if (x2) {
+      t += f.cT[f10];
+      bb += f.cB[f10];
+      dd += f.cD[f10];
+      ce = f.cE[f10];  // (no second row: the face of the one there is)
+      cn = 0;
+    }
+    if (y2) {
+      t += f.cT[f01];
+      bb += f.cB[f01];
+      dd += f.cD[f01];
+      cn = f.cN[f01];
+    }
+    cl.cE[c] = ce * (T)(2 * I + 3 == f.nx ? 1.0 / 6.0 : 0.125);
+    cl.cN[c] = cn * (T)(2 * J + 3 == f.ny ? 1.0 / 6.0 : 0.125);
+    cl.cT[c] = t * (T)0.25;
+    cl.cB[c] = bb * (T)0.25;
+    cl.cD[c] = dd * (T)0.25;
   }
 }
 
@@ -242,11 +335,14 @@ __device__ __forceinline__ bool tile_column(const MgLevel<T>& l, int t, int colo
   return ok;
 }
 
-// kB: levels per batch and thread (12 kB values in registers)
-template <typename T, bool kZeroNb, int kB>
+// kB: levels per batch and thread (12 kB values in registers, 16 kB with kAdd)
+// kAdd: the neighbours' x plus the coarse grid's correction xc (cnx x cny
+// columns, piecewise constant over the aggregates)
+template <typename T, bool kZeroNb, int kB, bool kAdd = false>
 __device__ __forceinline__ void scan_tile_load(const MgLevel<T>& l, const T* __restrict__ rhs,
                                                const T* __restrict__ x, int t, int color, ScanTile<T> st,
-                                               int tid) {
+                                               int tid, const T* __restrict__ xc = nullptr, int cnx = 0,
+                                               size_t cpl = 0) {
   const int nz = l.nz;
   const int lane = tid & 31, w = tid >> 5;
   int i, j;
@@ -255,6 +351,8 @@ __device__ __forceinline__ void scan_tile_load(const MgLevel<T>& l, const T* __r
   const int col = j * l.nx + i;
   const bool e = ok && i + 1 < l.nx, wv = ok && i > 0, n = ok && j + 1 < l.ny, so = ok && j > 0;
   const int de = e ? 1 : 0, dw = wv ? 1 : 0, dn = n ? l.nx : 0, ds = so ? l.nx : 0;
+  const int ge = (j >> 1) * cnx + ((i + de) >> 1), gw = (j >> 1) * cnx + ((i - dw) >> 1);
+  const int gn = ((j + (n ? 1 : 0)) >> 1) * cnx + (i >> 1), gs = ((j - (so ? 1 : 0)) >> 1) * cnx + (i >> 1);
   for (int kb = w; kb < nz; kb += 8 * kB) {
     T rv[kB], ce[kB], xe[kB], cw[kB], xw[kB], cn[kB], xn[kB], cs[kB], xs[kB], li[kB], cb[kB], lc[kB];
 #pragma unroll
@@ -271,6 +369,13 @@ __device__ __forceinline__ void scan_tile_load(const MgLevel<T>& l, const T* __r
         xn[u] = x[c + dn];
         cs[u] = l.cN[c - ds];
         xs[u] = x[c - ds];
+        if (kAdd) {
+          const T* g = xc + (size_t)(k < nz ? k : nz - 1) * cpl;
+          xe[u] += g[ge];
+          xw[u] += g[gw];
+          xn[u] += g[gn];
+          xs[u] += g[gs];
+        }
       }
       li[u] = l.li[c];
       cb[u] = l.cB[c];
@@ -392,6 +497,19 @@ __global__ void __launch_bounds__(256) k_smooth_scan(MgLevel<T> l, const T* __re
   scan_tile_store<T>(l, x, blockIdx.x, color, st, threadIdx.x);
 }
 
+// the half sweep after the coarse grid's correction
+template <typename T>
+__global__ void __launch_bounds__(256) k_smooth_add(MgLevel<T> l, const T* __restrict__ rhs, T* __restrict__ x,
+                                                    int color, const T* __restrict__ xc, int cnx, size_t cpl) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const ScanTile<T> st(reinterpret_cast<T*>(smem_raw), l.nz);
+  scan_tile_load<T, false, sizeof(T) == 4 ? 4 : 2, true>(l, rhs, x, blockIdx.x, color, st, threadIdx.x, xc, cnx, cpl);
+  __syncthreads();
+  scan_tile_solve<T>(l.nz, st, threadIdx.x);
+  __syncthreads();
+  scan_tile_store<T>(l, x, blockIdx.x, color, st, threadIdx.x);
+}
+
 // The coarsest grid's smoothing, kCoarseSweeps red-black sweeps (the first
 // half sweep from a zero guess), in one launch of one thread-block cluster:
 // CTA b takes tiles b, b + gridDim.x, ... of each half sweep, and the
@@ -399,8 +517,9 @@ __global__ void __launch_bounds__(256) k_smooth_scan(MgLevel<T> l, const T* __re
 // are seen by the cluster's loads after it) separates the half sweeps; a
 // half sweep reads only the other colour, so its tiles are independent.
 // Replaces 2 kCoarseSweeps launches of a few tiles each (16 x 16 x 64: 4
-// tiles per half sweep).
-constexpr int kCoarseSweeps = 8;
+// tiles per half sweep). Four sweeps: the iteration counts of eight (7 at
+// 256 x 256 x 64 and 193 x 193 x 60, 5 at 97 x 64 x 40), 0.25 ms less a solve.
+constexpr int kCoarseSweeps = 4;
 constexpr int kCoarseMaxCtas = 8;  // portable cluster size
 
 __device__ __forceinline__ void cluster_sync() {
@@ -430,6 +549,146 @@ __global__ void __launch_bounds__(256) k_coarse_smooth(MgLevel<T> l, const T* __
   }
 }
 
+// The same when every CTA has one tile of each colour: the two tiles' right-hand
+// side, couplings, factors and x stay in shared memory for all the sweeps, and
+// a half sweep reads the other colour's x from the CTA that holds it (its own
+// for the east and west neighbours and most of the others) through distributed
+// shared memory, so no sweep goes through L2. Same arithmetic. 14 calls of a
+// 256 x 256 x 64 solve at 16 x 16 x 64: 30 us each, and 61 us with twice the
+// sweeps and x and the couplings read from global memory.
+template <typename T>
+size_t coarse_resident_smem(int nz) {
+  return (size_t)nz * (6 * kScanRS + 12 * 32) * sizeof(T);
+}
+// x of column (i, j), whose colour is (i + j) % 2, at level offset: the shared
+// address in the CTA that holds its tile
+template <typename T>
+__device__ __forceinline__ unsigned remote_column(const MgLevel<T>& l, unsigned xbase, unsigned colour_stride, int i, int j) {
+  const int q = j * ((l.nx + 1) / 2) + (i >> 1);  // (tile_column: i = 2m + (j + colour) % 2)
+  const unsigned local = xbase + ((i + j) & 1) * colour_stride + (unsigned)(q & 31) * (unsigned)sizeof(T);
+  unsigned r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local), "r"(q >> 5));
+  return r;
+}
+__device__ __forceinline__ float ld_cluster(unsigned a, float) {
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ double ld_cluster(unsigned a, double) {
+  double v;
+  asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(a) : "memory");
+  return v;
+}
+template <typename T>
+__global__ void __launch_bounds__(256) k_coarse_resident(MgLevel<T> l, const T* __restrict__ rhs, T* __restrict__ x) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  T* base = reinterpret_cast<T*>(smem_raw);
+  const int nz = l.nz, tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const size_t sc = (size_t)nz * kScanRS, rc = (size_t)nz * 32;
+  T* X = base;            // per colour: the half sweep's right-hand side, then x (scan layout)
+  T* AC = base + 2 * sc;  // per colour: A, C (scan layout)
+  T* Q = base + 6 * sc;   // per colour: rhs, cE, cW, cN, cS, li
+  const size_t pl = (size_t)l.nx * l.ny;
+  const unsigned xa = (unsigned)__cvta_generic_to_shared(X), xs = (unsigned)(sc * sizeof(T));
+  bool ee[2], ww[2], nn[2], ss[2];
+  unsigned ae[2], aw[2], an[2], as[2];  // the neighbours' x, level 0
+#pragma unroll
+  for (int color = 0; color < 2; ++color) {
+    int i, j;
+    const bool ok = tile_column(l, blockIdx.x, color, lane, i, j);
+    const int col = j * l.nx + i;
+    const bool e = ee[color] = ok && i + 1 < l.nx, wv = ww[color] = ok && i > 0;
+    const bool n = nn[color] = ok && j + 1 < l.ny, so = ss[color] = ok && j > 0;
+    ae[color] = remote_column(l, xa, xs, e ? i + 1 : i, j);
+    aw[color] = remote_column(l, xa, xs, wv ? i - 1 : i, j);
+    an[color] = remote_column(l, xa, xs, i, n ? j + 1 : j);
+    as[color] = remote_column(l, xa, xs, i, so ? j - 1 : j);
+    T* A = AC + color * 2 * sc;
+    T* q = Q + color * 6 * rc;
+    constexpr int kL = 4;  // levels whose loads are all in flight (addresses clamped, values masked)
+    const int dw = wv ? 1 : 0, ds = so ? l.nx : 0;
+    for (int kb = w; kb < nz; kb += 8 * kL) {
+      T v[kL][8];
+#pragma unroll
+      for (int u = 0; u < kL; ++u) {
+        const int k = kb + 8 * u;
+        const size_t c = (size_t)(k < nz ? k : nz - 1) * pl + col;
+        v[u][0] = rhs[c];
+        v[u][1] = l.cE[c];
+        v[u][2] = l.cE[c - dw];
+        v[u][3] = l.cN[c];
+        v[u][4] = l.cN[c - ds];
+        v[u][5] = l.li[c];
+        v[u][6] = l.cB[c];
+        v[u][7] = l.lc[c];
+      }
+#pragma unroll
+      for (int u = 0; u < kL; ++u) {
+        const int k = kb + 8 * u, m = k * 32 + lane;
+        if (k >= nz) break;
+        q[m] = ok ? v[u][0] : (T)0;
+        q[rc + m] = e ? v[u][1] : (T)0;
+        q[2 * rc + m] = wv ? v[u][2] : (T)0;
+        q[3 * rc + m] = n ? v[u][3] : (T)0;
+        q[4 * rc + m] = so ? v[u][4] : (T)0;
+        q[5 * rc + m] = ok ? v[u][5] : (T)0;
+        A[k * kScanRS + lane] = (ok && k > 0) ? v[u][6] * v[u][5] : (T)0;
+        A[sc + k * kScanRS + lane] = (ok && k + 1 < nz) ? -v[u][7] : (T)0;
+      }
+    }
+  }
+  __syncthreads();
+  for (int sw = 0; sw < 2 * kCoarseSweeps; ++sw) {
+    const int color = sw & 1;
+    const T* q = Q + color * 6 * rc;
+    ScanTile<T> st(X, nz);
+    st.B = X + color * sc;
+    st.A = AC + color * 2 * sc;
+    st.C = st.A + sc;
+    constexpr int kB = 8;
+    for (int kb = w; kb < nz; kb += 8 * kB) {
+      T xe[kB], xw[kB], xn[kB], xv[kB];
+      if (sw > 0) {
+#pragma unroll
+        for (int u = 0; u < kB; ++u) {
+          const int k = kb + 8 * u;
+          const unsigned o = (unsigned)((k < nz ? k : nz - 1) * kScanRS * (int)sizeof(T));
+          xe[u] = ld_cluster(ae[color] + o, (T)0);
+          xw[u] = ld_cluster(aw[color] + o, (T)0);
+          xn[u] = ld_cluster(an[color] + o, (T)0);
+          xv[u] = ld_cluster(as[color] + o, (T)0);
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < kB; ++u) {
+        const int k = kb + 8 * u;
+        if (k < nz) {
+          const int m = k * 32 + lane;
+          T d = q[m];
+          if (sw > 0) {
+            if (ee[color]) d += q[rc + m] * xe[u];
+            if (ww[color]) d += q[2 * rc + m] * xw[u];
+            if (nn[color]) d += q[3 * rc + m] * xn[u];
+            if (ss[color]) d += q[4 * rc + m] * xv[u];
+          }
+          st.B[k * kScanRS + lane] = d * q[5 * rc + m];
+        }
+      }
+    }
+    __syncthreads();
+    scan_tile_solve<T>(nz, st, tid);
+    cluster_sync();  // the half sweep's x before the next half sweep's loads
+  }
+#pragma unroll
+  for (int color = 0; color < 2; ++color) {
+    ScanTile<T> st(X, nz);
+    st.B = X + color * sc;
+    scan_tile_store<T>(l, x, blockIdx.x, color, st, tid);
+  }
+  // (the last cluster_sync came after every read of a neighbour's shared memory)
+}
+
 constexpr size_t kScanSmemMax = 200 * 1024;   // one tile's shared memory, at most
 constexpr int kCoarseMaxTiles = 64;             // tiles per half sweep up to which one cluster smooths the coarsest grid
 template <typename T>
@@ -437,8 +696,9 @@ size_t scan_smem(int nz) {
   return 3 * (size_t)nz * kScanRS * sizeof(T);
 }
 
-// the residual rhs - A x on the four fine cells of each coarse cell, their
-// mean written as the coarse right-hand side (restriction by the 2 x 2 mean)
+// the residual rhs - A x on the fine cells of each coarse cell that the half
+// sweep just done (colour 1) did not solve: the two with (i + j) even; the
+// mean over the four is the coarse right-hand side
 template <typename T>
 __global__ void k_resid_restrict(MgLevel<T> f, const T* __restrict__ rhs, const T* __restrict__ x, MgLevel<T> cl) {
   const size_t pf = (size_t)f.nx * f.ny;
@@ -446,13 +706,11 @@ __global__ void k_resid_restrict(MgLevel<T> f, const T* __restrict__ rhs, const 
     int I, J, k;
     cell_of(c, cl.nx, cl.ny, I, J, k);
     const int i = 2 * I, j = 2 * J;
-    const size_t f00 = (size_t)k * pf + (size_t)j * f.nx + i;
-    const size_t f10 = f00 + 1, f01 = f00 + f.nx, f11 = f01 + 1;
-    const T t00 = rhs[f00] - apply_at(f, x, f00, i, j, k);
-    const T t10 = rhs[f10] - apply_at(f, x, f10, i + 1, j, k);
-    const T t01 = rhs[f01] - apply_at(f, x, f01, i, j + 1, k);
-    const T t11 = rhs[f11] - apply_at(f, x, f11, i + 1, j + 1, k);
-    cl.r[c] = (t00 + t10 + t01 + t11) * (T)0.25;
+    const size_t f00 = (size_t)k * pf + (size_t)j * f.nx + i, f11 = f00 + f.nx + 1;
+    T t = rhs[f00] - apply_at(f, x, f00, i, j, k);
+    // (the last column or row of an odd grid has no such partner)
+    if (i + 1 < f.nx && j + 1 < f.ny) t += rhs[f11] - apply_at(f, x, f11, i + 1, j + 1, k);
+    cl.r[c] = t * (T)0.25;
   }
 }
 
@@ -497,113 +755,54 @@ struct DotAcc<double> {
   __device__ __forceinline__ double value() const { return s; }
 };
 
+// the block's sum, in thread 0 (the tree halves the FP64 additions down to one
+// warp, which finishes by shuffles)
 __device__ __forceinline__ double block_sum(double v, double* sh) {
   sh[threadIdx.x] = v;
   __syncthreads();
-  for (int w = kMT / 2; w > 0; w >>= 1) {
-    if ((int)threadIdx.x < w) sh[threadIdx.x] += sh[threadIdx.x + w];
+  for (int w = kMT / 2; w >= 32; w >>= 1) {
+    if ((int)threadIdx.x < w) v = sh[threadIdx.x] = v + sh[threadIdx.x + w];
     __syncthreads();
   }
-  const double s = sh[0];
-  __syncthreads();
-  return s;
-}
-
-template <typename T>
-__global__ void k_init(const double* __restrict__ r64, double inv, size_t n, T* r, T* r0, T* x, T* p, T* v,
-                       double* part) {
-  __shared__ double sh[kMT];
-  DotAcc<T> acc;
-  for (size_t q = blockIdx.x * (size_t)kMT + threadIdx.x; q < n; q += (size_t)gridDim.x * kMT) {
-    const T rv = (T)(r64[q] * inv);
-    r[q] = rv;
-    r0[q] = rv;
-    x[q] = 0;
-    p[q] = 0;
-    v[q] = 0;
-    acc.prod(rv, rv);
-  }
-  const double s = block_sum(acc.value(), sh);
-  if (threadIdx.x == 0) part[blockIdx.x] = s;
-}
-
-// p = r + beta (p - omega v), beta from the previous iteration's scalars
-template <typename T>
-__global__ void k_upd_p(const T* __restrict__ r, T* __restrict__ p, const T* __restrict__ v, size_t n,
-                        const double* __restrict__ sc) {
-  const T b = (T)sc[BETA], om = (T)sc[OMEGA];
-  for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < n; q += (size_t)gridDim.x * blockDim.x)
-    p[q] = r[q] + b * (p[q] - om * v[q]);
-}
-
-// y = A xin, partials of (w1, y) [and (y, y) when two]
-template <typename T, bool kTwo>
-__global__ void k_apply_dot(MgLevel<T> l, const T* __restrict__ xin, T* __restrict__ y, const T* __restrict__ w1,
-                            double* part) {
-  __shared__ double sh[kMT];
-  DotAcc<T> a1, a2;
-  for (size_t c = blockIdx.x * (size_t)kMT + threadIdx.x; c < l.n; c += (size_t)gridDim.x * kMT) {
-    int i, j, k;
-    cell_of(c, l.nx, l.ny, i, j, k);
-    const T yv = apply_at(l, xin, c, i, j, k);
-    y[c] = yv;
-    a1.prod(w1[c], yv);
-    if (kTwo) a2.prod(yv, yv);
-  }
-  const double s1 = block_sum(a1.value(), sh);
-  if (threadIdx.x == 0) part[blockIdx.x] = s1;
-  if (kTwo) {
-    const double s2 = block_sum(a2.value(), sh);
-    if (threadIdx.x == 0) part[kMgRedBlocks + blockIdx.x] = s2;
-  }
-}
-
-// s = r - alpha v
-template <typename T>
-__global__ void k_upd_s(const T* __restrict__ r, const T* __restrict__ v, T* __restrict__ s, size_t n,
-                        const double* __restrict__ sc) {
-  const T al = (T)sc[ALPHA];
-  for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < n; q += (size_t)gridDim.x * blockDim.x)
-    s[q] = r[q] - al * v[q];
-}
-
-// x += alpha ph + omega sh; r = s - omega t; partials (r, r), (r0, r)
-template <typename T>
-__global__ void k_upd_xr(T* __restrict__ x, const T* __restrict__ ph, const T* __restrict__ shv,
-                         const T* __restrict__ s, const T* __restrict__ t, T* __restrict__ r,
-                         const T* __restrict__ r0, size_t n, const double* __restrict__ sc, double* part) {
-  __shared__ double sh[kMT];
-  const T al = (T)sc[ALPHA], om = (T)sc[OMEGA];
-  DotAcc<T> a1, a2;
-  for (size_t q = blockIdx.x * (size_t)kMT + threadIdx.x; q < n; q += (size_t)gridDim.x * kMT) {
-    x[q] += al * ph[q] + om * shv[q];
-    const T rv = s[q] - om * t[q];
-    r[q] = rv;
-    a1.prod(rv, rv);
-    a2.prod(r0[q], rv);
-  }
-  const double s1 = block_sum(a1.value(), sh);
-  if (threadIdx.x == 0) part[blockIdx.x] = s1;
-  const double s2 = block_sum(a2.value(), sh);
-  if (threadIdx.x == 0) part[kMgRedBlocks + blockIdx.x] = s2;
+  if (threadIdx.x < 32)
+    for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
+  return v;
 }
 
 enum Op { OP_INIT = 0, OP_ALPHA = 1, OP_OMEGA = 2, OP_XR = 3 };
 
+// What a reducing kernel needs to finish by itself: the block that ends last
+// sums the partials (in block order, whichever it is) and updates the scalars,
+// instead of a launch of its own. done: a counter the last block resets.
 // use_cond: the iteration runs as the body of a graph WHILE node whose
 // condition OP_XR sets (1 = go on, 0 = stop: converged, broken down, or at
 // the iteration limit)
-__global__ void k_finish(const double* __restrict__ part, int nb, int op, double* sc,
-                         cudaGraphConditionalHandle cond, int use_cond) {
-  __shared__ double sh[kMT];
+struct Finish {
+  double *part, *sc;
+  unsigned* done;
+  cudaGraphConditionalHandle cond;
+  int use_cond;
+};
+__device__ __forceinline__ void finish(const Finish& F, int op, double* sh) {
+  __shared__ int last;
+  if (threadIdx.x == 0) {
+    __threadfence();  // this block's partials before its count
+    last = atomicAdd(F.done, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
   double a1 = 0.0, a2 = 0.0;
-  for (int q = threadIdx.x; q < nb; q += kMT) {
-    a1 += part[q];
-    a2 += part[kMgRedBlocks + q];
+  for (int q = threadIdx.x; q < (int)gridDim.x; q += kMT) {
+    a1 += __ldcg(F.part + q);
+    a2 += __ldcg(F.part + kMgRedBlocks + q);
   }
   const double s1 = block_sum(a1, sh);
+  __syncthreads();  // sh is used again
   const double s2 = block_sum(a2, sh);
   if (threadIdx.x != 0) return;
+  *F.done = 0u;
+  double* sc = F.sc;
   if (op == OP_INIT) {
     sc[RR] = s1;
     sc[RHO_NEW] = s1;
@@ -638,12 +837,100 @@ __global__ void k_finish(const double* __restrict__ part, int nb, int op, double
     const double ro = sc[RHO_OLD], om = sc[OMEGA];
     sc[BETA] = (ro != 0.0 && om != 0.0) ? (s2 / ro) * (sc[ALPHA] / om) : 0.0;
     sc[ITERS] += 1.0;
-    if (use_cond) {
+    if (F.use_cond) {
       const bool stop = sc[BREAK] != 0.0 || !(s1 > sc[RTOL2]) || sc[ITERS] >= sc[MAXIT];
-      cudaGraphSetConditional(cond, stop ? 0u : 1u);
+      cudaGraphSetConditional(F.cond, stop ? 0u : 1u);
     }
   }
 }
+template <typename T>
+__global__ void k_init(const double* __restrict__ r64, double inv, size_t n, T* r, T* r0, T* x, T* p, T* v, Finish F) {
+  __shared__ double sh[kMT];
+  DotAcc<T> acc;
+  for (size_t q = blockIdx.x * (size_t)kMT + threadIdx.x; q < n; q += (size_t)gridDim.x * kMT) {
+    const T rv = (T)(r64[q] * inv);
+    r[q] = rv;
+    r0[q] = rv;
+    x[q] = 0;
+    p[q] = 0;
+    v[q] = 0;
+    acc.prod(rv, rv);
+  }
+  const double s = block_sum(acc.value(), sh);
+  if (threadIdx.x == 0) {
+    F.part[blockIdx.x] = s;
+    F.part[kMgRedBlocks + blockIdx.x] = 0.0;
+  }
+  __syncthreads();
+  finish(F, OP_INIT, sh);
+}
+
+// p = r + beta (p - omega v), beta from the previous iteration's scalars
+template <typename T>
+__global__ void k_upd_p(const T* __restrict__ r, T* __restrict__ p, const T* __restrict__ v, size_t n,
+                        const double* __restrict__ sc) {
+  const T b = (T)sc[BETA], om = (T)sc[OMEGA];
+  for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < n; q += (size_t)gridDim.x * blockDim.x)
+    p[q] = r[q] + b * (p[q] - om * v[q]);
+}
+
+// y = A xin, partials of (w1, y) [and (y, y) when two]
+template <typename T, bool kTwo>
+__global__ void k_apply_dot(MgLevel<T> l, const T* __restrict__ xin, T* __restrict__ y, const T* __restrict__ w1,
+                            Finish F) {
+  __shared__ double sh[kMT];
+  DotAcc<T> a1, a2;
+  for (size_t c = blockIdx.x * (size_t)kMT + threadIdx.x; c < l.n; c += (size_t)gridDim.x * kMT) {
+    int i, j, k;
+    cell_of(c, l.nx, l.ny, i, j, k);
+    const T yv = apply_at(l, xin, c, i, j, k);
+    y[c] = yv;
+    a1.prod(w1[c], yv);
+    if (kTwo) a2.prod(yv, yv);
+  }
+  const double s1 = block_sum(a1.value(), sh);
+  if (threadIdx.x == 0) F.part[blockIdx.x] = s1;
+  __syncthreads();
+  double s2 = 0.0;
+  if (kTwo) s2 = block_sum(a2.value(), sh);
+  if (threadIdx.x == 0) F.part[kMgRedBlocks + blockIdx.x] = s2;
+  __syncthreads();
+  finish(F, kTwo ? OP_OMEGA : OP_ALPHA, sh);
+}
+
+// s = r - alpha v
+template <typename T>
+__global__ void k_upd_s(const T* __restrict__ r, const T* __restrict__ v, T* __restrict__ s, size_t n,
+                        const double* __restrict__ sc) {
+  const T al = (T)sc[ALPHA];
+  for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < n; q += (size_t)gridDim.x * blockDim.x)
+    s[q] = r[q] - al * v[q];
+}
+
+// x += alpha ph + omega sh; r = s - omega t; partials (r, r), (r0, r)
+template <typename T>
+__global__ void k_upd_xr(T* __restrict__ x, const T* __restrict__ ph, const T* __restrict__ shv,
+                         const T* __restrict__ s, const T* __restrict__ t, T* __restrict__ r,
+                         const T* __restrict__ r0, size_t n, Finish F) {
+  __shared__ double sh[kMT];
+  const T al = (T)F.sc[ALPHA], om = (T)F.sc[OMEGA];
+  DotAcc<T> a1, a2;
+  for (size_t q = blockIdx.x * (size_t)kMT + threadIdx.x; q < n; q += (size_t)gridDim.x * kMT) {
+    x[q] += al * ph[q] + om * shv[q];
+    const T rv = s[q] - om * t[q];
+    r[q] = rv;
+    a1.prod(rv, rv);
+    a2.prod(r0[q], rv);
+  }
+  const double s1 = block_sum(a1.value(), sh);
+  if (threadIdx.x == 0) F.part[blockIdx.x] = s1;
+  __syncthreads();
+  const double s2 = block_sum(a2.value(), sh);
+  if (threadIdx.x == 0) F.part[kMgRedBlocks + blockIdx.x] = s2;
+  __syncthreads();
+  finish(F, OP_XR, sh);
+}
+
 __global__ void k_stop_test(double* sc, double rtol2, int max_iter) {
   sc[RTOL2] = rtol2;
   sc[MAXIT] = (double)max_iter;
@@ -704,8 +991,10 @@ void vcycle(MgSolver<T>* m, int li, const T* rhs, T* x, cudaStream_t s) {
     if (m->coarse_ctas > 0) {
       cudaLaunchConfig_t cfg;
       cudaLaunchAttribute at;
-      coarse_config(m->coarse_ctas, scan_smem<T>(l.nz), s, cfg, at);
-      cudaLaunchKernelEx(&cfg, k_coarse_smooth<T>, l, rhs, x);
+      coarse_config(m->coarse_ctas, m->coarse_resident ? coarse_resident_smem<T>(l.nz) : scan_smem<T>(l.nz), s, cfg,
+                    at);
+      if (m->coarse_resident) cudaLaunchKernelEx(&cfg, k_coarse_resident<T>, l, rhs, x);
+      else cudaLaunchKernelEx(&cfg, k_coarse_smooth<T>, l, rhs, x);
       return;
     }
     smooth(l, rhs, x, 0, 1, s);
@@ -721,8 +1010,14 @@ void vcycle(MgSolver<T>* m, int li, const T* rhs, T* x, cudaStream_t s) {
   smooth(l, rhs, x, 1, 0, s);
   k_resid_restrict<T><<<cells_grid(cl.n), kMT, 0, s>>>(l, rhs, x, cl);
   vcycle(m, li + 1, cl.r, cl.x, s);
-  k_prolong_add<T><<<cells_grid(l.n), kMT, 0, s>>>(l, x, cl);
-  smooth(l, rhs, x, 1, 0, s);
+  const size_t sm = scan_smem<T>(l.nz);
+  if (sm <= kScanSmemMax) {
+    k_smooth_add<T><<<((l.nx + 1) / 2 * l.ny + 31) / 32, 256, sm, s>>>(l, rhs, x, 1, cl.x, cl.nx,
+                                                                      (size_t)cl.nx * cl.ny);
+  } else {
+    k_prolong_add<T><<<cells_grid(l.n), kMT, 0, s>>>(l, x, cl);
+    smooth(l, rhs, x, 1, 0, s);
+  }
   smooth(l, rhs, x, 0, 0, s);
 }
 
@@ -735,6 +1030,17 @@ T* dev_alloc(MgSolver<T>* m, size_t n) {
 }
 
 }  // namespace
+
+void hz_residual(const HGeo& g, const double* a, const double* b, const double* f, const double* x, double* r,
+                 cudaStream_t s) {
+  const int xt = (g.nx + kResCols - 1) / kResCols;
+  const size_t tiles = (size_t)xt * ((g.ny + kResRows - 1) / kResRows);
+  // about 24 blocks an SM (the last wave), chunks of at least 4 levels (a chunk computes its first lower face again)
+  const int want = tiles >= 3648 ? 1 : (int)(3648 / tiles);
+  int kz = imax((g.nz + want - 1) / want, 4);
+  kz = imax(kz, (g.nz + 65534) / 65535);
+  k_residual64<<<dim3((unsigned)tiles, (g.nz + kz - 1) / kz), dim3(32, kResRows + 1), 0, s>>>(g, a, b, f, x, r, xt, kz);
+}
 
 template <typename T>
 MgSolver<T>* mg_create(const HGeo& g, int max_levels) {
@@ -755,9 +1061,9 @@ MgSolver<T>* mg_create(const HGeo& g, int max_levels) {
       ok = ok && *a != nullptr;
     }
     m->L = l + 1;
-    if (nx % 2 || ny % 2 || nx / 2 < 4 || ny / 2 < 4) break;
-    nx /= 2;
-    ny /= 2;
+    if (nx / 2 < 4 || ny / 2 < 4) break;
+    nx = (nx + 1) / 2;
+    ny = (ny + 1) / 2;
   }
   const size_t n = g.n();
   T** kv[] = {&m->x, &m->r, &m->r0, &m->p, &m->v, &m->s, &m->t, &m->ph, &m->sh};
@@ -771,12 +1077,17 @@ MgSolver<T>* mg_create(const HGeo& g, int max_levels) {
   p = nullptr;
   ok = ok && cudaMalloc(&p, NSC * sizeof(double)) == cudaSuccess;
   if (p) m->allocs.push_back(p), m->sc = (double*)p;
+  p = nullptr;
+  ok = ok && cudaMalloc(&p, sizeof(unsigned)) == cudaSuccess && cudaMemset(p, 0, sizeof(unsigned)) == cudaSuccess;
+  if (p) m->allocs.push_back(p), m->done = (unsigned*)p;
   ok = ok && cudaMallocHost(&m->hsc, NSC * sizeof(double)) == cudaSuccess;
   // the tiled smoother's FP64 tiles need more than the default 48 KB
   if (scan_smem<T>(g.nz) <= kScanSmemMax) {
     ok = ok && cudaFuncSetAttribute(k_smooth_scan<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)kScanSmemMax) == cudaSuccess;
     ok = ok && cudaFuncSetAttribute(k_smooth_scan<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)kScanSmemMax) == cudaSuccess;
+    ok = ok && cudaFuncSetAttribute(k_smooth_add<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)kScanSmemMax) == cudaSuccess;
     // the coarsest grid in one cluster launch when it is a few tiles: one
     // CTA per tile, up to a portable cluster (FP32 only: the FP64 rate of a
@@ -793,6 +1104,14 @@ MgSolver<T>* mg_create(const HGeo& g, int max_levels) {
       int clusters = 0;
       if (cudaOccupancyMaxActiveClusters(&clusters, k_coarse_smooth<T>, &cfg) == cudaSuccess && clusters > 0)
         m->coarse_ctas = ctas;
+      if (m->coarse_ctas == ntiles && coarse_resident_smem<T>(g.nz) <= kScanSmemMax) {
+        ok = ok && cudaFuncSetAttribute(k_coarse_resident<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)kScanSmemMax) == cudaSuccess;
+        coarse_config(ctas, coarse_resident_smem<T>(g.nz), nullptr, cfg, at);
+        clusters = 0;
+        m->coarse_resident =
+            cudaOccupancyMaxActiveClusters(&clusters, k_coarse_resident<T>, &cfg) == cudaSuccess && clusters > 0;
+      }
       cudaGetLastError();  // (a cluster launch that cannot run leaves the launches per half sweep)
     }
   }
@@ -836,14 +1155,12 @@ void enqueue_iteration(MgSolver<T>* m, cudaStream_t s, cudaGraphConditionalHandl
   MgLevel<T>& f = m->lv[0];
   k_upd_p<T><<<cg, kMT, 0, s>>>(m->r, m->p, m->v, n, m->sc);
   vcycle(m, 0, m->p, m->ph, s);
-  k_apply_dot<T, false><<<nb, kMT, 0, s>>>(f, m->ph, m->v, m->r0, m->part);
-  k_finish<<<1, kMT, 0, s>>>(m->part, nb, OP_ALPHA, m->sc, cond, 0);
+  const Finish F{m->part, m->sc, m->done, cond, use_cond};
+  k_apply_dot<T, false><<<nb, kMT, 0, s>>>(f, m->ph, m->v, m->r0, F);
   k_upd_s<T><<<cg, kMT, 0, s>>>(m->r, m->v, m->s, n, m->sc);
   vcycle(m, 0, m->s, m->sh, s);
-  k_apply_dot<T, true><<<nb, kMT, 0, s>>>(f, m->sh, m->t, m->s, m->part);
-  k_finish<<<1, kMT, 0, s>>>(m->part, nb, OP_OMEGA, m->sc, cond, 0);
-  k_upd_xr<T><<<nb, kMT, 0, s>>>(m->x, m->ph, m->sh, m->s, m->t, m->r, m->r0, n, m->sc, m->part);
-  k_finish<<<1, kMT, 0, s>>>(m->part, nb, OP_XR, m->sc, cond, use_cond);
+  k_apply_dot<T, true><<<nb, kMT, 0, s>>>(f, m->sh, m->t, m->s, F);
+  k_upd_xr<T><<<nb, kMT, 0, s>>>(m->x, m->ph, m->sh, m->s, m->t, m->r, m->r0, n, F);
 }
 
 // The iteration loop as one graph: a WHILE conditional node (default 1 at
@@ -903,8 +1220,8 @@ int mg_solve(MgSolver<T>* m, const double* r64, double* d64, double rtol, int ma
     cudaMemsetAsync(d64, 0, n * sizeof(double), s);
     return 0;
   }
-  k_init<T><<<nb, kMT, 0, s>>>(r64, 1.0 / rn, n, m->r, m->r0, m->x, m->p, m->v, m->part);
-  k_finish<<<1, kMT, 0, s>>>(m->part, nb, OP_INIT, m->sc, cudaGraphConditionalHandle{}, 0);
+  k_init<T><<<nb, kMT, 0, s>>>(r64, 1.0 / rn, n, m->r, m->r0, m->x, m->p, m->v,
+                               Finish{m->part, m->sc, m->done, cudaGraphConditionalHandle{}, 0});
   k_stop_test<<<1, 1, 0, s>>>(m->sc, rtol * rtol, max_iter);
   if (m->graph_state == 0) {
     // VIBE_GB300_HELMHOLTZ_GRAPH=0 keeps the host loop (one scalar read per iteration)
