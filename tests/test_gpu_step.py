@@ -161,6 +161,37 @@ def test_slow_tendency_mixed(vg, oc, scheme, levels, monkeypatch):
         assert_levels_close(vg, s, got, ref, 1e-4, range(n), "mixed slow tendency per level", lf)
 
 
+@pytest.mark.parametrize("levels", ["", "3"])
+@pytest.mark.parametrize("dims", [(33, 9, 11), (70, 18, 13), (20, 16, 12)])
+def test_slow_tendency_mixed_patchy_moisture(vg, oc, dims, levels, monkeypatch):
+    """Moisture in patches: whole tiles and columns of a species are zero,
+    others hold its edge, at tile corners, the ground, the lid and across the
+    starts of level chunks; one species has none at all. The mixed tendency
+    against the oracle's, at the tolerances of the smooth moist case."""
+    monkeypatch.setenv("VIBE_GB300_STAGE_LEVELS", levels)
+    nx, ny, nz = dims
+    s = small_setup(vg, nx=nx, ny=ny, nz=nz, moist=1, qv_surface=0.01, shear_u=0.004, bubble_xc=nx * 125.0,
+                    bubble_yc=ny * 125.0)
+    k, j, i = np.meshgrid(np.arange(nz), np.arange(ny), np.arange(nx), indexing="ij")
+    centre = {7: (0, 0, nx - 1), 8: (nz - 1, ny - 1, 0), 9: (4, 8, 31), 11: (nz // 2, ny // 2, 2)}
+    with vg.Model(s, vg.MIXED) as m:
+        o = oc.Model(oracle_setup(oc, s), "port")
+        for sp, (ck, cj, ci) in centre.items():
+            r = np.sqrt(((k - ck) / 4.0) ** 2 + ((j - cj) / 5.0) ** 2 + ((i - ci) / 6.0) ** 2)
+            a = o.get(sp).reshape(vg.storage_shape(s, sp))
+            vg.interior(s, sp, a)[...] = np.where(r < 1, 2e-3 * np.cos(0.5 * np.pi * np.minimum(r, 1)) ** 2, 0.0)
+            o.set(sp, a)
+            m.set(sp, a)
+        ref, got = o.slow_tendency(), m.slow_tendency()
+        floors = {sp: 1e-3 * np.abs(vg.interior(s, sp, o.get(sp))).max() for sp in range(12)}
+        vs = 1e-3 * velocity_scale(vg, s, o.state())
+        for sp in (0, 1, 2):
+            floors[sp] = max(floors[sp], vs)
+        assert_state_close(vg, s, got, ref, TOLMX, range(12), "patchy moisture", floors, velocity=False)
+        lf = {sp: 1e-2 * floors[sp] for sp in range(12)}
+        assert_levels_close(vg, s, got, ref, 1e-4, range(12), "patchy moisture per level", lf)
+
+
 @pytest.mark.parametrize("pgf", [0, 1])
 def test_acoustic_substep_fp64(vg, oc, pgf):
     s = small_setup(vg, pgf_perturbation=pgf)

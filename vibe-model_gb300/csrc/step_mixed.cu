@@ -53,33 +53,7 @@ struct MS64 {
 //  * the weights a_k = d_k/s_k^2 are normalised with one division:
 //    numerator and denominator scaled by (s0 s1 s2)^2, all terms positive
 //    and far inside the FP32 range (s_k in [1e-6, ~1e4]).
-__device__ __forceinline__ float weno_left(float qm2, float qm1, float q0, float q1, float q2, float s0, float s1,
-                                           float s2) {
-  const float v0 = (2.f * qm2 - 7.f * qm1 + 11.f * q0) * (1.f / 6.f);
-  const float v1 = (-qm1 + 5.f * q0 + 2.f * q1) * (1.f / 6.f);
-  const float v2 = (2.f * q0 + 5.f * q1 - q2) * (1.f / 6.f);
-  const float p01 = s0 * s1, p02 = s0 * s2, p12 = s1 * s2;
-  const float w0 = 0.1f * (p12 * p12), w1 = 0.6f * (p02 * p02), w2 = 0.3f * (p01 * p01);
-  return __fdividef(w0 * v0 + w1 * v1 + w2 * v2, w0 + w1 + w2);
-}
-__device__ __forceinline__ float weno_face_f(float qm2, float qm1, float q0, float q1, float q2, float vel) {
-  const float eps = 1e-6f;
-  const float e0 = qm2 - 2.f * qm1 + q0, f0 = qm2 - 4.f * qm1 + 3.f * q0;
-  const float e1 = qm1 - 2.f * q0 + q1, f1 = qm1 - q1;
-  const float e2 = q0 - 2.f * q1 + q2, f2 = 3.f * q0 - 4.f * q1 + q2;
-  const float s0 = eps + (13.f / 12.f) * (e0 * e0) + 0.25f * (f0 * f0);
-  const float s1 = eps + (13.f / 12.f) * (e1 * e1) + 0.25f * (f1 * f1);
-  const float s2 = eps + (13.f / 12.f) * (e2 * e2) + 0.25f * (f2 * f2);
-  const bool up = vel >= 0.f;  // upwind-ordered stencil (no divergence)
-  const float a0 = up ? qm2 : q2, a1 = up ? qm1 : q1, a3 = up ? q1 : qm1, a4 = up ? q2 : qm2;
-  const float t0 = up ? s0 : s2, t2 = up ? s2 : s0;
-  const float rec = weno_left(a0, a1, q0, a3, a4, t0, s1, t2);
-  if (fabsf(vel) >= 1e-3f) return vel * rec;
-  const float oth = weno_left(a4, a3, q0, a1, a0, t2, s1, t0);  // the other side
-  const float ql = up ? rec : oth, qr = up ? oth : rec;
-  return 0.5f * (vel * (ql + qr) - 1e-3f * (qr - ql));
-}
-
+//
 // ---- theta' and qv side by side: packed FP32 pairs ----
 // The stage kernel reconstructs theta' and qv at the same faces with the
 // same velocity, so their WENO5 arithmetic runs on f32x2 pairs (low:
@@ -118,8 +92,7 @@ __device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
 __device__ __forceinline__ F2 sel2(bool p, F2 a, F2 b) { return p ? a : b; }
 
 // WENO5 left-biased reconstruction of the stencil a0..a4 (centre a2) with
-// smoothness indicators s0..s2, as weno_left; the candidates are formed at
-// 6x and the 1/6 folded into the normalisation
+// smoothness indicators s0..s2; the candidates are formed at 6x and the 1/6 folded into the normalisation
 __device__ __forceinline__ F2 weno_left2(F2 a0, F2 a1, F2 a2, F2 a3, F2 a4, F2 s0, F2 s1, F2 s2) {
   const F2 V0 = fma2(dup2(11.f), a2, fma2(dup2(-7.f), a1, add2(a0, a0)));
   const F2 V1 = fma2(dup2(5.f), a2, sub2(add2(a3, a3), a1));
@@ -135,7 +108,7 @@ __device__ __forceinline__ F2 weno_left2(F2 a0, F2 a1, F2 a2, F2 a3, F2 a4, F2 s
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(i1) : "f"(d1));
   return mul2(num, mk2(i0, i1));
 }
-// WENO5 face flux of a pair (local Lax-Friedrichs, as weno_face_f) from the
+// WENO5 face flux of a pair (local Lax-Friedrichs) from the
 // stencil in upwind order: qm2 qm1 q0 q1 q2 for vel >= 0, its mirror image
 // q2 q1 q0 qm1 qm2 for vel < 0 (centre q0 either way). The smoothness
 // indicators of the mirrored stencil are the original ones in reverse
@@ -209,8 +182,13 @@ constexpr long long kSpinLimit = 1ll << 24;  // bounded mbarrier waits
 
 struct StageMaps {
   CUtensorMap m[NTILE];
+  CUtensorMap mq[5];  // qc, qr, qi, qs, qg (moist models)
   int xmax[NTILE], ymax[NTILE];
 };
+// Moisture beyond qv: a ring of three slots, one per pair (qc qr, qi qs, qg),
+// and each thread's top-face fluxes, in dynamic shared memory
+constexpr int kPairs = 3;
+constexpr unsigned kMoistSmem = (kPairs * 2 * SZ3 + kPairs * 2 * NT) * sizeof(float);
 
 // TMA-fed column kernel: a block owns 64 x 4 columns (two per thread); per
 // level one box per field, 72 floats wide from i0-4 (16-byte aligned x):
@@ -232,16 +210,6 @@ struct ColumnMaps {
   CUtensorMap m[kColBoxes];
   CUtensorMap back[kBackBoxes];  // w, rho', pi' of the output
 };
-
-// plain loader with the TMA box geometry (moisture species beyond qv)
-__device__ __forceinline__ void load_box3(float* __restrict__ dst, const float* __restrict__ plane, int P, int i0,
-                                          int j0, int xmax, int ymax) {
-  for (int e = threadIdx.y * TX + threadIdx.x; e < R3 * TW; e += NT) {
-    const int ty = e / TW, tx = e - ty * TW;
-    const int gi = iclamp(i0 - XO + tx, 0, xmax), gj = iclamp(j0 - 3 + ty, 0, ymax);
-    dst[e] = plane[gj * P + gi];
-  }
-}
 
 __device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void mbar_init(unsigned long long* b, unsigned count) {
@@ -287,6 +255,15 @@ __device__ __forceinline__ void issue_level(const StageMaps& M, float* buf, unsi
   tma_load_3d(buf + tile_off(TR), &M.m[TR], i0 - XO, j0 - 1, kc, bar);
 }
 
+// pair p's boxes of level k (p = 2: qg alone)
+__device__ __forceinline__ void issue_pair(const StageMaps& M, float* slot, unsigned long long* bar, int i0, int j0,
+                                           int k, int p) {
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  mbar_expect_tx(bar, (p < 2 ? 2 : 1) * R3 * TW * 4);
+  tma_load_3d(slot, &M.mq[2 * p], i0 - XO, j0 - 3, k, bar);
+  if (p < 2) tma_load_3d(slot + SZ3, &M.mq[2 * p + 1], i0 - XO, j0 - 3, k, bar);
+}
+
 // replace out-of-range box elements by the clamped ones: columns first, then
 // whole rows (so corners get clamp(x) and clamp(y))
 __device__ void fix_box(float* t, int rows, int halo, int i0, int j0, int xmax, int ymax, int tid) {
@@ -317,9 +294,10 @@ __device__ __forceinline__ void stage_body(const Dims& d, const Tab& t, const Fl
                                            const WS& win, const WS& w0, const WS& wout, const WS& rout, float dts,
                                            int kchunk, unsigned* err, int bx, int by, int bz) {
   __shared__ __align__(128) float sbuf[kStageRing][kBuf];
-  __shared__ __align__(128) float sQm[R3 * TW], sQm2[R3 * TW];  // a pair of moisture species beyond qv (plain loads)
+  extern __shared__ __align__(128) float sMoist[];  // moist models: kMoistSmem
   __shared__ float sFx[2][TY * (TX + 1)], sFy[2][(TY + 1) * TX];  // theta' / qv (or a moisture pair)
-  __shared__ __align__(8) unsigned long long sbar[kStageRing];
+  __shared__ __align__(8) unsigned long long sbar[kStageRing], sbarM[kPairs];
+  __shared__ int sfail;
   // the flags, fixed at compile time for the kSpec composition
   const bool f_weno = kSpec || fl.weno_scalars, f_adv = kSpec || fl.weno_advective;
   const bool f_moist = !kSpec && fl.moist, f_dd = !kSpec && fl.div_damp > 0.0;
@@ -351,6 +329,26 @@ __device__ __forceinline__ void stage_body(const Dims& d, const Tab& t, const Fl
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     for (int L = kb; L <= hi; ++L) issue_level(M, sbuf[L - kb], &sbar[L - kb], i0, j0, L, nz);
   }
+  // Moisture pairs: item n = (k - kb) kPairs + p is pair p of level k, in slot
+  // p, phase (k - kb) & 1; while item n is computed, n + 1 and n + 2 are in flight
+  const int items = (imin(klast, nz - 1) - kb + 1) * kPairs;
+  int m_next = 0, m_hi = -1;  // next item to wait for, last item issued
+  if (f_moist) {
+    if (tid == 0) {
+      sfail = 0;
+      for (int p = 0; p < kPairs; ++p) mbar_init(&sbarM[p], 1);
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+      for (int p = 0; p < 2; ++p) issue_pair(M, sMoist + p * 2 * SZ3, &sbarM[p], i0, j0, kb, p);
+    }
+    m_hi = 1;
+  }
+  // after a wait that ran out, thread 0: every copy still in flight, from level L up
+  auto drain = [&](int L) {
+    atomicOr(err, (unsigned)kErrWaitTimeout);
+    for (int l = L; l <= hi; ++l)
+      mbar_wait_bounded(&sbar[(l - kb) % kStageRing], (unsigned)((l - kb) / kStageRing) & 1u);
+    for (int n = m_next; n <= m_hi; ++n) mbar_wait_bounded(&sbarM[n % kPairs], (unsigned)(n / kPairs) & 1u);
+  };
   // bounded wait for level L by one thread, released to the block by the
   // barrier; on a timeout thread 0 drains every copy still in flight
   auto level_ready = [&](int L) -> bool {
@@ -358,11 +356,7 @@ __device__ __forceinline__ void stage_body(const Dims& d, const Tab& t, const Fl
     const bool arrived =
         (tid != 0) || mbar_wait_bounded(&sbar[lev % kStageRing], (unsigned)(lev / kStageRing) & 1u);
     if (__syncthreads_or(!arrived)) {
-      if (tid == 0) {
-        atomicOr(err, (unsigned)kErrWaitTimeout);
-        for (int l = L; l <= hi; ++l)
-          mbar_wait_bounded(&sbar[(l - kb) % kStageRing], (unsigned)((l - kb) / kStageRing) & 1u);
-      }
+      if (tid == 0) drain(L);
       return false;
     }
     return true;
@@ -414,6 +408,12 @@ __device__ __forceinline__ void stage_body(const Dims& d, const Tab& t, const Fl
     const unsigned c = (unsigned)k * pl + colc;
     const bool do_u = cells_here && in_box && j < ny, do_v = cells_here && in_box && i < nx;
     float bU = 0.f, bV = 0.f, bW = 0.f, bR = 0.f, bP = 0.f, bT = 0.f, bQ = 0.f;
+    float cond[5] = {0.f, 0.f, 0.f, 0.f, 0.f};  // qc, qr, qi, qs, qg at kc
+    if (f_moist && cell) {
+      const unsigned ckc = (unsigned)kc * pl + colc;
+#pragma unroll
+      for (int m = 0; m < 5; ++m) cond[m] = win.f[QC + m][ckc];
+    }
     if (has_base && !base_in) {
       if (do_u) bU = w0.f[U][c];
       if (do_v) bV = w0.f[V][c];
@@ -467,21 +467,8 @@ __device__ __forceinline__ void stage_body(const Dims& d, const Tab& t, const Fl
       bT = sT[o3];
       bQ = sQ[o3];
     }
-    // base value of q at this point: preloaded for the dynamic fields
-    auto base_of = [&](int q) -> float {
-      switch (q) {
-        case U: return bU;
-        case V: return bV;
-        case W: return bW;
-        case RHO: return bR;
-        case PI: return bP;
-        case THETA: return bT;
-        case QV: return bQ;
-        default: return w0.f[q][c];
-      }
-    };
-    auto emit = [&](int q, float r) {
-      const float o = has_base ? base_of(q) + dts * r : r;  // no base: raw tendency
+    auto emit = [&](int q, float r, float base) {
+      const float o = has_base ? base + dts * r : r;  // no base: raw tendency
       wout.f[q][c] = o;
       fsum += o;
       if (kRaw) rout.f[q][c] = r;
@@ -497,7 +484,7 @@ __device__ __forceinline__ void stage_body(const Dims& d, const Tab& t, const Fl
       float r = -(uc * ux + vc * uy + wc * uz);
       if (f_cor) r += (f_cor == 2 ? t.f0 + t.beta * (((float)j + 0.5f) * t.dy - 0.5f * (float)ny * t.dy) : t.f0) * vc;
       r -= cp * (0.5f * (sT[o3 + dim] + sT[o3 + ipu])) * (sP[o1 + ipu] - sP[o1 + dim]) * t.dx_inv;
-      emit(U, r);
+      emit(U, r, bU);
     }
     if (do_v) {  // v face (i, j, k)
       const int dp1 = jpv * TW, dm1 = djm * TW;
@@ -511,7 +498,7 @@ __device__ __forceinline__ void stage_body(const Dims& d, const Tab& t, const Fl
       float r = -(uc * vx + vc * vy + wc * vz);
       if (f_cor) r -= (f_cor == 2 ? t.f0 + t.beta * (((float)j + 0.5f) * t.dy - 0.5f * (float)ny * t.dy) : t.f0) * uc;
       r -= cp * (0.5f * (sT[o3 + djm * TW] + sT[o3 + jpv * TW])) * (sP[o1 + dp1] - sP[o1 + dm1]) * t.dy_inv;
-      emit(V, r);
+      emit(V, r, bV);
     }
     // w face (i, j, k), k = 0..nz; at k = nz the boxes other than w hold level nz-1 = kc
     const float wk = sW[o1];
@@ -530,11 +517,10 @@ __device__ __forceinline__ void stage_body(const Dims& d, const Tab& t, const Fl
       r -= cp * (0.5f * (thm + thc)) * (pic - pim) * t.idzw[k];
       float qcond = 0.f, qvc = wQ[3];  // qv(kc)
       if (f_moist) {
-        const unsigned ckc = (unsigned)kc * pl + colc;
-        qcond = win.f[QC][ckc] + win.f[QR][ckc] + win.f[QI][ckc] + win.f[QS][ckc] + win.f[QG][ckc];
+        qcond = cond[0] + cond[1] + cond[2] + cond[3] + cond[4];
       }
       r += (float)kG * (thc * t.th0inv[kc] + (float)kBuoyMoist * qvc - qcond);
-      emit(W, r);
+      emit(W, r, bW);
     }
     if (!cells_here) break;
     const float wt = g_wt;  // w at face k+1
@@ -544,7 +530,7 @@ __device__ __forceinline__ void stage_body(const Dims& d, const Tab& t, const Fl
       const float fy = sV[o1 + TW] * 0.5f * (rc + sR[o1 + TW]) - sV[o1] * 0.5f * (sR[o1 - TW] + rc);
       const float rkp = g_rk;
       const float fz = wt * 0.5f * (rc + rkp) - wk * 0.5f * (rprev + rc);
-      emit(RHO, -(fx * t.dx_inv + fy * t.dy_inv + fz * t.idzc[k]));
+      emit(RHO, -(fx * t.dx_inv + fy * t.dy_inv + fz * t.idzc[k]), bR);
       float r = 0.f;
       if (f_dd) {
         const float pc = sP[o1];
@@ -552,49 +538,22 @@ __device__ __forceinline__ void stage_body(const Dims& d, const Tab& t, const Fl
                           (sP[o1 + TW] - 2.f * pc + sP[o1 - TW]) * (t.dy_inv * t.dy_inv);
         r = -(float)fl.div_damp * lap;
       }
-      emit(PI, r);
+      emit(PI, r, bP);
     }
     // ---- scalars ----
     const float idz = t.idza[k];
     const bool vert = (k + 2 < nz || k >= 2);
     const float* sh = t.t0d + 6 * k;  // theta0(clamp(k+m)) - theta0(k), m = -3..2
     const float divh = (sU[o1 + 1] - sU[o1]) * t.dx_inv + (sV[o1 + TW] - sV[o1]) * t.dy_inv;
-    // A species' box at level k is Q. With WENO its horizontal face fluxes
-    // are first computed into sFx[slot] / sFy[slot] by all threads
-    // (hflux for one species, hflux_pair for two as an f32x2 pair: slots 0
-    // and 1), and after one barrier `scalar` reads them with the vertical
-    // face fluxes; theta' and qv share that barrier, as do the two species of
-    // a moisture pair.
-    auto hflux = [&](const float* Q, int slot) {
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const int t_ = tid + e * NT;
-        if (t_ < TY * (TX + 1)) {
-          const int fr = t_ / (TX + 1), ff = t_ - fr * (TX + 1);
-          float F = 0.f;
-          if (i0 + ff <= nx && j0 + fr < ny) {
-            const float* qq = Q + (fr + 3) * TW + ff + XO;  // cell i0+ff, the face's right cell
-            F = weno_face_f(qq[-3], qq[-2], qq[-1], qq[0], qq[1], sU[(fr + 1) * TW + ff + XO]);
-          }
-          sFx[slot][t_] = F;
-        }
-        if (t_ < (TY + 1) * TX) {
-          const int fg = t_ / TX, fcl = t_ - fg * TX;
-          float G = 0.f;
-          if (j0 + fg <= ny && i0 + fcl < nx) {
-            const float* qq = Q + (fg + 3) * TW + fcl + XO;
-            G = weno_face_f(qq[-3 * TW], qq[-2 * TW], qq[-TW], qq[0], qq[TW], sV[(fg + 1) * TW + fcl + XO]);
-          }
-          sFy[slot][t_] = G;
-        }
-      }
-    };
+    // A species' box at level k is Q. With WENO the horizontal face fluxes of
+    // two species are first computed into slots 0 and 1 of sFx / sFy by all
+    // threads (hflux_pair), and after one barrier `scalar` reads them with the
+    // vertical face fluxes.
     // theta' and qv together: every face of the tile, TY (TX+1) x faces and
     // (TY+1) TX y faces, reconstructs both species as one f32x2 pair (same
     // face velocity, same stencil addresses in the two boxes), the stencil
     // loaded in upwind order by choosing the addresses; x and y faces share
-    // one code path with the stencil stride chosen per face. Same face values
-    // as hflux up to rounding.
+    // one code path with the stencil stride chosen per face.
     auto hflux_pair = [&](const float* A, const float* B) {  // species A and B (theta', qv or a moisture pair)
       // one x and one y face pair per thread: its cell's left and lower
       // faces; the top row's y faces go to warp 0 and the right column's x
@@ -625,14 +584,18 @@ __device__ __forceinline__ void stage_body(const Dims& d, const Tab& t, const Fl
     };
     // species q's tendency from its horizontal face fluxes (slot) and its
     // vertical ones: ft through the top face, fb through the bottom face
-    // (WENO), or the column values z2 = q(k-1), z4 = q(k+1) (central)
-    auto scalar = [&](int q, const float* Q, int slot, float ft, float fb, float z2, float z4) {
+    // (WENO), or the column values z2 = q(k-1), z4 = q(k+1) (central).
+    // flat: the box is zero, its fluxes were not formed
+    auto scalar = [&](int q, const float* Q, int slot, float ft, float fb, float z2, float z4, float base, bool flat) {
       float r = 0.f;
       const float qc = Q[o3];
       if (f_weno) {
         if (cell) {
-          const float fe = sFx[slot][ty * (TX + 1) + tx + 1], fw = sFx[slot][ty * (TX + 1) + tx];
-          const float fn = sFy[slot][(ty + 1) * TX + tx], fs = sFy[slot][ty * TX + tx];
+          float fe = 0.f, fw = 0.f, fn = 0.f, fs = 0.f;
+          if (!flat) {
+            fe = sFx[slot][ty * (TX + 1) + tx + 1], fw = sFx[slot][ty * (TX + 1) + tx];
+            fn = sFy[slot][(ty + 1) * TX + tx], fs = sFy[slot][ty * TX + tx];
+          }
           r = -(fe - fw) * t.dx_inv - (fn - fs) * t.dy_inv;
           float div = divh;
           if (vert) {
@@ -652,7 +615,7 @@ __device__ __forceinline__ void stage_body(const Dims& d, const Tab& t, const Fl
       }
       if (cell) {
         if (q >= QV && qc <= 0.f && r < 0.f) r = 0.f;
-        emit(q, r);
+        emit(q, r, base);
       }
     };
     // theta' is advected as theta - theta0(k): the carried flux of level
@@ -679,40 +642,103 @@ __device__ __forceinline__ void stage_body(const Dims& d, const Tab& t, const Fl
       }
       __syncthreads();
     }
-    scalar(THETA, sT, 0, ftT, fbT, wT[2] + sh[2], wT[4] + sh[4]);
-    scalar(QV, sQ, 1, ftQ, fbQ, wQ[2], wQ[4]);
+    scalar(THETA, sT, 0, ftT, fbT, wT[2] + sh[2], wT[4] + sh[4], bT, false);
+    scalar(QV, sQ, 1, ftQ, fbQ, wQ[2], wQ[4], bQ, false);
     if (f_moist) {
-      // the moisture species in pairs (qc qr, qi qs, and qg with itself),
-      // each pair's faces reconstructed as one f32x2 pair like theta' and qv
-      for (int qa = QC; qa <= QG; qa += 2) {
-        const int qb = (qa + 1 <= QG) ? qa + 1 : qa;
-        __syncthreads();  // sQm, sQm2 and the flux slots are no longer read
-        load_box3(sQm, win.f[qa] + (unsigned)k * pl, P, i0, j0, nx - 1, ny - 1);
-        if (qb != qa) load_box3(sQm2, win.f[qb] + (unsigned)k * pl, P, i0, j0, nx - 1, ny - 1);
-        __syncthreads();
-        const float* const QB = (qb != qa) ? sQm2 : sQm;
-        if (f_weno) {
-          hflux_pair(sQm, QB);
-          __syncthreads();
-        }
+      // The moisture species in pairs (qc qr, qi qs, and qg with itself), each
+      // pair's faces reconstructed as one f32x2 pair like theta' and qv. The
+      // boxes come through the ring, the column's other values and the base
+      // are loaded before the wait, and the top face's pair is carried up in
+      // shared memory. Where a pair's box is all zero (cloud and rain away
+      // from clouds, ice in a warm-rain run) every horizontal flux is zero
+      // and none is formed; likewise the vertical ones of a warp whose
+      // columns are zero at the five levels. Bound by issue
+      // and barriers. 256 x 256 x 80, cloud and rain in a bubble, no ice: the
+      // stage takes 707 us, 1004 us with boxes loaded by the threads, every
+      // face formed and the vertical ones twice.
+#pragma unroll 1
+      for (int p = 0; p < kPairs; ++p) {
+        const int qa = QC + 2 * p, qb = (p < 2) ? qa + 1 : qa;
+        float* const QA = sMoist + p * 2 * SZ3;
+        float* const QB = (p < 2) ? QA + SZ3 : QA;
+        float* const carry = sMoist + kPairs * 2 * SZ3 + p * 2 * NT + tid;
         float za[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, zb[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-        float fta = 0.f, fba = 0.f, ftb = 0.f, fbb = 0.f;
+        float ba = 0.f, bb = 0.f;
         if (cell) {
+          const float *fa = win.f[qa] + colc, *fb = win.f[qb] + colc;
 #pragma unroll
-          for (int m = 0; m < 6; ++m) {
-            const unsigned o = (unsigned)iclamp(k + m - 3, 0, nz - 1) * pl + colc;
-            za[m] = win.f[qa][o];
-            zb[m] = win.f[qb][o];
+          for (int m = 1; m < 6; ++m) {
+            if (m == 3) continue;  // the box's centre
+            const unsigned o = (unsigned)iclamp(k + m - 3, 0, nz - 1) * pl;
+            za[m] = fa[o];
+            zb[m] = fb[o];
+          }
+          if (has_base && !base_in) {
+            ba = w0.f[qa][c];
+            bb = w0.f[qb][c];
+          }
+        }
+        const bool arrived = mbar_wait_bounded(&sbarM[p], (unsigned)(k - kb) & 1u);
+        if (!arrived) sfail = 1;
+        unsigned any = arrived ? 0u : 1u;
+        constexpr int n4 = R3 * TW / 4;
+        for (int e = tid; e < (p < 2 ? 2 * n4 : n4); e += NT) {
+          const uint4 v = *reinterpret_cast<const uint4*>(e < n4 ? QA + 4 * e : QB + 4 * (e - n4));
+          any |= (v.x | v.y | v.z | v.w) & 0x7fffffffu;
+        }
+        const bool flat = !__syncthreads_or((int)any);  // (also: the pair before is no longer read)
+        if (!flat && sfail) {
+          if (tid == 0) drain(k + 1);
+          return;
+        }
+        ++m_next;
+        if (m_hi + 1 < items) {
+          ++m_hi;
+          const int pn = m_hi % kPairs;
+          if (tid == 0) issue_pair(M, sMoist + pn * 2 * SZ3, &sbarM[pn], i0, j0, kb + m_hi / kPairs, pn);
+        }
+        if (!flat) {
+          if (edge) {
+            fix_box(QA, R3, 3, i0, j0, nx - 1, ny - 1, tid);
+            if (p < 2) fix_box(QB, R3, 3, i0, j0, nx - 1, ny - 1, tid);
+            __syncthreads();
           }
           if (f_weno) {
-            const F2 z1 = mk2(za[1], zb[1]), z2 = mk2(za[2], zb[2]), z4 = mk2(za[4], zb[4]);
-            const F2 qc2 = mk2(sQm[o3], QB[o3]);
-            un2(weno_vflux2(z1, z2, qc2, z4, mk2(za[5], zb[5]), wt), fta, ftb);
-            un2(weno_vflux2(mk2(za[0], zb[0]), z1, z2, qc2, z4, wk), fba, fbb);
+            hflux_pair(QA, QB);
+            __syncthreads();
           }
         }
-        scalar(qa, sQm, 0, fta, fba, za[2], za[4]);
-        if (qb != qa) scalar(qb, QB, 1, ftb, fbb, zb[2], zb[4]);
+        const float ca = QA[o3], cb = QB[o3];
+        if (base_in) {
+          ba = ca;
+          bb = cb;
+        }
+        float fta = 0.f, fba = 0.f, ftb = 0.f, fbb = 0.f;
+        if (f_weno) {
+          const unsigned col = __float_as_uint(za[1]) | __float_as_uint(za[2]) | __float_as_uint(za[4]) |
+                               __float_as_uint(za[5]) | __float_as_uint(zb[1]) | __float_as_uint(zb[2]) |
+                               __float_as_uint(zb[4]) | __float_as_uint(zb[5]) | __float_as_uint(ca) |
+                               __float_as_uint(cb);
+          if (cell) {
+            if (k > kb) {
+              fba = carry[0];
+              fbb = carry[NT];
+            } else {
+              const unsigned o = (unsigned)iclamp(k - 3, 0, nz - 1) * pl + colc;
+              un2(weno_vflux2(mk2(win.f[qa][o], win.f[qb][o]), mk2(za[1], zb[1]), mk2(za[2], zb[2]), mk2(ca, cb),
+                              mk2(za[4], zb[4]), wk), fba, fbb);
+            }
+          }
+          if (__any_sync(0xffffffffu, cell && (col & 0x7fffffffu) != 0u)) {
+            if (cell)
+              un2(weno_vflux2(mk2(za[1], zb[1]), mk2(za[2], zb[2]), mk2(ca, cb), mk2(za[4], zb[4]),
+                              mk2(za[5], zb[5]), wt), fta, ftb);
+          }
+          carry[0] = fta;
+          carry[NT] = ftb;
+        }
+        scalar(qa, QA, 0, fta, fba, za[2], za[4], ba, flat);
+        if (p < 2) scalar(qb, QB, 1, ftb, fbb, zb[2], zb[4], bb, flat);
       }
     }
     // slide the column registers up one level
@@ -1387,7 +1413,7 @@ bool box_map(const float* base, int xext, int yext, int zext, int P, size_t plan
   return true;
 }
 
-bool stage_maps(const Dims& d, const WS& win, StageMaps& M) {
+bool stage_maps(const Dims& d, const Flags& fl, const WS& win, StageMaps& M) {
   struct Spec { int q, xe, ye, ze, rows; };
   const Spec sp[NTILE] = {{THETA, d.nx, d.ny, d.nz, R3},     {QV, d.nx, d.ny, d.nz, R3},
                           {U, d.nx + 1, d.ny, d.nz, R1},     {V, d.nx, d.ny + 1, d.nz, R1},
@@ -1398,7 +1424,27 @@ bool stage_maps(const Dims& d, const WS& win, StageMaps& M) {
     M.xmax[b] = sp[b].xe - 1;
     M.ymax[b] = sp[b].ye - 1;
   }
+  if (fl.moist)
+    for (int m = 0; m < 5; ++m)
+      if (!box_map(win.f[QC + m], d.nx, d.ny, d.nz, d.P, d.plane, R3, &M.mq[m])) return false;
   return true;
+}
+struct StageArgs;
+template <bool kRaw, bool kSpec>
+__global__ void k_b_stage(const StageArgs* __restrict__ A, const int* __restrict__ start, int nd, unsigned* err);
+// the moisture ring's dynamic shared memory; false: it could not be raised
+bool stage_smem(const Flags& fl, unsigned* bytes) {
+  *bytes = fl.moist ? kMoistSmem : 0;
+  if (!fl.moist) return true;
+  bool ok = true;
+  auto raise = [&](auto* k) {
+    ok = ok && cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMoistSmem) == cudaSuccess;
+  };
+  raise(k_mx_stage<true, false>);
+  raise(k_mx_stage<false, false>);
+  raise(k_b_stage<true, false>);
+  raise(k_b_stage<false, false>);
+  return ok;
 }
 
 // boxes of the TMA-fed column kernel: every field over the whole padded
@@ -1418,7 +1464,8 @@ bool column_maps(const Dims& d, const WS& win, const WS& wout, ColumnMaps& C) {
 int mixed_stage(const Dims& d, const Tab& t, const Flags& fl, const WS& win, const WS& w0, const WS& wout,
                 const WS* rout, double dt_stage, unsigned* err, cudaStream_t stream) {
   StageMaps M;
-  if (!stage_maps(d, win, M)) return -1;
+  unsigned sm;
+  if (!stage_maps(d, fl, win, M) || !stage_smem(fl, &sm)) return -1;
   const dim3 b(TX, TY);
   const bool raw = rout != nullptr;
   const int kchunk = stage_kchunk(d, raw);
@@ -1427,11 +1474,11 @@ int mixed_stage(const Dims& d, const Tab& t, const Flags& fl, const WS& win, con
   if (raw && spec)
     k_mx_stage<true, true><<<g, b, 0, stream>>>(d, t, fl, M, win, w0, wout, *rout, (float)dt_stage, kchunk, err);
   else if (raw)
-    k_mx_stage<true, false><<<g, b, 0, stream>>>(d, t, fl, M, win, w0, wout, *rout, (float)dt_stage, kchunk, err);
+    k_mx_stage<true, false><<<g, b, sm, stream>>>(d, t, fl, M, win, w0, wout, *rout, (float)dt_stage, kchunk, err);
   else if (spec)
     k_mx_stage<false, true><<<g, b, 0, stream>>>(d, t, fl, M, win, w0, wout, wout, (float)dt_stage, kchunk, err);
   else
-    k_mx_stage<false, false><<<g, b, 0, stream>>>(d, t, fl, M, win, w0, wout, wout, (float)dt_stage, kchunk, err);
+    k_mx_stage<false, false><<<g, b, sm, stream>>>(d, t, fl, M, win, w0, wout, wout, (float)dt_stage, kchunk, err);
   return 0;
 }
 
@@ -2959,6 +3006,7 @@ struct MixedBatch {
   std::vector<Launch> seq;
   std::vector<void*> allocs;
   size_t hevi_smem = 0;
+  unsigned stage_smem = 0;
   int split = 0, nz = 0;  // split > 0: the level-split column body with that many levels per warp
   bool hevi_tma = false;  // TMA-fed column body (else the cp.async two-column body)
   bool defer = false;     // the TMA body defers its w/rho' corrections (u/v launches become fix-ups)
@@ -3008,7 +3056,7 @@ MixedBatch* mixed_batch_build(const std::vector<MixedDomain>& doms, const Flags&
   const double dts[3] = {dt / 3.0, dt / 2.0, dt};
   const int nd = (int)doms.size();
   auto sub_out = [&](const MixedDomain& m, int n) { return (n & 1) ? m.WB : m.WA; };
-  bool ok = true;
+  bool ok = stage_smem(fl, &b->stage_smem);
   for (int stage = 0; stage < 3 && ok; ++stage) {
     std::vector<StageArgs> sa(nd);
     std::vector<int> start(nd);
@@ -3019,7 +3067,7 @@ MixedBatch* mixed_batch_build(const std::vector<MixedDomain>& doms, const Flags&
       float* const* st_out = stage & 1 ? m.WSt1 : m.WSt0;
       const WS win = (stage == 0) ? ws_from(m.W0) : ws_mix(sub_out(m, n_sub - 1), (stage - 1) & 1 ? m.WSt1 : m.WSt0);
       StageArgs& a = sa[q];
-      ok = stage_maps(m.d, win, a.M);
+      ok = stage_maps(m.d, fl, win, a.M);
       a.d = m.d;
       a.t = m.t;
       a.fl = fl;
@@ -3124,11 +3172,11 @@ void mixed_batch_enqueue(const MixedBatch* b, cudaStream_t s) {
         if (L.raw && b->spec)
           k_b_stage<true, true><<<L.blocks, dim3(TX, TY), 0, s>>>((const StageArgs*)L.args, L.start, L.nd, b->err);
         else if (L.raw)
-          k_b_stage<true, false><<<L.blocks, dim3(TX, TY), 0, s>>>((const StageArgs*)L.args, L.start, L.nd, b->err);
+          k_b_stage<true, false><<<L.blocks, dim3(TX, TY), b->stage_smem, s>>>((const StageArgs*)L.args, L.start, L.nd, b->err);
         else if (b->spec)
           k_b_stage<false, true><<<L.blocks, dim3(TX, TY), 0, s>>>((const StageArgs*)L.args, L.start, L.nd, b->err);
         else
-          k_b_stage<false, false><<<L.blocks, dim3(TX, TY), 0, s>>>((const StageArgs*)L.args, L.start, L.nd, b->err);
+          k_b_stage<false, false><<<L.blocks, dim3(TX, TY), b->stage_smem, s>>>((const StageArgs*)L.args, L.start, L.nd, b->err);
         break;
       case 1:
         if (b->split)
