@@ -86,6 +86,30 @@ def test_kessler_tendency_matches_oracle(vg, oc, prec, offset):
             assert vg.interior(s, 7, got[7]).max() > 0.0  # condensation somewhere
 
 
+@pytest.mark.parametrize("dims", [(7, 5, 1), (33, 3, 7), (20, 5, 8), (31, 2, 9), (32, 4, 17)])
+@pytest.mark.parametrize("prec", ["FP64", "MIXED"])
+def test_kessler_level_tiles(vg, oc, prec, dims):
+    """Rain through every level, at the edges of the tiles of 32 columns by 8
+    levels the column is taken in (one level, a last tile of one level, a last
+    block of a few columns), at the tolerances of the cloudy state above."""
+    nx, ny, nz = dims
+    s = setup(vg, nx=nx, ny=ny, nz=nz, z_top=250.0 * nz, **({} if prec == "FP64" else dict(terrain_kind=0, ref_kind=0)))
+    kg, ko = kessler(vg, oc, 0)
+    rng = np.random.default_rng(11)
+    with vg.Model(s, getattr(vg, prec)) as m:
+        o = oc.Model(oracle_setup(oc, s), "port")
+        st = [a.copy() for a in m.state()]
+        for sp, amp in ((7, 2e-3), (8, 4e-3)):
+            a = vg.interior(s, sp, st[sp])
+            a[...] = amp * rng.uniform(0.1, 1.0, a.shape)
+        m.set_state(st)
+        o.set_state(st)
+        m.set_physics_kessler(kg)
+        got = m.physics_tendency(6.0)
+        ref = dict(zip((4, 6, 7, 8), oc.kessler_tendency(o, ko, 6.0)))
+        close(vg, s, got, ref, TOL_TEND64 if prec == "FP64" else TOL_TEND32, "tendency")
+
+
 @pytest.mark.parametrize("prec", ["FP64", "MIXED"])
 def test_rk3_steps_with_kessler_match_oracle(vg, oc, prec):
     """Two RK3 steps with the package coupled at every stage against the

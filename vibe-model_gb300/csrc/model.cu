@@ -733,13 +733,26 @@ __global__ void k_add_pt64(size_t n, const double* __restrict__ pt, double* __re
 }
 // mixed path: the stage kernel has written s = s0 + dt_s R; add dt_s pt, and
 // pt to the stage-3 tendency R the finish kernel folds into the FP64 state
-__global__ void k_add_pt32(size_t n, const float* __restrict__ pt, float* __restrict__ s, float dts,
-                           float* __restrict__ r) {
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
-    const float p = pt[e];
-    s[e] = s[e] + dts * p;
-    if (r) r[e] = r[e] + p;
-  }
+// (bound by memory: 12 or 20 bytes an element; planes are padded to whole
+// float4s. 256 x 256 x 81: 20 to 12.5 us)
+__global__ void k_add_pt32(size_t n4, const float4* __restrict__ pt, float4* __restrict__ s, float dts,
+                           float4* __restrict__ r) {
+  const size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+  if (e >= n4) return;
+  const float4 p = pt[e];
+  float4 v = s[e];
+  v.x = v.x + dts * p.x;
+  v.y = v.y + dts * p.y;
+  v.z = v.z + dts * p.z;
+  v.w = v.w + dts * p.w;
+  s[e] = v;
+  if (!r) return;
+  float4 t = r[e];
+  t.x = t.x + p.x;
+  t.y = t.y + p.y;
+  t.z = t.z + p.z;
+  t.w = t.w + p.w;
+  r[e] = t;
 }
 
 // zero the accumulators and let the package enqueue its work for this stage
@@ -847,8 +860,9 @@ int enqueue_one_step(vibe_gb300_model* m, double dt, int n_sub) {
             const size_t n = d.plane * (size_t)(d.nz + 1);
             for (int q : kPhysFields)
               if (m->phys_written & (1u << q))
-                k_add_pt32<<<1024, 256, 0, m->stream>>>(n, (const float*)m->pt[q], st_out[q], (float)dts[stage],
-                                                        stage == 2 ? m->WR[q] : nullptr);
+                k_add_pt32<<<(unsigned)((n / 4 + 255) / 256), 256, 0, m->stream>>>(
+                    n / 4, (const float4*)m->pt[q], (float4*)st_out[q], (float)dts[stage],
+                    stage == 2 ? (float4*)m->WR[q] : nullptr);
           }
         }
         const float dtau = (float)(dts[stage] / (double)n_sub);

@@ -12,13 +12,15 @@
 // PhysicsColumn::diagnose_layer_depth, physics_types.cpp:257-284) and the
 // tendencies are (after - before) / dt (physics_driver.cpp:271-288).
 //
-// One thread per column marching from the top level down. Every process of
-// the scheme at level k depends only on level k and on the rain flux falling
-// from level k+1, so the four passes of the column step (saturation
-// adjustment, autoconversion + accretion, sedimentation from the top, rain
-// evaporation) are done level by level in one top-down sweep with the same
-// result. tgamma(1 + b) and cbrt(Sc) of the reference are constants, taken
-// from the host's libm.
+// Every process of the scheme at level k depends only on level k and on the
+// rain flux falling from level k+1, so a block takes 32 columns and marches
+// down in tiles of 8 levels, one warp a level: the adjustment, conversion and
+// fall terms of a tile's levels at once, the flux through them in one warp
+// (one multiply-add, minimum and division a level), evaporation at once.
+// Bound by issue and the latency of the Newton iterations; one thread per
+// column left 13 warps an SM with all of a column's chain in each.
+// 256 x 256 x 80, mixed: 423 to 222 us. tgamma(1 + b) and cbrt(Sc) of the
+// reference are constants, taken from the host's libm.
 #include <cmath>
 
 #include "vibe_gb300.h"
@@ -135,11 +137,15 @@ template <class R> __device__ __forceinline__ R tot(const float* s, const double
   return (R)s[c] + (R)ref[c];
 }
 
+constexpr int kKessLevels = 8;  // levels of a tile, a warp each
+
 template <class T, class R>
-__global__ void k_kessler(const vibe_gb300_physics_args a, KesslerParams<R> o) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int j = blockIdx.y * blockDim.y + threadIdx.y;
-  if (i >= a.nx || j >= a.ny) return;
+__global__ void __launch_bounds__(32 * kKessLevels) k_kessler(const vibe_gb300_physics_args a, KesslerParams<R> o) {
+  __shared__ R s_mass[2][kKessLevels][32], s_out[2][kKessLevels][32];
+  const int lane = threadIdx.x, w = threadIdx.y;
+  const int q = blockIdx.x * 32 + lane;
+  const bool in = q < a.nx * a.ny;
+  const int j = in ? q / a.nx : 0, i = in ? q - j * a.nx : 0;
   const int nz = a.nz;
   const R dt = (R)a.dt;
   const size_t plane = (size_t)a.pitch * (a.ny + 1), col = (size_t)j * a.pitch + i;
@@ -155,63 +161,77 @@ __global__ void k_kessler(const vibe_gb300_physics_args a, KesslerParams<R> o) {
   T* t_qr = (T*)a.tend[QR];
   const bool mixed = sizeof(T) == sizeof(float);
   const R zs = (R)a.terrain[(size_t)j * a.nx + i], depth = (R)a.depth[(size_t)j * a.nx + i];
-  auto zc = [&](int k) { return zs + (R)a.zeta_mid[k] * depth; };  // Grid::z_center
-  R flux_in = (R)0;
-  // level heights around the current level, carried down the column
-  R z_up = (R)0, z_here = zc(nz - 1), z_dn = (nz > 1) ? zc(nz - 2) : (R)0;
-  for (int k = nz - 1; k >= 0; --k) {
-    const size_t c = (size_t)k * plane + col;
-    // layer depth (diagnose_layer_depth): interfaces halfway between centres,
-    // extrapolated at the bottom and top; 100 m for a single level
-    R dz;
-    if (nz == 1) {
-      dz = rmax((z_here + (R)0.5 * (R)100) - (z_here - (R)0.5 * (R)100), (R)1.0e-6);
-    } else {
-      const R z = z_here;
-      const R zlo = (k == 0) ? z - (R)0.5 * (z_up - z) : (R)0.5 * (z_dn + z);
-      const R zhi = (k == nz - 1) ? z + (R)0.5 * (z - z_dn) : (R)0.5 * (z + z_up);
-      dz = rmax(zhi - zlo, (R)1.0e-6);
-    }
-    z_up = z_here;
-    z_here = z_dn;
-    if (k >= 2) z_dn = zc(k - 2);
-    // state_to_column
-    const R pi0 = (R)a.ref_pi[c];
-    const R pis = mixed ? tot<R>(pi_s, a.ref_pi, c) : (R)pi_s[c];
-    const R pi = o.exner_offset ? pi0 + pis : pis;
-    const R p = (R)kP0 * rpow(rmax(pi, (R)1.0e-3), (R)1 / (R)kKappaPhys);
-    R theta = mixed ? tot<R>(th_s, a.ref_theta, c) : (R)th_s[c];
-    R qv = rmax((R)qv_s[c], (R)0), qc = rmax((R)qc_s[c], (R)0), qr = rmax((R)qr_s[c], (R)0);
-    R rho = mixed ? tot<R>(rho_s, a.ref_rho, c) : (R)rho_s[c];
-    if (!(rho > (R)0)) {  // density from p and the virtual temperature
-      const R qi = rmax((R)((const T*)a.state[QI])[c], (R)0), qsn = rmax((R)((const T*)a.state[QS])[c], (R)0),
-              qg = rmax((R)((const T*)a.state[QG])[c], (R)0);
-      const R tv = theta * exner_of(p) * ((R)1 + (R)0.608 * qv - qc - qi - qsn - qg);
-      rho = p / ((R)kRd * tv);
-    }
-    const R th0 = theta, qv0 = qv, qc0 = qc, qr0 = qr;
-    // 1. saturation adjustment
-    adjust(qv, qc, theta, p);
-    // 2. autoconversion + accretion
-    {
-      const R cq = rmax(qc, (R)0), rq = rmax(qr, (R)0);
-      const R rate = o.k1 * rmax(cq - o.qc0, (R)0) + o.k2 * rmax(cq, (R)0) * rmax(rq, (R)0);
-      const R dq = rmin(rate * dt, cq);
-      qc = cq - dq;
-      qr = rq + dq;
-    }
-    // 3. sedimentation: upstream flux from the level above, limited by the mass available
-    {
+  R flux_in = (R)0;  // warp 0: the rain flux into the tile
+  for (int ktop = nz - 1, b = 0; ktop >= 0; ktop -= kKessLevels, b ^= 1) {
+    const int k = ktop - w;
+    const bool here = in && k >= 0;
+    const size_t c = (size_t)imax(k, 0) * plane + col;
+    R theta = (R)0, qv = (R)0, qc = (R)0, qr = (R)0, rho = (R)0, p = (R)0, rhd = (R)1;
+    R th0 = (R)0, qv0 = (R)0, qc0 = (R)0, qr0 = (R)0;
+    // zeta at the levels below, at and above k: lanes 0..2 convert one each
+    const R zm = (R)a.zeta_mid[iclamp(k - 1 + imin(lane, 2), 0, nz - 1)];
+    const R zm_dn = __shfl_sync(0xffffffffu, zm, 0), zm_at = __shfl_sync(0xffffffffu, zm, 1),
+            zm_up = __shfl_sync(0xffffffffu, zm, 2);
+    if (here) {
+      // layer depth (diagnose_layer_depth): interfaces halfway between centres,
+      // extrapolated at the bottom and top; 100 m for a single level
+      // (Grid::z_center)
+      const R z = zs + zm_at * depth, z_up = zs + zm_up * depth, z_dn = zs + zm_dn * depth;
+      R dz;
+      if (nz == 1) {
+        dz = rmax((z + (R)0.5 * (R)100) - (z - (R)0.5 * (R)100), (R)1.0e-6);
+      } else {
+        const R zlo = (k == 0) ? z - (R)0.5 * (z_up - z) : (R)0.5 * (z_dn + z);
+        const R zhi = (k == nz - 1) ? z + (R)0.5 * (z - z_dn) : (R)0.5 * (z + z_up);
+        dz = rmax(zhi - zlo, (R)1.0e-6);
+      }
+      // state_to_column
+      const R pi0 = (R)a.ref_pi[c];
+      const R pis = mixed ? tot<R>(pi_s, a.ref_pi, c) : (R)pi_s[c];
+      const R pi = o.exner_offset ? pi0 + pis : pis;
+      p = (R)kP0 * rpow(rmax(pi, (R)1.0e-3), (R)1 / (R)kKappaPhys);
+      theta = mixed ? tot<R>(th_s, a.ref_theta, c) : (R)th_s[c];
+      qv = rmax((R)qv_s[c], (R)0), qc = rmax((R)qc_s[c], (R)0), qr = rmax((R)qr_s[c], (R)0);
+      rho = mixed ? tot<R>(rho_s, a.ref_rho, c) : (R)rho_s[c];
+      if (!(rho > (R)0)) {  // density from p and the virtual temperature
+        const R qi = rmax((R)((const T*)a.state[QI])[c], (R)0), qsn = rmax((R)((const T*)a.state[QS])[c], (R)0),
+                qg = rmax((R)((const T*)a.state[QG])[c], (R)0);
+        const R tv = theta * exner_of(p) * ((R)1 + (R)0.608 * qv - qc - qi - qsn - qg);
+        rho = p / ((R)kRd * tv);
+      }
+      th0 = theta, qv0 = qv, qc0 = qc, qr0 = qr;
+      // 1. saturation adjustment
+      adjust(qv, qc, theta, p);
+      // 2. autoconversion + accretion
+      {
+        const R cq = rmax(qc, (R)0), rq = rmax(qr, (R)0);
+        const R rate = o.k1 * rmax(cq - o.qc0, (R)0) + o.k2 * rmax(cq, (R)0) * rmax(rq, (R)0);
+        const R dq = rmin(rate * dt, cq);
+        qc = cq - dq;
+        qr = rq + dq;
+      }
+      // 3. sedimentation: upstream flux from the level above, limited by the mass available
       const R rh = rmax(rho, (R)1.0e-6), d = rmax(dz, (R)1.0e-6), rq = rmax(qr, (R)0);
-      const R mass = rh * rq * d;
-      const R vt = fall_speed(o, rh, rq);
-      const R available = mass + flux_in * dt;
-      const R out = rmin(rh * rq * vt * dt, rmax(available, (R)0));
-      qr = rmax(available - out, (R)0) / (rh * d);
-      flux_in = out / dt;
+      const R vt = (rq > (R)0) ? fall_speed(o, rh, rq) : (R)0;
+      const R load = rh * rq;
+      rhd = rh * d;
+      s_mass[b][w][lane] = load * d;
+      s_out[b][w][lane] = load * vt * dt;
     }
-    // 4. rain evaporation into subsaturated air
-    {
+    __syncthreads();
+    if (w == 0 && in) {
+      for (int u = 0; u < kKessLevels && u <= ktop; ++u) {
+        const R available = fma(flux_in, dt, s_mass[b][u][lane]);
+        const R out = rmin(s_out[b][u][lane], rmax(available, (R)0));
+        s_mass[b][u][lane] = available;
+        s_out[b][u][lane] = out;
+        flux_in = out / dt;
+      }
+    }
+    __syncthreads();  // (the other buffer's tile lies between this one's reads and its next writes)
+    if (here) {
+      qr = rmax(s_mass[b][w][lane] - s_out[b][w][lane], (R)0) / rhd;
+      // 4. rain evaporation into subsaturated air
       const R rq = rmax(qr, (R)0);
       if (rq > (R)0) {
         const R pk = exner_of(p);
@@ -231,18 +251,21 @@ __global__ void k_kessler(const vibe_gb300_physics_args a, KesslerParams<R> o) {
           }
         }
       }
+      // 5. positivity
+      if (o.positive_definite) {
+        qv = rmax(qv, (R)0);
+        qc = rmax(qc, (R)0);
+        qr = rmax(qr, (R)0);
+      }
+      // PhysicsTendency (accumulated onto the zeroed buffers; most air has none)
+      auto add = [&](T* t, R d) {
+        if (d != (R)0) t[c] += (T)(d / dt);
+      };
+      add(t_th, theta - th0);
+      add(t_qv, qv - qv0);
+      add(t_qc, qc - qc0);
+      add(t_qr, qr - qr0);
     }
-    // 5. positivity
-    if (o.positive_definite) {
-      qv = rmax(qv, (R)0);
-      qc = rmax(qc, (R)0);
-      qr = rmax(qr, (R)0);
-    }
-    // PhysicsTendency (accumulated onto the zeroed buffers)
-    t_th[c] += (T)((theta - th0) / dt);
-    t_qv[c] += (T)((qv - qv0) / dt);
-    t_qc[c] += (T)((qc - qc0) / dt);
-    t_qr[c] += (T)((qr - qr0) / dt);
   }
 }
 
@@ -289,7 +312,8 @@ int vibe_gb300_physics_kessler(void* user, vibe_gb300_physics_args* a) {
   for (int q : {THETA, QV, QC, QR})
     if (!a->tend[q]) return VIBE_GB300_EBADARG;
   const vibe_gb300_kessler& k = *static_cast<const vibe_gb300_kessler*>(user);
-  const dim3 b(32, 4), g((a->nx + 31) / 32, (a->ny + 3) / 4);
+  const dim3 b(32, kKessLevels);
+  const unsigned g = (unsigned)(((size_t)a->nx * a->ny + 31) / 32);
   cudaStream_t s = static_cast<cudaStream_t>(a->stream);
   a->written = (1u << THETA) | (1u << QV) | (1u << QC) | (1u << QR);
   if (a->precision == VIBE_GB300_MIXED) k_kessler<float, float><<<g, b, 0, s>>>(*a, params_of<float>(k));
