@@ -493,6 +493,36 @@ def test_level_split_column_kernel_edges(vg, oc, dims, dt, n_sub):
         assert_state_close(vg, t, m.state(), o.state(), 2 * TOLMX, range(7), "level-split column kernel %s" % (dims,))
 
 
+def test_column_kernel_dense_atmosphere(vg):
+    """Under 100 bar pi0/rho0 is so small that rho' is not taken from pi': the
+    built-in choice is the sweeping column kernel, with its bits, and a group
+    with such a member sweeps all of its members (1e-6: the same update)."""
+    kw = dict(nx=33, ny=9, nz=14, zeta_stretch=1.0, bubble_xc=4000.0, bubble_yc=1000.0, **STEP_CASES[3])
+    sets = [small_setup(vg, **kw), small_setup(vg, p_surf=1e7, **kw)]
+    swept = []
+    for t in sets:
+        with vg.Model(t, vg.MIXED) as m:
+            m.set_tuning(column_kernel=5)
+            try:
+                m.step(1.0, 3, 2)
+            finally:
+                m.set_tuning()
+            swept.append(m.state())
+    with vg.Model(sets[1], vg.MIXED) as m:
+        m.step(1.0, 3, 2)
+        for sp, (a, b) in enumerate(zip(m.state(), swept[1])):
+            assert np.array_equal(a, b), vg.SPECIES[sp]
+    grouped = [vg.Model(t, vg.MIXED) for t in sets]
+    try:
+        with vg.Group(grouped) as g:
+            g.step(1.0, 3, 2)
+            for m, t, ref in zip(grouped, sets, swept):
+                assert_state_close(vg, t, m.state(), ref, 1e-6, range(7), "in a group")
+    finally:
+        for m in grouped:
+            m.close()
+
+
 def test_autotune_keeps_the_update(vg):
     """The autotuner only chooses among launch shapes of the same update: a run
     after tuning matches the run before it to FP32 rounding (1e-6 of each

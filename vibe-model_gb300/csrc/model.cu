@@ -431,6 +431,9 @@ int build_tables(vibe_gb300_model* m) {
   auto R = [&](int w, int k) { return hs.ref[w][soff(cx, cy, 0, 0, k)]; };
   std::vector<double> r0(nz), t0(nz), p0(nz);
   for (int k = 0; k < nz; ++k) { t0[k] = R(0, k); p0[k] = R(1, k); r0[k] = R(2, k); }
+  m->fl.rho_from_pi = 1;
+  for (int k = 0; k < nz; ++k)
+    if (!((kRd / kCv) * (p0[k] / dmax(r0[k], 1e-8)) >= kKapMin)) m->fl.rho_from_pi = 0;
   const double zt = m->su.z_top;
   auto dzeta = [&](int k) { const int kk = iclamp(k, 0, nz - 1); return hs.zeta[kk + 1] - hs.zeta[kk]; };
   std::vector<float>& f = m->ftab_host;
@@ -872,7 +875,7 @@ int enqueue_one_step(vibe_gb300_model* m, double dt, int n_sub) {
           if (m->fl.acoustic_mode == 2) {
             // the u/v update of substep n-1 is applied inside substep n's column kernel
             Span sp(m, 1);
-            if (mixed_hevi_column(d, m->tab, m->fl, ws_of(in), ws_of(out), dtau, m->d_lu + (size_t)stage * 3 * d.nz,
+            if (mixed_hevi_column(d, m->tab, m->fl, ws_of(in), ws_of(out), ws_of(st_out), dtau, m->d_lu + (size_t)stage * 3 * d.nz,
                                   n > 0, n == n_sub - 1, m->d_err, m->stream))
               return fail(VIBE_GB300_EDEVICE, "TMA descriptor creation failed (cuTensorMapEncodeTiled)");
           } else {
@@ -2205,7 +2208,9 @@ int group_prepare(vibe_gb300_group* g, double dt, int n_sub) {
       md.S1 = m->S[1 - p];
       doms.push_back(md);
     }
-    g->batch[p] = mixed_batch_build(doms, g->ms[0]->fl, dt, n_sub, g->d_err);
+    Flags fl = g->ms[0]->fl;
+    for (const vibe_gb300_model* m : g->ms) fl.rho_from_pi = fl.rho_from_pi && m->fl.rho_from_pi;
+    g->batch[p] = mixed_batch_build(doms, fl, dt, n_sub, g->d_err);
     if (!g->batch[p]) return fail(VIBE_GB300_EDEVICE, "group launch set-up failed");
   }
   g->dt = dt;

@@ -110,9 +110,10 @@ int mixed_hevi_substep(const Dims& d, const Tab& t, const Flags& fl, const WS& w
                        const float* lu /* 3*nz: a, cprime, inv_denom */, unsigned* err, cudaStream_t stream);
 // returns nonzero when a TMA descriptor cannot be made. apply_uv: win is the
 // output of a substep whose u/v update (and deferred corrections) are still
-// to be applied; last: no further substep follows in the stage
-int mixed_hevi_column(const Dims& d, const Tab& t, const Flags& fl, const WS& win, const WS& wout, float dtau,
-                      const float* lu, bool apply_uv, bool last, unsigned* err, cudaStream_t stream);
+// to be applied; wst: the input of the stage's first substep, unchanged since;
+// last: no further substep follows in the stage
+int mixed_hevi_column(const Dims& d, const Tab& t, const Flags& fl, const WS& win, const WS& wout, const WS& wst,
+                      float dtau, const float* lu, bool apply_uv, bool last, unsigned* err, cudaStream_t stream);
 void mixed_uv_backward(const Dims& d, const Tab& t, const WS& win, const WS& wout, float dtau, cudaStream_t stream);
 // whether the column kernel chosen for this grid defers its w/rho'
 // corrections to the reader (then the last substep of a stage is finished

@@ -2390,23 +2390,31 @@ size_t hevi_tma_smem_bytes(int nz) {
 // 8-byte load or store; rows run on into each other, so only the P - nx
 // padding points idle) by one chunk; a block is the C = ceil(nz/kM) chunks of
 // its 64 points. Per-level constants lie in float4 tables with the step's
-// scalars folded in. The eliminated pi' never leaves the registers: 40 B/cell
-// of traffic, against 48 of the sweeping kernel.
-// All but a stage's last substep leave w and rho' as their explicit parts w~
-// and rho~ (the deferred form of hevi_tma_body<true>: the next substep applies
-// the implicit corrections to its input), so a chunk carries only its dp
-// values; the last one (`last`) reads its own w~ and rho~ back and corrects
-// them, and what remains of the stage is the u/v update.
-// Bound by latency at small grids (load, two barriers, store), by DRAM and the
-// loads in flight at large ones.
+// scalars folded in.
+// Every substep changes pi' by kap(k) times its change of rho' (both are the
+// same mass divergence), so rho' is not carried: the last substep writes
+// rho'(k) = rho'_0 + (pi'(k) - pi'_0) / kap(k) from the stage's state wst.
+// The eliminated pi' never leaves the registers: 32 B/cell of traffic, 40 with
+// rho', 48 in the sweeping kernel.
+// All but a stage's last substep leave w as its explicit part w~ (the deferred
+// form of hevi_tma_body<true>: the next substep applies the implicit
+// correction to its input), so a chunk carries only its dp values; the last
+// one (`last`) reads its own w~ back and corrects it, and what remains of the
+// stage is the u/v update.
+// Bound by latency at small grids (load, two barriers, store), by DRAM at large
+// ones: 512 x 512 x 80 158 us (4.3 TB/s; 175 with rho'), 193 x 193 x 60 17.0 (18.8),
+// three domains of 192 x 192 x 60 and below 29.3 (35.3). More loads in flight (a
+// ring of cp.async copies, 3 to 6 levels), bulk prefetches into L2 and
+// streaming hints made it slower or nothing: 170 to 232, 197, 176 to 178.
 size_t hevi_chunk_smem_bytes(int nz, int m) {
   const int C = (nz + m - 1) / m;
   return ((size_t)(3 * nz + 1)) * sizeof(float4) + (size_t)64 * C * sizeof(float2);
 }
 template <int kM>
 __device__ __forceinline__ void hevi_chunk_body(const Dims& d, const Tab& t, const Flags& fl, const WS& win,
-                                                const WS& wout, float dtau, const float* __restrict__ lu,
-                                                int apply_uv, int last, float cdx, float cdy, int bx) {
+                                                const WS& wout, const WS& wst, float dtau,
+                                                const float* __restrict__ lu, int apply_uv, int last, float cdx,
+                                                float cdy, int bx) {
   extern __shared__ float4 s_split[];
   const int nz = d.nz;
   const int C = blockDim.y;
@@ -2452,7 +2460,7 @@ __device__ __forceinline__ void hevi_chunk_body(const Dims& d, const Tab& t, con
     ta[k] = make_float4(dtau * ob * g, dtau * b * g, t.rfz[k], H);
   }
   const int vn = d.P;
-  const float dxi = t.dx_inv, dyi = t.dy_inv, db = dtau * b;
+  const float dxi = t.dx_inv, dyi = t.dy_inv;
   // single neighbours as in hevi2_body (the idle points read column 0 alone)
   const int ou2 = two ? 2 : 1;
   const int opw = (active && i > 0) ? -1 : 0;
@@ -2476,7 +2484,6 @@ __device__ __forceinline__ void hevi_chunk_body(const Dims& d, const Tab& t, con
       const int k = k0 + q;
       float2 wk1 = ld2(W, o + pl), pk1 = ld2(PI, k + 1 < nz ? o + pl : o);
       const float2 fu = ld2(U, o), fv0 = ld2(V, o), fv1 = ld2(V, o + vn);
-      float2 r = ld2(RHO, o);
       const float fu2 = ld1(U, o + ou2);
       float u0x = fu.x, u0y = fu.y, u1y = fu2, v0x = fv0.x, v0y = fv0.y, v1x = fv1.x, v1y = fv1.y, u1x;
       const float4 A0 = ta[k], A1 = ta[k + 1], B = tb[k], Ck = tc[k];
@@ -2495,8 +2502,6 @@ __device__ __forceinline__ void hevi_chunk_body(const Dims& d, const Tab& t, con
         v1y += ty_ * (fn.y - pk.y);
         wk1.x -= A1.y * gx;
         wk1.y -= A1.y * gy;
-        r.x += db * ((A0.z * wk.x - A1.z * wk1.x) * B.x);
-        r.y += db * ((A0.z * wk.y - A1.z * wk1.y) * B.x);
       } else {
         u1x = fu.y;
       }
@@ -2511,7 +2516,6 @@ __device__ __forceinline__ void hevi_chunk_body(const Dims& d, const Tab& t, con
         st2(W, o, wt);
         st2(U, o, make_float2(u0x, u0y));
         st2(V, o, make_float2(v0x, v0y));
-        st2(RHO, o, make_float2(r.x + dtau * sx_, r.y + dtau * sy_));
         if (last_i) wout.f[U][o + ou2] = two ? u1y : u1x;  // face nx
         if (last_j) st2(V, o + vn, make_float2(v1x, v1y));
       }
@@ -2582,15 +2586,14 @@ __device__ __forceinline__ void hevi_chunk_body(const Dims& d, const Tab& t, con
   for (int q = 0; q < kM; ++q)
     if (q < kn) {
       const int k = k0 + q;
-      const float4 A0 = ta[k], A1 = ta[k + 1];
-      const float iz = tb[k].x;
+      const float a = ta[k + 1].y, ik = dtau / tb[k].y;  // 1 / kap
       const bool top = q + 1 >= kn;
       const float2 xf = top ? in : dp[q + 1 < kM ? q + 1 : q];
       const float2 wf = top ? wt : back(W, o + pl);
-      const float2 wn = make_float2(wf.x - A1.y * (xf.x - dp[q].x), wf.y - A1.y * (xf.y - dp[q].y));
-      const float2 r = back(RHO, o);
-      st2(RHO, o, make_float2(r.x + db * ((A0.z * wb.x - A1.z * wn.x) * iz),
-                              r.y + db * ((A0.z * wb.y - A1.z * wn.y) * iz)));
+      const float2 wn = make_float2(wf.x - a * (xf.x - dp[q].x), wf.y - a * (xf.y - dp[q].y));
+      const float2 r = __ldg(reinterpret_cast<const float2*>(wst.f[RHO] + o));
+      const float2 p = __ldg(reinterpret_cast<const float2*>(wst.f[PI] + o));
+      st2(RHO, o, make_float2(r.x + (dp[q].x - p.x) * ik, r.y + (dp[q].y - p.y) * ik));
       st2(W, o, wb);
       wb = wn;
       o += pl;
@@ -2600,9 +2603,9 @@ __device__ __forceinline__ void hevi_chunk_body(const Dims& d, const Tab& t, con
 template <int kM, int kThreads, int kBlocks>
 __global__ void __launch_bounds__(kThreads, kBlocks) k_mx_hevi_chunk(
     const __grid_constant__ Dims d, const __grid_constant__ Tab t, const __grid_constant__ Flags fl,
-    const __grid_constant__ WS win, const __grid_constant__ WS wout, float dtau, const float* __restrict__ lu,
-    int apply_uv, int last, float cdx, float cdy) {
-  hevi_chunk_body<kM>(d, t, fl, win, wout, dtau, lu, apply_uv, last, cdx, cdy, blockIdx.x);
+    const __grid_constant__ WS win, const __grid_constant__ WS wout, const __grid_constant__ WS wst, float dtau,
+    const float* __restrict__ lu, int apply_uv, int last, float cdx, float cdy) {
+  hevi_chunk_body<kM>(d, t, fl, win, wout, wst, dtau, lu, apply_uv, last, cdx, cdy, blockIdx.x);
 }
 
 template <int kPF, int kRing>
@@ -2668,7 +2671,7 @@ int hevi_chunk_levels(int nz, long columns, const Flags& fl) {
     }
     env = v;
   }
-  if (env == 0 || fl.moist) return 0;
+  if (env == 0 || fl.moist || !fl.rho_from_pi) return 0;
   int m = env;
   if (m < 0) m = columns <= kChunkSmall ? 4 : nz <= 48 ? 6 : nz <= 64 ? 8 : 10;
   if ((nz + m - 1) / m > kMaxChunks) m = 10;
@@ -2742,8 +2745,8 @@ size_t hevi2_smem_bytes(int nz, int ring) {
   return ((((size_t)10 * (nz + 1) + 3) & ~(size_t)3) + (size_t)ring * 19 * 128) * sizeof(float);
 }
 
-int mixed_hevi_column(const Dims& d, const Tab& t, const Flags& fl, const WS& win, const WS& wout, float dtau,
-                      const float* lu, bool apply_uv, bool last, unsigned* err, cudaStream_t stream) {
+int mixed_hevi_column(const Dims& d, const Tab& t, const Flags& fl, const WS& win, const WS& wout, const WS& wst,
+                      float dtau, const float* lu, bool apply_uv, bool last, unsigned* err, cudaStream_t stream) {
   MixedTune tn;
   const bool tuned = tune_of(d, &tn) && tn.column >= 0;
   int r2 = hevi_two_ring(), ring = hevi_ring();
@@ -2755,8 +2758,8 @@ int mixed_hevi_column(const Dims& d, const Tab& t, const Flags& fl, const WS& wi
   if (v == 6) {
     const int m = hevi_chunk_levels(d.nz, (long)d.nx * d.ny, fl);
     const float cdx = -(float)kCp * dtau * t.dx_inv, cdy = -(float)kCp * dtau * t.dy_inv;
-    VGB_CHUNK_LAUNCH(k_mx_hevi_chunk, m, d.nz, hevi_chunk_blocks(d), stream, d, t, fl, win, wout, dtau, lu,
-                     apply_uv ? 1 : 0, last ? 1 : 0, cdx, cdy);
+    VGB_CHUNK_LAUNCH(k_mx_hevi_chunk, m, d.nz, hevi_chunk_blocks(d), stream, d, t, fl, win, wout, wst, dtau,
+                     lu, apply_uv ? 1 : 0, last ? 1 : 0, cdx, cdy);
     return 0;
   }
   if (v >= 0) {
@@ -2820,7 +2823,7 @@ void mixed_uv_fix(const Dims& d, const Tab& t, const Flags& fl, const WS& s, flo
 
 int mixed_hevi_substep(const Dims& d, const Tab& t, const Flags& fl, const WS& win, const WS& wout, float dtau,
                        const float* lu, unsigned* err, cudaStream_t stream) {
-  if (mixed_hevi_column(d, t, fl, win, wout, dtau, lu, false, true, err, stream)) return -1;
+  if (mixed_hevi_column(d, t, fl, win, wout, win, dtau, lu, false, true, err, stream)) return -1;
   // in place: u, v were copied by the column kernel
   if (mixed_hevi_defers(d, fl)) mixed_uv_fix(d, t, fl, wout, dtau, stream);
   else mixed_uv_backward(d, t, wout, wout, dtau, stream);
@@ -2923,6 +2926,7 @@ struct HeviArgs {  // 64-byte aligned through its CUtensorMap members
   Tab t;
   Flags fl;
   WS win, wout;
+  WS wst;  // the stage's state, input of its first substep
   float dtau, cdx, cdy;
   const float* lu;
   int apply_uv, last, gx, gy;
@@ -2996,7 +3000,7 @@ __global__ void __launch_bounds__(kThreads, kBlocks) k_b_hevi_chunk(const HeviAr
                                                                     const int* __restrict__ start, int nd) {
   const int dom = find_domain(start, nd);
   const HeviArgs& a = A[dom];
-  hevi_chunk_body<kM>(a.d, a.t, a.fl, a.win, a.wout, a.dtau, a.lu, a.apply_uv, a.last, a.cdx, a.cdy,
+  hevi_chunk_body<kM>(a.d, a.t, a.fl, a.win, a.wout, a.wst, a.dtau, a.lu, a.apply_uv, a.last, a.cdx, a.cdy,
                       (int)blockIdx.x - start[dom]);
 }
 
@@ -3135,6 +3139,7 @@ MixedBatch* mixed_batch_build(const std::vector<MixedDomain>& doms, const Flags&
         a.fl = fl;
         a.win = ws_from(in);
         a.wout = ws_from(sub_out(m, n));
+        a.wst = ws_from(stage & 1 ? m.WSt1 : m.WSt0);
         a.dtau = dtau;
         a.cdx = -(float)kCp * dtau * m.t.dx_inv;
         a.cdy = -(float)kCp * dtau * m.t.dy_inv;

@@ -94,6 +94,9 @@ constexpr int kHevi64M = 8;         // levels per warp of the FP64 level-split k
 constexpr int kHevi64Chunks = 20;   // warps per block at most: nz <= 160
 
 // Composition switches (same meaning as the setup struct in vibe_gb300.h).
+// below this kap(k) = (Rd/cv) pi0/rho0 the rounding of pi' would show in rho' = pi'/kap (an atmosphere
+// has 0.3 at the ground and more above)
+constexpr double kKapMin = 0.05;
 struct Flags {
   int advection;         // 2/4/6 central, 5 = weno5 id
   int weno_scalars;
@@ -107,6 +110,7 @@ struct Flags {
   int acoustic_mode;     // 0 explicit FB, 1 reference HEVI, 2 consistent HEVI
   double hevi_beta;
   int w_rigid;           // w = 0 on the ground and lid faces after every step
+  int rho_from_pi;       // every kap(k) >= kKapMin: rho' may follow from pi' (mixed level-split column kernel)
 };
 
 __host__ __device__ inline int iclamp(int v, int lo, int hi) { return v < lo ? lo : (v > hi ? hi : v); }
