@@ -603,7 +603,12 @@ int hevi_metric(vibe_gb300_model* m, double dtau, Metric* out) {
   }
   for (int k = 0; k < nz; ++k) {
     const double kap = (kRd / kCv) * (ref(1, k) / dmax(ref(2, k), 1e-8));
-    at(kH_idz, k) = 1.0 / dz(k);
+    const double iz = 1.0 / dz(k);
+    at(kH_oz, k) = (1.0 - b) * iz;
+    at(kH_bz, k) = b * iz;
+    at(kH_tz, k) = dtau * b * iz;
+    at(kH_dx, k) = -ref(2, k) / m->su.dx;
+    at(kH_dy, k) = -ref(2, k) / m->su.dy;
     at(kH_dk, k) = dtau * kap;
     at(kH_r0, k) = ref(2, k);
     at(kH_p0, k) = ref(1, k);

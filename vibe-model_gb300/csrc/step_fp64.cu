@@ -760,37 +760,57 @@ __global__ void k_chevi_column(Dims d, Metric m, Flags fl, CS s, double* __restr
 }
 
 #ifndef VGB_FP64_EXACT
+// zeros on the ghost points beside column (i, j), levels k0..k0+kn-1
+__device__ __forceinline__ void hevi_ghost(const Dims& d, int i, int j, int k0, int kn, double* __restrict__ w,
+                                           double* __restrict__ rho, double* __restrict__ pi) {
+  const bool ei = i == d.nx - 1, ej = j == d.ny - 1;
+  if (!ei && !ej) return;
+  const int kw = k0 + kn == d.nz ? kn + 1 : kn;  // the last chunk owns face nz
+  for (int q = 0; q < kw; ++q) {
+    const size_t o = IDX(i, j, k0 + q);
+    auto zero = [&](size_t g) {
+      w[g] = 0.0;
+      if (q < kn) rho[g] = pi[g] = 0.0;
+    };
+    if (ei) zero(o + 1);
+    if (ej) zero(o + d.P);
+    if (ei && ej) zero(o + d.P + 1);
+  }
+}
+
 // The same substep on flat grids with a uniform reference state, levels split
 // over warps. Its column matrix is one per level there, factored once on the
 // host (Metric::hevi): no division and no per-column coefficient is left, and
 // the two recurrences split into chunks of kHevi64M levels joined by carries
 // (as in the mixed path's level-split kernel: dp(k) = dp0(k) + G(k) dp(k0-1),
-// x(k) = x0(k) + H(k) x(k0+kn)). A warp is 32 consecutive points of the padded
-// plane by one chunk, a block the chunks of its columns. w, rho and pi are
-// updated in place: a chunk reads its inputs (its own and the two levels
-// beside it) before the first barrier and writes after the second. The points
-// of the ghost column and row get the zeros the substep leaves there.
+// x(k) = x0(k) + H(k) x(k0+kn)). A warp is 32 columns by one chunk or 16 by two,
+// a block the chunks of its columns. w, rho and pi are updated in place: a
+// chunk reads its inputs (its own and the two levels beside it) before the
+// first barrier and writes after the second. The points of the ghost column
+// and row get the zeros the substep leaves there.
 // Bound by the FP64 pipe: about 30 FP64 operations per cell, where the
-// sweeping kernel above spends ~250 (divisions, per-column coefficients).
-template <int kBlocks>
-__global__ void __launch_bounds__(32 * kHevi64Chunks / kBlocks, kBlocks)
-    k_chevi_chunk(Dims d, const double* __restrict__ tab, double inv_dx, double inv_dy, double b, double dtau, int pert,
+// sweeping kernel above spends ~250 (divisions, per-column coefficients). So
+// the fullest SM sets the time: blocks count cells' columns alone, and are of
+// 32 or 16 by hevi_cols below. Substep at
+// 96 x 96 x 50 57.7 to 31.6 us, 64 x 72 x 50 35.6 to 19.8 (adjoint 29.8 to 21.4),
+// 128 x 128 x 80 106 to 81, against blocks of 32 points of the padded plane.
+template <int kBlocks, int kCols>
+__global__ void __launch_bounds__(kCols * kHevi64Chunks / kBlocks, 32 / kCols * kBlocks)
+    k_chevi_chunk(Dims d, const double* __restrict__ tab, double b, double dtau, int pert,
                   const double* __restrict__ u, const double* __restrict__ v, double* __restrict__ w,
                   double* __restrict__ rho, double* __restrict__ pi) {
   constexpr int kM = kHevi64M;
   extern __shared__ double sh64[];
-  const int nz = d.nz, C = blockDim.y, R = nz + 1;
-  double* sf = sh64;            // C x 32: dp at each chunk's last level, zero carry
-  double* sx = sh64 + 32 * C;   // C x 32: x at each chunk's first level, zero carry
-  const int tx = threadIdx.x, c = threadIdx.y, tid = c * 32 + tx;
-  const int e = blockIdx.x * 32 + tx;
-  const int j = e / d.P, i = e - j * d.P;
-  const bool active = i < d.nx && j < d.ny;
-  const bool ghost = !active && i <= d.nx && j <= d.ny;
-  const int k0 = c * kM, kn = imin(kM, nz - k0);
-  const size_t pl = d.plane, col = active ? (size_t)e : 0;
+  const int nz = d.nz, C = (nz + kM - 1) / kM, R = nz + 1;
+  double* sf = sh64;                    // chunks x columns: dp at each chunk's last level, zero carry
+  double* sx = sh64 + 32 * blockDim.y;  // ... x at each chunk's first level, zero carry
+  const int tx = threadIdx.x % kCols, c = threadIdx.y * (32 / kCols) + threadIdx.x / kCols, tid = c * kCols + tx;
+  const int e = blockIdx.x * kCols + tx;
+  const int j = e / d.nx, i = e - j * d.nx;
+  const int k0 = c * kM, kn = imax(imin(kM, nz - k0), 0);
+  const bool active = j < d.ny && kn > 0;
+  const size_t pl = d.plane, col = active ? (size_t)j * d.P + i : 0;
   auto T = [&](int row, int k) { return __ldg(tab + row * R + k); };
-  const double ob = 1.0 - b;
   double pv[kM + 2], wv[kM + 1], rs[kM], dp[kM];
 #pragma unroll
   for (int q = 0; q < kM + 2; ++q) {
@@ -812,13 +832,13 @@ __global__ void __launch_bounds__(32 * kHevi64Chunks / kBlocks, kBlocks)
     if (q < kn && active) {
       const int k = k0 + q;
       const size_t o = (size_t)k * pl + col;
-      const double r1 = T(kH_rf, k + 1), iz = T(kH_idz, k);
+      const double r1 = T(kH_rf, k + 1);
       const double fo1 = r1 * wv[q + 1];
       wv[q + 1] -= T(kH_ae, k + 1) * (pv[q + 2] - pv[q + 1]);  // w~ at the upper face
       const double ft1 = r1 * wv[q + 1];
-      const double dh = -T(kH_r0, k) * ((u[o + 1] - u[o]) * inv_dx + (v[o + d.P] - v[o]) * inv_dy);
-      const double S = dh + (ob * iz) * (fo - fo1);
-      const double z = T(kH_dk, k) * (S + (b * iz) * (ft - ft1));
+      const double dh = T(kH_dx, k) * (u[o + 1] - u[o]) + T(kH_dy, k) * (v[o + d.P] - v[o]);
+      const double S = dh + T(kH_oz, k) * (fo - fo1);
+      const double z = T(kH_dk, k) * (S + T(kH_bz, k) * (ft - ft1));
       // the total first, as the reference forms it (its rounding at pi ~ 1 is part of its result)
       const double p0 = pert ? T(kH_p0, k) : 0.0;
       const double rhs = pert ? ((pv[q + 1] + p0) + z) - p0 : pv[q + 1] + z;
@@ -832,7 +852,7 @@ __global__ void __launch_bounds__(32 * kHevi64Chunks / kBlocks, kBlocks)
   sf[tid] = prev;
   __syncthreads();
   double below = 0.0;  // dp(k0 - 1)
-  for (int cc = 0; cc < c; ++cc) below = sf[cc * 32 + tx] + T(kH_G, (cc + 1) * kM - 1) * below;
+  for (int cc = 0; cc < c; ++cc) below = sf[cc * kCols + tx] + T(kH_G, (cc + 1) * kM - 1) * below;
   double nxt = 0.0;
 #pragma unroll
   for (int q = kM - 1; q >= 0; --q)
@@ -844,16 +864,9 @@ __global__ void __launch_bounds__(32 * kHevi64Chunks / kBlocks, kBlocks)
   sx[tid] = dp[0];
   __syncthreads();
   double above = 0.0;  // x(k0 + kn)
-  for (int cc = C - 1; cc > c; --cc) above = sx[cc * 32 + tx] + T(kH_H, cc * kM) * above;
-  if (ghost) {
-    const size_t g = (size_t)e;
-    for (int q = 0; q < kn; ++q) {
-      const size_t o = (size_t)(k0 + q) * pl + g;
-      w[o] = rho[o] = pi[o] = 0.0;
-    }
-    if (k0 + kn == nz) w[(size_t)nz * pl + g] = 0.0;
-  }
+  for (int cc = C - 1; cc > c; --cc) above = sx[cc * kCols + tx] + T(kH_H, cc * kM) * above;
   if (!active) return;
+  hevi_ghost(d, i, j, k0, kn, w, rho, pi);
 #pragma unroll
   for (int q = 0; q < kM; ++q)
     if (q < kn) dp[q] += T(kH_H, k0 + q) * above;
@@ -868,7 +881,7 @@ __global__ void __launch_bounds__(32 * kHevi64Chunks / kBlocks, kBlocks)
       const double xf = (q + 1 < kn) ? dp[q + 1 < kM ? q + 1 : q] : above;
       const double wn = wv[q + 1] - T(kH_ai, k + 1) * (xf - dp[q]);
       const double fn1 = T(kH_rf, k + 1) * wn;
-      rho[o] = rs[q] + (dtau * b * T(kH_idz, k)) * (fn - fn1);
+      rho[o] = rs[q] + T(kH_tz, k) * (fn - fn1);
       pi[o] = dp[q] + (pert ? T(kH_p0, k) : 0.0);
       w[o] = wb;
       wb = wn;
@@ -1150,23 +1163,22 @@ __global__ void k_hevi_ad_column(Dims d, Metric m, Flags fl, double* __restrict_
 // the column part of k_hevi_ad_column with the transposed factors of
 // Metric::hevi, in place on bar_w and bar_pi; bar of Dh goes to k_dh_ad_chunk.
 // bar_rho passes through. The ghost points' bars do not reach the input.
-template <int kBlocks>
-__global__ void __launch_bounds__(32 * kHevi64Chunks / kBlocks, kBlocks)
+template <int kBlocks, int kCols>
+__global__ void __launch_bounds__(kCols * kHevi64Chunks / kBlocks, 32 / kCols * kBlocks)
     k_hevi_ad_chunk(Dims d, const double* __restrict__ tab, double b, double dtau, const double* __restrict__ bu,
                     const double* __restrict__ bv, double* __restrict__ bw, double* __restrict__ brho,
                     double* __restrict__ bpi, double* __restrict__ bdh) {
   constexpr int kM = kHevi64M;
   extern __shared__ double sh64[];
-  const int nz = d.nz, C = blockDim.y, R = nz + 1;
-  double* sf = sh64;
-  double* sx = sh64 + 32 * C;
-  const int tx = threadIdx.x, c = threadIdx.y, tid = c * 32 + tx;
-  const int e = blockIdx.x * 32 + tx;
-  const int j = e / d.P, i = e - j * d.P;
-  const bool active = i < d.nx && j < d.ny;
-  const bool ghost = !active && i <= d.nx && j <= d.ny;
-  const int k0 = c * kM, kn = imin(kM, nz - k0);
-  const size_t pl = d.plane, col = active ? (size_t)e : 0;
+  const int nz = d.nz, C = (nz + kM - 1) / kM, R = nz + 1;
+  double* sf = sh64;                    // chunks x columns
+  double* sx = sh64 + 32 * blockDim.y;  // (likewise)
+  const int tx = threadIdx.x % kCols, c = threadIdx.y * (32 / kCols) + threadIdx.x / kCols, tid = c * kCols + tx;
+  const int e = blockIdx.x * kCols + tx;
+  const int j = e / d.nx, i = e - j * d.nx;
+  const int k0 = c * kM, kn = imax(imin(kM, nz - k0), 0);
+  const bool active = j < d.ny && kn > 0;
+  const size_t pl = d.plane, col = active ? (size_t)j * d.P + i : 0;
   auto T = [&](int row, int k) { return __ldg(tab + row * R + k); };
   const double ob = 1.0 - b, db = dtau * b;
   double br[kM + 2], bn[kM + 1], y[kM];  // bar_rho(k0-1+q); bar of w_new, faces k0..k0+kn; bar_x, then y
@@ -1199,7 +1211,7 @@ __global__ void __launch_bounds__(32 * kHevi64Chunks / kBlocks, kBlocks)
   sf[tid] = prev;
   __syncthreads();
   double below = 0.0;
-  for (int cc = 0; cc < c; ++cc) below = sf[cc * 32 + tx] + T(kH_GT, (cc + 1) * kM - 1) * below;
+  for (int cc = 0; cc < c; ++cc) below = sf[cc * kCols + tx] + T(kH_GT, (cc + 1) * kM - 1) * below;
   double nxt = 0.0;
 #pragma unroll
   for (int q = kM - 1; q >= 0; --q)
@@ -1211,16 +1223,9 @@ __global__ void __launch_bounds__(32 * kHevi64Chunks / kBlocks, kBlocks)
   sx[tid] = y[0];
   __syncthreads();
   double above = 0.0;  // y(k0 + kn)
-  for (int cc = C - 1; cc > c; --cc) above = sx[cc * 32 + tx] + T(kH_HT, cc * kM) * above;
-  if (ghost) {
-    const size_t g = (size_t)e;
-    for (int q = 0; q < kn; ++q) {
-      const size_t o = (size_t)(k0 + q) * pl + g;
-      bw[o] = brho[o] = bpi[o] = 0.0;
-    }
-    if (k0 + kn == nz) bw[(size_t)nz * pl + g] = 0.0;
-  }
+  for (int cc = C - 1; cc > c; --cc) above = sx[cc * kCols + tx] + T(kH_HT, cc * kM) * above;
   if (!active) return;
+  hevi_ghost(d, i, j, k0, kn, bw, brho, bpi);
 #pragma unroll
   for (int q = 0; q < kM; ++q)
     if (q < kn) y[q] += T(kH_HT, k0 + q) * above;
@@ -1369,18 +1374,41 @@ void FP64_FN(fp64_fb_substep_ad)(const Dims& d, const Metric& m, double* const* 
                                                                                bar[W], dtau);
 }
 
+#ifndef VGB_FP64_EXACT
+// Columns a block of the level-split kernels: those that leave the fullest SM
+// less to do, counted in warps by levels (a warp of 16 columns by two chunks
+// runs the longer one's levels). 96 x 96 x 50: 2 blocks of 32 columns on the
+// fullest of 152 SMs (1.9 on average), 128 x 128 x 80: 4 (3.4) or 7 of 16 (6.7).
+static int hevi_cols(const Dims& d) {
+  int dev = 0, sms = 1;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const long n = (long)d.nx * d.ny;
+  long pairs = 0;
+  for (int k = 0; k < d.nz; k += 2 * kHevi64M) pairs += imin(kHevi64M, d.nz - k);
+  auto fullest = [&](int cols, long levels) { return ((n + cols - 1) / cols + sms - 1) / sms * levels; };
+  return fullest(16, pairs) < fullest(32, d.nz) ? 16 : 32;
+}
+#define VGB_HEVI64_LAUNCH(Kernel, d, stream, ...)                                                     \
+  do {                                                                                                \
+    const int cols = hevi_cols(d), C = ((d).nz + kHevi64M - 1) / kHevi64M;                            \
+    const dim3 b(32, (C * cols + 31) / 32);                                                           \
+    const int g = (int)(((long)(d).nx * (d).ny + cols - 1) / cols);                                   \
+    const size_t sm = 64 * (size_t)b.y * sizeof(double);                                              \
+    const bool half = C <= kHevi64Chunks / 2;                                                         \
+    if (cols == 16 && half) Kernel<2, 16><<<g, b, sm, stream>>>(__VA_ARGS__);                         \
+    else if (cols == 16) Kernel<1, 16><<<g, b, sm, stream>>>(__VA_ARGS__);                            \
+    else if (half) Kernel<2, 32><<<g, b, sm, stream>>>(__VA_ARGS__);                                  \
+    else Kernel<1, 32><<<g, b, sm, stream>>>(__VA_ARGS__);                                            \
+  } while (0)
+#endif
+
 void FP64_FN(fp64_hevi_substep_ad)(const Dims& d, const Metric& m, const Flags& fl, double* const* bar, double* bdh,
                                    double* scratch, double dtau, unsigned* err, cudaStream_t stream) {
 #ifndef VGB_FP64_EXACT
   if (m.hevi) {
-    const int C = (d.nz + kHevi64M - 1) / kHevi64M, g = (int)((d.plane + 31) / 32);
-    const size_t sm = 64 * (size_t)C * sizeof(double);
-    if (C <= kHevi64Chunks / 2)
-      k_hevi_ad_chunk<2><<<g, dim3(32, C), sm, stream>>>(d, m.hevi, fl.hevi_beta, dtau, bar[U], bar[V], bar[W],
-                                                         bar[RHO], bar[PI], bdh);
-    else
-      k_hevi_ad_chunk<1><<<g, dim3(32, C), sm, stream>>>(d, m.hevi, fl.hevi_beta, dtau, bar[U], bar[V], bar[W],
-                                                         bar[RHO], bar[PI], bdh);
+    VGB_HEVI64_LAUNCH(k_hevi_ad_chunk, d, stream, d, m.hevi, fl.hevi_beta, dtau, bar[U], bar[V], bar[W], bar[RHO],
+                      bar[PI], bdh);
     k_dh_ad_chunk<<<grid3(d, d.nx + 1, d.ny + 1, d.nz, kBlk), kBlk, 0, stream>>>(d, m.hevi, m.inv_dx, m.inv_dy, bdh,
                                                                                 bar[U], bar[V]);
     return;
@@ -1417,14 +1445,8 @@ void FP64_FN(fp64_cons_hevi_substep)(const Dims& d, const Metric& m, const Flags
                             double* scratch, double dtau, unsigned* err, cudaStream_t stream) {
 #ifndef VGB_FP64_EXACT
   if (m.hevi) {
-    const int C = (d.nz + kHevi64M - 1) / kHevi64M, g = (int)((d.plane + 31) / 32);
-    const size_t sm = 64 * (size_t)C * sizeof(double);
-    if (C <= kHevi64Chunks / 2)
-      k_chevi_chunk<2><<<g, dim3(32, C), sm, stream>>>(d, m.hevi, m.inv_dx, m.inv_dy, fl.hevi_beta, dtau, fl.pgf_pert,
-                                                       st[U], st[V], st[W], st[RHO], st[PI]);
-    else
-      k_chevi_chunk<1><<<g, dim3(32, C), sm, stream>>>(d, m.hevi, m.inv_dx, m.inv_dy, fl.hevi_beta, dtau, fl.pgf_pert,
-                                                       st[U], st[V], st[W], st[RHO], st[PI]);
+    VGB_HEVI64_LAUNCH(k_chevi_chunk, d, stream, d, m.hevi, fl.hevi_beta, dtau, fl.pgf_pert, st[U], st[V], st[W],
+                      st[RHO], st[PI]);
     k_uv_chunk<<<grid3(d, d.nx, d.ny, d.nz, kBlk), kBlk, 0, stream>>>(d, m.hevi, st[PI], st[U], st[V]);
     return;
   }

@@ -71,7 +71,11 @@ enum Hevi64Row {
   kH_ae,   // face: dtau (1-b) cp theta0_f / dz_f
   kH_ai,   // face: dtau b cp theta0_f / dz_f
   kH_rf,   // face: rho0_f
-  kH_idz,  // 1/dz
+  kH_oz,   // (1-b)/dz
+  kH_bz,   // b/dz
+  kH_tz,   // dtau b/dz
+  kH_dx,   // -rho0/dx
+  kH_dy,   // -rho0/dy
   kH_dk,   // dtau kappa
   kH_r0,   // rho0
   kH_p0,   // pi0
