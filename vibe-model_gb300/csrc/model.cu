@@ -836,9 +836,7 @@ int enqueue_one_step(vibe_gb300_model* m, double dt, int n_sub) {
         Span sp(m, 2);
         m->f64->nonfinite(d, S1, m->d_err, m->stream);
         if (stage < 2 && m->rec_stage[stage])
-          for (int q = 0; q < NSPECIES; ++q)
-            CUDA_OK(cudaMemcpyAsync(m->rec_stage[stage][q], S1[q], d.plane * (size_t)(d.nz + 1) * sizeof(double),
-                                    cudaMemcpyDeviceToDevice, m->stream));
+          state_copy(d.plane * (size_t)(d.nz + 1), m->rec_stage[stage], S1, m->stream);
       }
       Span sp(m, 2);
       m->f64->sponge(d, m->met, S1, m->kmin, dt, m->stream);
@@ -899,9 +897,7 @@ int enqueue_one_step(vibe_gb300_model* m, double dt, int n_sub) {
         if (stage < 2 && m->rec_stage[stage]) {
           // the next stage's input as FP64 totals; what the working copy does
           // not hold (inactive species, points off the boxes) from the step's start
-          for (int q = 0; q < NSPECIES; ++q)
-            CUDA_OK(cudaMemcpyAsync(m->rec_stage[stage][q], S0[q], d.plane * (size_t)(d.nz + 1) * sizeof(double),
-                                    cudaMemcpyDeviceToDevice, m->stream));
+          state_copy(d.plane * (size_t)(d.nz + 1), m->rec_stage[stage], S0, m->stream);
           WS next = ws_compose(in, m->WSt[stage & 1]);
           if (!m->fl.moist)
             for (int q = QV + 1; q < NSPECIES; ++q) next.f[q] = nullptr;
@@ -2522,8 +2518,8 @@ namespace {
 size_t state_count(const vibe_gb300_model* m) { return m->d.plane * (size_t)(m->d.nz + 1); }
 
 int copy_state(vibe_gb300_model* m, double* const* dst, double* const* src) {
-  for (int q = 0; q < NSPECIES; ++q)
-    CUDA_OK(cudaMemcpyAsync(dst[q], src[q], state_count(m) * sizeof(double), cudaMemcpyDeviceToDevice, m->stream));
+  state_copy(state_count(m), dst, src, m->stream);
+  CUDA_OK(cudaGetLastError());
   return 0;
 }
 
@@ -2681,11 +2677,10 @@ int stl_step_tl(vibe_gb300_model* m, double dt, int n_sub, double* const* const*
   const bool f32 = m->precision == VIBE_GB300_MIXED;
   double* const* x0 = m->stl[0];
   double* const* r = m->stl[2];
-  if (int rc = copy_state(m, x0, x)) return rc;
   const double dts[3] = {dt / 3.0, dt / 2.0, dt};
   for (int st = 0; st < 3; ++st) {
-    tend_tl(m->d, m->met, m->fl, base[st], st == 0 ? x0 : x, r, m->stl_face, f32, m->stream);
-    for (int q = 0; q < NSPECIES; ++q) lin_axpy(n, x0[q], r[q], dts[st], x[q], m->stream);
+    tend_tl(m->d, m->met, m->fl, base[st], x, r, m->stl_face, f32, m->stream);
+    tl_stage(n, x, x0, r, dts[st], st == 0, m->stream);
     if (int rc = stl_substeps(m, st, dts[st] / n_sub, n_sub, x, false)) return rc;
   }
   return stl_sponge_rigid(m, dt, x);
@@ -2697,25 +2692,17 @@ int stl_step_ad(vibe_gb300_model* m, double dt, int n_sub, double* const* const*
   const bool f32 = m->precision == VIBE_GB300_MIXED;
   double* const* acc = m->stl[0];
   double* const* r = m->stl[2];
-  double* const* prev = m->stl[5];
   if (int rc = stl_sponge_rigid(m, dt, x)) return rc;
-  for (int q = 0; q < NSPECIES; ++q) CUDA_OK(cudaMemsetAsync(acc[q], 0, n * sizeof(double), m->stream));
   const double dts[3] = {dt / 3.0, dt / 2.0, dt};
   for (int st = 2; st >= 0; --st) {
     if (int rc = stl_substeps(m, st, dts[st] / n_sub, n_sub, x, true)) return rc;
-    for (int q = 0; q < NSPECIES; ++q) {
-      lin_scale_add(n, x[q], 1.0, acc[q], m->stream);           // through x0 directly
-      lin_axpy(n, m->stl_zero, x[q], dts[st], r[q], m->stream);  // bar of R = dt_stage * bar
-      CUDA_OK(cudaMemsetAsync(prev[q], 0, n * sizeof(double), m->stream));
-    }
-    tend_ad(m->d, m->met, m->fl, base[st], r, prev, m->stl_face, m->stl_cell, f32, m->stream);
-    if (st == 0) {
-      for (int q = 0; q < NSPECIES; ++q) lin_scale_add(n, prev[q], 1.0, acc[q], m->stream);
-    } else if (int rc = copy_state(m, x, prev)) {
-      return rc;
-    }
+    // acc: through x0 directly; r: bar of R = dt_stage * bar; x: bar of the stage's input, from zero
+    ad_stage(n, x, acc, r, dts[st], st == 2, m->stream);
+    tend_ad(m->d, m->met, m->fl, base[st], r, x, m->stl_face, m->stl_cell, f32, m->stream);
   }
-  return copy_state(m, x, acc);
+  ad_close(n, x, acc, m->stream);
+  CUDA_OK(cudaGetLastError());
+  return 0;
 }
 
 // one step from the model's current state that records its stage inputs;

@@ -179,8 +179,12 @@ void tend_tl(const Dims& d, const Metric& m, const Flags& fl, double* const* bas
 void tend_ad(const Dims& d, const Metric& m, const Flags& fl, double* const* base, double* const* bar_out,
              double* const* bar_in, double* face, double* cell_scr, bool f32, cudaStream_t s);
 // whole-array helpers: out = x0 + a r; acc += a x; conversions
-void lin_axpy(size_t n, const double* x0, const double* r, double a, double* out, cudaStream_t s);
-void lin_scale_add(size_t n, const double* x, double a, double* acc, cudaStream_t s);
+// the twelve fields of n doubles (n even), one launch each: dst = src; x = x0 + a r
+// (first: x0 = x before); acc = x (first) or acc + x, r = a x, x = 0; x += acc
+void state_copy(size_t n, double* const* dst, double* const* src, cudaStream_t s);
+void tl_stage(size_t n, double* const* x, double* const* x0, double* const* r, double a, bool first, cudaStream_t s);
+void ad_stage(size_t n, double* const* x, double* const* acc, double* const* r, double a, bool first, cudaStream_t s);
+void ad_close(size_t n, double* const* x, double* const* acc, cudaStream_t s);
 void lin_to_f32(size_t n, const double* x, float* y, cudaStream_t s);
 void lin_to_f64(size_t n, const float* x, double* y, cudaStream_t s);
 // FP32 working state (perturbation form) -> FP64 total fields (species with a
