@@ -890,7 +890,7 @@ int enqueue_one_step(vibe_gb300_model* m, double dt, int n_sub) {
         if (m->fl.acoustic_mode == 2 && stage < 2) {  // the last substep's u/v update, in place
           Span sp(m, 3);
           if (mixed_hevi_defers(d, m->fl)) mixed_uv_fix(d, m->tab, m->fl, ws_of(in), dtau, m->stream);
-          else mixed_uv_backward(d, m->tab, ws_of(in), ws_of(in), dtau, m->stream);
+          else mixed_uv_backward(d, m->tab, ws_of(in), dtau, m->stream);
         }
         final_sub = in;
         last_dtau = dtau;

@@ -114,7 +114,8 @@ int mixed_hevi_substep(const Dims& d, const Tab& t, const Flags& fl, const WS& w
 // last: no further substep follows in the stage
 int mixed_hevi_column(const Dims& d, const Tab& t, const Flags& fl, const WS& win, const WS& wout, const WS& wst,
                       float dtau, const float* lu, bool apply_uv, bool last, unsigned* err, cudaStream_t stream);
-void mixed_uv_backward(const Dims& d, const Tab& t, const WS& win, const WS& wout, float dtau, cudaStream_t stream);
+// u/v backward update of a stage's last substep, in place
+void mixed_uv_backward(const Dims& d, const Tab& t, const WS& s, float dtau, cudaStream_t stream);
 // whether the column kernel chosen for this grid defers its w/rho'
 // corrections to the reader (then the last substep of a stage is finished
 // by mixed_uv_fix instead of mixed_uv_backward, and mixed_finish gets defer)

@@ -831,11 +831,11 @@ __global__ void k_mx_fb_mass(Dims d, Tab t, WS win, WS wout, float dtau) {
   wout.f[PI][c] = win.f[PI][c] + dtau * (t.kap[k] * drho);
 }
 // momentum backward with the new pi' (read from wout)
-__device__ __forceinline__ void fb_mom_body(const Dims& d, const Tab& t, const WS& win, const WS& wout, float dtau,
-                                            int do_w, int bx, int by, int bz) {
-  const int i = bx * blockDim.x + threadIdx.x;
-  const int j = by * blockDim.y + threadIdx.y;
-  const int k = bz;
+__global__ void k_mx_fb_mom(const __grid_constant__ Dims d, const __grid_constant__ Tab t,
+                            const __grid_constant__ WS win, const __grid_constant__ WS wout, float dtau) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int j = blockIdx.y * blockDim.y + threadIdx.y;
+  const int k = blockIdx.z;
   if (i > d.nx || j > d.ny || k > d.nz) return;
   const size_t c = IX(i, j, k);
   const float* __restrict__ pn = wout.f[PI];
@@ -848,10 +848,41 @@ __device__ __forceinline__ void fb_mom_body(const Dims& d, const Tab& t, const W
     const int jp = imin(j, d.ny - 1), jm = imax(j - 1, 0);
     wout.f[V][c] = win.f[V][c] + dtau * (-cp * t.t0c[k] * (pn[IX(i, jp, k)] - pn[IX(i, jm, k)]) * t.dy_inv);
   }
-  if (do_w && i < d.nx && j < d.ny) {
+  if (i < d.nx && j < d.ny) {
     const int kc = imin(k, d.nz - 1), km = imax(k - 1, 0);
     wout.f[W][c] = win.f[W][c] + dtau * (-cp * t.tfz[k] * (pn[IX(i, j, kc)] - pn[IX(i, j, km)]) * t.idzw[k]);
   }
+}
+
+// u and v alone, in place: the faces between two cells (the clamped ones see no
+// gradient). Two columns a thread, 8-byte accesses. Bound by memory (20 B a cell):
+// 512 x 512 x 80 74 us, 126 with one column a thread.
+__device__ __forceinline__ void uv_body(const Dims& d, const Tab& t, const WS& s, float dtau, int bx, int by, int bz) {
+  const int i = 2 * (bx * blockDim.x + threadIdx.x);
+  const int j = by * blockDim.y + threadIdx.y;
+  const int k = bz;
+  if (i >= d.nx || j >= d.ny) return;
+  const size_t c = IX(i, j, k);
+  const bool two = i + 1 < d.nx;
+  const float cp = (float)kCp, t0 = t.t0c[k];
+  const float* __restrict__ pn = s.f[PI];
+  const float2 p = *reinterpret_cast<const float2*>(pn + c);
+  float2 u = *reinterpret_cast<const float2*>(s.f[U] + c);
+  const float pw = i > 0 ? pn[c - 1] : p.x;
+  u.x = u.x + dtau * (-cp * t0 * (p.x - pw) * t.dx_inv);
+  u.y = two ? u.y + dtau * (-cp * t0 * (p.y - p.x) * t.dx_inv) : u.y;  // (else face nx, or a padding point)
+  *reinterpret_cast<float2*>(s.f[U] + c) = u;
+  if (j > 0) {
+    const float2 ps = *reinterpret_cast<const float2*>(pn + c - d.P);
+    float2 v = *reinterpret_cast<const float2*>(s.f[V] + c);
+    v.x = v.x + dtau * (-cp * t0 * (p.x - ps.x) * t.dy_inv);
+    v.y = two ? v.y + dtau * (-cp * t0 * (p.y - ps.y) * t.dy_inv) : v.y;
+    *reinterpret_cast<float2*>(s.f[V] + c) = v;
+  }
+}
+__global__ void k_mx_uv(const __grid_constant__ Dims d, const __grid_constant__ Tab t, const __grid_constant__ WS s,
+                        float dtau) {
+  uv_body(d, t, s, dtau, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 
 // ---- consistent vertically implicit substep in FP32 ---------------------
@@ -862,11 +893,6 @@ __device__ __forceinline__ void fb_mom_body(const Dims& d, const Tab& t, const W
 // 40 KB per block at nz = 80, so 5 blocks -- 20 warps -- fit an SM); the
 // backward sweep re-derives the explicit terms from the same inputs, which
 // the forward sweep has just pulled through L2.
-__global__ void k_mx_fb_mom(const __grid_constant__ Dims d, const __grid_constant__ Tab t,
-                            const __grid_constant__ WS win, const __grid_constant__ WS wout, float dtau, int do_w) {
-  fb_mom_body(d, t, win, wout, dtau, do_w, blockIdx.x, blockIdx.y, blockIdx.z);
-}
-
 // apply_uv: the u/v backward update of the previous substep is applied here,
 // on the fly, from this substep's input pi' (the previous substep's result):
 // u(i) += dtau (-cp theta0(k) (pi'(ip) - pi'(im)) / dx) with the clamped
@@ -1188,7 +1214,7 @@ __device__ __forceinline__ double widen(float f) {
 // added to the FP64 state with one conversion and one FP64 add per field.
 // rin == nullptr: no tendency (single-substep entry points, S1 == S0).
 // Also writes the next step's FP32 working copy W0.
-// uv_dtau != 0: the last substep's u/v backward update (fb_mom_body, u and
+// uv_dtau != 0: the last substep's u/v backward update (uv_body, u and
 // v) is applied here on the fly instead of by its own in-place launch
 // The deferred corrections of a kDefer column kernel's w and rho' (see
 // hevi_tma_body below), for 1 <= k <= nz-1 with cb = dtau beta cp:
@@ -1204,11 +1230,14 @@ __device__ __forceinline__ float defer_fix_rho(const Tab& t, float db, float rt,
 
 // defer: wfin is a kDefer column kernel's output; its w and rho' get their
 // corrections (with dtau = uv_dtau) on the fly
+// Two columns a thread, 8- and 16-byte accesses (rows are padded to whole pairs;
+// what lies past a field's box is read and not used). Bound by memory: 216 B a
+// cell, 512 x 512 x 80 672 us (6.7 TB/s), 801 with one column a thread.
 __device__ __forceinline__ void finish_body(const Dims& d, const Tab& t, const Flags& fl, const WS& wfin,
                                             const WS& wst, const WS& w0, const WS& rin, float dtf, const CS64& s0,
                                             const MS64& s1, unsigned* err, int bx, int by, int bz,
                                             float uv_dtau = 0.f, bool defer = false) {
-  const int i = bx * blockDim.x + threadIdx.x;
+  const int i = 2 * (bx * blockDim.x + threadIdx.x);
   const int j = by * blockDim.y + threadIdx.y;
   const int k = bz;
   if (i > d.nx || j > d.ny || k > d.nz) return;
@@ -1222,74 +1251,98 @@ __device__ __forceinline__ void finish_body(const Dims& d, const Tab& t, const F
   // unchanged, so only the FP64 additions remain
   const bool plain = __double_as_longlong(wd) == 0x3ff0000000000000ll && __double_as_longlong(sdt) == 0ll;
   bool bad = false;
-  auto incr = [&](int q) { return rin.f[q] ? dtf * rin.f[q][c] : 0.f; };
-  const float cb = uv_dtau * (float)fl.hevi_beta * (float)kCp, db = uv_dtau * (float)fl.hevi_beta;
-  auto w_at = [&](int kf) {  // w at face kf of this column, corrected when deferred
-    const float wt = wfin.f[W][IX(i, j, kf)];
-    if (!defer || kf < 1 || kf >= d.nz) return wt;
-    return defer_fix_w(t, d.nz, cb, wt, wfin.f[PI][IX(i, j, kf)], wfin.f[PI][IX(i, j, kf - 1)], kf);
-  };
-  auto face = [&](int q) {
-    float wv = (q == W) ? w_at(k) : wfin.f[q][c];
-    if (uv_dtau != 0.f && q != W) {  // as fb_mom_body: k < nz and the face's clamped pi' neighbours
-      const float* __restrict__ pn = wfin.f[PI];
-      const float cp = (float)kCp;
-      if (q == U) {
-        const int ip = imin(i, d.nx - 1), im = imax(i - 1, 0);
-        wv = wv + uv_dtau * (-cp * t.t0c[k] * (pn[IX(ip, j, k)] - pn[IX(im, j, k)]) * t.dx_inv);
-      } else {
-        const int jp = imin(j, d.ny - 1), jm = imax(j - 1, 0);
-        wv = wv + uv_dtau * (-cp * t.t0c[k] * (pn[IX(i, jp, k)] - pn[IX(i, jm, k)]) * t.dy_inv);
-      }
-    }
-    const double a = s0.f[q][c] + widen(incr(q) + (wv - wst.f[q][c]));
-    const double v = plain ? a : wd * a;
-    s1.f[q][c] = v;
-    w0.f[q][c] = wf * wv;
-    bad |= !finite64(v);
-  };
-  if (j < d.ny && k < d.nz) face(U);
-  if (i < d.nx && k < d.nz) face(V);
-  if (i < d.nx && j < d.ny) {
-    if (fl.w_rigid && (k == 0 || k == d.nz)) {
-      s1.f[W][c] = 0.0;
-      w0.f[W][c] = 0.f;
+  auto ld = [&](const float* f) { return *reinterpret_cast<const float2*>(f + c); };
+  // the second column is in the field's box too
+  auto put = [&](int q, double2 v, float2 w, bool two) {
+    bad |= !finite64(v.x) || (two && !finite64(v.y));
+    if (two) {
+      *reinterpret_cast<double2*>(s1.f[q] + c) = v;
+      *reinterpret_cast<float2*>(w0.f[q] + c) = w;
     } else {
-      face(W);
+      s1.f[q][c] = v.x;
+      w0.f[q][c] = w.x;
+    }
+  };
+  // S0 + increment, with the acoustic part da
+  auto total = [&](int q, float2 da) {
+    const double2 a = *reinterpret_cast<const double2*>(s0.f[q] + c);
+    const float2 r = rin.f[q] ? ld(rin.f[q]) : make_float2(0.f, 0.f);
+    const float ix = rin.f[q] ? dtf * r.x : 0.f, iy = rin.f[q] ? dtf * r.y : 0.f;
+    return make_double2(a.x + widen(ix + da.x), a.y + widen(iy + da.y));
+  };
+  const float cb = uv_dtau * (float)fl.hevi_beta * (float)kCp, db = uv_dtau * (float)fl.hevi_beta;
+  // w at face kf of column i + m, corrected when deferred
+  auto w_at = [&](int m, int kf) {
+    const float wt = wfin.f[W][IX(i + m, j, kf)];
+    if (!defer || kf < 1 || kf >= d.nz) return wt;
+    return defer_fix_w(t, d.nz, cb, wt, wfin.f[PI][IX(i + m, j, kf)], wfin.f[PI][IX(i + m, j, kf - 1)], kf);
+  };
+  const float cp = (float)kCp;
+  const float* __restrict__ pn = wfin.f[PI];
+  auto face = [&](int q, float2 wv, bool two) {
+    const float2 ws = ld(wst.f[q]);
+    double2 v = total(q, make_float2(wv.x - ws.x, wv.y - ws.y));
+    if (!plain) v = make_double2(wd * v.x, wd * v.y);
+    put(q, v, make_float2(wf * wv.x, wf * wv.y), two);
+  };
+  const bool lev = k < d.nz;
+  const bool cell = i < d.nx && j < d.ny, cell2 = i + 1 < d.nx;
+  if (lev && j < d.ny) {
+    float2 wv = ld(wfin.f[U]);
+    if (uv_dtau != 0.f) {  // as uv_body: faces 0 and nx see no gradient
+      const float2 p = ld(pn);
+      const float gx = (i > 0 && i < d.nx) ? p.x - pn[c - 1] : 0.f, gy = cell2 ? p.y - p.x : 0.f;
+      wv.x = wv.x + uv_dtau * (-cp * t.t0c[k] * gx * t.dx_inv);
+      wv.y = wv.y + uv_dtau * (-cp * t.t0c[k] * gy * t.dx_inv);
+    }
+    face(U, wv, i + 1 <= d.nx);
+  }
+  if (lev && i < d.nx) {
+    float2 wv = ld(wfin.f[V]);
+    if (uv_dtau != 0.f) {
+      float2 g = make_float2(0.f, 0.f);
+      if (j > 0 && j < d.ny) {
+        const float2 p = ld(pn), ps = ld(pn - d.P);
+        g = make_float2(p.x - ps.x, p.y - ps.y);
+      }
+      wv.x = wv.x + uv_dtau * (-cp * t.t0c[k] * g.x * t.dy_inv);
+      wv.y = wv.y + uv_dtau * (-cp * t.t0c[k] * g.y * t.dy_inv);
+    }
+    face(V, wv, cell2);
+  }
+  if (cell) {
+    if (fl.w_rigid && (k == 0 || k == d.nz)) {
+      put(W, make_double2(0.0, 0.0), make_float2(0.f, 0.f), cell2);
+    } else {
+      face(W, defer ? make_float2(w_at(0, k), w_at(1, k)) : ld(wfin.f[W]), cell2);
     }
   }
-  if (i < d.nx && j < d.ny && k < d.nz) {
+  if (cell && lev) {
     {
-      float wv = wfin.f[RHO][c];
-      if (defer) wv = defer_fix_rho(t, db, wv, w_at(k), w_at(k + 1), k);
-      const double a = s0.f[RHO][c] + widen(incr(RHO) + (wv - wst.f[RHO][c]));
-      const double v = plain ? a : wd * (a + sdt * t.r0d[kc]);
-      s1.f[RHO][c] = v;
-      w0.f[RHO][c] = wf * wv;
-      bad |= !finite64(v);
+      float2 wv = ld(wfin.f[RHO]);
+      if (defer) {
+        wv.x = defer_fix_rho(t, db, wv.x, w_at(0, k), w_at(0, k + 1), k);
+        wv.y = defer_fix_rho(t, db, wv.y, w_at(1, k), w_at(1, k + 1), k);
+      }
+      const float2 ws = ld(wst.f[RHO]);
+      double2 v = total(RHO, make_float2(wv.x - ws.x, wv.y - ws.y));
+      if (!plain) v = make_double2(wd * (v.x + sdt * t.r0d[kc]), wd * (v.y + sdt * t.r0d[kc]));
+      put(RHO, v, make_float2(wf * wv.x, wf * wv.y), cell2);
     }
     {
-      const float wv = wfin.f[PI][c];
-      const double a = s0.f[PI][c] + widen(incr(PI) + (wv - wst.f[PI][c]));
-      const double v = plain ? a : wd * (a + sdt * t.p0d[kc]);
-      s1.f[PI][c] = v;
-      w0.f[PI][c] = wf * wv;
-      bad |= !finite64(v);
+      const float2 wv = ld(wfin.f[PI]), ws = ld(wst.f[PI]);
+      double2 v = total(PI, make_float2(wv.x - ws.x, wv.y - ws.y));
+      if (!plain) v = make_double2(wd * (v.x + sdt * t.p0d[kc]), wd * (v.y + sdt * t.p0d[kc]));
+      put(PI, v, make_float2(wf * wv.x, wf * wv.y), cell2);
     }
     {
-      double v = s0.f[THETA][c] + widen(incr(THETA));
-      if (!plain) v = wd * (v + sdt * t.t0dd[kc]);
-      s1.f[THETA][c] = v;
-      w0.f[THETA][c] = wf * wst.f[THETA][c];
-      bad |= !finite64(v);
+      const float2 ws = ld(wst.f[THETA]);
+      double2 v = total(THETA, make_float2(0.f, 0.f));
+      if (!plain) v = make_double2(wd * (v.x + sdt * t.t0dd[kc]), wd * (v.y + sdt * t.t0dd[kc]));
+      put(THETA, v, make_float2(wf * ws.x, wf * ws.y), cell2);
     }
     const int last = fl.moist ? QG : QV;
-    for (int q = QV; q <= last; ++q) {
-      const double v = s0.f[q][c] + widen(incr(q));
-      s1.f[q][c] = v;
-      w0.f[q][c] = wst.f[q][c];
-      bad |= !finite64(v);
-    }
+    for (int q = QV; q <= last; ++q) put(q, total(q, make_float2(0.f, 0.f)), ld(wst.f[q]), cell2);
   }
   if (bad) atomicOr(err, (unsigned)kErrNonFinite);
 }
@@ -1521,7 +1574,7 @@ int mixed_stage(const Dims& d, const Tab& t, const Flags& fl, const WS& win, con
 }
 
 // ---- adjoint of the FP32 forward-backward substep (k_mx_fb_mass, then
-// fb_mom_body with w): the transposed momentum phase (each cell gathers the
+// k_mx_fb_mom): the transposed momentum phase (each cell gathers the
 // pressure-gradient coefficients of its faces, uniform per level) and then
 // the transposed mass phase (each face gathers the divergence of its two
 // cells, with Z = bar_rho' + kappa bar_pi'); in place on the bars.
@@ -1688,7 +1741,7 @@ void mixed_fb_substep(const Dims& d, const Tab& t, const Flags& fl, const WS& wi
                       cudaStream_t stream) {
   const dim3 b(32, 4);
   k_mx_fb_mass<<<g3(d.nx, d.ny, d.nz, b), b, 0, stream>>>(d, t, win, wout, dtau);
-  k_mx_fb_mom<<<g3(d.nx + 1, d.ny + 1, d.nz + 1, b), b, 0, stream>>>(d, t, win, wout, dtau, 1);
+  k_mx_fb_mom<<<g3(d.nx + 1, d.ny + 1, d.nz + 1, b), b, 0, stream>>>(d, t, win, wout, dtau);
 }
 
 __device__ __forceinline__ void cp_async8(float* smem, const float* gmem) {
@@ -2271,7 +2324,7 @@ __global__ void __launch_bounds__(128, 7) k_mx_hevi_tmad(const __grid_constant__
 }
 
 // After a stage's last substep of the kDefer column kernel: its u/v backward
-// update (as fb_mom_body) and the w/rho' corrections, in place, in one
+// update (as uv_body) and the w/rho' corrections, in place, in one
 // launch: a thread owns a column position of the (nx+1) x (ny+1) face grid
 // and marches up the levels, reading w~(k+1) (and correcting it) before it
 // writes w(k+1), so no other thread's read races a write (pi' itself is not
@@ -2809,9 +2862,9 @@ int mixed_hevi_column(const Dims& d, const Tab& t, const Flags& fl, const WS& wi
   return 0;
 }
 
-void mixed_uv_backward(const Dims& d, const Tab& t, const WS& win, const WS& wout, float dtau, cudaStream_t stream) {
+void mixed_uv_backward(const Dims& d, const Tab& t, const WS& s, float dtau, cudaStream_t stream) {
   const dim3 b(32, 4);
-  k_mx_fb_mom<<<g3(d.nx + 1, d.ny + 1, d.nz, b), b, 0, stream>>>(d, t, win, wout, dtau, 0);
+  k_mx_uv<<<g3((d.nx + 1) / 2, d.ny, d.nz, b), b, 0, stream>>>(d, t, s, dtau);
 }
 
 bool mixed_hevi_defers(const Dims& d, const Flags& fl) { return hevi_tma_variant(d, fl) == 5; }
@@ -2826,7 +2879,7 @@ int mixed_hevi_substep(const Dims& d, const Tab& t, const Flags& fl, const WS& w
   if (mixed_hevi_column(d, t, fl, win, wout, win, dtau, lu, false, true, err, stream)) return -1;
   // in place: u, v were copied by the column kernel
   if (mixed_hevi_defers(d, fl)) mixed_uv_fix(d, t, fl, wout, dtau, stream);
-  else mixed_uv_backward(d, t, wout, wout, dtau, stream);
+  else mixed_uv_backward(d, t, wout, dtau, stream);
   return 0;
 }
 
@@ -2836,7 +2889,7 @@ void mixed_finish(const Dims& d, const Tab& t, const Flags& fl, const WS& wfin, 
   const dim3 b(32, 4);
   WS none;
   for (int q = 0; q < NSPECIES; ++q) none.f[q] = nullptr;
-  k_mx_finish<<<g3(d.nx + 1, d.ny + 1, d.nz + 1, b), b, 0, stream>>>(d, t, fl, wfin, wst, w0, rin ? *rin : none,
+  k_mx_finish<<<g3(d.nx / 2 + 1, d.ny + 1, d.nz + 1, b), b, 0, stream>>>(d, t, fl, wfin, wst, w0, rin ? *rin : none,
                                                                      (float)dt, cs64(s0), ms64(s1), err, uv_dtau,
                                                                      defer ? 1 : 0);
 }
@@ -3008,7 +3061,7 @@ __global__ void k_b_uv(const UvArgs* __restrict__ A, const int* __restrict__ sta
   const int dom = find_domain(start, nd);
   const UvArgs& a = A[dom];
   const int l = (int)blockIdx.x - start[dom];
-  fb_mom_body(a.d, a.t, a.win, a.wout, a.dtau, 0, l % a.gx, (l / a.gx) % a.gy, l / (a.gx * a.gy));
+  uv_body(a.d, a.t, a.wout, a.dtau, l % a.gx, (l / a.gx) % a.gy, l / (a.gx * a.gy));
 }
 __global__ void __launch_bounds__(128, 8) k_b_fix(const UvArgs* __restrict__ A, const int* __restrict__ start, int nd) {
   const int dom = find_domain(start, nd);
@@ -3166,8 +3219,8 @@ MixedBatch* mixed_batch_build(const std::vector<MixedDomain>& doms, const Flags&
       a.win = ws_from(sub_out(m, n_sub - 1));
       a.wout = a.win;
       a.dtau = dtau;
-      a.gx = ceil_div(m.d.nx + 1, b->defer ? 32 * kFixPos : 32);  // (the fix-up: kFixPos positions per thread)
-      a.gy = ceil_div(m.d.ny + 1, 4);
+      a.gx = b->defer ? ceil_div(m.d.nx + 1, 32 * kFixPos) : ceil_div(m.d.nx, 64);  // kFixPos or two columns per thread
+      a.gy = ceil_div(m.d.ny + (b->defer ? 1 : 0), 4);
       a.gz = b->defer ? 1 : m.d.nz;  // the deferred fix-up marches the levels
       start[q] = ub;
       ub += a.gx * a.gy * a.gz;
@@ -3193,7 +3246,7 @@ MixedBatch* mixed_batch_build(const std::vector<MixedDomain>& doms, const Flags&
       a.s0 = cs64(m.S0);
       a.s1 = ms64(m.S1);
       a.defer = b->defer ? 1 : 0;
-      a.gx = ceil_div(m.d.nx + 1, 32);
+      a.gx = ceil_div(m.d.nx + 1, 64);
       a.gy = ceil_div(m.d.ny + 1, 4);
       a.gz = m.d.nz + 1;
       start[q] = fb;
