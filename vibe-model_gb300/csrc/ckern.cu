@@ -643,27 +643,39 @@ constexpr int kCflThreads = 256;
 // CFL scan (c_kernels.c:148-186): per cell dz = max(dzeta[k]*scale, 1),
 // speed = sqrt(u^2+v^2+w^2), cfl = dt*(|u|/dx + |v|/dy + |w|/dz); block maxima
 // of (cfl, speed) and min of dz, then one block merges.
+// The three are never negative nor NaN, so they order as their bits: the merges
+// are integer comparisons (FP64 ones would issue at the FP64 rate).
+__device__ __forceinline__ long long order_bits(double x) { return __double_as_longlong(x); }
+__device__ __forceinline__ int order_bits(float x) { return __float_as_int(x); }
+__device__ __forceinline__ double from_order(long long b) { return __longlong_as_double(b); }
+__device__ __forceinline__ float from_order(int b) { return __int_as_float(b); }
 template <typename T>
-__device__ __forceinline__ void max3_block(T& a, T& b, T& c) {  // max, max, min
-  __shared__ T s1[32], s2[32], s3[32];
-  for (int off = 16; off > 0; off >>= 1) {
-    a = fmax(a, __shfl_down_sync(0xffffffffu, a, off));
-    b = fmax(b, __shfl_down_sync(0xffffffffu, b, off));
-    c = fmin(c, __shfl_down_sync(0xffffffffu, c, off));
-  }
+__device__ __forceinline__ void max3_block(T& ta, T& tb, T& tc) {  // max, max, min
+  using I = decltype(order_bits(T()));
+  __shared__ I s1[32], s2[32], s3[32];
+  I a = order_bits(ta), b = order_bits(tb), c = order_bits(tc);
+  auto merge = [&]() {
+    for (int off = 16; off > 0; off >>= 1) {
+      const I x = __shfl_down_sync(0xffffffffu, a, off), y = __shfl_down_sync(0xffffffffu, b, off),
+              z = __shfl_down_sync(0xffffffffu, c, off);
+      a = x > a ? x : a;
+      b = y > b ? y : b;
+      c = z < c ? z : c;
+    }
+  };
+  merge();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
   if (lane == 0) { s1[warp] = a; s2[warp] = b; s3[warp] = c; }
   __syncthreads();
   if (warp == 0) {
-    a = lane < nw ? s1[lane] : (T)0;
-    b = lane < nw ? s2[lane] : (T)0;
-    c = lane < nw ? s3[lane] : (T)1e30;
-    for (int off = 16; off > 0; off >>= 1) {
-      a = fmax(a, __shfl_down_sync(0xffffffffu, a, off));
-      b = fmax(b, __shfl_down_sync(0xffffffffu, b, off));
-      c = fmin(c, __shfl_down_sync(0xffffffffu, c, off));
-    }
+    a = lane < nw ? s1[lane] : 0;
+    b = lane < nw ? s2[lane] : 0;
+    c = lane < nw ? s3[lane] : order_bits((T)1e30);
+    merge();
   }
+  ta = from_order(a);
+  tb = from_order(b);
+  tc = from_order(c);
 }
 // Most cells cannot raise a maximum, and finding that out in FP64 costs three
 // divisions a cell. So a cell's CFL number and squared speed are first bounded
@@ -692,6 +704,9 @@ __device__ __forceinline__ float trunc_signed(double x) {  // rounded toward zer
 __device__ __forceinline__ float trunc_signed(float x) { return x; }
 __device__ __forceinline__ unsigned down_bits(double x) { return __float_as_uint(__double2float_rd(x)); }
 __device__ __forceinline__ unsigned down_bits(float x) { return __float_as_uint(x); }
+// What is left of FP64: one subtraction a thread and tile, the column's smallest dz
+// in the bottom tiles, the cells evaluated. 384 x 384 x 60 (floor 31 us): 61 us; 89 with
+// the extent of dzeta, the merges and the roots in every warp (FP64 pipe 76 % busy).
 constexpr int kCflLevels = 4;  // levels of one tile
 template <typename T>
 __global__ void __launch_bounds__(kCflThreads, 4) k_cfl_partial(const T* __restrict__ u, const T* __restrict__ v,
@@ -714,23 +729,31 @@ __global__ void __launch_bounds__(kCflThreads, 4) k_cfl_partial(const T* __restr
   if (threadIdx.x < 2) best[threadIdx.x] = seen[0][threadIdx.x] = 0u;
   __syncthreads();
   int par = 0;
-  T dlo = (T)NAN, dhi = (T)NAN;
-  for (int k = threadIdx.x & 31; k < nz; k += 32) {
-    dlo = fmin(dlo, dzeta[k]);
-    dhi = fmax(dhi, dzeta[k]);
+  __shared__ T dext[2];  // the smallest and the largest dzeta, for the blocks that have bottom tiles
+  if (blockIdx.x < ctiles && threadIdx.x < 32) {
+    T dlo = (T)NAN, dhi = (T)NAN;
+    for (int k = threadIdx.x; k < nz; k += 32) {
+      dlo = fmin(dlo, dzeta[k]);
+      dhi = fmax(dhi, dzeta[k]);
+    }
+    for (int off = 16; off > 0; off >>= 1) {
+      dlo = fmin(dlo, __shfl_xor_sync(0xffffffffu, dlo, off));
+      dhi = fmax(dhi, __shfl_xor_sync(0xffffffffu, dhi, off));
+    }
+    if (threadIdx.x == 0) {
+      dext[0] = dlo;
+      dext[1] = dhi;
+    }
   }
-  for (int off = 16; off > 0; off >>= 1) {
-    dlo = fmin(dlo, __shfl_xor_sync(0xffffffffu, dlo, off));
-    dhi = fmax(dhi, __shfl_xor_sync(0xffffffffu, dhi, off));
-  }
+  __syncthreads();
   for (size_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
     const size_t kt = tile / ctiles, col = (tile - kt * ctiles) * kCflThreads + threadIdx.x;
     const int k0 = (int)kt * kCflLevels;
     const bool in = col < nxy;
     const T scale = zs ? (in ? z_top - zs[col] : (T)1) : z_top;
-    const float fscale = (float)scale;
+    const float fscale = trunc_signed(scale);
     if (in && k0 == 0) {
-      T dz = fmin(dlo * scale, dhi * scale);
+      T dz = fmin(dext[0] * scale, dext[1] * scale);
       if (dz < (T)1) dz = (T)1;
       mdz = fmin(mdz, dz);
     }
@@ -790,11 +813,10 @@ __global__ void __launch_bounds__(kCflThreads, 4) k_cfl_partial(const T* __restr
     par ^= 1;
     __syncthreads();  // seen[par] is clear, best is settled
   }
-  T mw = sqrt(mw2);
-  max3_block(worst, mw, mdz);
+  max3_block(worst, mw2, mdz);
   if (threadIdx.x == 0) {
     partials[3 * blockIdx.x] = worst;
-    partials[3 * blockIdx.x + 1] = mw;
+    partials[3 * blockIdx.x + 1] = sqrt(mw2);
     partials[3 * blockIdx.x + 2] = mdz;
   }
 }
