@@ -879,7 +879,7 @@ int enqueue_one_step(vibe_gb300_model* m, double dt, int n_sub) {
             // the u/v update of substep n-1 is applied inside substep n's column kernel
             Span sp(m, 1);
             if (mixed_hevi_column(d, m->tab, m->fl, ws_of(in), ws_of(out), ws_of(st_out), dtau, m->d_lu + (size_t)stage * 3 * d.nz,
-                                  n > 0, n == n_sub - 1, m->d_err, m->stream))
+                                  n > 0, n == n_sub - 1 && stage < 2, m->d_err, m->stream))
               return fail(VIBE_GB300_EDEVICE, "TMA descriptor creation failed (cuTensorMapEncodeTiled)");
           } else {
             Span sp(m, 1);
@@ -908,7 +908,8 @@ int enqueue_one_step(vibe_gb300_model* m, double dt, int n_sub) {
       const WS wr = ws_of(m->WR);
       // stage 3's last u/v update is folded into the finish kernel
       mixed_finish(d, m->tab, m->fl, ws_of(final_sub), ws_of(m->WSt[0]), w0, &wr, dt, S0, S1, m->d_err, m->stream,
-                   m->fl.acoustic_mode == 2 ? last_dtau : 0.f, m->fl.acoustic_mode == 2 && mixed_hevi_defers(d, m->fl));
+                   m->fl.acoustic_mode == 2 ? last_dtau : 0.f,
+                   m->fl.acoustic_mode == 2 ? mixed_hevi_finish(d, m->fl) : 0);
     }
     m->cur = 1 - m->cur;
   }

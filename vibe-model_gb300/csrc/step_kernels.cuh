@@ -118,8 +118,10 @@ int mixed_hevi_column(const Dims& d, const Tab& t, const Flags& fl, const WS& wi
 void mixed_uv_backward(const Dims& d, const Tab& t, const WS& s, float dtau, cudaStream_t stream);
 // whether the column kernel chosen for this grid defers its w/rho'
 // corrections to the reader (then the last substep of a stage is finished
-// by mixed_uv_fix instead of mixed_uv_backward, and mixed_finish gets defer)
+// by mixed_uv_fix instead of mixed_uv_backward)
 bool mixed_hevi_defers(const Dims& d, const Flags& fl);
+// mixed_finish's defer after that kernel's stage 3 without `last`
+int mixed_hevi_finish(const Dims& d, const Flags& fl);
 // u/v backward update and the deferred w/rho' corrections, in place
 void mixed_uv_fix(const Dims& d, const Tab& t, const Flags& fl, const WS& s, float dtau, cudaStream_t stream);
 // adjoint of mixed_fb_substep, in place on bars of (u, v, w, rho', pi')
@@ -132,7 +134,7 @@ void mixed_hevi_substep_ad(const Dims& d, const Tab& t, const Flags& fl, const W
 // in-place mixed_uv_backward launch is then left out)
 void mixed_finish(const Dims& d, const Tab& t, const Flags& fl, const WS& wfin, const WS& wst, const WS& w0,
                   const WS* rin, double dt, double* const* s0, double* const* s1, unsigned* err,
-                  cudaStream_t stream, float uv_dtau = 0.f, bool defer = false);
+                  cudaStream_t stream, float uv_dtau = 0.f, int defer = 0);
 // ---- several domains per launch (work-list), mixed path, HEVI mode ----
 struct MixedDomain {
   Dims d;

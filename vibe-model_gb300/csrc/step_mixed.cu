@@ -1228,15 +1228,18 @@ __device__ __forceinline__ float defer_fix_rho(const Tab& t, float db, float rt,
   return rt + db * (-(t.rfz[k + 1] * wk1 - t.rfz[k] * wk) * t.idzc[k]);
 }
 
-// defer: wfin is a kDefer column kernel's output; its w and rho' get their
-// corrections (with dtau = uv_dtau) on the fly
+// defer: what of the last substep's output is still to be corrected here, on the
+// fly (with dtau = uv_dtau): kDeferSweep the w and rho' of a kDefer column kernel,
+// kDeferChunk those of the level-split kernel, whose rho' follows from pi'
+// (hevi_chunk_body: 16 B a cell less than by its last substep)
+enum FinishDefer { kDeferNone = 0, kDeferSweep = 1, kDeferChunk = 2 };
 // Two columns a thread, 8- and 16-byte accesses (rows are padded to whole pairs;
 // what lies past a field's box is read and not used). Bound by memory: 216 B a
 // cell, 512 x 512 x 80 672 us (6.7 TB/s), 801 with one column a thread.
 __device__ __forceinline__ void finish_body(const Dims& d, const Tab& t, const Flags& fl, const WS& wfin,
                                             const WS& wst, const WS& w0, const WS& rin, float dtf, const CS64& s0,
                                             const MS64& s1, unsigned* err, int bx, int by, int bz,
-                                            float uv_dtau = 0.f, bool defer = false) {
+                                            float uv_dtau = 0.f, int defer = kDeferNone) {
   const int i = 2 * (bx * blockDim.x + threadIdx.x);
   const int j = by * blockDim.y + threadIdx.y;
   const int k = bz;
@@ -1319,13 +1322,22 @@ __device__ __forceinline__ void finish_body(const Dims& d, const Tab& t, const F
   }
   if (cell && lev) {
     {
-      float2 wv = ld(wfin.f[RHO]);
-      if (defer) {
-        wv.x = defer_fix_rho(t, db, wv.x, w_at(0, k), w_at(0, k + 1), k);
-        wv.y = defer_fix_rho(t, db, wv.y, w_at(1, k), w_at(1, k + 1), k);
-      }
       const float2 ws = ld(wst.f[RHO]);
-      double2 v = total(RHO, make_float2(wv.x - ws.x, wv.y - ws.y));
+      float2 wv, da;
+      if (defer == kDeferChunk) {
+        const float2 pe = ld(wfin.f[PI]), ps = ld(wst.f[PI]);
+        const float ik = 1.f / t.kap[k];
+        da = make_float2((pe.x - ps.x) * ik, (pe.y - ps.y) * ik);
+        wv = make_float2(ws.x + da.x, ws.y + da.y);
+      } else {
+        wv = ld(wfin.f[RHO]);
+        if (defer) {
+          wv.x = defer_fix_rho(t, db, wv.x, w_at(0, k), w_at(0, k + 1), k);
+          wv.y = defer_fix_rho(t, db, wv.y, w_at(1, k), w_at(1, k + 1), k);
+        }
+        da = make_float2(wv.x - ws.x, wv.y - ws.y);
+      }
+      double2 v = total(RHO, da);
       if (!plain) v = make_double2(wd * (v.x + sdt * t.r0d[kc]), wd * (v.y + sdt * t.r0d[kc]));
       put(RHO, v, make_float2(wf * wv.x, wf * wv.y), cell2);
     }
@@ -1353,8 +1365,7 @@ __global__ void k_mx_finish(const __grid_constant__ Dims d, const __grid_constan
                             const __grid_constant__ WS wst, const __grid_constant__ WS w0,
                             const __grid_constant__ WS rin, float dtf, const __grid_constant__ CS64 s0,
                             const __grid_constant__ MS64 s1, unsigned* err, float uv_dtau, int defer) {
-  finish_body(d, t, fl, wfin, wst, w0, rin, dtf, s0, s1, err, blockIdx.x, blockIdx.y, blockIdx.z, uv_dtau,
-              defer != 0);
+  finish_body(d, t, fl, wfin, wst, w0, rin, dtf, s0, s1, err, blockIdx.x, blockIdx.y, blockIdx.z, uv_dtau, defer);
 }
 
 __global__ void k_mx_unpack_f32(Dims d, int nsx, int nsy, int nsz, int ni, int nj, int nk, const float* __restrict__ src,
@@ -2891,6 +2902,10 @@ void mixed_uv_backward(const Dims& d, const Tab& t, const WS& s, float dtau, cud
 }
 
 bool mixed_hevi_defers(const Dims& d, const Flags& fl) { return hevi_tma_variant(d, fl) == 5; }
+int mixed_hevi_finish(const Dims& d, const Flags& fl) {
+  const int v = hevi_tma_variant(d, fl);
+  return v == 5 ? kDeferSweep : v == 6 ? kDeferChunk : kDeferNone;
+}
 
 void mixed_uv_fix(const Dims& d, const Tab& t, const Flags& fl, const WS& s, float dtau, cudaStream_t stream) {
   const dim3 b(32, 4);
@@ -2908,13 +2923,13 @@ int mixed_hevi_substep(const Dims& d, const Tab& t, const Flags& fl, const WS& w
 
 void mixed_finish(const Dims& d, const Tab& t, const Flags& fl, const WS& wfin, const WS& wst, const WS& w0,
                   const WS* rin, double dt, double* const* s0, double* const* s1, unsigned* err,
-                  cudaStream_t stream, float uv_dtau, bool defer) {
+                  cudaStream_t stream, float uv_dtau, int defer) {
   const dim3 b(32, 4);
   WS none;
   for (int q = 0; q < NSPECIES; ++q) none.f[q] = nullptr;
   k_mx_finish<<<g3(d.nx / 2 + 1, d.ny + 1, d.nz + 1, b), b, 0, stream>>>(d, t, fl, wfin, wst, w0, rin ? *rin : none,
                                                                      (float)dt, cs64(s0), ms64(s1), err, uv_dtau,
-                                                                     defer ? 1 : 0);
+                                                                     defer);
 }
 
 void mixed_unpack_f32(const Dims& d, int nsx, int nsy, int nsz, int ni, int nj, int nk, const float* src, double* dst,
@@ -3098,7 +3113,7 @@ __global__ void k_b_finish(const FinishArgs* __restrict__ A, const int* __restri
   const FinishArgs& a = A[dom];
   const int l = (int)blockIdx.x - start[dom];
   finish_body(a.d, a.t, a.fl, a.wfin, a.wst, a.w0, a.rin, a.dtf, a.s0, a.s1, err, l % a.gx, (l / a.gx) % a.gy,
-              l / (a.gx * a.gy), a.uv_dtau, a.defer != 0);
+              l / (a.gx * a.gy), a.uv_dtau, a.defer);
 }
 
 WS ws_from(float* const* a) {
@@ -3221,7 +3236,7 @@ MixedBatch* mixed_batch_build(const std::vector<MixedDomain>& doms, const Flags&
         a.cdy = -(float)kCp * dtau * m.t.dy_inv;
         a.lu = m.lu + (size_t)stage * 3 * nz;
         a.apply_uv = n > 0;
-        a.last = n == n_sub - 1;
+        a.last = n == n_sub - 1 && stage < 2;  // (stage 3's corrections: the finish)
         if (b->hevi_tma && !column_maps(m.d, a.win, a.wout, a.C)) ok = false;
         a.gx = ceil_div(m.d.nx, 64);  // two columns per thread
         a.gy = ceil_div(m.d.ny, 4);
@@ -3268,7 +3283,7 @@ MixedBatch* mixed_batch_build(const std::vector<MixedDomain>& doms, const Flags&
       a.uv_dtau = (float)(dt / (double)n_sub);
       a.s0 = cs64(m.S0);
       a.s1 = ms64(m.S1);
-      a.defer = b->defer ? 1 : 0;
+      a.defer = b->split ? kDeferChunk : b->defer ? kDeferSweep : kDeferNone;
       a.gx = ceil_div(m.d.nx + 1, 64);
       a.gy = ceil_div(m.d.ny + 1, 4);
       a.gz = m.d.nz + 1;
