@@ -930,16 +930,18 @@ def main():
     peak, peak_kind = measured_peak()
     # algorithmic bytes per cell of one launch of each kernel class (FP32 fields 4 B, FP64 8 B):
     # stage: 56 (stage 1: win = w0), 84 (stage 2), 112 (stage 3, + its tendency);
-    # column: read u v w rho pi, write w rho pi u v; finish: read S0, R3, 5 substep
-    # fields, 7 stage fields, write S1, W0; after a stage's last substep, in
-    # place: u/v update (read u v pi, write u v) and, when the column kernel
-    # defers its w/rho' corrections (variant 5, the built-in one), those
+    # column: read u v w pi, write the same (the level-split kernel, the built-in
+    # one: rho follows once a stage, + 12 B in a stage's last substep but the
+    # third's) or also rho (the others); finish: read S0, R3, the substep fields, 7
+    # stage fields, write S1, W0; after a stage's last substep, in place: u/v update
+    # (read u v pi, write u v) and, after the deferring sweep (variant 5), its w/rho'
     # corrections too in the same column march (+ read w rho, write w rho)
     col = tuning.get("column_kernel", -1) if isinstance(tuning, dict) else -1
-    defer = col in (-1, 5)
-    per_cell = {0: (56.0 + 84.0 + 112.0) / 3.0, 1: 40.0, 2: 216.0, 3: 36.0 if defer else 20.0}
-    names = {0: "k_mx_stage", 1: "k_mx_hevi_tmad" if defer else "k_mx_hevi_tma", 2: "k_mx_finish",
-             3: "k_mx_fix" if defer else "k_mx_fb_mom(u,v)"}
+    split, defer = col == -1, col == 5
+    per_cell = {0: (56.0 + 84.0 + 112.0) / 3.0, 1: 32.0 + 2 * 12.0 / (3 * NSUB) if split else 40.0,
+                2: 212.0 if split else 216.0, 3: 36.0 if defer else 20.0}
+    names = {0: "k_mx_stage", 1: "k_mx_hevi_chunk" if split else "k_mx_hevi_tmad" if defer else "k_mx_hevi_tma",
+             2: "k_mx_finish", 3: "k_mx_fix" if defer else "k_mx_uv"}
     dom = max(ktimes, key=lambda c: ktimes[c][0])
     tot_ms, spans = ktimes[dom]
     avg_s = tot_ms / max(spans, 1) * 1e-3

@@ -290,9 +290,9 @@ int vibe_gb300_hevi_substep(vibe_gb300_model *m, double dtau);
  * 1 cp.async ring, 2/3 two columns per thread, 4 two columns per thread fed
  * by TMA boxes, 5 the same with the w/rho' corrections of the implicit
  * sweep applied by the next reader of those fields, which cuts the
- * backward sweep's traffic to pi' alone -- the built-in choice; -1 = the
- * built-in choice) and
- * the stage kernel's levels per block -- and keeps the fastest for every
+ * backward sweep's traffic to pi' alone; -1 = the built-in choice: the
+ * levels split over warps, and 5 for moist models, columns too tall for the
+ * split and reference states of very high pressure) and the stage kernel's levels per block -- and keeps the fastest for every
  * single model of this grid in the process (groups keep the built-in column
  * kernel). Variants differ only by FP32 rounding (FMA contraction, vertical
  * fluxes recomputed at level-chunk starts). The model's state is left as it
