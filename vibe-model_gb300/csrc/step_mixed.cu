@@ -2486,6 +2486,11 @@ size_t hevi_tma_smem_bytes(int nz) {
 // three domains of 192 x 192 x 60 and below 29.3 (35.3). More loads in flight (a
 // ring of cp.async copies, 3 to 6 levels), bulk prefetches into L2 and
 // streaming hints made it slower or nothing: 170 to 232, 197, 176 to 178.
+// The form with this many levels a warp, that of the small grids, is launched early:
+// its blocks leave SMs free, so the next launch's tables are made meanwhile (64 x 64 x
+// 40, four steps: 1.24 to 1.15 ms). Larger grids have no SM free, and blocks that wait
+// keep other streams' out (193 x 193 x 60, three models in turn: 1.3 % slower).
+constexpr int kChunkEarly = 4;
 size_t hevi_chunk_smem_bytes(int nz, int m) {
   const int C = (nz + m - 1) / m;
   return ((size_t)(3 * nz + 1)) * sizeof(float4) + (size_t)64 * C * sizeof(float2);
@@ -2514,17 +2519,36 @@ __device__ __forceinline__ void hevi_chunk_body(const Dims& d, const Tab& t, con
   const unsigned pl = (unsigned)d.plane;
   const unsigned col = active ? (unsigned)e : 0u;
   // 32-bit offsets from the fields' bases (the mixed path's fields have fewer
-  // than 2^32 points); the inputs are other buffers than the outputs, so the
-  // read-only loads may pass the stores
-  auto ld2 = [&](int q, unsigned o) { return __ldg(reinterpret_cast<const float2*>(win.f[q] + o)); };
-  auto ld1 = [&](int q, unsigned o) { return __ldg(win.f[q] + o); };
+  // than 2^32 points); the inputs are other buffers than the outputs, so these
+  // loads may pass the stores. Launched early they may not pass the wait for the
+  // launch before, which hands them their offset, nor be read-only ones: that
+  // launch writes their fields while this one already runs.
+  constexpr bool kEarly = kM == kChunkEarly;
+  auto ldf2 = [](const float* p) {
+    if (!kEarly) return __ldg(reinterpret_cast<const float2*>(p));
+    float2 v;
+    asm("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
+    return v;
+  };
+  auto ld2 = [&](int q, unsigned o) { return ldf2(win.f[q] + o); };
+  auto ld1 = [&](int q, unsigned o) {
+    if (!kEarly) return __ldg(win.f[q] + o);
+    float v;
+    asm("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(win.f[q] + o));
+    return v;
+  };
   auto st2 = [&](int q, unsigned o, float2 v) {
     if (two) *reinterpret_cast<float2*>(wout.f[q] + o) = v;
     else wout.f[q][o] = v.x;
   };
   unsigned o = (unsigned)k0 * pl + col;
-  float2 pk = ld2(PI, o), wk = ld2(W, o);
-  const float2 pm = ld2(PI, k0 > 0 ? o - pl : o);
+  float2 pk, wk, pm;
+  auto first = [&]() {
+    pk = ld2(PI, o);
+    wk = ld2(W, o);
+    pm = ld2(PI, k0 > 0 ? o - pl : o);
+  };
+  if (!kEarly) first();
   const float b = (float)fl.hevi_beta, ob = 1.f - b;
   const float cpf = (float)kCp;
   for (int k = tid; k <= nz; k += 32 * C) {
@@ -2543,6 +2567,15 @@ __device__ __forceinline__ void hevi_chunk_body(const Dims& d, const Tab& t, con
   const int ope = !active ? 0 : (i + 2 < d.nx) ? 2 : (two ? 1 : 0);
   const int ops = (active && j > 0) ? -vn : 0, opn = (active && j + 1 < d.ny) ? vn : 0;
   const bool last_j = (j == d.ny - 1), last_i = (i + 2 >= d.nx);
+  if (kEarly) {
+    // (programmatic dependent launch) All above reads tables that no launch of the
+    // step writes and runs beside the launch before this one, which is complete and
+    // visible behind the wait. Nothing is written before it. The next launch may
+    // start once every block is here; it waits likewise.
+    asm volatile("griddepcontrol.wait;" : "+r"(o) : : "memory");
+    asm volatile("griddepcontrol.launch_dependents;" : : : "memory");
+    first();
+  }
   __syncthreads();
   float2 dp[kM], wt, prev = make_float2(0.f, 0.f);
   {
@@ -2649,7 +2682,7 @@ __device__ __forceinline__ void hevi_chunk_body(const Dims& d, const Tab& t, con
     in = make_float2(f.x + h * in.x, f.y + h * in.y);
   }
   if (!active) return;
-  o = (unsigned)k0 * pl + col;
+  o = kEarly ? o - (unsigned)kn * pl : (unsigned)k0 * pl + col;  // (early: still the wait's)
 #pragma unroll
   for (int q = 0; q < kM; ++q)
     if (q < kn) {
@@ -2678,8 +2711,7 @@ __device__ __forceinline__ void hevi_chunk_body(const Dims& d, const Tab& t, con
       const float2 xf = top ? in : dp[q + 1 < kM ? q + 1 : q];
       const float2 wf = top ? wt : back(W, o + pl);
       const float2 wn = make_float2(wf.x - a * (xf.x - dp[q].x), wf.y - a * (xf.y - dp[q].y));
-      const float2 r = __ldg(reinterpret_cast<const float2*>(wst.f[RHO] + o));
-      const float2 p = __ldg(reinterpret_cast<const float2*>(wst.f[PI] + o));
+      const float2 r = ldf2(wst.f[RHO] + o), p = ldf2(wst.f[PI] + o);
       st2(RHO, o, make_float2(r.x + (dp[q].x - p.x) * ik, r.y + (dp[q].y - p.y) * ik));
       st2(W, o, wb);
       wb = wn;
@@ -2769,14 +2801,22 @@ int hevi_chunk_blocks(const Dims& d) { return ((d.ny - 1) * d.P + d.nx + 63) / 6
 #define VGB_CHUNK_LAUNCH(Kernel, m, nz, blocks, st, ...)                                                        \
   do {                                                                                                          \
     const int C_ = ((nz) + (m) - 1) / (m);                                                                      \
-    const dim3 b_(32, C_);                                                                                      \
-    const size_t sm_ = hevi_chunk_smem_bytes(nz, m);                                                            \
-    if ((m) == 4) Kernel<4, 640, 1><<<blocks, b_, sm_, st>>>(__VA_ARGS__);                                      \
-    else if ((m) == 6) Kernel<6, 256, 4><<<blocks, b_, sm_, st>>>(__VA_ARGS__);                                 \
-    else if ((m) == 8 && C_ <= 8) Kernel<8, 256, 4><<<blocks, b_, sm_, st>>>(__VA_ARGS__);                      \
-    else if ((m) == 8) Kernel<8, 640, 1><<<blocks, b_, sm_, st>>>(__VA_ARGS__);                                 \
-    else if (C_ <= 8) Kernel<10, 256, 4><<<blocks, b_, sm_, st>>>(__VA_ARGS__);                                 \
-    else Kernel<10, 640, 1><<<blocks, b_, sm_, st>>>(__VA_ARGS__);                                              \
+    cudaLaunchAttribute at_;                                                                                    \
+    at_.id = cudaLaunchAttributeProgrammaticStreamSerialization;                                                \
+    at_.val.programmaticStreamSerializationAllowed = 1;                                                         \
+    cudaLaunchConfig_t cf_ = {};                                                                                \
+    cf_.gridDim = dim3(blocks);                                                                                 \
+    cf_.blockDim = dim3(32, C_);                                                                                \
+    cf_.dynamicSmemBytes = hevi_chunk_smem_bytes(nz, m);                                                        \
+    cf_.stream = st;                                                                                            \
+    cf_.attrs = &at_;                                                                                           \
+    cf_.numAttrs = (m) == kChunkEarly ? 1 : 0;                                                                  \
+    if ((m) == 4) cudaLaunchKernelEx(&cf_, Kernel<4, 640, 1>, __VA_ARGS__);                                     \
+    else if ((m) == 6) cudaLaunchKernelEx(&cf_, Kernel<6, 256, 4>, __VA_ARGS__);                                \
+    else if ((m) == 8 && C_ <= 8) cudaLaunchKernelEx(&cf_, Kernel<8, 256, 4>, __VA_ARGS__);                     \
+    else if ((m) == 8) cudaLaunchKernelEx(&cf_, Kernel<8, 640, 1>, __VA_ARGS__);                                \
+    else if (C_ <= 8) cudaLaunchKernelEx(&cf_, Kernel<10, 256, 4>, __VA_ARGS__);                                \
+    else cudaLaunchKernelEx(&cf_, Kernel<10, 640, 1>, __VA_ARGS__);                                             \
   } while (0)
 
 // Ring depth of the two-columns-per-thread kernel (0 = off);
