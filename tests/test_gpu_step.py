@@ -544,6 +544,34 @@ def test_early_launched_substeps_repeat_bits(vg, dims, n_sub):
                 assert np.array_equal(st[sp], ref[sp]), vg.SPECIES[sp]
 
 
+@pytest.mark.parametrize("moist", [0, 1])
+@pytest.mark.parametrize("dims", [(5, 3, 7), (33, 17, 8), (8, 6, 4)])
+def test_snapshot_restore_repeats_bits(vg, dims, moist):
+    """A restored snapshot is the saved state, ghost points and species that are
+    not prognostic included, and steps from it repeat their bits, mixed (state
+    and working copy in one pass, odd and even rows) and FP64."""
+    nx, ny, nz = dims
+    s = small_setup(vg, nx=nx, ny=ny, nz=nz, zeta_stretch=1.0, bubble_xc=nx * 125.0, bubble_yc=ny * 125.0, moist=moist,
+                    qv_surface=0.01, **STEP_CASES[3])
+    rng = np.random.default_rng(5)
+    for prec in (vg.MIXED, vg.FP64):
+        with vg.Model(s, prec) as m:
+            for sp in range(12):
+                a = m.get(sp)
+                m.set(sp, a + 1e-4 * rng.uniform(0.0, 1.0, a.shape) * (a != 0 if sp < 7 else 1))
+            saved = [m.get(sp) for sp in range(12)]
+            m.save_snapshot()
+            m.step(0.5, 2, 3)
+            first = [m.get(sp) for sp in range(12)]
+            for _ in range(2):
+                m.restore_snapshot()
+                for sp in range(12):
+                    assert np.array_equal(m.get(sp), saved[sp]), vg.SPECIES[sp]
+                m.step(0.5, 2, 3)
+                for sp in range(12):
+                    assert np.array_equal(m.get(sp), first[sp]), vg.SPECIES[sp]
+
+
 def test_autotune_keeps_the_update(vg):
     """The autotuner only chooses among launch shapes of the same update: a run
     after tuning matches the run before it to FP32 rounding (1e-6 of each

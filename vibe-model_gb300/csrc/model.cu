@@ -997,6 +997,16 @@ int sync_working(vibe_gb300_model* m) {
   return 0;
 }
 
+// the current state = from, with its working copy
+int restore_state(vibe_gb300_model* m, double* const* from) {
+  if (m->precision == VIBE_GB300_MIXED)
+    mixed_restore(m->d, m->tab, from, m->S[m->cur], working_targets(m, m->W0), m->stream);
+  else
+    state_copy(m->d.plane * (size_t)(m->d.nz + 1), m->S[m->cur], from, m->stream);
+  CUDA_OK(cudaGetLastError());
+  return 0;
+}
+
 }  // namespace
 
 // ===========================================================================
@@ -1964,15 +1974,13 @@ int vibe_gb300_snapshot(vibe_gb300_model* m, int op) {
     if (!m->snap[0])
       for (int q = 0; q < NSPECIES; ++q)
         if (int rc = dalloc(m, &m->snap[q], n)) return rc;
-    for (int q = 0; q < NSPECIES; ++q)
-      CUDA_OK(cudaMemcpyAsync(m->snap[q], m->S[m->cur][q], n * sizeof(double), cudaMemcpyDeviceToDevice, m->stream));
+    state_copy(n, m->snap, m->S[m->cur], m->stream);
+    CUDA_OK(cudaGetLastError());
     m->has_snap = true;
     return 0;
   }
   if (!m->has_snap) return fail(VIBE_GB300_EBADARG, "no snapshot saved");
-  for (int q = 0; q < NSPECIES; ++q)
-    CUDA_OK(cudaMemcpyAsync(m->S[m->cur][q], m->snap[q], n * sizeof(double), cudaMemcpyDeviceToDevice, m->stream));
-  return sync_working(m);
+  return restore_state(m, m->snap);
 }
 
 int vibe_gb300_sponge(vibe_gb300_model* m, double dt) {
@@ -2531,8 +2539,7 @@ int window_checkpoint(vibe_gb300_window* w, int c) {
   return sync_working(w->m);
 }
 int window_restart(vibe_gb300_window* w, int c) {
-  if (int rc = copy_state(w->m, w->m->S[w->m->cur], w->ckpt[c].data())) return rc;
-  return sync_working(w->m);
+  return restore_state(w->m, w->ckpt[c].data());
 }
 int window_begin(vibe_gb300_window* w) {
   CUDA_OK(cudaEventRecord(w->e0, w->m->stream));

@@ -161,6 +161,9 @@ void mixed_batch_destroy(MixedBatch* b);
 void mixed_unpack_f32(const Dims& d, int nsx, int nsy, int nsz, int ni, int nj, int nk, const float* src, double* dst,
                       cudaStream_t stream);
 void mixed_to_working(const Dims& d, const Tab& t, double* const* s, const WS& w, cudaStream_t stream);
+// to = from (all points of the twelve fields) and its working copy, in one pass
+void mixed_restore(const Dims& d, const Tab& t, double* const* from, double* const* to, const WS& w,
+                   cudaStream_t stream);
 // the same conversion on the columns of the box [ia, ia + ni) x [ja, ja + nj)
 // (clipped to the grid)
 void mixed_to_working_region(const Dims& d, const Tab& t, double* const* s, const WS& w, int ia, int ja, int ni,

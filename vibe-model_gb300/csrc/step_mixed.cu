@@ -1422,6 +1422,33 @@ __global__ void k_mx_to_working(const __grid_constant__ Dims d, const __grid_con
                                 const __grid_constant__ CS64 s, const __grid_constant__ WS w) {
   to_working_body(d, t, s, w, blockIdx.x, blockIdx.y, blockIdx.z);
 }
+// The whole arrays of a state copied and the working copy made of them on the way (as
+// to_working_point), one launch for the twelve fields instead of a copy each and a
+// pass that reads them again; two points a thread. Bound by memory: 512 x 512 x 80
+// 681 us (6.8 TB/s), copies and pass 1078.
+__global__ void k_mx_restore(const __grid_constant__ Dims d, const __grid_constant__ Tab t,
+                             const __grid_constant__ CS64 from, const __grid_constant__ MS64 to,
+                             const __grid_constant__ WS w) {
+  const unsigned e = 2 * (blockIdx.x * blockDim.x + threadIdx.x);
+  if (e >= d.plane) return;
+  const int k = blockIdx.y, j = (int)(e / (unsigned)d.P), i = (int)(e - (unsigned)j * d.P);  // (rows hold whole pairs)
+  const size_t c = (size_t)k * d.plane + e;
+  const bool cells = k < d.nz;
+#pragma unroll
+  for (int q = 0; q < NSPECIES; ++q) {
+    const double2 v = *reinterpret_cast<const double2*>(from.f[q] + c);
+    *reinterpret_cast<double2*>(to.f[q] + c) = v;
+    if (!w.f[q]) continue;  // not prognostic
+    const bool rows = q == U || q == W ? j < d.ny : j <= d.ny;
+    if (!rows || (q != W && !cells)) continue;
+    const int iend = q == V || q == W ? d.nx - 1 : d.nx;  // the last column of the field's box, ghosts included
+    const double r = q == RHO ? t.r0d[k] : q == THETA ? t.t0dd[k] : q == PI ? t.p0d[k] : 0.0;
+    const bool dep = q == RHO || q == THETA || q == PI;
+    const float2 f = make_float2(narrow(dep ? v.x - r : v.x), narrow(dep ? v.y - r : v.y));
+    if (i + 1 <= iend) *reinterpret_cast<float2*>(w.f[q] + c) = f;
+    else if (i <= iend) w.f[q][c] = f.x;
+  }
+}
 // the columns of a box [ia, ib) x [ja, jb)
 __global__ void k_mx_to_working_region(const __grid_constant__ Dims d, const __grid_constant__ Tab t,
                                        const __grid_constant__ CS64 s, const __grid_constant__ WS w, int ia, int ja,
@@ -3027,6 +3054,11 @@ void mixed_to_working_region(const Dims& d, const Tab& t, double* const* s, cons
   if (a1 <= a0 || b1 <= b0) return;
   const dim3 b(32, 4);
   k_mx_to_working_region<<<g3(a1 - a0, b1 - b0, d.nz + 1, b), b, 0, stream>>>(d, t, cs64(s), w, a0, b0, a1, b1);
+}
+
+void mixed_restore(const Dims& d, const Tab& t, double* const* from, double* const* to, const WS& w,
+                   cudaStream_t stream) {
+  k_mx_restore<<<dim3((unsigned)((d.plane / 2 + 255) / 256), d.nz + 1), 256, 0, stream>>>(d, t, cs64(from), ms64(to), w);
 }
 
 void mixed_to_working(const Dims& d, const Tab& t, double* const* s, const WS& w, cudaStream_t stream) {
