@@ -1029,6 +1029,15 @@ T* dev_alloc(MgSolver<T>* m, size_t n) {
   return (T*)p;
 }
 
+// the arrays of one size in one allocation, each on a 256-byte boundary
+template <typename T, size_t N>
+bool dev_alloc_all(MgSolver<T>* m, T** (&arrs)[N], size_t n) {
+  const size_t na = (n + 63) / 64 * 64;
+  T* const base = dev_alloc(m, N * na);
+  for (size_t q = 0; q < N; ++q) *arrs[q] = base ? base + q * na : nullptr;
+  return base != nullptr;
+}
+
 }  // namespace
 
 void hz_residual(const HGeo& g, const double* a, const double* b, const double* f, const double* x, double* r,
@@ -1056,10 +1065,7 @@ MgSolver<T>* mg_create(const HGeo& g, int max_levels) {
     L.nz = g.nz;
     L.n = (size_t)nx * ny * g.nz;
     T** arrs[] = {&L.cE, &L.cN, &L.cT, &L.cB, &L.cD, &L.lc, &L.li, &L.x, &L.r};
-    for (T** a : arrs) {
-      *a = dev_alloc(m, L.n);
-      ok = ok && *a != nullptr;
-    }
+    ok = dev_alloc_all(m, arrs, L.n) && ok;
     m->L = l + 1;
     if (nx / 2 < 4 || ny / 2 < 4) break;
     nx = (nx + 1) / 2;
@@ -1067,10 +1073,7 @@ MgSolver<T>* mg_create(const HGeo& g, int max_levels) {
   }
   const size_t n = g.n();
   T** kv[] = {&m->x, &m->r, &m->r0, &m->p, &m->v, &m->s, &m->t, &m->ph, &m->sh};
-  for (T** a : kv) {
-    *a = dev_alloc(m, n);
-    ok = ok && *a != nullptr;
-  }
+  ok = dev_alloc_all(m, kv, n) && ok;
   void* p = nullptr;
   ok = ok && cudaMalloc(&p, 2 * kMgRedBlocks * sizeof(double)) == cudaSuccess;
   if (p) m->allocs.push_back(p), m->part = (double*)p;
