@@ -718,3 +718,18 @@ def test_neumaier_integer_sum(vg, kind, n):
     assert abs(got - ref) <= 4 * eps * abs(ref) + 4 * n * eps * eps * np.abs(x).sum() + 5e-324, (got, ref)
     x[n // 2] = np.inf  # the compensation of an infinite sum is inf - inf, as in the reference
     assert np.isnan(vg.neumaier_sum(x))
+
+
+@pytest.mark.parametrize("big", [7.0e305, 1e306, 1.7e308, 1e300, 1.0])
+@pytest.mark.parametrize("odd", [(np.inf, -np.inf), (np.nan,), (-np.nan,), (np.nan, -np.nan), (np.inf,), (-np.inf,)])
+@pytest.mark.parametrize("n", [8, 5000])
+def test_neumaier_nonfinite_beside_the_largest(vg, big, odd, n):
+    """Infinities and NaN make the compensated sum NaN, as in the reference,
+    also beside finite elements up to the largest double."""
+    x = np.zeros(n)
+    x[0] = big
+    x[1:1 + len(odd)] = odd
+    x[1 + len(odd)] = -big
+    assert np.isnan(vg.neumaier_sum(x))
+    x[1:1 + len(odd)] = 0.0
+    assert vg.neumaier_sum(x) == 0.0

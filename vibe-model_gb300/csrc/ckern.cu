@@ -526,6 +526,7 @@ __device__ Neu<T> neu_block(Neu<T> v) {
 // pair as before. value() is exact to the two doubles of a pair.
 struct ExactSum {
   static constexpr int kSpan = 54, kAbove = 8, kRounds = 1024;
+  static constexpr int kTopBase = 0x7fe - kSpan;  // a window ends at the largest finite exponent field
   unsigned long long lo = 0;
   long long hi = 0;
   int base = 1 << 20;  // no window yet
@@ -564,7 +565,7 @@ struct ExactSum {
   __device__ __forceinline__ void window(int top, Neu<double>& pair) {
     if (top == 0 || (unsigned)(top - base) <= (unsigned)kSpan || (top < base && base < 4096)) return;
     flush(pair);
-    base = top + kAbove - kSpan;
+    base = min(top + kAbove - kSpan, kTopBase);
   }
   __device__ __forceinline__ void add(double x, Neu<double>& pair) {
     const unsigned long long bits = (unsigned long long)__double_as_longlong(x);
