@@ -733,3 +733,30 @@ def test_neumaier_nonfinite_beside_the_largest(vg, big, odd, n):
     assert np.isnan(vg.neumaier_sum(x))
     x[1:1 + len(odd)] = 0.0
     assert vg.neumaier_sum(x) == 0.0
+
+
+@pytest.mark.parametrize("case", ["winds", "depth", "dzeta"])
+def test_cfl_scan_bounds_beyond_single_precision(vg, oc, case):
+    """Winds under 2^-126 beside tiny spacings, and dzeta and depths that single
+    precision cuts to zero while their product is an ordinary thickness: the
+    scan equals the oracle's bit for bit."""
+    nx, ny, nz = 3, 1, 2
+    n = nx * ny * nz
+    u, v, w = np.zeros(n), np.zeros(n), np.zeros(n)
+    dz, zs, z_top, dx = np.full(nz, 0.01), np.zeros(nx * ny), 20000.0, 1e-9
+    if case == "winds":  # both winds of the first cell count as 2^-126, together above the second's
+        u[0], v[0], v[1] = 1e-300, 1e-300, 2e-38
+    else:  # w = 5 m/s where dz is 3.63 m has the larger bound and the smaller number than 2 m/s where it is 1.32 m
+        dx = 1000.0
+        w[0], w[nx * ny + 1] = 5.0, 2.0
+        if case == "depth":
+            dz[:], z_top = (1.1e-38, 4e-39), 3.3e38
+        else:
+            dz[:], z_top = (2e38, 3e38), 1e-38
+            w[0], w[nx * ny + 1] = 5.0, 6.0  # dz = 2 m and 3 m: equal bounds per wind, 2.5 /s and 2 /s
+    a, b = ctypes.c_double(), ctypes.c_double()
+    ro = oc.port_lib().vo_cfl_scan(u.ctypes.data, v.ctypes.data, w.ctypes.data, dz.ctypes.data, zs.ctypes.data, nx, ny,
+                                    nz, dx, dx, z_top, 6.0, ctypes.byref(a), ctypes.byref(b))
+    r, mw, mdz = vg.cfl_scan(u, v, w, dz, zs, nx, ny, nz, dx, dx, z_top, 6.0)
+    assert (r, mdz) == (ro, b.value), (r, ro, mdz, b.value)
+    assert mw == a.value or abs(mw - a.value) <= 2.3e-16 * a.value

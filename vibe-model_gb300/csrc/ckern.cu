@@ -687,6 +687,10 @@ __device__ __forceinline__ void max3_block(T& ta, T& tb, T& tc) {  // max, max, 
 // must win: a handful of cells per block. The maxima are those of the FP64
 // values, bit for bit. The bounds assume ordinary positive dt, dx, dy
 // (`plain`); else, and where a bound is not finite, cells are evaluated.
+// What FP32 cannot hold makes a bound larger than the cell by any factor, so a
+// tile whose largest bound is no more than such floors (winds count from 2^-126
+// up) sets no limit, and a cell whose dzeta or depth is past 1e30, beside which
+// the other may have been cut to zero, has no bound.
 // The minimum of dz over a column is dz at the smallest (or, where the column's
 // depth is negative, the largest) dzeta: a product rounds monotonically.
 __device__ __forceinline__ float trunc_abs(double x) {  // |x| rounded toward zero; tiny values up to 2^-126
@@ -720,6 +724,7 @@ __global__ void __launch_bounds__(kCflThreads, 4) k_cfl_partial(const T* __restr
   const bool plain = dt >= (T)1e-30 && dt <= (T)1e30 && dx >= (T)1e-30 && dx <= (T)1e30 && dy >= (T)1e-30 && dy <= (T)1e30;
   const float up = 1.00002f;  // above the rounding of the bounds (a few 1e-6)
   const float bdt = (float)dt * up, bdx = 1.f / (float)dx, bdy = 1.f / (float)dy;
+  const float cfloor = fmaxf(bdt * (bdx + bdy + 1.f) * 1e-30f, 1e-30f);
   // the largest squared speed, one square root at the end: a correctly
   // rounded square root is monotone, so the maximum of the roots is the root
   // of the maximum, bit for bit
@@ -753,6 +758,7 @@ __global__ void __launch_bounds__(kCflThreads, 4) k_cfl_partial(const T* __restr
     const bool in = col < nxy;
     const T scale = zs ? (in ? z_top - zs[col] : (T)1) : z_top;
     const float fscale = trunc_signed(scale);
+    const bool deep = !(fabsf(fscale) < 1e30f);
     if (in && k0 == 0) {
       T dz = fmin(dext[0] * scale, dext[1] * scale);
       if (dz < (T)1) dz = (T)1;
@@ -773,10 +779,11 @@ __global__ void __launch_bounds__(kCflThreads, 4) k_cfl_partial(const T* __restr
       const int k = k0 + m < nz ? k0 + m : nz - 1;
       const float fu = trunc_abs(qu[m]), fv = trunc_abs(qv[m]), fw = trunc_abs(qw[m]);
       const float some = (fu + fv + fw > 0.f) ? 1e-36f : 0.f;  // products below 2^-126 count as that much
-      float fdz = trunc_signed(dzeta[k]) * fscale;
+      const float fzeta = trunc_signed(dzeta[k]);
+      float fdz = fzeta * fscale;
       if (fdz < 1.f) fdz = 1.f;
       ec[m] = bdt * (fu * bdx + fv * bdy + fw * __frcp_rn(fdz)) + some;
-      if (fdz > 3e38f) ec[m] = __int_as_float(0x7f800000);  // out of FP32's range: no bound
+      if (deep || !(fabsf(fzeta) < 1e30f) || fdz > 3e38f) ec[m] = __int_as_float(0x7f800000);  // no bound
       es[m] = up * (fu * fu + fv * fv + fw * fw) + some;
       tc = fmaxf(tc, ec[m]);
       ts = fmaxf(ts, es[m]);
@@ -794,7 +801,7 @@ __global__ void __launch_bounds__(kCflThreads, 4) k_cfl_partial(const T* __restr
     const float bc = __uint_as_float(best[0]), bs = __uint_as_float(best[1]);
     const float mc = __uint_as_float(seen[par][0]), ms = __uint_as_float(seen[par][1]);
     // under these a cell cannot be the tile's maximum (no such limit where a bound is tiny or not finite)
-    const float lc = (mc > 1e-30f && mc < 3e38f) ? mc * 0.99995f : 0.f, ls = (ms > 1e-30f && ms < 3e38f) ? ms * 0.99995f : 0.f;
+    const float lc = (mc > cfloor && mc < 3e38f) ? mc * 0.99995f : 0.f, ls = (ms > 1e-30f && ms < 3e38f) ? ms * 0.99995f : 0.f;
     if (threadIdx.x < 2) seen[par ^ 1][threadIdx.x] = 0u;
 #pragma unroll
     for (int m = 0; m < kCflLevels; ++m) {
