@@ -760,3 +760,22 @@ def test_cfl_scan_bounds_beyond_single_precision(vg, oc, case):
     r, mw, mdz = vg.cfl_scan(u, v, w, dz, zs, nx, ny, nz, dx, dx, z_top, 6.0)
     assert (r, mdz) == (ro, b.value), (r, ro, mdz, b.value)
     assert mw == a.value or abs(mw - a.value) <= 2.3e-16 * a.value
+
+
+@pytest.mark.parametrize("where", ["zs", "dzeta", "rho", "q", "w"])
+@pytest.mark.parametrize("nan", [np.nan, -np.nan])
+def test_flux_advection_nan_reaches_the_result(vg, oc, where, nan):
+    """A NaN in the metric or a field makes the cells that use it NaN, as in
+    the oracle, and no others."""
+    nx, ny, nz = 34, 10, 6
+    rng = np.random.default_rng(1)
+    n = nx * ny * nz
+    f = dict(q=rng.random(n), rho=0.5 + rng.random(n), u=rng.random(n) - 0.5, v=rng.random(n) - 0.5,
+             w=rng.random(n) - 0.5, dzeta=0.01 + 0.01 * rng.random(nz), zs=500.0 * rng.random(nx * ny))
+    f[where][f[where].size // 2] = nan
+    got = vg.advect_scalar_flux(f["q"], f["rho"], f["u"], f["v"], f["w"], f["dzeta"], f["zs"], nx, ny, nz, 900.0,
+                                1100.0, 20000.0)
+    ref = np.zeros(n)
+    oc.port_lib().vo_advect_scalar_flux(*[f[k].ctypes.data for k in ("q", "rho", "u", "v", "w", "dzeta", "zs")], nx, ny,
+                                         nz, 900.0, 1100.0, 20000.0, ref.ctypes.data)
+    assert np.isnan(ref).any() and np.array_equal(np.isnan(got), np.isnan(ref))

@@ -852,9 +852,12 @@ __global__ void k_cfl_final(const T* __restrict__ partials, int nb, T* __restric
 // FP64 operations, the bound, where one thread per cell with its six faces
 // spent 70 and three index divisions. The halves of the two means are exact
 // powers of two and are applied once.
-// x < 1 and x > 1e-12 on the integer pipe (a NaN rho makes the fluxes NaN
-// whatever the divisor)
-__device__ __forceinline__ bool below_one(double x) { return __double2hiint(x) < 0x3ff00000; }
+// x < 1 and x > 1e-12 on the integer pipe (a NaN x, of either sign, is not below
+// one; a NaN rho makes the fluxes NaN whatever the divisor)
+__device__ __forceinline__ bool below_one(double x) {
+  const int h = __double2hiint(x);
+  return h < 0x3ff00000 && (unsigned)h <= 0xfff00000u;
+}
 __device__ __forceinline__ bool below_one(float x) { return x < 1.f; }
 __device__ __forceinline__ bool above_floor(double x) { return __double_as_longlong(x) > __double_as_longlong(1e-12); }
 __device__ __forceinline__ bool above_floor(float x) { return x > 1e-12f; }
