@@ -115,6 +115,28 @@ def test_slow_tendency_fp64_exact(vg, oc, scheme):
             assert np.array_equal(vg.interior(s, sp, a), vg.interior(s, sp, b)), vg.SPECIES[sp]
 
 
+def test_slow_tendency_ground_above_the_top(vg, oc):
+    """A hill higher than the model top turns its columns' thicknesses negative;
+    the divergence and the pressure gradient use 1 m there (max(dz, 1)), as the
+    oracle does. The bounds of the tendencies above."""
+    s = small_setup(vg, terrain_kind=1, hill_h=4500.0, hill_a=1500.0, hill_xc=2500.0, hill_yc=2000.0, coriolis=1)
+    rng = np.random.default_rng(3)
+    with vg.Model(s, vg.FP64) as m:
+        o = oc.Model(oracle_setup(oc, s), "port")
+        assert o.terrain().max() > s.z_top > o.terrain().min()
+        for sp, amp in ((2, 1.0), (3, 0.01), (4, 1.0), (5, 1e-3)):  # the split terms vanish on the base state
+            f = o.get(sp).reshape(vg.storage_shape(s, sp))
+            vg.interior(s, sp, f)[...] += amp * rng.standard_normal(vg.interior(s, sp, f).shape)
+            o.set(sp, f)
+            m.set(sp, f)
+        floors = {sp: 1e-3 * np.abs(vg.interior(s, sp, o.get(sp))).max() for sp in range(7)}
+        vs = 1e-3 * velocity_scale(vg, s, o.state())
+        for sp in (0, 1, 2):
+            floors[sp] = max(floors[sp], vs)
+        got, ref = m.slow_tendency(), o.slow_tendency()
+        assert_state_close(vg, s, got, ref, TOL_TEND, range(7), "slow tendency", floors, velocity=False)
+
+
 MIXED_SCHEMES = [
     dict(),
     dict(advection=2, weno_scalars=0),

@@ -279,3 +279,35 @@ def test_own_step_refusals(vg):
         dx = perturb(vg, s, m, 11)
         with pytest.raises(vg.VibeError):
             m.step_tl(DT, NSUB, dx)
+
+
+def test_tendency_tl_ground_above_the_top(vg, oc):
+    """With central scalars the slow tendency is quadratic in the state, so the
+    oracle's central difference is the tangent-linear up to rounding: under a
+    hill higher than the model top, where max(dz, 1) sets the thickness of the
+    divergence and the pressure gradient to 1 m. Rounding: eps |R| of
+    terms up to 1e3 of the result, under 1e-9; the adjoint to the bound of the dot
+    products above."""
+    s = vg.Setup.defaults(nx=20, ny=16, nz=8, dx=3000.0, dy=3000.0, z_top=3000.0, ref_kind=1, bv_n=0.01,
+                          u_background=10.0, shear_u=0.001, advection=2, weno_scalars=0, weno_advective=0,
+                          pgf_perturbation=1, split_fast=1, acoustic_mode=0, qv_surface=0.0, terrain_kind=1,
+                          hill_h=4500.0, hill_a=18000.0, hill_xc=30000.0, hill_yc=24000.0)
+    with vg.Model(s, vg.FP64) as m:
+        assert m.terrain().max() > s.z_top
+        dx, y = perturb(vg, s, m, 21), perturb(vg, s, m, 22)
+        m.set_state([a + b for a, b in zip(m.state(), perturb(vg, s, m, 23))])  # off the base state
+        x0, tl = m.state(), m.tendency_tl(dx)
+        setup = oc.Setup()
+        for name, _ in oc.Setup._fields_:
+            setattr(setup, name, getattr(s, name))
+        o, r = oc.Model(setup, "port"), []
+        for sign in (1.0, -1.0):
+            for sp in range(7):
+                o.set(sp, x0[sp] + sign * dx[sp])
+            r.append(o.slow_tendency())
+        for sp in range(6):
+            fd = (vg.interior(s, sp, r[0][sp]) - vg.interior(s, sp, r[1][sp])) / 2.0
+            t = vg.interior(s, sp, tl[sp])
+            assert np.abs(fd - t).max() <= 1e-9 * max(np.abs(t).max(), 1e-3), vg.SPECIES[sp]
+        lhs, rhs = vdot(tl, y), vdot(dx, m.tendency_ad(y))
+        assert abs(lhs - rhs) <= 1e-10 * max(abs(lhs), abs(rhs))

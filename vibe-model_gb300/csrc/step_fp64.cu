@@ -203,7 +203,8 @@ __device__ inline double ac_w(const CS& s, const Metric& m, const Dims& d, const
 __device__ inline double idz_at(const Metric& m, const Dims& d, int i, int j, int k) {
   return m.inv_dzeta[iclamp(k, 0, d.nz - 1)] * m.inv_scale[(size_t)iclamp(j, 0, d.ny - 1) * d.nx + iclamp(i, 0, d.nx - 1)];
 }
-__device__ inline double floor1(double idz) { return idz > 1.0 ? 1.0 : idz; }  // 1 / max(dz, 1)
+// 1 / max(dz, 1) of idz = 1 / dz: 1 for dz under 1 m, negative (ground above the model top) or NaN
+__device__ inline double floor1(double idz) { return (unsigned)__double2hiint(idz) < 0x3ff00000u ? idz : 1.0; }
 // theta less what split_fast moves to the substeps, pi or pi'
 __device__ inline double th_slow(const CS& s, const Metric& m, const Flags& fl, size_t c) {
   return fl.split_fast ? s.f[THETA][c] - m.th0[c] : s.f[THETA][c];

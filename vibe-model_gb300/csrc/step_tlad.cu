@@ -141,7 +141,8 @@ constexpr int kMaxLoads = 48;  // more than any point function below reads
 __device__ __forceinline__ double idz_(const Metric& m, const Dims& d, int i, int j, int k) {
   return m.inv_dzeta[iclamp(k, 0, d.nz - 1)] * m.inv_scale[(size_t)iclamp(j, 0, d.ny - 1) * d.nx + iclamp(i, 0, d.nx - 1)];
 }
-__device__ __forceinline__ double floor1_(double idz) { return idz > 1.0 ? 1.0 : idz; }  // 1 / max(dz, 1)
+// 1 / max(dz, 1) of idz = 1 / dz: 1 for dz under 1 m, negative (ground above the model top) or NaN
+__device__ __forceinline__ double floor1_(double idz) { return (unsigned)__double2hiint(idz) < 0x3ff00000u ? idz : 1.0; }
 __device__ __forceinline__ double ref_(const double* f, const Dims& d, int i, int j, int k) {
   return f[d.idx(i, j, k)];
 }
