@@ -199,3 +199,21 @@ def test_fp64_physics_graph_replay_and_errors(vg):
         b.step(2.0, 4, 3)
         for x, y in zip(a.state(), b.state()):
             assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("dt", [0.0, float("nan")])
+def test_kessler_rates_over_no_time(vg, oc, dt):
+    """(after - before) / dt has no value for a dt of zero or NaN, also in
+    cloudless cells, where after equals before: NaN where the oracle has it."""
+    s = setup(vg)
+    kg, ko = kessler(vg, oc, 0)
+    with vg.Model(s, vg.FP64) as m:
+        o = oc.Model(oracle_setup(oc, s), "port")
+        o.set_state(m.state())
+        m.set_physics_kessler(kg)
+        got = m.physics_tendency(dt)
+        with np.errstate(all="ignore"):
+            ref = dict(zip((4, 6, 7, 8), oc.kessler_tendency(o, ko, dt)))
+        for sp in (4, 6, 7, 8):
+            g, r = vg.interior(s, sp, got[sp]), vg.interior(s, sp, ref[sp])
+            assert np.isnan(r).any() and np.array_equal(np.isnan(g), np.isnan(r)), vg.SPECIES[sp]

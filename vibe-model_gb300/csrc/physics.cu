@@ -148,6 +148,7 @@ __global__ void __launch_bounds__(32 * kKessLevels) k_kessler(const vibe_gb300_p
   const int j = in ? q / a.nx : 0, i = in ? q - j * a.nx : 0;
   const int nz = a.nz;
   const R dt = (R)a.dt;
+  const bool odd_dt = !(dt < (R)0 || dt > (R)0);
   const size_t plane = (size_t)a.pitch * (a.ny + 1), col = (size_t)j * a.pitch + i;
   const T* th_s = (const T*)a.state[THETA];
   const T* pi_s = (const T*)a.state[PI];
@@ -257,9 +258,10 @@ __global__ void __launch_bounds__(32 * kKessLevels) k_kessler(const vibe_gb300_p
         qc = rmax(qc, (R)0);
         qr = rmax(qr, (R)0);
       }
-      // PhysicsTendency (accumulated onto the zeroed buffers; most air has none)
+      // PhysicsTendency (accumulated onto the zeroed buffers; most air has none,
+      // which only a dt of zero or NaN turns into something else)
       auto add = [&](T* t, R d) {
-        if (d != (R)0) t[c] += (T)(d / dt);
+        if (d != (R)0 || odd_dt) t[c] += (T)(d / dt);
       };
       add(t_th, theta - th0);
       add(t_qv, qv - qv0);
