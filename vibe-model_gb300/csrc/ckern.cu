@@ -149,9 +149,12 @@ __global__ void k_thomas_batched(const T* __restrict__ a, const T* __restrict__ 
 // where one thread per system took 2.50 ms and read DRAM 13 times over). The modified super-diagonal and the
 // eliminated right-hand side stay in shared memory, level-major, and the back
 // substitution stores x through the same staging, so DRAM sees each element
-// once and no workspace is needed. FP64 multiplies by one reciprocal per row
-// (pivots under 1e-290, where it could overflow, divide), as the pipe is the
-// bound there: about 13 FP64 operations a row; FP32 divides twice.
+// once and no workspace is needed. FP64 takes one reciprocal per row and
+// corrects each product with it by its residual num - q den (Markstein's
+// quotient), which rounds as a division does: about 17 FP64 operations a row,
+// the bound there, where two divisions take 25 (products alone, 13 operations,
+// are 1.35 times as far from 64-bit results). Pivots and quotients outside the
+// range where that holds divide. FP32 divides twice.
 // A system with a zero pivot leaves x as it was.
 template <typename T>
 struct Sweep {
@@ -165,14 +168,21 @@ __device__ __forceinline__ void cp_async_elem(T* smem, const T* gmem) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], %2;\n" ::"r"(sa), "l"(gmem), "n"((int)sizeof(T)) : "memory");
 }
 // one row: x_k = (d - a x_{k-1}) / den, c'_k = c / den
+__device__ __forceinline__ bool ordinary(double x, unsigned lo, unsigned hi) {  // |x| by its upper word
+  return ((unsigned)__double2hiint(x) & 0x7fffffffu) - lo < hi - lo;
+}
+__device__ __forceinline__ double quotient(double num, double den, double r) {  // r = 1 / den
+  const double q = num * r;
+  return fma(fma(-q, den, num), r, q);
+}
 __device__ __forceinline__ void sweep_row(double den, double num, double c, double& x, double& cp) {
-  if ((__double2hiint(den) & 0x7fffffff) < 0x03d00000) {  // |den| < 1e-290
+  const double r = 1.0 / den;
+  x = quotient(num, den, r);
+  cp = quotient(c, den, r);
+  // (a quotient that is not finite, or of a pivot under 1e-290 or past 2^1021)
+  if (!ordinary(den, 0x03d00000u, 0x7fc00000u) || !ordinary(x, 0u, 0x7ff00000u) || !ordinary(cp, 0u, 0x7ff00000u)) {
     x = num / den;
     cp = c / den;
-  } else {
-    const double r = 1.0 / den;
-    x = num * r;
-    cp = c * r;
   }
 }
 __device__ __forceinline__ void sweep_row(float den, float num, float c, float& x, float& cp) {
@@ -194,7 +204,14 @@ __global__ void __launch_bounds__(32) k_thomas_sweep(const T* __restrict__ a, co
   const T* ds = d + (size_t)s0 * n;
   const T* as = a ? a + (size_t)s0 * (n - 1) : nullptr;
   const T* cs = c ? c + (size_t)s0 * (n - 1) : nullptr;
-  for (int e = lane; e < 8 * A; e += 32) st[e] = (T)0;  // absent a, c and idle lanes read zeros
+  // an absent a or c reads zeros; idle lanes read a = 0, b = c = d = 1, as a zero
+  // pivot or numerator would take their warp through the slow path of the
+  // division on every row (FP32, 33 systems of 128 rows: 48 us, with ones 29)
+  if (!as || !cs)
+    for (int e = lane; e < 8 * A; e += 32) st[e] = (T)0;
+  __syncwarp();
+  if (lane >= ns)
+    for (int e = 0; e < 8 * K; ++e) st[e / K * A + lane * R + e % K] = e / K % 4 == 0 ? (T)0 : (T)1;
   __syncwarp();
   const int nch = (n + K - 1) / K;
   auto load = [&](int ch) {
@@ -232,8 +249,8 @@ __global__ void __launch_bounds__(32) k_thomas_sweep(const T* __restrict__ a, co
         const T am = k > 0 ? q[kk] : (T)0;
         const T den = q[A + kk] - am * cp;
         sing |= den == (T)0;
-        sweep_row(den, q[3 * A + kk] - am * xp, k + 1 < n ? q[2 * A + kk] : (T)0, xp, cp);
         if (n == 1) xp = q[3 * A] / den;
+        else sweep_row(den, q[3 * A + kk] - am * xp, k + 1 < n ? q[2 * A + kk] : (T)0, xp, cp);
         Y[k * 32 + lane] = xp;
         CP[k * 32 + lane] = cp;
       }
