@@ -100,14 +100,14 @@ void vibe_advect_scalar_flux_f64(const double *q, const double *rho,
 /* n_sys independent systems of size n, each stored contiguously
  * (system s uses a + s*(n-1), b + s*n, ...). A warp sweeps 32 systems whose
  * columns it keeps on chip (up to 200 KB of shared memory: 380 rows in FP64,
- * 764 in FP32) for n <= 128 or n_sys >= 256; else one warp per
- * system (each lane eliminates a chunk of rows, the chunks' end unknowns are
- * joined by a 2x2 block-tridiagonal solve), whose results agree with the
- * single sweep to rounding. A system whose chunk
- * pivots or interface blocks are zero or tiny (b[r0] = 0 at a chunk start,
- * non-dominant diagonals) is solved again with the single sweep, so the error
- * contract stays the reference's: VIBE_C_ERR_SINGULAR only on an exactly zero
- * sweep pivot (c_kernels.c:26,34,40).
+ * 764 in FP32) for n <= 128, and above where the systems are so many that it
+ * is the faster form; else one warp per system (each lane eliminates a chunk
+ * of rows, the chunks' end unknowns are joined by a 2x2 block-tridiagonal
+ * solve), whose results agree with the single sweep to rounding. A system
+ * whose chunk pivots or interface blocks are zero or tiny (b[r0] = 0 at a
+ * chunk start, non-dominant diagonals) is solved again with the single sweep,
+ * so the error contract stays the reference's: VIBE_C_ERR_SINGULAR only on an
+ * exactly zero sweep pivot (c_kernels.c:26,34,40).
  * status (device, n_sys ints) receives the per-system return code; may be
  * NULL. Returns VIBE_C_OK or VIBE_C_ERR_BAD_ARG/VIBE_C_ERR_DEVICE (launch).
  * The sweep needs no scratch; that of the warp-per-system form (3*n*n_sys

@@ -813,3 +813,38 @@ def test_thomas_sweep_error_against_64_bits(vg, n):
     if np.finfo(np.longdouble).nmant <= 52:
         pytest.skip("no wider type on this host")
     assert err(got.reshape(2000, n)) <= 1.02 * err(twice)
+
+
+@pytest.mark.parametrize("bits,n", [(64, 3), (64, 4), (64, 5), (64, 128), (64, 129), (64, 380), (64, 381), (32, 7),
+                                    (32, 8), (32, 9), (32, 128), (32, 129), (32, 764), (32, 765)])
+@pytest.mark.parametrize("n_sys", [1, 32, 255, 257, 2999])
+def test_thomas_sweep_and_solver_limits(vg, oc, bits, n, n_sys):
+    """At the edges of the on-chip sweep's stages (4 and 8 levels), at the tallest
+    columns it holds and just above, for few systems and many, whichever kernel
+    the batched call takes: against the oracle at the bounds above (1e-12; FP32
+    1e-5), with a singular system between others."""
+    import torch
+    dt = torch.float64 if bits == 64 else torch.float32
+    vp, i32 = ctypes.c_void_p, ctypes.c_int
+    f = _dev(vg, "vibe_tridiagonal_solve_batched_f%d_dev" % bits, [vp] * 4 + [i32, i32, vp, vp, vp])
+    rng = np.random.default_rng(n * 10000 + n_sys)
+    a, c = (-rng.random((n_sys, n - 1)) for _ in range(2))
+    b, d = 2.5 + rng.random((n_sys, n)), rng.random((n_sys, n)) - 0.5
+    bad = n_sys // 3 if n_sys > 1 else -1
+    if bad >= 0:
+        b[bad, 0] = 0.0
+    t = [torch.tensor(v, dtype=dt, device="cuda") for v in (a, b, c, d)]
+    x = torch.full((n_sys, n), 7.0, dtype=dt, device="cuda")
+    st = torch.full((n_sys,), -1, dtype=torch.int32, device="cuda")
+    assert f(*[v.data_ptr() for v in t], n, n_sys, x.data_ptr(), st.data_ptr(),
+             torch.cuda.current_stream().cuda_stream) == 0
+    torch.cuda.synchronize()
+    host = [np.ascontiguousarray(v.double().cpu().numpy()) for v in t]
+    got, status = x.double().cpu().numpy(), st.cpu().numpy()
+    tol = 1e-12 if bits == 64 else 1e-5
+    xo, ws = np.zeros(n), np.zeros(n)
+    for s in range(n_sys):
+        rc = oc.port_lib().vo_tridiagonal_solve(*[h[s].ctypes.data for h in host], n, xo.ctypes.data, ws.ctypes.data)
+        assert status[s] == rc == (1 if s == bad else 0)
+        if rc == 0:
+            assert np.abs(got[s] - xo).max() <= tol * np.abs(xo).max()

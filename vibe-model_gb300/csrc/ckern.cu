@@ -8,6 +8,7 @@
 // warp shuffles inside a block, one partial per block in device scratch, and
 // a single-block pass that merges the partials in block order, so results are
 // deterministic run to run.
+#include <algorithm>
 #include <atomic>
 #include <cmath>
 #include <cstring>
@@ -971,14 +972,28 @@ using vgb_cabi::DevScratch;
 using vgb_cabi::HostCall;
 
 // The staged sweep runs whenever its columns fit in shared memory and n is at
-// most kTallN, or there are enough systems: it takes n * 0.18 us a wave of 32 x
-// 152 systems, the warp-per-system solver 0.7 ns * n a system (65536 systems of
-// 200 rows: 9.1 ms), which meet near 260 systems.
+// most kTallN, or the systems are many enough that it is done before the
+// warp-per-system solver would be. A wave of the sweep (32 systems a block, as
+// many blocks an SM as their columns leave room for) takes 0.73 us a row in
+// FP64 and 0.25 in FP32; the other is bound by latency for few systems and by
+// its traffic for many. Measured, sweep against solver: FP64 1000 x 129 94 and
+// 154 us, 256 x 300 212 and 121, 1000 x 380 267 and 223, 4864 x 380 268 and 854;
+// FP32 1000 x 129 33 and 23, 4864 x 129 34 and 50, 1000 x 760 170 and 74, 4864 x 760
+// 170 and 446.
 constexpr size_t kSweepSmem = 200 * 1024;
 constexpr int kSweepSystems = 256;
 template <typename T>
 bool thomas_sweeps(int n, int n_sys) {
-  return Sweep<T>::smem(n) <= kSweepSmem && (n <= kTallN || n_sys >= kSweepSystems);
+  const size_t sm = Sweep<T>::smem(n);
+  if (sm > kSweepSmem) return false;
+  if (n <= kTallN) return true;
+  if (n_sys < kSweepSystems) return false;
+  const bool d = sizeof(T) == 8;
+  const long blocks = (n_sys + 31L) / 32, wave = 152L * (long)(227 * 1024 / (sm + 1024));
+  const double sweep = (double)((blocks + wave - 1) / wave) * n * (d ? 0.73 : 0.25);
+  const double latency = d ? 73.0 + 0.16 * n : 13.0 + 0.045 * n;
+  const double each = d ? 0.10 + 1.9e-4 * n : (4.5e-5 + 7e-8 * n) * n;
+  return sweep <= std::max(latency, 0.4 * latency + each * n_sys);
 }
 template <typename T>
 size_t thomas_work(int n, int n_sys) {
