@@ -132,10 +132,11 @@ int vibe_tridiagonal_solve_batched_f64_dev(const double *a, const double *b,
  * device pointers as in the _dev form. The first call on each device
  * resolves the array's device address (cudaGetSymbolAddress) and keeps it for
  * the life of the process; make that first call before any stream capture,
- * and do not call this form on a device after cudaDeviceReset of it. It runs
- * the one-thread-per-system sweep for every n, so for n > 128 it agrees with
- * the _dev form to rounding (and reports VIBE_C_ERR_SINGULAR on the sweep's
- * exact-zero pivot only). All calls share the one array:
+ * and do not call this form on a device after cudaDeviceReset of it. It
+ * sweeps for every n (on chip up to 380 rows, above with one thread per system
+ * and the array), so where the _dev form takes the warp-per-system solver the
+ * two agree to rounding (and this one reports VIBE_C_ERR_SINGULAR on the
+ * sweep's exact-zero pivot only). All calls share the one array:
  * calls whose kernels can overlap on the GPU (different streams, no
  * ordering between them) race on it. */
 int vibe_tridiagonal_solve_batched_f64_dev_noalloc(const double *a, const double *b,

@@ -95,3 +95,37 @@ def test_noalloc_tall_systems_and_null_status(vg):
     scale = float(x_ref.abs().max())
     assert float((x_na - x_ref).abs().max()) <= 1e-12 * scale
     assert torch.equal(x_na, x_nul)
+
+
+@pytest.mark.parametrize("n,n_sys", [(80, 3000), (300, 800), (380, 600), (381, 688), (1000, 262), (262144, 1), (5000, 52)])
+def test_noalloc_against_the_oracle(vg, oc, n, n_sys):
+    """Columns the sweep holds on chip (up to 380 rows) and taller ones, which
+    take the fixed array, against the oracle, on two calls in a row with
+    different systems, one of them singular; the allocating form agrees."""
+    torch = pytest.importorskip("torch")
+    noalloc, alloc = _bind(vg)
+    dev = torch.device("cuda", 0)
+    stream = torch.cuda.current_stream(dev).cuda_stream
+    assert n * n_sys <= LIMIT
+    rng = np.random.default_rng(n)
+    for call in range(2):
+        b, d = 4.0 + rng.random((n_sys, n)), rng.standard_normal((n_sys, n))
+        a, c = -rng.random((n_sys, n - 1)), -rng.random((n_sys, n - 1))
+        bad = n_sys // 2 if n_sys > 1 else -1
+        if bad >= 0:
+            b[bad, 0] = 0.0
+        t = [torch.tensor(v, device=dev) for v in (a, b, c, d)]
+        x = [torch.full((n_sys, n), 7.0, dtype=torch.float64, device=dev) for _ in range(2)]
+        st = [torch.full((n_sys,), -1, dtype=torch.int32, device=dev) for _ in range(2)]
+        for k, f in enumerate((noalloc, alloc)):
+            assert f(*[v.data_ptr() for v in t], n, n_sys, x[k].data_ptr(), st[k].data_ptr(), stream) == 0
+        torch.cuda.synchronize(dev)
+        xo, ws = np.zeros(n), np.zeros(n)
+        got, status = [v.cpu().numpy() for v in x], [v.cpu().numpy() for v in st]
+        for s in range(n_sys):
+            rc = oc.port_lib().vo_tridiagonal_solve(a[s].ctypes.data, b[s].ctypes.data, c[s].ctypes.data,
+                                                     d[s].ctypes.data, n, xo.ctypes.data, ws.ctypes.data)
+            assert status[0][s] == status[1][s] == rc == (1 if s == bad else 0)
+            if rc == 0:
+                for g in got:
+                    assert np.abs(g[s] - xo).max() <= 1e-12 * np.abs(xo).max()

@@ -1387,13 +1387,12 @@ int vibe_tridiagonal_solve_batched_f64_dev_noalloc(const double* a, const double
     return VIBE_C_ERR_BAD_ARG;
   }
   if (n_sys == 0) return VIBE_C_OK;
-  if (Sweep<double>::smem(n) <= kSweepSmem)  // on chip: no workspace at all
-    return thomas_sweep_launch<double>(a, b, c, d, n, n_sys, x, status, (cudaStream_t)stream);
   const int dev = cur_dev();
   if (dev < 0 || dev >= 64) { g_cerr = "device ordinal out of range"; return VIBE_C_ERR_DEVICE; }
   double* work = nullptr;
   {
-    // set-up on the first call per device: resolve the array's device address
+    // set-up on the first call per device, of any size (a later call may be
+    // captured): resolve the array's device address
     std::lock_guard<std::mutex> lk(g_noalloc_mu);
     if (!g_noalloc_ptr[dev]) {
       void* p = nullptr;
@@ -1402,6 +1401,8 @@ int vibe_tridiagonal_solve_batched_f64_dev_noalloc(const double* a, const double
     }
     work = g_noalloc_ptr[dev];
   }
+  if (Sweep<double>::smem(n) <= kSweepSmem)  // on chip: the workspace is not needed
+    return thomas_sweep_launch<double>(a, b, c, d, n, n_sys, x, status, (cudaStream_t)stream);
   // the workspace needs no clearing: every system writes cp[k] before it reads it
   k_thomas_batched<double><<<(n_sys + 127) / 128, 128, 0, (cudaStream_t)stream>>>(a, b, c, d, n, n_sys, x, work,
                                                                                  status);
