@@ -848,3 +848,48 @@ def test_thomas_sweep_and_solver_limits(vg, oc, bits, n, n_sys):
         assert status[s] == rc == (1 if s == bad else 0)
         if rc == 0:
             assert np.abs(got[s] - xo).max() <= tol * np.abs(xo).max()
+
+
+@pytest.mark.parametrize("bits", [64, 32])
+@pytest.mark.parametrize("thin", [False, True])
+def test_flux_advection_error_against_wider_type(vg, bits, thin):
+    """The tiled kernel is no further from the result in a wider type than the
+    formula with its two divisions a cell, rounded at every operation (FP64: but
+    for the product that a fused multiply-add takes into a difference of
+    fluxes): 2-norms over 31 x 40 x 20 cells, to 2 %; thin: layers under 1 m
+    count as 1 m."""
+    import torch
+    dt, np_t = (torch.float64, np.float64) if bits == 64 else (torch.float32, np.float32)
+    if bits == 64 and np.finfo(np.longdouble).nmant <= 52:
+        pytest.skip("no wider type on this host")
+    nx, ny, nz = 31, 40, 20
+    rng = np.random.default_rng(bits)
+    u, v, w = ((a * rng.random((nz, ny, nx)) - 0.5 * a).astype(np_t) for a in (40.0, 30.0, 4.0))
+    q, rho = (300.0 + 5.0 * rng.random((nz, ny, nx))).astype(np_t), (0.2 + rng.random((nz, ny, nx))).astype(np_t)
+    dz = ((2e-5 if thin else 0.01) * (1.0 + rng.random(nz))).astype(np_t)
+    zs = (800.0 * rng.random((ny, nx))).astype(np_t)
+    f = _dev(vg, "vibe_advect_scalar_flux_f%d_dev" % bits, [ctypes.c_void_p] * 7 + [ctypes.c_int] * 3 +
+             [ctypes.c_double if bits == 64 else ctypes.c_float] * 3 + [ctypes.c_void_p] * 2)
+    t = [torch.tensor(a, dtype=dt, device="cuda") for a in (q, rho, u, v, w, dz, zs)]
+    out = torch.empty((nz, ny, nx), dtype=dt, device="cuda")
+    assert f(*[a.data_ptr() for a in t], nx, ny, nz, 900.0, 1100.0, 20000.0, out.data_ptr(),
+             torch.cuda.current_stream().cuda_stream) == 0
+
+    def formula(wide, r):  # r rounds to the kernel's type (or not at all)
+        U, V, W, Q, R, D, S = (a.astype(wide) for a in (u, v, w, q, rho, dz, zs))
+        thick = np.maximum(r(D[:, None, None] * r(wide(20000.0) - S)), 1)
+
+        def diff(vel, ax):  # of the fluxes through a cell's two faces
+            f = r(vel * r(R + np.roll(R, 1, ax))) * r(Q + np.roll(Q, 1, ax))
+            return r(np.roll(f if bits == 64 else r(f), -1, ax) - r(f)) / 4
+
+        h = r(r(diff(U, 2) * r(wide(1) / wide(900.0))) + r(diff(V, 1) * r(wide(1) / wide(1100.0))))
+        z = diff(W, 0)
+        z[0], z[-1] = 0, 0
+        return -r(r(h + r(z / thick)) / R)
+
+    wide = np.longdouble if bits == 64 else np.float64
+    exact = formula(wide, lambda a: a)
+    twice = formula(wide, lambda a: np.asarray(a, np_t).astype(wide))
+    err = lambda a: float(np.sqrt(((a - exact) ** 2).sum()))  # noqa: E731
+    assert err(out.cpu().numpy().astype(wide)) <= 1.02 * err(twice)
