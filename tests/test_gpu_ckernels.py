@@ -762,12 +762,13 @@ def test_cfl_scan_bounds_beyond_single_precision(vg, oc, case):
     assert mw == a.value or abs(mw - a.value) <= 2.3e-16 * a.value
 
 
+@pytest.mark.parametrize("dims", [(34, 10, 6), (62, 24, 45)])  # a thread per cell, tiles
 @pytest.mark.parametrize("where", ["zs", "dzeta", "rho", "q", "w"])
 @pytest.mark.parametrize("nan", [np.nan, -np.nan])
-def test_flux_advection_nan_reaches_the_result(vg, oc, where, nan):
+def test_flux_advection_nan_reaches_the_result(vg, oc, where, nan, dims):
     """A NaN in the metric or a field makes the cells that use it NaN, as in
     the oracle, and no others."""
-    nx, ny, nz = 34, 10, 6
+    nx, ny, nz = dims
     rng = np.random.default_rng(1)
     n = nx * ny * nz
     f = dict(q=rng.random(n), rho=0.5 + rng.random(n), u=rng.random(n) - 0.5, v=rng.random(n) - 0.5,
@@ -856,13 +857,13 @@ def test_flux_advection_error_against_wider_type(vg, bits, thin):
     """The tiled kernel is no further from the result in a wider type than the
     formula with its two divisions a cell, rounded at every operation (FP64: but
     for the product that a fused multiply-add takes into a difference of
-    fluxes): 2-norms over 31 x 40 x 20 cells, to 2 %; thin: layers under 1 m
+    fluxes): 2-norms over 62 x 40 x 40 cells, to 2 %; thin: layers under 1 m
     count as 1 m."""
     import torch
     dt, np_t = (torch.float64, np.float64) if bits == 64 else (torch.float32, np.float32)
     if bits == 64 and np.finfo(np.longdouble).nmant <= 52:
         pytest.skip("no wider type on this host")
-    nx, ny, nz = 31, 40, 20
+    nx, ny, nz = 62, 40, 40
     rng = np.random.default_rng(bits)
     u, v, w = ((a * rng.random((nz, ny, nx)) - 0.5 * a).astype(np_t) for a in (40.0, 30.0, 4.0))
     q, rho = (300.0 + 5.0 * rng.random((nz, ny, nx))).astype(np_t), (0.2 + rng.random((nz, ny, nx))).astype(np_t)
@@ -893,3 +894,32 @@ def test_flux_advection_error_against_wider_type(vg, bits, thin):
     twice = formula(wide, lambda a: np.asarray(a, np_t).astype(wide))
     err = lambda a: float(np.sqrt(((a - exact) ** 2).sum()))  # noqa: E731
     assert err(out.cpu().numpy().astype(wide)) <= 1.02 * err(twice)
+
+
+@pytest.mark.parametrize("bits", [64, 32])
+@pytest.mark.parametrize("dims", [(63, 17, 120), (94, 25, 61), (31, 8, 400), (62, 9, 200), (124, 48, 11), (186, 16, 25),
+                                  (5, 700, 30), (4000, 1, 20), (16, 512, 9), (33, 33, 33)])
+def test_flux_advection_tiles_and_cells(vg, oc, bits, dims):
+    """Grids large enough for the tiled kernel, with ragged last tiles and level
+    chunks, and grids that fill its tiles badly and take a thread per cell:
+    against the oracle at the bounds above (1e-12; FP32 1e-4)."""
+    import torch
+    nx, ny, nz = dims
+    dt = torch.float64 if bits == 64 else torch.float32
+    f = _dev(vg, "vibe_advect_scalar_flux_f%d_dev" % bits, [ctypes.c_void_p] * 7 + [ctypes.c_int] * 3 +
+             [ctypes.c_double if bits == 64 else ctypes.c_float] * 3 + [ctypes.c_void_p] * 2)
+    rng = np.random.default_rng(nx + ny)
+    n = nx * ny * nz
+    fields = [rng.random(n), 0.5 + rng.random(n), 20 * rng.random(n) - 10, 20 * rng.random(n) - 10, rng.random(n) - 0.5,
+              0.01 + 0.01 * rng.random(nz), 500.0 * rng.random(nx * ny)]
+    t = [torch.tensor(v, dtype=dt, device="cuda") for v in fields]
+    host = [np.ascontiguousarray(v.double().cpu().numpy()) for v in t]
+    for zs in (True, False):
+        out = torch.full((n,), float("nan"), dtype=dt, device="cuda")
+        assert f(*[v.data_ptr() for v in t[:6]], t[6].data_ptr() if zs else None, nx, ny, nz, 900.0, 1100.0, 20000.0,
+                 out.data_ptr(), torch.cuda.current_stream().cuda_stream) == 0
+        ref = np.full(n, np.nan)
+        oc.port_lib().vo_advect_scalar_flux(*[h.ctypes.data for h in host[:6]], host[6].ctypes.data if zs else None,
+                                             nx, ny, nz, 900.0, 1100.0, 20000.0, ref.ctypes.data)
+        tol = 1e-12 if bits == 64 else 1e-4
+        assert np.abs(out.double().cpu().numpy() - ref).max() <= tol * np.abs(ref).max()

@@ -961,6 +961,43 @@ __global__ void __launch_bounds__(32 * (kFluxRows + 1)) k_flux_adv(
   }
 }
 
+// The same, one thread per cell with its six faces, for grids that fill the
+// tiles badly (flux_tiles below).
+template <typename T>
+__global__ void k_flux_cell(const T* __restrict__ q, const T* __restrict__ rho, const T* __restrict__ u,
+                           const T* __restrict__ v, const T* __restrict__ w, const T* __restrict__ dzeta,
+                           const T* __restrict__ zs, int nx, int ny, int nz, T dx, T dy, T z_top, T* __restrict__ dqdt) {
+  const size_t nxy = (size_t)nx * ny, n = nxy * nz;
+  const T inv_dx = (T)1 / dx, inv_dy = (T)1 / dy, hf = (T)0.5;
+  for (size_t idx = blockIdx.x * (size_t)blockDim.x + threadIdx.x; idx < n; idx += (size_t)gridDim.x * blockDim.x) {
+    const int k = (int)(idx / nxy);
+    const int j = (int)((idx / nx) % ny);
+    const int i = (int)(idx % nx);
+    const size_t base_k = (size_t)k * nxy;
+    const T scale = zs ? (z_top - zs[(size_t)j * nx + i]) : z_top;
+    T dz = dzeta[k] * scale;
+    if (dz < (T)1) dz = (T)1;
+    const size_t c = idx;
+    const size_t e = base_k + (size_t)j * nx + (size_t)((i + 1) % nx);
+    const size_t ws = base_k + (size_t)j * nx + (size_t)((i + nx - 1) % nx);
+    const T fxE = u[e] * (hf * (rho[c] + rho[e])) * (hf * (q[c] + q[e]));
+    const T fxW = u[c] * (hf * (rho[ws] + rho[c])) * (hf * (q[ws] + q[c]));
+    const size_t nn = base_k + (size_t)((j + 1) % ny) * nx + (size_t)i;
+    const size_t ss = base_k + (size_t)((j + ny - 1) % ny) * nx + (size_t)i;
+    const T fyN = v[nn] * (hf * (rho[c] + rho[nn])) * (hf * (q[c] + q[nn]));
+    const T fyS = v[c] * (hf * (rho[ss] + rho[c])) * (hf * (q[ss] + q[c]));
+    T fzT = 0, fzB = 0;
+    if (k > 0 && k + 1 < nz) {
+      const size_t t = c + nxy, b = c - nxy;
+      fzT = w[t] * (hf * (rho[c] + rho[t])) * (hf * (q[c] + q[t]));
+      fzB = w[c] * (hf * (rho[b] + rho[c])) * (hf * (q[b] + q[c]));
+    }
+    const T div = (fxE - fxW) * inv_dx + (fyN - fyS) * inv_dy + (fzT - fzB) / dz;
+    const T rr = (rho[idx] > (T)1e-12) ? rho[idx] : (T)1e-12;
+    dqdt[idx] = -div / rr;
+  }
+}
+
 // ---- allocation-free batched Thomas ------------------------------------
 // Some callers of this library may not allocate device memory at all: a host
 // model whose own allocator has reserved the device's memory and forbids any
@@ -1221,6 +1258,19 @@ T neu_host(const T* x, size_t n) {
   return ok ? r : (T)NAN;
 }
 
+// The tiled kernel where it is the faster one. FP64: it takes 75 ps a cell of its
+// tiles, the cells beyond the grid included, and no less than 15 us (at least
+// four levels a block in turn); a thread per cell takes 7 us and 130 ps a cell.
+// Tiles against cells: 48 x 48 x 20 15.0 and 14.7 us, 96 x 96 x 10 14.9 and 19.0,
+// 16 x 512 x 60 (half of each tile used) 76 and 70, 1 x 1000 x 40 97 and 15. FP32, bound by memory:
+// 16 x 512 x 60 10.8 and 10.6, 3 x 4096 x 40 31 and 11, 384 x 384 x 60 82 and 117.
+template <typename T>
+bool flux_tiles(size_t tiles, int nz, size_t cells) {
+  const size_t padded = tiles * kFluxCols * kFluxRows * nz;
+  if (sizeof(T) == 4) return padded <= 2 * cells;
+  return std::max(15.0, 7.5e-5 * (double)padded) <= 7.0 + 1.3e-4 * (double)cells;
+}
+
 template <typename T>
 int flux_dev(const T* q, const T* rho, const T* u, const T* v, const T* w, const T* dzeta, const T* zs, int nx, int ny,
              int nz, T dx, T dy, T z_top, T* dqdt, vibe_stream_t stream) {
@@ -1231,6 +1281,11 @@ int flux_dev(const T* q, const T* rho, const T* u, const T* v, const T* w, const
   // of at least 4 levels (a chunk computes its first lower face again)
   const int xt = (nx + kFluxCols - 1) / kFluxCols;
   const size_t tiles = (size_t)xt * ((ny + kFluxRows - 1) / kFluxRows);
+  if (!flux_tiles<T>(tiles, nz, n)) {
+    const int blocks = (int)((n + 255) / 256 < 65535 ? (n + 255) / 256 : 65535);
+    k_flux_cell<T><<<blocks, 256, 0, (cudaStream_t)stream>>>(q, rho, u, v, w, dzeta, zs, nx, ny, nz, dx, dy, z_top, dqdt);
+    return device_ok(cudaGetLastError(), "flux advection launch") ? VIBE_C_OK : VIBE_C_ERR_DEVICE;
+  }
   const int want = tiles >= 3648 ? 1 : (int)(3648 / tiles);
   int kz = (nz + want - 1) / want;
   if (kz < 4) kz = 4;
