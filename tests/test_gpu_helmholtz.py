@@ -130,6 +130,23 @@ def test_multigrid_odd_grids(vg, oc, dims, levels):
                 assert np.array_equal(h.solve(a, b, f)[1], x)
 
 
+@pytest.mark.parametrize("dims", [(31, 33, 12), (33, 70, 9), (64, 48, 10), (65, 129, 5), (7, 150, 8), (40, 30, 12)])
+def test_mixed_passes_gain_as_much_each(vg, oc, dims):
+    """FP32 passes of 1e-4 each: with a third one, or two that overshoot as on
+    even grids, a tol of 1e-10 ends no further than one more pass from the FP64
+    residual's rounding: 1e-13 on grids of odd size, which take the third, and
+    below the tolerance on the others. The odd ones with and without coarser levels."""
+    nx, ny, nz = dims
+    s = hc.si_setup(oc, nx=nx, ny=ny, nz=nz, zeta_first=20000.0 / nz, zeta_stretch=1.0)
+    a, b, f, dzeta, zs = hc.si_problem(oc, s)
+    port = oc.Model(s, "port")
+    fn = np.sqrt(np.sum(oc.interior(s, 3, f) ** 2))
+    with make(vg, s, 4, dzeta, zs, tol=1e-10) as h:
+        rc, x = h.solve(a, b, f)
+        assert rc == 0
+        assert port.helmholtz_residual_l2(a, b, f, x) / fn < (1e-13 if nx % 2 or ny % 2 else 1e-10)
+
+
 def test_bad_arguments(vg, oc):
     s = hc.si_setup(oc, nx=8, ny=8, nz=4)
     dzeta = np.full(4, 0.25)

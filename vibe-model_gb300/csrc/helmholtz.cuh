@@ -62,6 +62,8 @@ template <typename T>
 void mg_destroy(MgSolver<T>* m);
 template <typename T>
 int mg_levels(const MgSolver<T>* m);
+template <typename T>
+bool mg_odd(const MgSolver<T>* m);  // whether the grid is of odd size and has coarser levels
 // builds every level's couplings and column factors from the FP64 a, b
 template <typename T>
 int mg_set_coefficients(MgSolver<T>* m, const double* a, const double* b, cudaStream_t s);

@@ -1136,6 +1136,11 @@ void mg_destroy(MgSolver<T>* m) {
 }
 
 template <typename T>
+bool mg_odd(const MgSolver<T>* m) {
+  return m->L > 1 && (m->lv[0].nx % 2 || m->lv[0].ny % 2);
+}
+
+template <typename T>
 int mg_levels(const MgSolver<T>* m) {
   return m->L;
 }
@@ -1265,6 +1270,7 @@ template MgSolver<float>* mg_create<float>(const HGeo&, int);
 template MgSolver<double>* mg_create<double>(const HGeo&, int);
 template void mg_destroy<float>(MgSolver<float>*);
 template void mg_destroy<double>(MgSolver<double>*);
+template bool mg_odd<float>(const MgSolver<float>*);
 template int mg_levels<float>(const MgSolver<float>*);
 template int mg_levels<double>(const MgSolver<double>*);
 template int mg_set_coefficients<float>(MgSolver<float>*, const double*, const double*, cudaStream_t);
