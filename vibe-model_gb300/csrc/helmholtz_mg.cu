@@ -26,7 +26,7 @@
 // equation is kept in the volume-weighted form (sums over the cells there
 // are), which keeps the couplings of its faces symmetric. Residuals are restricted by the 2x2 mean (computed and
 // restricted in one pass) and corrections prolonged piecewise constant.
-// V(1,1) cycle, the coarsest grid smoothed kCoarseSweeps times in one cluster
+// V(1,1) cycle, the coarsest grid smoothed 4 or 8 times in one cluster
 // launch. The half sweep before a restriction leaves the residual zero on its
 // colour, so only the other colour's is computed and restricted; the one after
 // a prolongation overwrites its colour, so the correction is added where it
@@ -73,6 +73,7 @@ struct MgSolver {
   // yet, 1 = built, -1 = not available: the host loop runs instead)
   int graph_state = 0;
   int coarse_ctas = 0;  // CTAs of the one-cluster coarsest smoothing (0: one launch per half sweep)
+  int coarse_sweeps = 8;
   bool coarse_resident = false;  // ... whose CTAs keep their one tile per colour in shared memory
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t gexec = nullptr;
@@ -510,16 +511,21 @@ __global__ void __launch_bounds__(256) k_smooth_add(MgLevel<T> l, const T* __res
   scan_tile_store<T>(l, x, blockIdx.x, color, st, threadIdx.x);
 }
 
-// The coarsest grid's smoothing, kCoarseSweeps red-black sweeps (the first
+// The coarsest grid's smoothing, `sweeps` red-black sweeps (the first
 // half sweep from a zero guess), in one launch of one thread-block cluster:
 // CTA b takes tiles b, b + gridDim.x, ... of each half sweep, and the
 // cluster barrier (release/acquire at cluster scope, so x's global stores
 // are seen by the cluster's loads after it) separates the half sweeps; a
 // half sweep reads only the other colour, so its tiles are independent.
-// Replaces 2 kCoarseSweeps launches of a few tiles each (16 x 16 x 64: 4
-// tiles per half sweep). Four sweeps: the iteration counts of eight (7 at
-// 256 x 256 x 64 and 193 x 193 x 60, 5 at 97 x 64 x 40), 0.25 ms less a solve.
-constexpr int kCoarseSweeps = 4;
+// Replaces 2 sweeps launches of a few tiles each (16 x 16 x 64: 4 tiles per half
+// sweep).
+// Four sweeps leave the residuals that eight do where the coarsest grid is short
+// (a sweep carries a correction two columns on) and coarse enough that its
+// columns couple weakly: 256 x 256 x 64, coarsest 16 x 16 of the fifth level, 2.4e-14
+// either way after 7 iterations, 0.25 ms less a solve. Else they do not: 12 x 2000
+// x 16, coarsest 6 x 1000, 2.9e-11 and 8.6e-12 after 5; 40 x 30 x 20, coarsest 20 x 15 of
+// the second level, 3.3e-10 and 2.0e-11 after 5.
+constexpr int kCoarseExtent = 32, kCoarseLevels = 3;
 constexpr int kCoarseMaxCtas = 8;  // portable cluster size
 
 __device__ __forceinline__ void cluster_sync() {
@@ -527,12 +533,13 @@ __device__ __forceinline__ void cluster_sync() {
 }
 
 template <typename T>
-__global__ void __launch_bounds__(256) k_coarse_smooth(MgLevel<T> l, const T* __restrict__ rhs, T* __restrict__ x) {
+__global__ void __launch_bounds__(256) k_coarse_smooth(MgLevel<T> l, const T* __restrict__ rhs, T* __restrict__ x,
+                                                       int sweeps) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const ScanTile<T> st(reinterpret_cast<T*>(smem_raw), l.nz);
   const int ntiles = ((l.nx + 1) / 2 * l.ny + 31) / 32;
   constexpr int kB = sizeof(T) == 4 ? 8 : 4;
-  for (int sw = 0; sw < 2 * kCoarseSweeps; ++sw) {
+  for (int sw = 0; sw < 2 * sweeps; ++sw) {
     const int color = sw & 1;
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
       if (sw == 0)
@@ -581,7 +588,8 @@ __device__ __forceinline__ double ld_cluster(unsigned a, double) {
   return v;
 }
 template <typename T>
-__global__ void __launch_bounds__(256) k_coarse_resident(MgLevel<T> l, const T* __restrict__ rhs, T* __restrict__ x) {
+__global__ void __launch_bounds__(256) k_coarse_resident(MgLevel<T> l, const T* __restrict__ rhs, T* __restrict__ x,
+                                                         int sweeps) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* base = reinterpret_cast<T*>(smem_raw);
   const int nz = l.nz, tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
@@ -639,7 +647,7 @@ __global__ void __launch_bounds__(256) k_coarse_resident(MgLevel<T> l, const T* 
     }
   }
   __syncthreads();
-  for (int sw = 0; sw < 2 * kCoarseSweeps; ++sw) {
+  for (int sw = 0; sw < 2 * sweeps; ++sw) {
     const int color = sw & 1;
     const T* q = Q + color * 6 * rc;
     ScanTile<T> st(X, nz);
@@ -993,13 +1001,14 @@ void vcycle(MgSolver<T>* m, int li, const T* rhs, T* x, cudaStream_t s) {
       cudaLaunchAttribute at;
       coarse_config(m->coarse_ctas, m->coarse_resident ? coarse_resident_smem<T>(l.nz) : scan_smem<T>(l.nz), s, cfg,
                     at);
-      if (m->coarse_resident) cudaLaunchKernelEx(&cfg, k_coarse_resident<T>, l, rhs, x);
-      else cudaLaunchKernelEx(&cfg, k_coarse_smooth<T>, l, rhs, x);
+      const int sweeps = m->coarse_sweeps;
+      if (m->coarse_resident) cudaLaunchKernelEx(&cfg, k_coarse_resident<T>, l, rhs, x, sweeps);
+      else cudaLaunchKernelEx(&cfg, k_coarse_smooth<T>, l, rhs, x, sweeps);
       return;
     }
     smooth(l, rhs, x, 0, 1, s);
     smooth(l, rhs, x, 1, 0, s);
-    for (int it = 1; it < kCoarseSweeps; ++it) {
+    for (int it = 1; it < m->coarse_sweeps; ++it) {
       smooth(l, rhs, x, 0, 0, s);
       smooth(l, rhs, x, 1, 0, s);
     }
@@ -1071,6 +1080,8 @@ MgSolver<T>* mg_create(const HGeo& g, int max_levels) {
     nx = (nx + 1) / 2;
     ny = (ny + 1) / 2;
   }
+  const MgLevel<T>& last = m->lv[m->L - 1];
+  m->coarse_sweeps = m->L >= kCoarseLevels && imax(last.nx, last.ny) <= kCoarseExtent ? 4 : 8;
   const size_t n = g.n();
   T** kv[] = {&m->x, &m->r, &m->r0, &m->p, &m->v, &m->s, &m->t, &m->ph, &m->sh};
   ok = dev_alloc_all(m, kv, n) && ok;
