@@ -698,6 +698,7 @@ __global__ void __launch_bounds__(256) k_coarse_resident(MgLevel<T> l, const T* 
 }
 
 constexpr size_t kScanSmemMax = 200 * 1024;   // one tile's shared memory, at most
+constexpr int kOddTiles = 200;                  // tiles up to which an odd grid is its own coarsest (mg_create)
 constexpr int kCoarseMaxTiles = 64;             // tiles per half sweep up to which one cluster smooths the coarsest grid
 template <typename T>
 size_t scan_smem(int nz) {
@@ -1066,7 +1067,7 @@ MgSolver<T>* mg_create(const HGeo& g, int max_levels) {
   m->g = g;
   int nx = g.nx, ny = g.ny;
   const int cap = max_levels < 1 ? 1 : (max_levels > kMgMaxLevels ? kMgMaxLevels : max_levels);
-  bool ok = true;
+  bool ok = true, odd = false;
   for (int l = 0; l < cap; ++l) {
     MgLevel<T>& L = m->lv[l];
     L.nx = nx;
@@ -1077,6 +1078,19 @@ MgSolver<T>* mg_create(const HGeo& g, int max_levels) {
     ok = dev_alloc_all(m, arrs, L.n) && ok;
     m->L = l + 1;
     if (nx / 2 < 4 || ny / 2 < 4) break;
+    if (nx % 2 || ny % 2) {
+      // A first odd grid of this many tiles a half sweep would save iterations with
+      // coarser levels, but their launches cost more: 97 x 64 x 40 (98 tiles), FP32
+      // 3060 us with five levels, 2590 with one; FP64 4390 and 3820. In FP32 up to
+      // kCoarseMaxTiles the one level would be smoothed by a single cluster (63 x
+      // 63 x 24: 2770 us with five levels, 7800 with one), unless it is of a tile a
+      // CTA, which is fast (40 x 30 x 20, second level 20 x 15). Larger grids are bound
+      // by their work (193 x 193 x 60, FP64: 7950 and 13700).
+      const int tiles = ((nx + 1) / 2 * ny + 31) / 32;
+      const bool few = sizeof(T) == 4 && l > 0 && tiles <= kCoarseMaxCtas;
+      if (!odd && (few || (tiles > (sizeof(T) == 4 ? kCoarseMaxTiles : 16) && tiles <= kOddTiles))) break;
+      odd = true;
+    }
     nx = (nx + 1) / 2;
     ny = (ny + 1) / 2;
   }
