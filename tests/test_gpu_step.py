@@ -696,3 +696,36 @@ def test_energy_budget_matches_oracle(vg, oc, prec):
         got, ref = m.energy_budget(), oc.energy_budget(o)
         for key in ref:
             assert abs(got[key] - ref[key]) <= 1e-12 * abs(ref[key]) + 1e-300, (key, got[key], ref[key])
+
+
+@pytest.mark.parametrize("dims,dx", [((64, 64, 40), 250.0), ((120, 100, 60), 1000.0)])
+def test_level_split_error_against_64_bits(vg, dims, dx):
+    """Four steps with the level-split column kernel are no further from the FP64
+    model's than with the sweeping one (variant 5): 2-norms of w and v over a
+    perturbed state, to 2 %, short and long chunks."""
+    nx, ny, nz = dims
+    s = small_setup(vg, nx=nx, ny=ny, nz=nz, dx=dx, dy=dx, z_top=40.0 * dx if dx < 500 else 20.0 * dx,
+                    zeta_first=50.0, zeta_stretch=1.03, ref_kind=1, bv_n=0.01, acoustic_mode=2, hevi_beta=0.5,
+                    bubble_xc=0.5 * nx * dx, bubble_yc=0.5 * ny * dx, qv_surface=0.0, u_background=10.0, shear_u=0.0)
+    rng = np.random.default_rng(3)
+    with vg.Model(s, vg.FP64) as m:
+        start = m.state()
+        for sp, amp in ((0, 0.5), (1, 0.5), (2, 0.05), (4, 0.5)):
+            f = vg.interior(s, sp, start[sp])
+            f += amp * rng.standard_normal(f.shape) * (1 if sp != 2 else np.arange(nz + 1)[:, None, None] % nz > 0)
+        m.set_state(start)
+        m.step(dx / 125.0 if dx < 500 else 6.0, 6, 4)
+        ref = m.state()
+    err = {}
+    for variant in (5, -1):
+        with vg.Model(s, vg.MIXED) as m:
+            m.set_state(start)
+            m.set_tuning(column_kernel=variant)
+            try:
+                m.step(dx / 125.0 if dx < 500 else 6.0, 6, 4)
+            finally:
+                m.set_tuning()
+            got = m.state()
+        err[variant] = [float(np.linalg.norm(vg.interior(s, sp, got[sp]) - vg.interior(s, sp, ref[sp]))) for sp in (1, 2)]
+    for a, b in zip(err[-1], err[5]):
+        assert 0.0 < a <= 1.02 * b, err

@@ -2486,18 +2486,22 @@ size_t hevi_tma_smem_bytes(int nz) {
 
 // ---- the HEVI column update with the levels split over warps ---------------
 // The column system's LU factors depend on the level only, so both
-// recurrences, dp(k) = rhs(k) li(k) - m(k) dp(k-1) with m = la li and
+// recurrences, dp(k) = (rhs(k) - la(k) dp(k-1)) li(k) and
 // x(k) = dp(k) - lc(k) x(k+1), split into chunks of kM levels: each thread
-// solves its chunk with a zero carry and adds the chunk's carry times
-// G(k) = prod_{l=k0..k} (-m(l)), or H(k) = prod_{l=k..k0+kn-1} (-lc(l)). Every
-// warp folds the carries of the chunks below (above) it by itself, so a block
+// runs its chunk with a zero carry, and once more with the carry that the chunks
+// below (above) it make, each of which passes on its last (first) value plus its
+// own carry times prod(-la li), or prod(-lc), over its levels. (Adding that
+// product's part to the first run's values, and la li in one factor, left w and v 1
+// to 3 % further from 64-bit results over four steps.) Every
+// warp folds those carries by itself, so a block
 // meets at two barriers instead of two per level, and a column's latency is
 // that of one chunk instead of 2 nz levels. A warp is 64 consecutive points of
 // the padded plane (two adjacent columns a lane, every row access an aligned
 // 8-byte load or store; rows run on into each other, so only the P - nx
 // padding points idle) by one chunk; a block is the C = ceil(nz/kM) chunks of
 // its 64 points. Per-level constants lie in float4 tables with the step's
-// scalars folded in.
+// scalars folded in, but for 1/dz of a pressure gradient, which is multiplied last:
+// folded in, its rounding is the same in every substep and adds up (another 3 %).
 // Every substep changes pi' by kap(k) times its change of rho' (both are the
 // same mass divergence), so rho' is not carried: the last substep writes
 // rho'(k) = rho'_0 + (pi'(k) - pi'_0) / kap(k) from the stage's state wst.
@@ -2520,7 +2524,7 @@ size_t hevi_tma_smem_bytes(int nz) {
 constexpr int kChunkEarly = 4;
 size_t hevi_chunk_smem_bytes(int nz, int m) {
   const int C = (nz + m - 1) / m;
-  return ((size_t)(3 * nz + 1)) * sizeof(float4) + (size_t)64 * C * sizeof(float2);
+  return ((size_t)(3 * nz + 1)) * sizeof(float4) + (size_t)65 * C * sizeof(float2);
 }
 template <int kM>
 __device__ __forceinline__ void hevi_chunk_body(const Dims& d, const Tab& t, const Flags& fl, const WS& win,
@@ -2530,11 +2534,12 @@ __device__ __forceinline__ void hevi_chunk_body(const Dims& d, const Tab& t, con
   extern __shared__ float4 s_split[];
   const int nz = d.nz;
   const int C = blockDim.y;
-  float4* ta = s_split;          // nz+1: face k: explicit and implicit pressure-gradient factor, rfz; level k: H
+  float4* ta = s_split;          // nz+1: face k: explicit and implicit pressure-gradient factor, rfz, idzw
   float4* tb = ta + (nz + 1);    // nz: idzc, dtau kap, r0, t0
-  float4* tc = tb + nz;          // nz: li, m = la li, lc, G
+  float4* tc = tb + nz;          // nz: li, la, lc
   float2* sf = reinterpret_cast<float2*>(tc + nz);  // C x 32: dp at each chunk's last level, zero carry
   float2* sx = sf + 32 * C;                         // C x 32: x at each chunk's first level, zero carry
+  float2* gh = sx + 32 * C;                         // C: the chunk's prod(-la li) and prod(-lc)
   const int tx = threadIdx.x, c = threadIdx.y;
   const int tid = c * 32 + tx;
   const int e = bx * 64 + 2 * tx;
@@ -2579,12 +2584,12 @@ __device__ __forceinline__ void hevi_chunk_body(const Dims& d, const Tab& t, con
   const float b = (float)fl.hevi_beta, ob = 1.f - b;
   const float cpf = (float)kCp;
   for (int k = tid; k <= nz; k += 32 * C) {
-    const float g = (k > 0 && k < nz) ? cpf * t.tfz[k] * t.idzw[k] : 0.f;  // no gradient on the ground and the lid
+    const float tf = (k > 0 && k < nz) ? t.tfz[k] : 0.f;  // no gradient on the ground and the lid
     if (k < nz) {
       tb[k] = make_float4(t.idzc[k], dtau * t.kap[k], t.r0c[k], t.t0c[k]);
-      tc[k] = make_float4(lu[2 * nz + k], lu[k] * lu[2 * nz + k], lu[nz + k], 1.f);
+      tc[k] = make_float4(lu[2 * nz + k], lu[k], lu[nz + k], 0.f);
     }
-    ta[k] = make_float4(dtau * ob * g, dtau * b * g, t.rfz[k], 1.f);
+    ta[k] = make_float4(dtau * ob * cpf * tf, dtau * b * cpf * tf, t.rfz[k], t.idzw[k]);
   }
   const int vn = d.P;
   const float dxi = t.dx_inv, dyi = t.dy_inv;
@@ -2609,10 +2614,10 @@ __device__ __forceinline__ void hevi_chunk_body(const Dims& d, const Tab& t, con
     const float4 A = ta[k0];
     const float gx = pk.x - pm.x, gy = pk.y - pm.y;
     if (apply_uv) {  // the input's deferred correction of w
-      wk.x -= A.y * gx;
-      wk.y -= A.y * gy;
+      wk.x -= A.y * gx * A.w;
+      wk.y -= A.y * gy * A.w;
     }
-    wt = make_float2(wk.x - A.x * gx, wk.y - A.x * gy);
+    wt = make_float2(wk.x - A.x * gx * A.w, wk.y - A.x * gy * A.w);
   }
 #pragma unroll
   for (int q = 0; q < kM; ++q) {
@@ -2636,18 +2641,18 @@ __device__ __forceinline__ void hevi_chunk_body(const Dims& d, const Tab& t, con
         v0y += ty_ * (pk.y - fs.y);
         v1x += ty_ * (fn.x - pk.x);
         v1y += ty_ * (fn.y - pk.y);
-        wk1.x -= A1.y * gx;
-        wk1.y -= A1.y * gy;
+        wk1.x -= A1.y * gx * A1.w;
+        wk1.y -= A1.y * gy * A1.w;
       } else {
         u1x = fu.y;
       }
-      const float2 wt1 = make_float2(wk1.x - A1.x * gx, wk1.y - A1.x * gy);
+      const float2 wt1 = make_float2(wk1.x - A1.x * gx * A1.w, wk1.y - A1.x * gy * A1.w);
       const float sx_ = ob * ((A0.z * wk.x - A1.z * wk1.x) * B.x) - B.z * ((u1x - u0x) * dxi + (v1x - v0x) * dyi);
       const float sy_ = ob * ((A0.z * wk.y - A1.z * wk1.y) * B.x) - B.z * ((u1y - u0y) * dxi + (v1y - v0y) * dyi);
       const float rx = pk.x + B.y * (sx_ + b * ((A0.z * wt.x - A1.z * wt1.x) * B.x));
       const float ry = pk.y + B.y * (sy_ + b * ((A0.z * wt.y - A1.z * wt1.y) * B.x));
-      prev = make_float2(rx * Ck.x - Ck.y * prev.x, ry * Ck.x - Ck.y * prev.y);
-      dp[q] = prev;
+      dp[q] = make_float2(rx, ry);
+      prev = make_float2((rx - Ck.y * prev.x) * Ck.x, (ry - Ck.y * prev.y) * Ck.x);
       if (active) {
         st2(W, o, wt);
         st2(U, o, make_float2(u0x, u0y));
@@ -2665,57 +2670,55 @@ __device__ __forceinline__ void hevi_chunk_body(const Dims& d, const Tab& t, con
   }
   if (active && k0 + kn == nz) st2(W, o, wt);
   sf[tid] = prev;
-  // the carries' products, first needed behind the barrier, from the tables:
+  // the chunks' products, first needed behind the barrier, from the tables:
   // formed with the tables, from memory, they held the start up (substep at
   // 64 x 64 x 40 6.9 to 6.2 us, 193 x 193 x 60 17.0 to 16.3)
-  for (int k = tid; k < nz; k += 32 * C) {
-    const int lo = k / kM * kM, hi = imin(lo + kM, nz);
+  if (tid < C) {
+    const int lo = tid * kM, hi = imin(lo + kM, nz);
     float G = 1.f, H = 1.f;
-    for (int l = lo; l <= k; ++l) G *= -tc[l].y;
-    for (int l = k; l < hi; ++l) H *= -tc[l].z;
-    tc[k].w = G;
-    ta[k].w = H;
+    for (int l = lo; l < hi; ++l) {
+      G *= -tc[l].y * tc[l].x;
+      H *= -tc[l].z;
+    }
+    gh[tid] = make_float2(G, H);
   }
   __syncthreads();
   float2 in = make_float2(0.f, 0.f);  // dp(k0 - 1)
   for (int cc = 0; cc < c; ++cc) {
     const float2 f = sf[cc * 32 + tx];
-    const float g = tc[(cc + 1) * kM - 1].w;
+    const float g = gh[cc].x;
     in = make_float2(f.x + g * in.x, f.y + g * in.y);
   }
+  const float2 below = in;  // which gives x(k0 - 1) below
 #pragma unroll
   for (int q = 0; q < kM; ++q)
     if (q < kn) {
-      const float g = tc[k0 + q].w;
-      dp[q].x += g * in.x;
-      dp[q].y += g * in.y;
+      const float4 Ck = tc[k0 + q];
+      in = dp[q] = make_float2((dp[q].x - Ck.y * in.x) * Ck.x, (dp[q].y - Ck.y * in.y) * Ck.x);
     }
   float2 nx = make_float2(0.f, 0.f);
 #pragma unroll
   for (int q = kM - 1; q >= 0; --q)
     if (q < kn) {  // x with zero carry from above
       const float l = tc[k0 + q].z;
-      dp[q].x -= l * nx.x;
-      dp[q].y -= l * nx.y;
-      nx = dp[q];
+      nx = make_float2(dp[q].x - l * nx.x, dp[q].y - l * nx.y);
     }
-  sx[tid] = dp[0];
+  sx[tid] = nx;
   __syncthreads();
-  const float2 below = in;  // dp(k0 - 1), which gives x(k0 - 1) below
   in = make_float2(0.f, 0.f);  // x(k0 + kn)
   for (int cc = C - 1; cc > c; --cc) {
     const float2 f = sx[cc * 32 + tx];
-    const float h = ta[cc * kM].w;
+    const float h = gh[cc].y;
     in = make_float2(f.x + h * in.x, f.y + h * in.y);
   }
   if (!active) return;
   o = kEarly ? o - (unsigned)kn * pl : (unsigned)k0 * pl + col;  // (early: still the wait's)
+  nx = in;
 #pragma unroll
-  for (int q = 0; q < kM; ++q)
+  for (int q = kM - 1; q >= 0; --q)
     if (q < kn) {
-      const float h = ta[k0 + q].w;
-      dp[q].x += h * in.x;
-      dp[q].y += h * in.y;
+      const float l = tc[k0 + q].z;
+      nx = dp[q] = make_float2(dp[q].x - l * nx.x, dp[q].y - l * nx.y);
       st2(PI, o + q * pl, dp[q]);
     }
   if (!last) return;
@@ -2725,19 +2728,19 @@ __device__ __forceinline__ void hevi_chunk_body(const Dims& d, const Tab& t, con
   };
   float2 wb = back(W, o);  // w at the level's lower face
   if (c > 0) {
-    const float l = tc[k0 - 1].z, a = ta[k0].y;
-    wb.x -= a * (dp[0].x - (below.x - l * dp[0].x));
-    wb.y -= a * (dp[0].y - (below.y - l * dp[0].y));
+    const float l = tc[k0 - 1].z, a = ta[k0].y, iz = ta[k0].w;
+    wb.x -= a * (dp[0].x - (below.x - l * dp[0].x)) * iz;
+    wb.y -= a * (dp[0].y - (below.y - l * dp[0].y)) * iz;
   }
 #pragma unroll
   for (int q = 0; q < kM; ++q)
     if (q < kn) {
       const int k = k0 + q;
-      const float a = ta[k + 1].y, ik = dtau / tb[k].y;  // 1 / kap
+      const float a = ta[k + 1].y, iz = ta[k + 1].w, ik = dtau / tb[k].y;  // 1 / kap
       const bool top = q + 1 >= kn;
       const float2 xf = top ? in : dp[q + 1 < kM ? q + 1 : q];
       const float2 wf = top ? wt : back(W, o + pl);
-      const float2 wn = make_float2(wf.x - a * (xf.x - dp[q].x), wf.y - a * (xf.y - dp[q].y));
+      const float2 wn = make_float2(wf.x - a * (xf.x - dp[q].x) * iz, wf.y - a * (xf.y - dp[q].y) * iz);
       const float2 r = ldf2(wst.f[RHO] + o), p = ldf2(wst.f[PI] + o);
       st2(RHO, o, make_float2(r.x + (dp[q].x - p.x) * ik, r.y + (dp[q].y - p.y) * ik));
       st2(W, o, wb);
