@@ -87,3 +87,31 @@ def test_group_after_members_reconfigured_for_another_dt(vg):
     finally:
         for m in grouped + single:
             m.close()
+
+
+@pytest.mark.parametrize("n_sub", [1, 6])
+@pytest.mark.parametrize("nz", [13, 57, 70])
+def test_large_groups_match_the_oracle(vg, oc, nz, n_sub):
+    """Members of more than 9000 columns together, the work-list column kernel
+    with 6, 8 and 10 levels a warp (last chunks of one level, full ones): every
+    member against the oracle over two steps, at the mixed path's bound on
+    ragged grids, 2e-5 of each field's scale."""
+    sizes = [(80, 70), (33, 65), (64, 41)]
+    setups = [member(vg, nx, ny, q) for q, (nx, ny) in enumerate(sizes)]
+    for s in setups:
+        s.nz, s.zeta_stretch, s.z_top = nz, 1.0, 200.0 * nz
+    models = [vg.Model(s, vg.MIXED) for s in setups]
+    try:
+        with vg.Group(models) as g:
+            g.step(0.3 * n_sub, n_sub, 2)
+        for m, s in zip(models, setups):
+            t = oc.Setup()
+            for name, _ in oc.Setup._fields_:
+                setattr(t, name, getattr(s, name))
+            o = oc.Model(t, "port")
+            assert o.rk3_step(0.3 * n_sub, n_sub) == 0 and o.rk3_step(0.3 * n_sub, n_sub) == 0
+            assert_rounding_close(vg, s, [m.get(sp) for sp in range(7)], [o.get(sp) for sp in range(7)], 2e-5,
+                                  "group %s" % ((s.nx, s.ny, s.nz),))
+    finally:
+        for m in models:
+            m.close()

@@ -729,3 +729,19 @@ def test_level_split_error_against_64_bits(vg, dims, dx):
         err[variant] = [float(np.linalg.norm(vg.interior(s, sp, got[sp]) - vg.interior(s, sp, ref[sp]))) for sp in (1, 2)]
     for a, b in zip(err[-1], err[5]):
         assert 0.0 < a <= 1.02 * b, err
+
+
+@pytest.mark.parametrize("dt,n_sub", [(0.5, 1), (1.0, 3)])
+@pytest.mark.parametrize("dims", [(97, 95, 48), (97, 95, 49), (101, 93, 57), (193, 47, 64), (130, 71, 65)])
+def test_level_split_column_kernel_levels_a_warp(vg, oc, dims, dt, n_sub):
+    """Grids of more than 9000 columns take 6, 8 or 10 levels a warp by their
+    height (48, 49 to 64, above): with a last chunk of one level, full ones and
+    ragged rows against the oracle, at the bound of the kernel's edges above."""
+    nx, ny, nz = dims
+    t = small_setup(vg, nx=nx, ny=ny, nz=nz, zeta_stretch=1.0, bubble_xc=nx * 125.0, bubble_yc=ny * 125.0,
+                    **STEP_CASES[3])
+    with vg.Model(t, vg.MIXED) as m:
+        o = oc.Model(oracle_setup(oc, t), "port")
+        m.step(dt, n_sub, 2)
+        assert o.rk3_step(dt, n_sub) == 0 and o.rk3_step(dt, n_sub) == 0
+        assert_state_close(vg, t, m.state(), o.state(), 2 * TOLMX, range(7), "level-split column kernel %s" % (dims,))
