@@ -736,11 +736,12 @@ def test_neumaier_nonfinite_beside_the_largest(vg, big, odd, n):
 
 
 @pytest.mark.parametrize("case", ["winds", "depth", "dzeta"])
-def test_cfl_scan_bounds_beyond_single_precision(vg, oc, case):
+@pytest.mark.parametrize("dims", [(3, 1, 2), (300, 16, 18), (300, 77, 21)])
+def test_cfl_scan_bounds_beyond_single_precision(vg, oc, case, dims):
     """Winds under 2^-126 beside tiny spacings, and dzeta and depths that single
     precision cuts to zero while their product is an ordinary thickness: the
     scan equals the oracle's bit for bit."""
-    nx, ny, nz = 3, 1, 2
+    nx, ny, nz = dims
     n = nx * ny * nz
     u, v, w = np.zeros(n), np.zeros(n), np.zeros(n)
     dz, zs, z_top, dx = np.full(nz, 0.01), np.zeros(nx * ny), 20000.0, 1e-9
@@ -750,9 +751,11 @@ def test_cfl_scan_bounds_beyond_single_precision(vg, oc, case):
         dx = 1000.0
         w[0], w[nx * ny + 1] = 5.0, 2.0
         if case == "depth":
-            dz[:], z_top = (1.1e-38, 4e-39), 3.3e38
+            dz[:], z_top = 1.1e-38, 3.3e38
+            dz[1] = 4e-39
         else:
-            dz[:], z_top = (2e38, 3e38), 1e-38
+            dz[:], z_top = 2e38, 1e-38
+            dz[1] = 3e38
             w[0], w[nx * ny + 1] = 5.0, 6.0  # dz = 2 m and 3 m: equal bounds per wind, 2.5 /s and 2 /s
     a, b = ctypes.c_double(), ctypes.c_double()
     ro = oc.port_lib().vo_cfl_scan(u.ctypes.data, v.ctypes.data, w.ctypes.data, dz.ctypes.data, zs.ctypes.data, nx, ny,
@@ -923,3 +926,76 @@ def test_flux_advection_tiles_and_cells(vg, oc, bits, dims):
                                              nx, ny, nz, 900.0, 1100.0, 20000.0, ref.ctypes.data)
         tol = 1e-12 if bits == 64 else 1e-4
         assert np.abs(out.double().cpu().numpy() - ref).max() <= tol * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("kind", ["white", "uniform", "near", "calm", "tiny", "huge", "nonfinite", "odd_metric", "steps"])
+@pytest.mark.parametrize("dims", [(260, 16, 17), (97, 65, 33), (300, 77, 21), (511, 257, 6)])
+def test_cfl_scan_tiles_change_no_bit(vg, oc, kind, dims):
+    """The tiled scan (two and four levels a tile) equals the oracle's bit for bit:
+    also where most cells lie at the best (a uniform wind, one that differs in its
+    last bits, one that grows from cell to cell)."""
+    nx, ny, nz = dims
+    n = nx * ny * nz
+    rng = np.random.default_rng(n)
+    u, v, w = (20.0 * rng.standard_normal(n) for _ in range(3))
+    dz, zs, dt = 0.01 + 0.02 * rng.random(nz), 500.0 * rng.random(nx * ny), 6.0
+    if kind == "uniform":
+        u[:], v[:], w[:] = -10.0, 5.0, 0.0
+    elif kind == "near":
+        u, v, w = 10.0 + 1e-14 * rng.standard_normal(n), 1e-6 * v, 1e-7 * w
+    elif kind == "calm":
+        u, v, w = np.zeros(n), np.zeros(n), np.zeros(n)
+    elif kind == "tiny":
+        u, v, w = (1e-40 * a for a in (u, v, w))
+        u[n // 2] = 1e-310
+    elif kind == "huge":
+        u, v, w = (10.0 ** rng.uniform(20, 150, n) * np.sign(a) for a in (u, v, w))
+    elif kind == "nonfinite":
+        u[n // 3], v[n // 2], w[n - 1], zs[0] = np.nan, -np.inf, np.nan, np.nan
+    elif kind == "odd_metric":
+        dz, zs = rng.standard_normal(nz) * 10.0 ** rng.uniform(-3, 3, nz), 40000.0 * rng.random(nx * ny)
+    elif kind == "steps":
+        u, v, w = 10.0 + 1e-9 * np.arange(n), -3.0 - 1e-9 * np.arange(n)[::-1], np.full(n, 0.5)
+    with np.errstate(all="ignore"):
+        for step in (dt, -dt, 1e-40):
+            r, mw, mdz = vg.cfl_scan(u, v, w, dz, zs, nx, ny, nz, 900.0, 1100.0, 20000.0, step)
+            a, b = ctypes.c_double(), ctypes.c_double()
+            ro = oc.port_lib().vo_cfl_scan(u.ctypes.data, v.ctypes.data, w.ctypes.data, dz.ctypes.data, zs.ctypes.data,
+                                            nx, ny, nz, 900.0, 1100.0, 20000.0, step, ctypes.byref(a), ctypes.byref(b))
+            assert (r, mdz) == (ro, b.value), (step, r, ro, mdz, b.value)
+            assert mw == a.value or abs(mw - a.value) <= 2.3e-16 * a.value, (mw, a.value)  # the sum's FMA contraction
+
+
+@pytest.mark.parametrize("kind", ["white", "uniform", "near", "calm", "nonfinite"])
+@pytest.mark.parametrize("dims", [(512, 257, 65), (255, 130, 40)])
+def test_cfl_scan_f32_against_torch(vg, kind, dims):
+    """FP32, tiled (8.6 M cells) and cell by cell, against the same formula in
+    torch's FP32: bit for bit but for the speed, whose sum may be contracted."""
+    import torch
+    nx, ny, nz = dims
+    g = torch.Generator(device="cuda").manual_seed(nx)
+    u, v, w = (20.0 * torch.randn(nz, ny, nx, device="cuda", generator=g) for _ in range(3))
+    dz = 0.01 + 0.02 * torch.rand(nz, device="cuda", generator=g)
+    zs = 500.0 * torch.rand(ny, nx, device="cuda", generator=g)
+    if kind == "uniform":
+        u, v, w = torch.full_like(u, 10.0), torch.full_like(u, -5.0), torch.zeros_like(u)
+    elif kind == "near":
+        u, v, w = 10.0 + 1e-6 * u, 1e-4 * v, 1e-5 * w
+    elif kind == "calm":
+        u, v, w = (torch.zeros_like(u) for _ in range(3))
+    elif kind == "nonfinite":
+        u.view(-1)[5], v.view(-1)[u.numel() // 2], w.view(-1)[-1] = float("nan"), float("nan"), float("nan")
+    f = _dev(vg, "vibe_cfl_scan_f32_dev", [ctypes.c_void_p] * 5 + [ctypes.c_int] * 3 + [ctypes.c_float] * 4 +
+             [ctypes.c_void_p] * 2)
+    out = torch.empty(3, device="cuda")
+    for step in (6.0, -6.0):
+        assert f(u.data_ptr(), v.data_ptr(), w.data_ptr(), dz.data_ptr(), zs.data_ptr(), nx, ny, nz, 900.0, 1100.0,
+                 20000.0, step, out.data_ptr(), torch.cuda.current_stream().cuda_stream) == 0
+        thick = (dz[:, None, None] * (20000.0 - zs)).clamp(min=1.0)
+        dx, dy = torch.full_like(u, 900.0), torch.full_like(u, 1100.0)  # (torch multiplies by a number's reciprocal)
+        c = step * (u.abs() / dx + v.abs() / dy + w.abs() / thick)
+        s = (u * u + v * v + w * w).sqrt()
+        got = out.tolist()
+        assert got[0] == max(0.0, float(c.nan_to_num(nan=0.0).max()))
+        assert abs(got[1] - float(s.nan_to_num(nan=0.0).max())) <= 2.4e-7 * got[1]
+        assert got[2] == float(thick.min())

@@ -725,13 +725,31 @@ __device__ __forceinline__ float trunc_signed(double x) {  // rounded toward zer
   return copysignf(f, __int_as_float(h));
 }
 __device__ __forceinline__ float trunc_signed(float x) { return x; }
-__device__ __forceinline__ unsigned down_bits(double x) { return __float_as_uint(__double2float_rd(x)); }
-__device__ __forceinline__ unsigned down_bits(float x) { return __float_as_uint(x); }
+template <typename T>
+__device__ __forceinline__ float round_down(T x) {  // of x >= 0
+  return fminf(trunc_signed(x), 3.402823466e38f);
+}
 // What is left of FP64: one subtraction a thread and tile, the column's smallest dz
 // in the bottom tiles, the cells evaluated. 384 x 384 x 60 (floor 31 us): 61 us; 89 with
 // the extent of dzeta, the merges and the roots in every warp (FP64 pipe 76 % busy).
-constexpr int kCflLevels = 4;  // levels of one tile
+constexpr int kCflLevels = 4;  // levels of one tile, half of them where that leaves SMs without one
+// A block's best CFL number and squared speed (as order bits), and the inputs of
+// the last cell of each thread that had the best of its time. Both round
+// monotonically in |u|, |v|, |w| (and the first falls with dz), so a cell with none larger
+// cannot raise them: in fields with many equal cells, a uniform wind above all,
+// every bound lies above the best. FP64 cells near the best, of which a nearly
+// uniform wind has many, are compared by products with the reciprocals (5 FP64
+// operations, where the three divisions take 31) before they are evaluated. Both
+// scan kernels, 384 x 384 x 60: white noise 69 us, a uniform wind 163 and a nearly uniform one 319,
+// where every cell evaluated took 997 and 620 (and 1066 and 679 with the bounds alone).
 template <typename T>
+struct CflBest {
+  using I = decltype(order_bits(T()));
+  static constexpr int kOf = sizeof(T) == 8 ? kCflThreads : 1;  // (FP32: not used)
+  I best[2], top_c[4][kOf], top_s[3][kOf];
+  T up_dt, inv_dx, inv_dy;
+};
+template <typename T, int kL>
 __global__ void __launch_bounds__(kCflThreads, 4) k_cfl_partial(const T* __restrict__ u, const T* __restrict__ v,
                                                              const T* __restrict__ w, const T* __restrict__ dzeta,
                                                              const T* __restrict__ zs, int nx, int ny, int nz, T dx,
@@ -746,12 +764,16 @@ __global__ void __launch_bounds__(kCflThreads, 4) k_cfl_partial(const T* __restr
   // the largest squared speed, one square root at the end: a correctly
   // rounded square root is monotone, so the maximum of the roots is the root
   // of the maximum, bit for bit
-  T worst = 0, mw2 = 0, mdz = (T)1e30;
-  // best[0..1]: the block's maxima of the two, rounded down, as float bits
-  // (non-negative floats order as their bits); seen[..]: a tile's largest bounds
-  __shared__ unsigned best[2], seen[2][2];
-  if (threadIdx.x < 2) best[threadIdx.x] = seen[0][threadIdx.x] = 0u;
-  __syncthreads();
+  T mdz = (T)1e30;
+  __shared__ CflBest<T> sh;
+  __shared__ unsigned seen[2][2];  // a tile's largest bounds, as float bits (non-negative floats order as their bits)
+  const int tid = threadIdx.x;
+  if constexpr (sizeof(T) == 8) {
+    for (int q = 0; q < 3; ++q) sh.top_c[q][tid] = sh.top_s[q][tid] = 0;
+    sh.top_c[3][tid] = 0;
+  }
+  if (tid < 2) sh.best[tid] = 0, seen[0][tid] = 0u;
+  if (tid == 0) sh.up_dt = dt * (T)(1.0 + 0x1p-48), sh.inv_dx = (T)1 / dx, sh.inv_dy = (T)1 / dy;
   int par = 0;
   __shared__ T dext[2];  // the smallest and the largest dzeta, for the blocks that have bottom tiles
   if (blockIdx.x < ctiles && threadIdx.x < 32) {
@@ -772,7 +794,7 @@ __global__ void __launch_bounds__(kCflThreads, 4) k_cfl_partial(const T* __restr
   __syncthreads();
   for (size_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
     const size_t kt = tile / ctiles, col = (tile - kt * ctiles) * kCflThreads + threadIdx.x;
-    const int k0 = (int)kt * kCflLevels;
+    const int k0 = (int)kt * kL;
     const bool in = col < nxy;
     const T scale = zs ? (in ? z_top - zs[col] : (T)1) : z_top;
     const float fscale = trunc_signed(scale);
@@ -782,18 +804,19 @@ __global__ void __launch_bounds__(kCflThreads, 4) k_cfl_partial(const T* __restr
       if (dz < (T)1) dz = (T)1;
       mdz = fmin(mdz, dz);
     }
-    T qu[kCflLevels], qv[kCflLevels], qw[kCflLevels];
+    T qu[kL], qv[kL], qw[kL];
+    const size_t e0 = (size_t)k0 * nxy + col;
 #pragma unroll
-    for (int m = 0; m < kCflLevels; ++m) {
-      const size_t e = (size_t)(k0 + m) * nxy + col;
+    for (int m = 0; m < kL; ++m) {
+      const size_t e = e0 + m * nxy;
       const bool on = in && k0 + m < nz;
       qu[m] = on ? u[e] : (T)0;
       qv[m] = on ? v[e] : (T)0;
       qw[m] = on ? w[e] : (T)0;
     }
-    float ec[kCflLevels], es[kCflLevels], tc = 0.f, ts = 0.f;
+    float ec[kL], es[kL], tc = 0.f, ts = 0.f;
 #pragma unroll
-    for (int m = 0; m < kCflLevels; ++m) {
+    for (int m = 0; m < kL; ++m) {
       const int k = k0 + m < nz ? k0 + m : nz - 1;
       const float fu = trunc_abs(qu[m]), fv = trunc_abs(qv[m]), fw = trunc_abs(qw[m]);
       const float some = (fu + fv + fw > 0.f) ? 1e-36f : 0.f;  // products below 2^-126 count as that much
@@ -816,29 +839,77 @@ __global__ void __launch_bounds__(kCflThreads, 4) k_cfl_partial(const T* __restr
     }
     __syncthreads();
     // (another warp may raise best meanwhile: any value read is a maximum already reached)
-    const float bc = __uint_as_float(best[0]), bs = __uint_as_float(best[1]);
+    const float bc = round_down(from_order(sh.best[0])), bs = round_down(from_order(sh.best[1]));
     const float mc = __uint_as_float(seen[par][0]), ms = __uint_as_float(seen[par][1]);
     // under these a cell cannot be the tile's maximum (no such limit where a bound is tiny or not finite)
     const float lc = (mc > cfloor && mc < 3e38f) ? mc * 0.99995f : 0.f, ls = (ms > 1e-30f && ms < 3e38f) ? ms * 0.99995f : 0.f;
     if (threadIdx.x < 2) seen[par ^ 1][threadIdx.x] = 0u;
+    if constexpr (sizeof(T) == 4) {  // evaluation is cheap
 #pragma unroll
-    for (int m = 0; m < kCflLevels; ++m) {
-      const int k = k0 + m;
-      const T uu = qu[m], vv = qv[m], ww = qw[m];
-      if (in && k < nz && (!plain || (!(ec[m] <= bc) && !(ec[m] < lc)))) {
-        T dz = dzeta[k] * scale;
-        if (dz < (T)1) dz = (T)1;
-        worst = fmax(worst, dt * (fabs(uu) / dx + fabs(vv) / dy + fabs(ww) / dz));
-        atomicMax(&best[0], down_bits(worst));
+      for (int m = 0; m < kL; ++m) {
+        const int k = k0 + m;
+        const T uu = qu[m], vv = qv[m], ww = qw[m];
+        if (in && k < nz && (!plain || (!(ec[m] <= bc) && !(ec[m] < lc)))) {
+          T dz = dzeta[k] * scale;
+          if (dz < (T)1) dz = (T)1;
+          const T c = dt * (fabs(uu) / dx + fabs(vv) / dy + fabs(ww) / dz);
+          if (c > from_order(sh.best[0])) atomicMax(&sh.best[0], order_bits(c));
+        }
+        if (in && k < nz && (!plain || (!(es[m] <= bs) && !(es[m] < ls)))) {
+          const T s2 = uu * uu + vv * vv + ww * ww;
+          if (s2 > from_order(sh.best[1])) atomicMax(&sh.best[1], order_bits(s2));
+        }
       }
-      if (in && k < nz && (!plain || (!(es[m] <= bs) && !(es[m] < ls)))) {
-        mw2 = fmax(mw2, uu * uu + vv * vv + ww * ww);
-        atomicMax(&best[1], down_bits(mw2));
+    } else {
+      // the few cells that are left are read again: kept, they would take the registers of a block an SM
+      unsigned left = 0u;
+#pragma unroll
+      for (int m = 0; m < kL; ++m)
+        if (in && k0 + m < nz) {
+          if (!plain || (!(ec[m] <= bc) && !(ec[m] < lc))) left |= 1u << m;
+          if (!plain || (!(es[m] <= bs) && !(es[m] < ls))) left |= 0x10000u << m;
+        }
+      while (left) {
+        const int m = (__ffs(left) - 1) & 15;
+        const size_t e = e0 + m * nxy;
+        const T au = fabs(u[e]), av = fabs(v[e]), aw = fabs(w[e]);
+        const auto bu = order_bits(au), bv = order_bits(av), bw = order_bits(aw);
+        if (left >> m & 1u) {
+          T dz = dzeta[k0 + m] * scale;
+          if (dz < (T)1) dz = (T)1;
+          const auto bz = order_bits(dz);
+          const T b = from_order(sh.best[0]);
+          bool go = true;
+          if (plain) {
+            go = bu > sh.top_c[0][tid] || bv > sh.top_c[1][tid] || bw > sh.top_c[2][tid] ||
+                 (bz < sh.top_c[3][tid] && bw != 0);
+            if (go && b > (T)1e-250) {  // (what underflows in the products is nothing beside such a best)
+              const T rdz = (T)(fmaxf(__frcp_rn(trunc_signed(dz)), 3e-39f) * 1.000001f);  // 1/dz or more
+              go = !((aw * rdz + (av * sh.inv_dy + au * sh.inv_dx)) * sh.up_dt <= b);
+            }
+          }
+          if (go) {
+            const T c = dt * (au / dx + av / dy + aw / dz);
+            if (c >= b) {
+              sh.top_c[0][tid] = bu, sh.top_c[1][tid] = bv, sh.top_c[2][tid] = bw, sh.top_c[3][tid] = bz;
+              if (c > b) atomicMax(&sh.best[0], order_bits(c));
+            }
+          }
+        }
+        if ((left >> m & 0x10000u) && (bu > sh.top_s[0][tid] || bv > sh.top_s[1][tid] || bw > sh.top_s[2][tid])) {
+          const T s2 = au * au + av * av + aw * aw, b = from_order(sh.best[1]);
+          if (s2 >= b) {
+            sh.top_s[0][tid] = bu, sh.top_s[1][tid] = bv, sh.top_s[2][tid] = bw;
+            if (s2 > b) atomicMax(&sh.best[1], order_bits(s2));
+          }
+        }
+        left &= ~(0x10001u << m);
       }
     }
     par ^= 1;
     __syncthreads();  // seen[par] is clear, best is settled
   }
+  T worst = tid == 0 ? from_order(sh.best[0]) : (T)0, mw2 = tid == 0 ? from_order(sh.best[1]) : (T)0;
   max3_block(worst, mw2, mdz);
   if (threadIdx.x == 0) {
     partials[3 * blockIdx.x] = worst;
@@ -846,6 +917,48 @@ __global__ void __launch_bounds__(kCflThreads, 4) k_cfl_partial(const T* __restr
     partials[3 * blockIdx.x + 2] = mdz;
   }
 }
+// The same with every cell evaluated, a grid-stride loop, for grids that the tiles
+// are not worth their barriers on.
+template <typename T>
+__global__ void k_cfl_cells(const T* __restrict__ u, const T* __restrict__ v, const T* __restrict__ w,
+                              const T* __restrict__ dzeta, const T* __restrict__ zs, int nx, int ny, int nz, T dx, T dy,
+                              T z_top, T dt, T* __restrict__ partials) {
+  const size_t n = (size_t)nx * ny * nz, nxy = (size_t)nx * ny;  // (no negative dimension reaches here)
+  // the largest squared speed, one square root at the end: a correctly
+  // rounded square root is monotone, so the maximum of the roots is the root
+  // of the maximum, bit for bit
+  T worst = 0, mw2 = 0, mdz = (T)1e30;
+  const size_t S = (size_t)gridDim.x * blockDim.x;
+  size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+  if (e < n) {
+    // the cell's level and column, stepped along with e (no division per cell)
+    size_t k = e / nxy, col = e - k * nxy;
+    const size_t sk = S / nxy, sc = S - sk * nxy;
+    for (; e < n; e += S) {
+      const T uu = u[e], vv = v[e], ww = w[e];
+      const T scale = zs ? (z_top - zs[col]) : z_top;
+      T dz = dzeta[k] * scale;
+      if (dz < (T)1) dz = (T)1;
+      mdz = fmin(mdz, dz);
+      mw2 = fmax(mw2, uu * uu + vv * vv + ww * ww);
+      worst = fmax(worst, dt * (fabs(uu) / dx + fabs(vv) / dy + fabs(ww) / dz));
+      col += sc;
+      k += sk;
+      if (col >= nxy) {
+        col -= nxy;
+        ++k;
+      }
+    }
+  }
+  T mw = sqrt(mw2);
+  max3_block(worst, mw, mdz);
+  if (threadIdx.x == 0) {
+    partials[3 * blockIdx.x] = worst;
+    partials[3 * blockIdx.x + 1] = mw;
+    partials[3 * blockIdx.x + 2] = mdz;
+  }
+}
+
 template <typename T>
 __global__ void k_cfl_final(const T* __restrict__ partials, int nb, T* __restrict__ out3) {
   T a = 0, b = 0, c = (T)1e30;
@@ -1173,13 +1286,29 @@ T bilinear_host(const T* f, int halo, int nsx, int nsy, int nz, T xi, T yj, int 
   return ok ? r : (T)NAN;
 }
 
+// From this many cells on the tiled scan is the faster one whatever the winds: FP64 by
+// the divisions it saves (97 x 65 x 33, white noise 16 us against 30, nearly uniform 31 and
+// 30; 40 x 30 x 20 14.6 and 16.8, 18.7 and 16.7), FP32 by memory (384 x 384 x 60 43 to 76
+// against 78 to 109; 300 x 300 x 48 25 to 40 and 25 to 39, nearly uniform 31 and 25).
+template <typename T>
+constexpr size_t kCflCells = sizeof(T) == 8 ? (size_t)1 << 16 : (size_t)1 << 23;
+
 template <typename T>
 int cfl_launch(const T* u, const T* v, const T* w, const T* dzeta, const T* zs, int nx, int ny, int nz, T dx, T dy,
                T z_top, T dt, T* out3, T* part, cudaStream_t st) {
   const size_t ctiles = ((size_t)nx * ny + kCflThreads - 1) / kCflThreads;
-  const size_t tiles = ctiles * (((size_t)nz + kCflLevels - 1) / kCflLevels);
-  const int nb = (int)(tiles < 1 ? 1 : tiles < (size_t)kCflBlocks ? tiles : (size_t)kCflBlocks);
-  k_cfl_partial<T><<<nb, kCflThreads, 0, st>>>(u, v, w, dzeta, zs, nx, ny, nz, dx, dy, z_top, dt, tiles, part);
+  size_t tiles = ctiles * (((size_t)nz + kCflLevels - 1) / kCflLevels);
+  int nb = (int)(tiles < 1 ? 1 : tiles < (size_t)kCflBlocks ? tiles : (size_t)kCflBlocks);
+  if ((size_t)nx * ny * nz < kCflCells<T>) {
+    nb = kCflBlocks / 2;
+    k_cfl_cells<T><<<nb, kRedThreads, 0, st>>>(u, v, w, dzeta, zs, nx, ny, nz, dx, dy, z_top, dt, part);
+  } else if (sizeof(T) == 8 && tiles <= kCflBlocks / 2) {
+    tiles = ctiles * (((size_t)nz + kCflLevels / 2 - 1) / (kCflLevels / 2));
+    nb = (int)(tiles < (size_t)kCflBlocks ? tiles : (size_t)kCflBlocks);
+    k_cfl_partial<T, kCflLevels / 2><<<nb, kCflThreads, 0, st>>>(u, v, w, dzeta, zs, nx, ny, nz, dx, dy, z_top, dt, tiles, part);
+  } else {
+    k_cfl_partial<T, kCflLevels><<<nb, kCflThreads, 0, st>>>(u, v, w, dzeta, zs, nx, ny, nz, dx, dy, z_top, dt, tiles, part);
+  }
   k_cfl_final<T><<<1, kRedThreads, 0, st>>>(part, nb, out3);
   return device_ok(cudaGetLastError(), "cfl launch") ? VIBE_C_OK : VIBE_C_ERR_DEVICE;
 }
