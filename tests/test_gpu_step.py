@@ -745,3 +745,22 @@ def test_level_split_column_kernel_levels_a_warp(vg, oc, dims, dt, n_sub):
         m.step(dt, n_sub, 2)
         assert o.rk3_step(dt, n_sub) == 0 and o.rk3_step(dt, n_sub) == 0
         assert_state_close(vg, t, m.state(), o.state(), 2 * TOLMX, range(7), "level-split column kernel %s" % (dims,))
+
+
+def test_mixed_model_memory(vg):
+    """A mixed model holds 27 FP64 fields (two states, three reference fields), 58
+    FP32 ones (working copies, stages, tendencies), one staging array, in
+    allocations of whole 2 MB, and small tables: no field that only the FP64
+    tendency or the TL/AD reads."""
+    import torch
+    s = small_setup(vg, nx=384, ny=384, nz=60, zeta_stretch=1.0, **STEP_CASES[3])
+    with vg.Model(small_setup(vg, **STEP_CASES[3]), vg.MIXED) as m:  # what the first model of a process loads
+        m.step(0.5, 1, 1)
+    free0 = torch.cuda.mem_get_info()[0]
+    with vg.Model(s, vg.MIXED) as m:
+        used = free0 - torch.cuda.mem_get_info()[0]
+        staging = max(m.size(sp) for sp in range(12))
+    points = 392 * 385 * 61
+    up = lambda n: -(-(n + 256) // (2 << 20)) * (2 << 20)  # noqa: E731
+    held = 27 * up(8 * points) + 58 * up(4 * points) + up(8 * staging)
+    assert used <= held + (32 << 20), (used, held)

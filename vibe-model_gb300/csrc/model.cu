@@ -385,6 +385,18 @@ __global__ void k_inv_floor1(size_t n, const double* __restrict__ x, double* __r
     out[e] = 1.0 / dmax(x[e], 1.0);
 }
 
+// the reciprocals of theta0 for those that read them: the fast FP64 tendency,
+// and the TL/AD of every model (a field of 168 MB at 512 x 512 x 80)
+int inv_theta0(vibe_gb300_model* m) {
+  if (m->d_inv_th0) return 0;
+  const size_t n = m->d.plane * (size_t)(m->d.nz + 1);
+  if (int rc = dalloc(m, &m->d_inv_th0, n)) return rc;
+  k_inv_floor1<<<1024, 256, 0, m->stream>>>(n, m->d_th0, m->d_inv_th0);
+  CUDA_OK(cudaGetLastError());
+  m->met.inv_th0 = m->d_inv_th0;
+  return 0;
+}
+
 // rigid ground and lid (w_rigid): w = 0 on the k = 0 and k = nz faces
 __global__ void k_rigid_w(Dims d, double* __restrict__ w) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
@@ -1103,7 +1115,6 @@ int vibe_gb300_model_create(const vibe_gb300_setup* s, int precision, vibe_gb300
   rc = rc ? rc : dalloc(m, &m->d_rho0, nfield);
   rc = rc ? rc : dalloc(m, &m->d_inv_dzeta, (size_t)nz);
   rc = rc ? rc : dalloc(m, &m->d_inv_scale, (size_t)nx * ny);
-  rc = rc ? rc : dalloc(m, &m->d_inv_th0, nfield);
   rc = rc ? rc : dalloc(m, &m->d_err, (size_t)1);
   rc = rc ? rc : dalloc(m, &m->d_tri, 3 * (size_t)nz);
   if (!rc && precision == VIBE_GB300_FP64) {
@@ -1138,7 +1149,7 @@ int vibe_gb300_model_create(const vibe_gb300_setup* s, int precision, vibe_gb300
   if (cudaMemcpy(m->d_inv_dzeta, dz.data(), nz * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess ||
       cudaMemcpy(m->d_inv_scale, sc.data(), sc.size() * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess)
     return bail(fail(VIBE_GB300_EDEVICE, "metric upload failed"));
-  m->met.inv_dzeta = m->d_inv_dzeta; m->met.inv_scale = m->d_inv_scale; m->met.inv_th0 = m->d_inv_th0;
+  m->met.inv_dzeta = m->d_inv_dzeta; m->met.inv_scale = m->d_inv_scale;
   m->met.dx = s->dx; m->met.dy = s->dy; m->met.z_top = s->z_top;
   m->met.inv_dx = 1.0 / s->dx; m->met.inv_dy = 1.0 / s->dy;
   m->met.dzeta = m->d_dzeta; m->met.scale = m->d_scale; m->met.sponge = m->d_sponge;
@@ -1148,7 +1159,7 @@ int vibe_gb300_model_create(const vibe_gb300_setup* s, int precision, vibe_gb300
     dst[0] = m->d_th0;
     if ((rc = upload_storage(m, RHO, m->hs.ref[0].data(), dst, 1))) return bail(rc);
     CUDA_OK(cudaStreamSynchronize(m->stream));
-    k_inv_floor1<<<1024, 256, 0, m->stream>>>(nfield, m->d_th0, m->d_inv_th0);
+    if (precision == VIBE_GB300_FP64 && m->f64 == &kFp64Fast && (rc = inv_theta0(m))) return bail(rc);
     dst[0] = m->d_pi0;
     if ((rc = upload_storage(m, RHO, m->hs.ref[1].data(), dst, 1))) return bail(rc);
     CUDA_OK(cudaStreamSynchronize(m->stream));
@@ -2580,6 +2591,7 @@ int stl_supported(const vibe_gb300_model* m) {
 
 int stl_ensure(vibe_gb300_model* m) {
   if (m->stl_zero) return 0;
+  if (int rc = inv_theta0(m)) return rc;
   const size_t n = state_count(m);
   for (auto& st : m->stl)
     for (int q = 0; q < NSPECIES; ++q)
@@ -2736,7 +2748,6 @@ int stl_upload(vibe_gb300_model* m, const double* const* host, double* const* de
   }
   return 0;
 }
-// device -> FieldT: the boxes from dev, every other point from keep
 // Host arrays that the caller has only reserved get their pages here, while
 // the device works on what is enqueued: a device copy into pages that do not
 // exist yet faults on each of them (12 arrays of 4.6 MB: the call took 58 ms
@@ -2751,6 +2762,7 @@ void stl_prefault(const vibe_gb300_model* m, double* const* out) {
   }
 }
 
+// device -> FieldT: the boxes from dev, every other point from keep
 int stl_download(vibe_gb300_model* m, double* const* dev, const double* const* keep, double* const* host) {
   const dim3 b(32, 4);
   for (int q = 0; q < NSPECIES; ++q) {
