@@ -797,7 +797,7 @@ __device__ __forceinline__ void hevi_ghost(const Dims& d, int i, int j, int k0, 
 // 128 x 128 x 80 106 to 81, against blocks of 32 points of the padded plane.
 template <int kBlocks, int kCols>
 __global__ void __launch_bounds__(kCols * kHevi64Chunks / kBlocks, 32 / kCols * kBlocks)
-    k_chevi_chunk(Dims d, const double* __restrict__ tab, double b, double dtau, int pert,
+    k_chevi_chunk(Dims d, const double* __restrict__ tab, double dtau, int pert,
                   const double* __restrict__ u, const double* __restrict__ v, double* __restrict__ w,
                   double* __restrict__ rho, double* __restrict__ pi) {
   constexpr int kM = kHevi64M;
@@ -1446,7 +1446,7 @@ void FP64_FN(fp64_cons_hevi_substep)(const Dims& d, const Metric& m, const Flags
                             double* scratch, double dtau, unsigned* err, cudaStream_t stream) {
 #ifndef VGB_FP64_EXACT
   if (m.hevi) {
-    VGB_HEVI64_LAUNCH(k_chevi_chunk, d, stream, d, m.hevi, fl.hevi_beta, dtau, fl.pgf_pert, st[U], st[V], st[W],
+    VGB_HEVI64_LAUNCH(k_chevi_chunk, d, stream, d, m.hevi, dtau, fl.pgf_pert, st[U], st[V], st[W],
                       st[RHO], st[PI]);
     k_uv_chunk<<<grid3(d, d.nx, d.ny, d.nz, kBlk), kBlk, 0, stream>>>(d, m.hevi, st[PI], st[U], st[V]);
     return;

@@ -1577,19 +1577,10 @@ bool stage_maps(const Dims& d, const Flags& fl, const WS& win, StageMaps& M) {
 struct StageArgs;
 template <bool kRaw, bool kSpec>
 __global__ void k_b_stage(const StageArgs* __restrict__ A, const int* __restrict__ start, int nd, unsigned* err);
-// the moisture ring's dynamic shared memory; false: it could not be raised
-bool stage_smem(const Flags& fl, unsigned* bytes) {
-  *bytes = fl.moist ? kMoistSmem : 0;
-  if (!fl.moist) return true;
-  bool ok = true;
-  auto raise = [&](auto* k) {
-    ok = ok && cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMoistSmem) == cudaSuccess;
-  };
-  raise(k_mx_stage<true, false>);
-  raise(k_mx_stage<false, false>);
-  raise(k_b_stage<true, false>);
-  raise(k_b_stage<false, false>);
-  return ok;
+// lets k (a moist stage kernel) have the moisture ring's dynamic shared memory
+template <class K>
+bool raise_moist(K* k) {
+  return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMoistSmem) == cudaSuccess;
 }
 
 // boxes of the TMA-fed column kernel: every field over the whole padded
@@ -1609,10 +1600,11 @@ bool column_maps(const Dims& d, const WS& win, const WS& wout, ColumnMaps& C) {
 int mixed_stage(const Dims& d, const Tab& t, const Flags& fl, const WS& win, const WS& w0, const WS& wout,
                 const WS* rout, double dt_stage, unsigned* err, cudaStream_t stream) {
   StageMaps M;
-  unsigned sm;
-  if (!stage_maps(d, fl, win, M) || !stage_smem(fl, &sm)) return -1;
-  const dim3 b(TX, TY);
   const bool raw = rout != nullptr;
+  const unsigned sm = fl.moist ? kMoistSmem : 0;
+  if (!stage_maps(d, fl, win, M)) return -1;
+  if (fl.moist && !(raw ? raise_moist(k_mx_stage<true, false>) : raise_moist(k_mx_stage<false, false>))) return -1;
+  const dim3 b(TX, TY);
   const int kchunk = stage_kchunk(d, raw);
   const dim3 g((d.nx + TX) / TX, (d.ny + TY) / TY, (d.nz + kchunk - 1) / kchunk);
   const bool spec = stage_spec(fl);
@@ -3264,7 +3256,8 @@ MixedBatch* mixed_batch_build(const std::vector<MixedDomain>& doms, const Flags&
   const double dts[3] = {dt / 3.0, dt / 2.0, dt};
   const int nd = (int)doms.size();
   auto sub_out = [&](const MixedDomain& m, int n) { return (n & 1) ? m.WB : m.WA; };
-  bool ok = stage_smem(fl, &b->stage_smem);
+  b->stage_smem = fl.moist ? kMoistSmem : 0;
+  bool ok = !fl.moist || (raise_moist(k_b_stage<true, false>) && raise_moist(k_b_stage<false, false>));
   for (int stage = 0; stage < 3 && ok; ++stage) {
     std::vector<StageArgs> sa(nd);
     std::vector<int> start(nd);
