@@ -858,10 +858,8 @@ def test_thomas_sweep_and_solver_limits(vg, oc, bits, n, n_sys):
 @pytest.mark.parametrize("thin", [False, True])
 def test_flux_advection_error_against_wider_type(vg, bits, thin):
     """The tiled kernel is no further from the result in a wider type than the
-    formula with its two divisions a cell, rounded at every operation (FP64: but
-    for the product that a fused multiply-add takes into a difference of
-    fluxes): 2-norms over 62 x 40 x 40 cells, to 2 %; thin: layers under 1 m
-    count as 1 m."""
+    formula with its two divisions a cell, rounded at every operation: 2-norms
+    over 62 x 40 x 40 cells, to 1 %; thin: layers under 1 m count as 1 m."""
     import torch
     dt, np_t = (torch.float64, np.float64) if bits == 64 else (torch.float32, np.float32)
     if bits == 64 and np.finfo(np.longdouble).nmant <= 52:
@@ -884,8 +882,8 @@ def test_flux_advection_error_against_wider_type(vg, bits, thin):
         thick = np.maximum(r(D[:, None, None] * r(wide(20000.0) - S)), 1)
 
         def diff(vel, ax):  # of the fluxes through a cell's two faces
-            f = r(vel * r(R + np.roll(R, 1, ax))) * r(Q + np.roll(Q, 1, ax))
-            return r(np.roll(f if bits == 64 else r(f), -1, ax) - r(f)) / 4
+            f = r(r(vel * r(R + np.roll(R, 1, ax))) * r(Q + np.roll(Q, 1, ax)))
+            return r(np.roll(f, -1, ax) - f) / 4
 
         h = r(r(diff(U, 2) * r(wide(1) / wide(900.0))) + r(diff(V, 1) * r(wide(1) / wide(1100.0))))
         z = diff(W, 0)
@@ -896,7 +894,7 @@ def test_flux_advection_error_against_wider_type(vg, bits, thin):
     exact = formula(wide, lambda a: a)
     twice = formula(wide, lambda a: np.asarray(a, np_t).astype(wide))
     err = lambda a: float(np.sqrt(((a - exact) ** 2).sum()))  # noqa: E731
-    assert err(out.cpu().numpy().astype(wide)) <= 1.02 * err(twice)
+    assert err(out.cpu().numpy().astype(wide)) <= 1.01 * err(twice)
 
 
 @pytest.mark.parametrize("bits", [64, 32])

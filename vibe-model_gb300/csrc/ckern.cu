@@ -1017,12 +1017,12 @@ __global__ void k_cfl_final(const T* __restrict__ partials, int nb, T* __restric
 // warp is 32 consecutive columns, whose west fluxes serve the 31 cells between
 // them (the neighbour's by shuffle); a block's nine rows of south fluxes serve
 // eight rows of cells through shared memory; a thread marches up the levels
-// and keeps its lower face's flux. With one reciprocal per cell that is about 33
+// and keeps its lower face's flux. With one reciprocal per cell that is about 36
 // FP64 operations, the bound, where one thread per cell with its six faces
 // spent 70 and three index divisions. The halves of the two means are exact
-// powers of two and are applied once. Faces pass on their mass flux and their q
-// apart, so that a difference of two fluxes rounds one product and not both:
-// fluxes nearly cancel, and their rounding is most of the result's.
+// powers of two and are applied once. The upper face's flux stands in its
+// difference unrounded (fluxes nearly cancel, and their rounding is most of the
+// result's), as one face of each pair did in the kernel before.
 // x < 1 and x > 1e-12 on the integer pipe (a NaN x, of either sign, is not below
 // one; a NaN rho makes the fluxes NaN whatever the divisor)
 __device__ __forceinline__ bool below_one(double x) {
@@ -1032,12 +1032,12 @@ __device__ __forceinline__ bool below_one(double x) {
 __device__ __forceinline__ bool below_one(float x) { return x < 1.f; }
 __device__ __forceinline__ bool above_floor(double x) { return __double_as_longlong(x) > __double_as_longlong(1e-12); }
 __device__ __forceinline__ bool above_floor(float x) { return x > 1e-12f; }
-// (h + z / dz) / r: one reciprocal of dz r, the quotient corrected by its
-// residual, that product's own rounding included, so it rounds once where the
-// two divisions (some nine FP64 operations more) round twice
+// (h + z / dz) / r with both quotients rounded as divisions round: one reciprocal
+// of dz r gives those of dz and r, and each quotient is corrected by its residual
+// (eight FP64 operations less than two divisions)
 __device__ __forceinline__ double flux_quotient(double h, double z, double dz, double r) {
-  const double num = fma(h, dz, z), den = dz * r, low = fma(dz, r, -den), i = 1.0 / den;
-  const double q = num * i, x = fma(fma(-q, low, fma(-q, den, num)), i, q);
+  const double den = dz * r, i = 1.0 / den;
+  const double x = quotient(h + quotient(z, dz, r * i), r, dz * i);
   return ordinary(den, 0x03d00000u, 0x7fc00000u) && ordinary(x, 0u, 0x7ff00000u) ? x : (h + z / dz) / r;
 }
 __device__ __forceinline__ float flux_quotient(float h, float z, float dz, float r) { return (h + z / dz) / r; }
@@ -1047,9 +1047,7 @@ __global__ void __launch_bounds__(32 * (kFluxRows + 1)) k_flux_adv(
     const T* __restrict__ q, const T* __restrict__ rho, const T* __restrict__ u, const T* __restrict__ v,
     const T* __restrict__ w, const T* __restrict__ dzeta, const T* __restrict__ zs, int nx, int ny, int nz, T dx, T dy,
     T z_top, T* __restrict__ dqdt, int xtiles, int kz) {
-  // (FP32, bound by latency, has no registers left for it in x and y: 120 us against 82)
-  constexpr bool kApart = sizeof(T) == 8;
-  __shared__ T sm[2][kFluxRows + 1][32], sq[kApart ? 2 : 1][kApart ? kFluxRows + 1 : 1][32];
+  __shared__ T sy[2][kFluxRows + 1][32];
   const size_t nxy = (size_t)nx * ny;
   const int lane = threadIdx.x, row = threadIdx.y;
   const int i0 = (int)(blockIdx.x % (unsigned)xtiles) * kFluxCols, j0 = (int)(blockIdx.x / (unsigned)xtiles) * kFluxRows;
@@ -1065,28 +1063,22 @@ __global__ void __launch_bounds__(32 * (kFluxRows + 1)) k_flux_adv(
   T qc = q[o + c], rc = rho[o + c], fb = 0;
   if (cells && k0 > 0) fb = w[o + c] * (rho[o - nxy + c] + rc) * (q[o - nxy + c] + qc);
   for (int k = k0; k < k1; ++k, o += nxy) {
-    const T ms = v[o + c] * (rho[o + cs] + rc), qs = q[o + cs] + qc;
-    const T fs = ms * qs;
-    sm[k & 1][row][lane] = kApart ? ms : fs;
-    if constexpr (kApart) sq[k & 1][row][lane] = qs;
-    T qt = 0, rt = 0, mt = 0, fw = 0, mw = 0, qw = 0, me = 0, qe = 0;  // me, qe: the east face's (FP32, me: its flux)
+    const T fs = v[o + c] * (rho[o + cs] + rc) * (q[o + cs] + qc);
+    sy[k & 1][row][lane] = fs;
+    T qt = 0, rt = 0, mt = 0, fw = 0, fe = 0;
     if (k + 1 < nz) {
       qt = q[o + nxy + c];
       rt = rho[o + nxy + c];
     }
     if (cells) {
       if (k + 1 < nz) mt = w[o + nxy + c] * (rc + rt);
-      T rw = __shfl_up_sync(0xffffffffu, rc, 1);
-      qw = __shfl_up_sync(0xffffffffu, qc, 1);
+      T qw = __shfl_up_sync(0xffffffffu, qc, 1), rw = __shfl_up_sync(0xffffffffu, rc, 1);
       if (lane == 0) {
         qw = q[o + cw];
         rw = rho[o + cw];
       }
-      mw = u[o + c] * (rw + rc);
-      qw += qc;
-      fw = mw * qw;
-      me = __shfl_down_sync(0xffffffffu, kApart ? mw : fw, 1);
-      if constexpr (kApart) qe = __shfl_down_sync(0xffffffffu, qw, 1);
+      fw = u[o + c] * (rw + rc) * (qw + qc);
+      fe = __shfl_down_sync(0xffffffffu, fw, 1);
     }
     __syncthreads();  // (the buffer of two levels ago: every thread read it before the barrier in between)
     const T qm = qc + qt;
@@ -1094,15 +1086,7 @@ __global__ void __launch_bounds__(32 * (kFluxRows + 1)) k_flux_adv(
       T dz = dzeta[k] * scale;
       if (below_one(dz)) dz = (T)1;
       const T rr = above_floor(rc) ? rc : (T)1e-12;
-      T fx = me, fy = sm[k & 1][row + 1][lane];
-      if constexpr (kApart) {
-        fx = fma(fx, qe, -fw);
-        fy = fma(fy, sq[k & 1][row + 1][lane], -fs);
-      } else {
-        fx -= fw;
-        fy -= fs;
-      }
-      const T h = fx * ax + fy * ay;
+      const T h = (fe - fw) * ax + (sy[k & 1][row + 1][lane] - fs) * ay;
       const T z = (k > 0 && k + 1 < nz) ? (T)0.25 * fma(mt, qm, -fb) : (T)0;
       dqdt[o + c] = -flux_quotient(h, z, dz, rr);
     }
@@ -1429,7 +1413,7 @@ T neu_host(const T* x, size_t n) {
 // tiles, the cells beyond the grid included, and no less than 15 us (at least
 // four levels a block in turn); a thread per cell takes 7 us and 130 ps a cell.
 // Tiles against cells: 48 x 48 x 20 15.0 and 14.7 us, 96 x 96 x 10 14.9 and 19.0,
-// 16 x 512 x 60 (half of each tile used) 76 and 70, 1 x 1000 x 40 97 and 15. FP32, bound by memory:
+// 16 x 512 x 60 (half of each tile used) 82 and 70, 1 x 1000 x 40 97 and 15. FP32, bound by memory:
 // 16 x 512 x 60 10.8 and 10.6, 3 x 4096 x 40 31 and 11, 384 x 384 x 60 82 and 117.
 template <typename T>
 bool flux_tiles(size_t tiles, int nz, size_t cells) {
