@@ -145,17 +145,18 @@ __global__ void k_thomas_batched(const T* __restrict__ a, const T* __restrict__ 
 // system) comes in by cp.async with four (FP32: eight) lanes on consecutive
 // elements, so each fetched sector is used, and is transposed by the odd row
 // stride of the staging buffer (no bank conflicts when lanes read their own
-// rows). Two chunks are in flight; chunks of two sectors leave room for three
-// warps an SM instead of four at n = 80 (0.80 ms against 0.71 at 262144 x 80,
-// where one thread per system took 2.50 ms and read DRAM 13 times over). The modified super-diagonal and the
-// eliminated right-hand side stay in shared memory, level-major, and the back
-// substitution stores x through the same staging, so DRAM sees each element
-// once and no workspace is needed. FP64 takes one reciprocal per row and
-// corrects each product with it by its residual num - q den (Markstein's
-// quotient), which rounds as a division does: about 17 FP64 operations a row,
-// the bound there, where two divisions take 25 (products alone, 13 operations,
-// are 1.35 times as far from 64-bit results). Pivots and quotients outside the
-// range where that holds divide. FP32 divides twice.
+// rows). Two chunks are in flight; chunks of two sectors leave room for fewer
+// warps an SM (1.04 ms against 0.87 at 262144 x 80, where one thread per system
+// took 2.50 and read DRAM 13 times over; 1.95 against 0.99 at 65536 x 200, one warp
+// per system 9.08). The modified super-diagonal and the eliminated right-hand
+// side stay in shared memory, level-major, and the back substitution stores x
+// through the same staging, so DRAM sees each element once and no workspace is
+// needed. FP64 takes one reciprocal per row and corrects each product with it by
+// its residual num - q den (Markstein's quotient), which rounds as a division
+// does: about 17 FP64 operations a row, the bound there, where two divisions take
+// 25 (products alone, 13 operations, are 1.35 times as far from 64-bit results).
+// Pivots and quotients outside the range where that holds divide. FP32 divides
+// twice.
 // A system with a zero pivot leaves x as it was.
 template <typename T>
 struct Sweep {
@@ -768,8 +769,9 @@ __device__ __forceinline__ float round_down(T x) {  // of x >= 0
   return fminf(trunc_signed(x), 3.402823466e38f);
 }
 // What is left of FP64: one subtraction a thread and tile, the column's smallest dz
-// in the bottom tiles, the cells evaluated. 384 x 384 x 60 (floor 31 us): 61 us; 89 with
-// the extent of dzeta, the merges and the roots in every warp (FP64 pipe 76 % busy).
+// in the bottom tiles, the cells evaluated. 384 x 384 x 60 (floor 31 us): 66 us; the
+// extent of dzeta, the merges and the roots in every warp took 28 more (FP64 pipe
+// 76 % busy).
 constexpr int kCflLevels = 4;  // levels of one tile, half of them where that leaves SMs without one
 // A block's best CFL number and squared speed (as order bits), and the inputs of
 // the last cell of each thread that had the best of its time. Both round
@@ -1017,9 +1019,10 @@ __global__ void k_cfl_final(const T* __restrict__ partials, int nb, T* __restric
 // warp is 32 consecutive columns, whose west fluxes serve the 31 cells between
 // them (the neighbour's by shuffle); a block's nine rows of south fluxes serve
 // eight rows of cells through shared memory; a thread marches up the levels
-// and keeps its lower face's flux. With one reciprocal per cell that is about 36
-// FP64 operations, the bound, where one thread per cell with its six faces
-// spent 70 and three index divisions. The halves of the two means are exact
+// and keeps its lower face's flux. With the cell's two quotients from one reciprocal
+// that is about 41 FP64 operations, the bound (384 x 384 x 60 674 us, the pipe 86 %
+// busy), where one thread per cell with its six faces spent 70 and three index
+// divisions (1180 us). The halves of the two means are exact
 // powers of two and are applied once. The upper face's flux stands in its
 // difference unrounded (fluxes nearly cancel, and their rounding is most of the
 // result's), as one face of each pair did in the kernel before.

@@ -1235,7 +1235,7 @@ __device__ __forceinline__ float defer_fix_rho(const Tab& t, float db, float rt,
 enum FinishDefer { kDeferNone = 0, kDeferSweep = 1, kDeferChunk = 2 };
 // Two columns a thread, 8- and 16-byte accesses (rows are padded to whole pairs;
 // what lies past a field's box is read and not used). Bound by memory: 216 B a
-// cell, 512 x 512 x 80 672 us (6.7 TB/s), 801 with one column a thread.
+// cell, 512 x 512 x 80 685 us (6.6 TB/s), 801 with one column a thread.
 __device__ __forceinline__ void finish_body(const Dims& d, const Tab& t, const Flags& fl, const WS& wfin,
                                             const WS& wst, const WS& w0, const WS& rin, float dtf, const CS64& s0,
                                             const MS64& s1, unsigned* err, int bx, int by, int bz,
@@ -2505,10 +2505,11 @@ size_t hevi_tma_smem_bytes(int nz) {
 // one (`last`) reads its own w~ back and corrects it, and what remains of the
 // stage is the u/v update.
 // Bound by latency at small grids (load, two barriers, store), by DRAM at large
-// ones: 512 x 512 x 80 158 us (4.3 TB/s; 175 with rho'), 193 x 193 x 60 17.0 (18.8),
-// three domains of 192 x 192 x 60 and below 29.3 (35.3). More loads in flight (a
-// ring of cp.async copies, 3 to 6 levels), bulk prefetches into L2 and
-// streaming hints made it slower or nothing: 170 to 232, 197, 176 to 178.
+// ones: a launch in the step 512 x 512 x 80 152 us (4.5 TB/s), 193 x 193 x 60 16.3,
+// three domains of 192 x 192 x 60 and below 28.7; carrying rho' cost 175 against
+// 158, 18.8 against 17.0 and 35.3 against 29.3 then. More loads in flight (a ring of
+// cp.async copies, 3 to 6 levels), bulk prefetches into L2 and streaming hints
+// made the kernel that carried it slower or nothing: 170 to 232, 197, 176 to 178.
 // The form with this many levels a warp, that of the small grids, is launched early:
 // its blocks leave SMs free, so the next launch's tables are made meanwhile (64 x 64 x
 // 40, four steps: 1.24 to 1.15 ms). Larger grids have no SM free, and blocks that wait
@@ -2795,13 +2796,14 @@ size_t hevi_smem_bytes(int nz, int ring) {
 // columns, 0 = the sweeping kernels. VIBE_GB300_HEVI_PAR=0 turns it off, 4 or
 // 8 fixes the levels. Eight chunks (256 threads, 4 blocks an SM at 64
 // registers) measured best from 128 x 128 up; below, where the blocks do not
-// fill the SMs twice, shorter chunks without the register limit (a launch at
-// 64 x 64 x 40: 10.8 us, 14.7 with 8 levels; the sweeping kernel 50.8; at
-// 193 x 193 x 60 23 against 75, at 512 x 512 x 80 179 against 187).
-// Moist models keep the sweeping kernel: the carries round differently, and
-// the saturation adjustment turns a difference in the last bits of theta and
-// pi into 6e-5 of qc within two steps (cloud water is the small difference of
-// vapour and saturation), though either rounding is as good.
+// fill the SMs twice, shorter chunks without the register limit. Event spans of
+// single launches, with 4, 8 and, at 80 levels, 10 levels a warp, and of the
+// sweeping kernel: 64 x 64 x 40 10.3 us, 14.6 and 51; 193 x 193 x 60 30.9, 20.5 and
+// 74; 512 x 512 x 80 224, 184, 155 and 186.
+// Moist models keep the sweeping kernel, and with it the bits of their results:
+// the carries round differently, and the saturation adjustment makes 6e-5 of qc
+// of a difference in the last bits of theta and pi within two steps (cloud water
+// is the small difference of vapour and saturation). Either rounding is as good.
 int hevi_chunk_levels(int nz, long columns, const Flags& fl) {
   static int env = -2;
   if (env == -2) {
